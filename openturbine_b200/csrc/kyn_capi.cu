@@ -27,8 +27,6 @@ using namespace kyn;
 
 namespace {
 
-constexpr int kMaxDynSmem = 232448 - 1024;  // 227 KB per CTA on sm_100, minus static use
-constexpr int kSmemPerSM = 233472;      // 228 KB per SM
 constexpr int kBucketStreams = 8;
 
 struct DevModel {

@@ -163,7 +163,6 @@ __host__ __device__ inline int sec_doubles(int Q) { return ((3 * Q + 1) & ~1) + 
 // resident CTAs overlap more beams' serial sections (LU pivots); more warps
 // per CTA shorten the parallel phases of one beam.
 constexpr int kGroupScratch = 256;      // doubles of per-group scratch for QP math
-constexpr int kPanel = 8;               // LU panel width
 constexpr int kConStride = 96;          // doubles per constraint record in smem
 constexpr int kHubSmem = 208;           // doubles of the hub record (hubsm)
 constexpr int kDriveSmem = 600;         // doubles of the hub record of a drive train
@@ -200,8 +199,7 @@ struct Smem {
     int resid;          // double [N][6]
     int b;              // double [n6]  permuted rhs
     int xs;             // double [n6]  permuted solution
-    int rpiv;           // double [n6]  reciprocal pivots
-    int stage;          // double [64]  U12 tile staged by warp 0 during the LU
+    int droot;          // double [n6]  drive train: root corrections per unit shaft rotation
     int con;            // double [nc][kConStride]
     int red;            // double [2][NT/32 + 8]  (offset 0: cluster exchange)
     int hub;            // double [kHubSmem or kDriveSmem] hub state and records, or -1
@@ -228,8 +226,17 @@ __host__ __device__ constexpr int gj_slot_entries(int real_bytes, int nt) {
 __host__ __device__ inline int gj_vec_offset(int real_bytes, int nt) {
     return (2 * gj_slot_entries(real_bytes, nt) * real_bytes + 15) & ~15;
 }
-__host__ __device__ inline int gj_scratch_bytes(int N, int real_bytes, int nt) {
-    return gj_vec_offset(real_bytes, nt) + 4 * 6 * N * 8 + 64 * 8;
+// The block elimination keeps its diagonal-block inverses (64 doubles per 8
+// rows) in the place of the pivot buffers; only a drive train (hub = 2) needs
+// the vectors beside them.
+__host__ __device__ inline int solve_vec_offset(int N, int real_bytes, int nt, int hub) {
+    const int gj = gj_vec_offset(real_bytes, nt), lu = ((6 * N + 7) / 8) * 64 * 8;
+    return hub > 1 && lu > gj ? lu : gj;
+}
+__host__ __device__ inline int solve_scratch_bytes(int N, int real_bytes, int nt, int hub) {
+    const int vec = solve_vec_offset(N, real_bytes, nt, hub) + 4 * 6 * N * 8 + 64 * 8;
+    const int lu = ((6 * N + 7) / 8) * 64 * 8;
+    return vec > lu ? vec : lu;
 }
 
 // The system matrix and the quadrature scratch never live at the same time:
@@ -237,7 +244,7 @@ __host__ __device__ inline int gj_scratch_bytes(int N, int real_bytes, int nt) {
 // two share one region; so do the sections staged for the next quadrature
 // phase, copied in once the solve has read A for the last time.
 // hub: 0 none, 1 a hub node, 2 a drive train (hub chain of 2 or 3 nodes).
-__host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, int nt, int hub = 0) {
+__host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, int nc, int hub, int ldA) {
     Smem S{};
     int o = 0;
     auto take = [&](int bytes) {
@@ -246,7 +253,7 @@ __host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, 
         return r;
     };
     const int n6 = 6 * N;
-    S.ldA = n6 + 1;
+    S.ldA = ldA;
     // The cluster exchange areas come first, so that every CTA of a model's
     // cluster finds them at the same offset whatever its beam's size.
     S.red = take(2 * (nt / 32 + 8) * 8);
@@ -262,7 +269,7 @@ __host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, 
     // k-steps of two points (m16n8k8), so an odd Q gets one zero pad point.
     {
         const int g_bytes = 4 * (real_bytes == 4 ? (Q + 1) & ~1 : Q) * 56 * real_bytes;
-        const int s_bytes = gj_scratch_bytes(N, real_bytes, nt);
+        const int s_bytes = solve_scratch_bytes(N, real_bytes, nt, hub);
         S.G = take(g_bytes > s_bytes ? g_bytes : s_bytes);
     }
     S.Fc = take(Q * 6 * 8);
@@ -281,13 +288,30 @@ __host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, 
     S.resid = take(N * 6 * 8);
     S.b = take(n6 * 8);
     S.xs = take(n6 * 8);
-    S.rpiv = take(n6 * 8);
-    S.stage = take(64 * 8);
+    S.droot = hub > 1 ? take(n6 * 8) : -1;
     S.con = take((nc > 0 ? nc : 1) * kConStride * 8);
     S.pos = take(N * 4);
     S.bar = take(8);
     S.bytes = o;
     return S;
+}
+
+// Leading dimension of the system.  The right-hand sides follow the m free
+// columns, and the elimination's last column tile may reach past them, so a
+// row holds n6 + 1 columns and ceil8(m + 2).  Rows 8 values (mod 16) apart put
+// the two rows of a quarter-warp's pair loads into different halves of the
+// banks; where that padding would cost a resident CTA, or the fit, the rows
+// are packed to the next even length.
+constexpr int kSmemPerSM = 233472;          // 228 KB per SM, 1 KB of it taken per resident CTA
+constexpr int kMaxDynSmem = 232448 - 1024;  // 227 KB per CTA on sm_100, minus static use
+__host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, int nt, int hub = 0) {
+    const int n6 = 6 * N, tile = (n6 - 6 * nc + 9) & ~7;
+    const int tight = n6 + 2 > tile ? n6 + 2 : tile;
+    const Smem P = plan_smem(N, Q, real_bytes, nt, nc, hub, ((n6 + 8) & ~15) + 8);
+    const Smem T = plan_smem(N, Q, real_bytes, nt, nc, hub, tight);
+    const int most = 512 / nt;  // resident CTAs that the register budget allows
+    const int cp = kSmemPerSM / (P.bytes + 1024), ct = kSmemPerSM / (T.bytes + 1024);
+    return P.bytes <= kMaxDynSmem && (cp < most ? cp : most) >= (ct < most ? ct : most) ? P : T;
 }
 
 // Column layout of the integration GEMM's B operand G (56 columns).  The 54
@@ -433,11 +457,15 @@ __device__ __forceinline__ void store_pair_block(TR* A, int ldA, const int* pos,
     }
 }
 
-// ---- dense LU pieces (free block of the beam system in shared memory) -------------
-// The pivot chains (diagonal blocks, panel solves, block back substitution)
-// compute in the storage type TR: FP64 in the plain form, FP32 in the FP32
-// form.  Trailing updates run on the FP64 tensor cores in both forms (FP32
-// operands are exact in FP64; the result is rounded once to TR on store).
+// ---- block elimination of the free block in shared memory --------------------------
+// Right-looking elimination in 8-row panels on the FP64 tensor cores, in both
+// forms (FP32 operands are exact in FP64; a result is rounded once to TR on
+// store).  Panel k multiplies its rows by the inverse of its 8x8 diagonal
+// block, U_kj = D_k^-1 A_kj, in registers, and subtracts A_ik U_kj from the
+// rows below; A_kj and A_ik stay as they are, so no panel of L is solved and
+// nothing but trailing tiles is stored.  Fragments use the k order
+// (0,2,4,6 | 1,3,5,7): a lane's accumulator pair of U^T is then its B operand
+// of the update, and every A operand is one two-value load.
 
 // Reciprocal of a pivot: hardware approximation refined by Newton-Raphson
 // steps r <- r + r (1 - d r) (each step squares the relative error): two in
@@ -455,250 +483,186 @@ __device__ __forceinline__ float pivot_rcp(float d) {
     return fmaf(r, fmaf(-d, r, 1.f), r);
 }
 
-// Warp-level factorisation of the kb x kb diagonal block of the panel of
-// columns [p0, p0+kb): lane r holds row p0+r; pivots broadcast by shuffles.
-template <typename TR>
-__device__ __forceinline__ void factor_diag(TR* A, int ldA, int m, int p0, double* rpiv, int lane,
-                                            int* flag) {
-    const int kb = min(kPanel, m - p0);
-    TR v[kPanel];
-#pragma unroll
-    for (int c = 0; c < kPanel; ++c) v[c] = (lane < kb && c < kb) ? A[(p0 + lane) * ldA + p0 + c] : TR(0);
-#pragma unroll
-    for (int j = 0; j < kPanel; ++j) {
-        if (j < kb) {
-            const TR d = __shfl_sync(0xffffffffu, v[j], j);
-            TR u[kPanel];
-#pragma unroll
-            for (int c = j + 1; c < kPanel; ++c) u[c] = __shfl_sync(0xffffffffu, v[c], j);
-            const TR rp = pivot_rcp(d);
-            if (lane == 0) {
-                rpiv[p0 + j] = static_cast<double>(rp);
-                if (!(fabs(d) > TR(0)) || !isfinite(rp)) *flag |= 2;
-            }
-            if (lane > j) {
-                const TR l = v[j] * rp;
-                v[j] = l;
-#pragma unroll
-                for (int c = j + 1; c < kPanel; ++c) v[c] -= l * u[c];
-            }
-        }
-    }
-    if (lane < kb) {
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c)
-            if (c < kb) A[(p0 + lane) * ldA + p0 + c] = v[c];
-    }
+// Two adjacent values of the system (even column, even leading dimension).
+__device__ __forceinline__ double2 load_pair(const double* p) { return *reinterpret_cast<const double2*>(p); }
+__device__ __forceinline__ double2 load_pair(const float* p) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
+}
+__device__ __forceinline__ void store_pair(double* p, double a, double b) {
+    *reinterpret_cast<double2*>(p) = make_double2(a, b);
+}
+__device__ __forceinline__ void store_pair(float* p, double a, double b) {
+    *reinterpret_cast<float2*>(p) = make_float2(static_cast<float>(a), static_cast<float>(b));
 }
 
-// L21 = A21 U11^{-1} for rows [r_begin, m) of the panel [p0, p0+kb), rows
-// strided by `stride` starting at r_begin + idx.
-template <typename TR>
-__device__ __forceinline__ void solve_l21(TR* A, int ldA, int m, int p0, const double* rpiv,
-                                          int r_begin, int idx, int stride) {
-    const int kb = min(kPanel, m - p0);
-#pragma unroll 2
-    for (int r = r_begin + idx; r < m; r += stride) {
-        TR u[kPanel];
+// In-place inverse of an 8x8 block held by one warp in accumulator layout
+// (lane l: row l/4, columns 2(l%4) and +1), Gauss-Jordan over four 2x2 pivot
+// blocks D, each inverted through its determinant.  With s the row's pivot
+// entries times adj(D) and u the pivot rows' entries of the lane's columns,
+// every entry becomes base - (s u) / det; pivot rows and columns differ only
+// in s, u and a zero base, so the four steps are free of branches and hold one
+// reciprocal each.  Bound by the latency of that chain (shuffles, two products,
+// the reciprocal, one product per step).  A zero or non-finite determinant
+// sets bit 2 of *flag.
+__device__ __forceinline__ void invert_block8(double& v0, double& v1, int lane, int* flag) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int r = lane >> 2, t = lane & 3;
 #pragma unroll
-        for (int c = 0; c < kPanel; ++c) u[c] = (c < kb) ? A[r * ldA + p0 + c] : TR(0);
-#pragma unroll
-        for (int j = 0; j < kPanel; ++j) {
-            if (j < kb) {
-                u[j] *= static_cast<TR>(rpiv[p0 + j]);
-#pragma unroll
-                for (int k = j + 1; k < kPanel; ++k)
-                    if (k < kb) u[k] -= u[j] * A[(p0 + j) * ldA + p0 + k];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c)
-            if (c < kb) A[r * ldA + p0 + c] = u[c];
+    for (int p = 0; p < 4; ++p) {
+        const double a = __shfl_sync(kAll, v0, 9 * p), b = __shfl_sync(kAll, v1, 9 * p);
+        const double c = __shfl_sync(kAll, v0, 9 * p + 4), d = __shfl_sync(kAll, v1, 9 * p + 4);
+        const double x0 = __shfl_sync(kAll, v0, (lane & 28) + p), x1 = __shfl_sync(kAll, v1, (lane & 28) + p);
+        const double w00 = __shfl_sync(kAll, v0, 8 * p + t), w01 = __shfl_sync(kAll, v1, 8 * p + t);
+        const double w10 = __shfl_sync(kAll, v0, 8 * p + 4 + t), w11 = __shfl_sync(kAll, v1, 8 * p + 4 + t);
+        const double det = fma(a, d, -(b * c));
+        const double rd = pivot_rcp(det);
+        if (lane == 0 && (!(fabs(det) > 0.) || !isfinite(rd))) atomicOr(flag, 2);
+        const bool row0 = r == 2 * p, row1 = r == 2 * p + 1, col = t == p;
+        double s0 = fma(x0, d, -(x1 * c)), s1 = fma(x1, a, -(x0 * b));
+        s0 = row0 ? -d : row1 ? c : s0;
+        s1 = row0 ? b : row1 ? -a : s1;
+        const double u00 = col ? 1. : w00, u01 = col ? 0. : w01;
+        const double u10 = col ? 0. : w10, u11 = col ? 1. : w11;
+        const bool clear = row0 || row1 || col;
+        v0 = fma(-rd, fma(s0, u00, s1 * u10), clear ? 0. : v0);
+        v1 = fma(-rd, fma(s0, u01, s1 * u11), clear ? 0. : v1);
     }
 }
 
-// Warp-level factorisation of the panel of columns [p0, p0+kb): diagonal
-// block, then L21 for the rows below (one row per lane per pass).
+// B operands of the update by panel k in column tile c0, the lane's pair of
+// -U^T = -(A_kj^T D_k^-T): the panel's rows are read as they stand.
 template <typename TR>
-__device__ __forceinline__ void factor_panel(TR* A, int ldA, int m, int p0, double* rpiv, int lane,
-                                             int* flag) {
-    factor_diag(A, ldA, m, p0, rpiv, lane, flag);
-    __syncwarp();
-    solve_l21(A, ldA, m, p0, rpiv, p0 + min(kPanel, m - p0), lane, 32);
+__device__ __forceinline__ double2 panel_multiplier(const TR* A, int ldA, int k0, int c0, double2 dinv, int lane) {
+    const TR* a = A + (k0 + 2 * (lane & 3)) * ldA + c0 + (lane >> 2);
+    double u0 = 0., u1 = 0.;
+    dmma884(u0, u1, static_cast<double>(a[0]), dinv.x);
+    dmma884(u0, u1, static_cast<double>(a[ldA]), dinv.y);
+    return make_double2(-u0, -u1);
 }
 
-// One warp applies panel [k0, k0+kb) to the column tile [c0, c0+8) (columns
-// beyond m masked) for rows [rb0, rb1): U12 = L11^{-1} A12 for the tile, then
-// A22 -= L21 U12 on the FP64 tensor cores (8x8x4 tiles, two k-steps).
-// Where U12 goes:
-//   kU12InPlace  - lanes 0..7 solve one column each and overwrite A12 (the
-//                  tile of U12 is part of the factorisation);
-//   kU12ToStage  - same, but into stage[8][8]; the caller copies it into A once
-//                  no other warp reads that A12 tile any more;
-//   kU12InRegs   - every lane solves column c0 + lane/4 in registers and
-//                  nothing is written (a helper warp on rows of a tile whose
-//                  U12 another warp stores).
-enum U12Mode { kU12InPlace = 0, kU12ToStage = 1, kU12InRegs = 2 };
+// Inverts diagonal block k0 (rows and columns from m on count as identity)
+// after subtracting, for k0 > 0, the update of the panel before it, and
+// writes the inverse (row-major 8x8) to dinv_out.  A last block of fewer than
+// eight columns shares its tile with right-hand sides, whose update is stored.
+// One warp.
+template <typename TR>
+__device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0, const double* dinv_prev,
+                                                  double* dinv_out, int lane, int* flag) {
+    const int r = k0 + (lane >> 2), c = k0 + 2 * (lane & 3);
+    double2 d = load_pair(A + r * ldA + c);
+    if (k0 > 0) {
+        const double2 dp = load_pair(dinv_prev + 2 * lane);
+        const double2 l = load_pair(A + r * ldA + c - 8);
+        const double2 u = panel_multiplier(A, ldA, k0 - 8, k0, dp, lane);
+        dmma884(d.x, d.y, l.x, u.x);
+        dmma884(d.x, d.y, l.y, u.y);
+    }
+    if (k0 + 8 > m) {
+        if (r < m && c >= m) store_pair(A + r * ldA + c, d.x, d.y);
+        if (r >= m || c >= m) d.x = (r == c) ? 1. : 0.;
+        if (r >= m || c + 1 >= m) d.y = (r == c + 1) ? 1. : 0.;
+    }
+    invert_block8(d.x, d.y, lane, flag);
+    store_pair(dinv_out + 2 * lane, d.x, d.y);
+}
 
-template <int kMode, typename TR>
-__device__ __forceinline__ void update_tile(TR* A, int ldA, int m, int k0, int kb, int c0, int rb0,
-                                            int rb1, double* stage, int lane) {
-    const int r0 = k0 + kb;
-    const int s4 = lane & 3;
-    const int kk0 = k0 + s4, kk1 = k0 + 4 + s4;
-    double b0, b1;
-    if (kMode != kU12InRegs) {
-        if (lane < 8 && c0 + lane <= m) {
-            const int c = c0 + lane;
-            TR u[kPanel];
-#pragma unroll
-            for (int j = 0; j < kPanel; ++j) u[j] = (j < kb) ? A[(k0 + j) * ldA + c] : TR(0);
-#pragma unroll
-            for (int q = 0; q < kPanel - 1; ++q) {
-#pragma unroll
-                for (int j = q + 1; j < kPanel; ++j)
-                    if (j < kb) u[j] -= A[(k0 + j) * ldA + k0 + q] * u[q];
-            }
-            if (kMode == kU12InPlace) {
-#pragma unroll
-                for (int j = 1; j < kPanel; ++j)
-                    if (j < kb) A[(k0 + j) * ldA + c] = u[j];
-            } else {
-#pragma unroll
-                for (int j = 0; j < kPanel; ++j) stage[j * 8 + lane] = static_cast<double>(u[j]);
-            }
-        }
-        __syncwarp();
-        const int bcol = c0 + (lane >> 2);
-        const bool bok = bcol <= m;
-        if (kMode == kU12InPlace) {
-            b0 = (kk0 < r0 && bok) ? static_cast<double>(A[kk0 * ldA + bcol]) : 0.;
-            b1 = (kk1 < r0 && bok) ? static_cast<double>(A[kk1 * ldA + bcol]) : 0.;
+// Eliminates the free block A[0:m][0:m] with its right-hand sides in columns
+// m .. m + nrhs - 1 of a system with leading dimension ldA (a multiple of 8 no
+// smaller than the tiles' extent; columns past the right-hand sides are
+// scratch).  dinv: the inverses of the diagonal blocks, 64 doubles each.
+//
+// Warp 0 runs the serial chain (the next panel's diagonal block: update,
+// inversion) while the other warps share the trailing tiles of panel k in
+// equal contiguous runs down the columns; one barrier per panel.  The former
+// form (two barriers per panel, an unblocked 8x8 factorisation and a panel of
+// L solved by all threads) spent 62k of 126k cycles per Newton iteration on a
+// 13-node beam and 102k of 187k on a 21-node beam, two thirds of them in warp
+// 0's chain.
+template <typename TR, int NT>
+__device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int nrhs, double* dinv, int* flag) {
+    constexpr int NWK = NT / 32 - 1;  // warps on the trailing tiles
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = (m + 7) >> 3, nct = (m + nrhs + 7) >> 3;
+    const int fr = lane >> 2, fc = 2 * (lane & 3);
+    if (warp == 0) factor_diag_block(A, ldA, m, 0, dinv, dinv, lane, flag);
+    __syncthreads();
+    for (int k = 0; k + 1 < nb; ++k) {
+        const int k0 = 8 * k;
+        if (warp == 0) {
+            factor_diag_block(A, ldA, m, k0 + 8, dinv + 64 * k, dinv + 64 * (k + 1), lane, flag);
         } else {
-            b0 = (kk0 < r0 && bok) ? stage[s4 * 8 + (lane >> 2)] : 0.;
-            b1 = (kk1 < r0 && bok) ? stage[(4 + s4) * 8 + (lane >> 2)] : 0.;
+            // trailing tiles in column-major order without the first (warp 0's)
+            const int ni = nb - k - 1, total = ni * (nct - k - 1) - 1;
+            const int lo = total * (warp - 1) / NWK + 1, hi = total * warp / NWK + 1;
+            const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
+            int j = lo / ni, i = lo - j * ni;
+            for (int left = hi - lo; left > 0;) {
+                const int c0 = 8 * (k + 1 + j);
+                const double2 u = panel_multiplier(A, ldA, k0, c0, dk, lane);
+                const int cnt = min(ni - i, left);
+                TR* row = A + (8 * (k + 1 + i) + fr) * ldA;
+                const TR* ap = row + k0 + fc;
+                TR* cp = row + c0 + fc;
+                int rows_left = m - 8 * (k + 1 + i) - fr;  // rows from m on are not stored
+#pragma unroll 4
+                for (int e = 0; e < cnt; ++e) {
+                    const double2 l = load_pair(ap);
+                    double2 d = load_pair(cp);
+                    dmma884(d.x, d.y, l.x, u.x);
+                    dmma884(d.x, d.y, l.y, u.y);
+                    if (rows_left > 0) store_pair(cp, d.x, d.y);
+                    ap += 8 * ldA;
+                    cp += 8 * ldA;
+                    rows_left -= 8;
+                }
+                left -= cnt;
+                ++j;
+                i = 0;
+            }
         }
-    } else {
-        const int col = c0 + (lane >> 2);
-        const bool cok = col <= m;
-        TR u[kPanel];
-#pragma unroll
-        for (int j = 0; j < kPanel; ++j) u[j] = (j < kb && cok) ? A[(k0 + j) * ldA + (cok ? col : c0)] : TR(0);
-#pragma unroll
-        for (int q = 0; q < kPanel - 1; ++q) {
-#pragma unroll
-            for (int j = q + 1; j < kPanel; ++j)
-                if (j < kb) u[j] -= A[(k0 + j) * ldA + k0 + q] * u[q];
-        }
-        b0 = u[0];
-        b1 = u[4];
-#pragma unroll
-        for (int t = 1; t < 4; ++t) {
-            b0 = (s4 == t) ? u[t] : b0;
-            b1 = (s4 == t) ? u[4 + t] : b1;
-        }
-        if (kk0 >= r0) b0 = 0.;
-        if (kk1 >= r0) b1 = 0.;
-    }
-    const int dcol = c0 + 2 * s4;
-    const bool c0ok = dcol <= m, c1ok = dcol + 1 <= m;
-#pragma unroll 2
-    for (int rb = rb0; rb < rb1; rb += 8) {
-        const int row = rb + (lane >> 2);
-        const bool rv = row < rb1;
-        const double a0 = (rv && kk0 < r0) ? -static_cast<double>(A[row * ldA + kk0]) : 0.;
-        const double a1 = (rv && kk1 < r0) ? -static_cast<double>(A[row * ldA + kk1]) : 0.;
-        double d0 = (rv && c0ok) ? static_cast<double>(A[row * ldA + dcol]) : 0.;
-        double d1 = (rv && c1ok) ? static_cast<double>(A[row * ldA + dcol + 1]) : 0.;
-        dmma884(d0, d1, a0, b0);
-        dmma884(d0, d1, a1, b1);
-        if (rv && c0ok) A[row * ldA + dcol] = static_cast<TR>(d0);
-        if (rv && c1ok) A[row * ldA + dcol + 1] = static_cast<TR>(d1);
+        __syncthreads();
     }
 }
 
-// Solves L U y = r for the right-hand side in column rc (rows [0, m)) by one
-// warp, in place, with the factors as the LU leaves them (unit L below the
-// diagonal, U with its pivots on it, reciprocal pivots in rpiv): forward then
-// back substitution, one column per step.
+// Back substitution x_k = D_k^-1 (y_k - sum_{j>k} A_kj x_j) by one warp, y in
+// column rhs, x to xs[0:m].  Lanes (row, column pair) of a block row; the four
+// partial sums of a row and the product with the inverse go through shuffles.
 template <typename TR>
-__device__ void solve_factored_column(TR* A, int ldA, int m, int rc, const double* rpiv, int lane) {
-    for (int j = 0; j < m; ++j) {
-        const double yj = static_cast<double>(A[j * ldA + rc]);
-        for (int i = j + 1 + lane; i < m; i += 32)
-            A[i * ldA + rc] = static_cast<TR>(static_cast<double>(A[i * ldA + rc]) -
-                                              static_cast<double>(A[i * ldA + j]) * yj);
-        __syncwarp();
-    }
-    for (int j = m - 1; j >= 0; --j) {
-        const double yj = static_cast<double>(A[j * ldA + rc]) * rpiv[j];
-        __syncwarp();
-        if (lane == 0) A[j * ldA + rc] = static_cast<TR>(yj);
-        for (int i = lane; i < j; i += 32)
-            A[i * ldA + rc] = static_cast<TR>(static_cast<double>(A[i * ldA + rc]) -
-                                              static_cast<double>(A[i * ldA + j]) * yj);
-        __syncwarp();
-    }
-}
-
-// Replaces the kb x kb upper-triangular diagonal block of panel p0 (pivots in
-// rpiv) by its inverse; lane j < kb computes column j by back substitution
-// (lanes >= kb compute on padding and store nothing).
-template <typename TR>
-__device__ __forceinline__ void invert_diag_block(TR* A, int ldA, int m, int p0, const double* rpiv,
-                                                  int lane) {
-    const int kb = min(kPanel, m - p0);
-    const int jc = lane & 7;
-    TR x[kPanel];
-#pragma unroll
-    for (int i = 0; i < kPanel; ++i) x[i] = (i == jc) ? TR(1) : TR(0);
-#pragma unroll
-    for (int c = kPanel - 1; c >= 0; --c) {
-        if (c < kb) {  // warp-uniform; x[c] = 0 for c > jc, so no lane test is needed
-            x[c] *= static_cast<TR>(rpiv[p0 + c]);
-#pragma unroll
-            for (int i = 0; i < c; ++i) x[i] -= A[(p0 + i) * ldA + p0 + c] * x[c];
+__device__ __forceinline__ void back_substitute_blocks(const TR* A, int ldA, int m, int rhs, const double* dinv,
+                                                       double* xs, int lane) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int nb = (m + 7) >> 3;
+    const int fr = lane >> 2, t = lane & 3;
+    double xk = 0.;  // x of the block after, row fr
+    for (int k = nb - 1; k >= 0; --k) {
+        const int row = 8 * k + fr;
+        const TR* ar = A + row * ldA;
+        const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
+        double z0 = (t == 0 && row < m) ? static_cast<double>(ar[rhs]) : 0., z1 = 0.;
+#pragma unroll 4
+        for (int c = 8 * (k + 2) + 2 * t; c < m; c += 8) {  // m is even: a pair is in or out
+            const double2 a = load_pair(ar + c);
+            const double2 x = load_pair(xs + c);
+            z0 = fma(-a.x, x.x, z0);
+            z1 = fma(-a.y, x.y, z1);
         }
-    }
-    __syncwarp();
-    if (lane < kb) {
-#pragma unroll
-        for (int i = 0; i < kPanel; ++i)
-            if (i <= lane) A[(p0 + i) * ldA + p0 + lane] = x[i];
-    }
-}
-
-// Block back substitution U x = y by one warp (y in column m), with the
-// diagonal blocks already inverted: x_b = U_bb^{-1} y_b, then the rows above
-// the block take y_i -= U_i,b x_b.  Arithmetic in TR; the solution is written
-// to xs in FP64.
-template <typename TR>
-__device__ __forceinline__ void back_substitute_blocked(const TR* A, int ldA, int m, double* xs, int lane) {
-    for (int i = lane; i < m; i += 32) xs[i] = static_cast<double>(A[i * ldA + m]);
-    __syncwarp();
-    const int nblk = (m + kPanel - 1) / kPanel;
-    for (int b = nblk - 1; b >= 0; --b) {
-        const int k0 = b * kPanel, kb = min(kPanel, m - k0);
-        TR xv = TR(0);
-        if (lane < kb) {
-#pragma unroll
-            for (int c = 0; c < kPanel; ++c)
-                if (c >= lane && c < kb) xv += A[(k0 + lane) * ldA + k0 + c] * static_cast<TR>(xs[k0 + c]);
+        if (k + 1 < nb) {
+            const double x0 = __shfl_sync(kAll, xk, 8 * t), x1 = __shfl_sync(kAll, xk, 8 * t + 4);
+            if (8 * (k + 1) + 2 * t < m) {
+                const double2 a = load_pair(ar + 8 * (k + 1) + 2 * t);
+                z0 = fma(-a.x, x0, z0);
+                z1 = fma(-a.y, x1, z1);
+            }
         }
-        __syncwarp();
-        if (lane < kb) xs[k0 + lane] = static_cast<double>(xv);
-        __syncwarp();
-        TR xb[kPanel];
-#pragma unroll
-        for (int c = 0; c < kPanel; ++c) xb[c] = (c < kb) ? static_cast<TR>(xs[k0 + c]) : TR(0);
-#pragma unroll 2
-        for (int i = lane; i < k0; i += 32) {
-            TR acc = static_cast<TR>(xs[i]);
-#pragma unroll
-            for (int c = 0; c < kPanel; ++c)
-                if (c < kb) acc -= A[i * ldA + k0 + c] * xb[c];
-            xs[i] = static_cast<double>(acc);
-        }
+        z0 += z1;
+        z0 += __shfl_xor_sync(kAll, z0, 1);
+        z0 += __shfl_xor_sync(kAll, z0, 2);
+        const double za = __shfl_sync(kAll, z0, 8 * t), zb = __shfl_sync(kAll, z0, 8 * t + 4);
+        xk = fma(dk.x, za, dk.y * zb);
+        xk += __shfl_xor_sync(kAll, xk, 1);
+        xk += __shfl_xor_sync(kAll, xk, 2);
+        if (t == 0 && row < m) xs[row] = xk;
         __syncwarp();
     }
 }
@@ -2734,8 +2698,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     double* resid = reinterpret_cast<double*>(smem_raw + S.resid);
     double* bp = reinterpret_cast<double*>(smem_raw + S.b);
     double* xs = reinterpret_cast<double*>(smem_raw + S.xs);
-    double* rpiv = reinterpret_cast<double*>(smem_raw + S.rpiv);
-    double* stage = reinterpret_cast<double*>(smem_raw + S.stage);
+    double* droot = drive ? reinterpret_cast<double*>(smem_raw + S.droot) : nullptr;
     double* con = reinterpret_cast<double*>(smem_raw + S.con);
     double* gscr = reinterpret_cast<double*>(smem_raw + S.A);  // quadrature phase only
     double* red = reinterpret_cast<double*>(smem_raw + S.red);
@@ -3152,8 +3115,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         }
         if (drive && tid < nc) {
             // roots: x_root = c_r + theta d_r from the corrections of the record
-            // they join; d_r waits in rpiv's constrained rows (the LU uses rpiv
-            // below m only) for the second right-hand side
+            // they join; d_r waits in droot for the second right-hand side
             double* cr = con + tid * kConStride;
             const int pr = 6 * pos[KB.con_node[tid]];
             double c6[6], d6[6];
@@ -3175,7 +3137,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
             for (int k = 0; k < 6; ++k) {
                 xs[pr + k] = c6[k];
-                rpiv[pr + k] = d6[k];
+                droot[pr + k] = d6[k];
                 cr[conrec::dr + k] = d6[k];
             }
         } else if (tid < nc) {
@@ -3205,22 +3167,33 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         // (S2) free-row right-hand side, folded into column m of A (and kept in
         //      FP64 in bp[0:m]); a drive train adds the second right-hand side
         //      -A_fr d_r in column m + 1 (FP64 copy in rhs2)
-        double* gjv = reinterpret_cast<double*>(smem_raw + S.G + gj_vec_offset(sizeof(TR), NT));
+        double* gjv = reinterpret_cast<double*>(smem_raw + S.G + solve_vec_offset(N, sizeof(TR), NT, drive ? 2 : 0));
         double* r64 = gjv;                 // [n6] residual of the linear solve
         double* rhs2 = gjv + n6;           // [n6] second right-hand side (drive train)
         double* x2 = gjv + 2 * n6;         // [n6] its solution
         double* red4 = gjv + 4 * n6;       // [64] reductions of the refinement
-        for (int i = tid; i < m; i += NT) {
-            double r = bp[i], r2 = 0.;
-            for (int j = m; j < n6; ++j) {
-                r -= static_cast<double>(A[i * ldA + j]) * xs[j];
-                if (drive) r2 -= static_cast<double>(A[i * ldA + j]) * rpiv[j];
+        // (eight lanes per row: the rows start in only two different banks)
+        for (int i0 = 4 * warp; i0 < m; i0 += 4 * NW) {
+            const int i = i0 + (lane >> 3), ic = min(i, m - 1);
+            double r = 0., r2 = 0.;
+            for (int j = m + (lane & 7); j < n6; j += 8) {
+                const double aij = static_cast<double>(A[ic * ldA + j]);
+                r -= aij * xs[j];
+                if (drive) r2 -= aij * droot[j];
             }
-            A[i * ldA + m] = static_cast<TR>(r);
-            bp[i] = r;
-            if (drive) {
-                A[i * ldA + m + 1] = static_cast<TR>(r2);
-                rhs2[i] = r2;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                r += __shfl_xor_sync(0xffffffffu, r, o);
+                if (drive) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+            }
+            if ((lane & 7) == 0 && i < m) {
+                r += bp[i];
+                A[i * ldA + m] = static_cast<TR>(r);
+                bp[i] = r;
+                if (drive) {
+                    A[i * ldA + m + 1] = static_cast<TR>(r2);
+                    rhs2[i] = r2;
+                }
             }
         }
         __syncthreads();
@@ -3361,68 +3334,15 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
           }
         } else {
-            // (S3) LU without pivoting of the free block A[0:m][0:m]; the right-hand
-            //      side in column m is eliminated with it.  Right-looking, panels of
-            //      kPanel columns, two CTA barriers per panel:
-            //      phase 1 - warp 0 applies panel k to the next panel's diagonal rows
-            //                (its U12 tile goes to a stage) and factors the next
-            //                diagonal block; the other warps apply panel k to the rows
-            //                below it and to every other column tile;
-            //      phase 2 - the stage is copied into A and all threads solve the next
-            //                panel's L21 rows (one row per thread).
-            //      Multipliers are stored scaled; rpiv keeps the reciprocal pivots.
+            // block elimination, then the back substitution of each right-hand
+            // side by a warp of its own
+            double* dinv = reinterpret_cast<double*>(smem_raw + S.G);
             if (m > 0) {
-                if (warp == 0) factor_diag(A, ldA, m, 0, rpiv, lane, &s_flag);
-                __syncthreads();
-                solve_l21(A, ldA, m, 0, rpiv, min(kPanel, m), tid, NT);
-                __syncthreads();
-                for (int k0 = 0; k0 < m; k0 += kPanel) {
-                    const int kb = min(kPanel, m - k0);
-                    const int r0 = k0 + kb;
-                    const int nct = (m + 1 - r0 + 7) / 8;  // column tiles of [r0, m], rhs included
-                    const int top = min(r0 + kPanel, m);   // rows of the next diagonal block
-                    if (warp == 0) {
-                        update_tile<kU12ToStage>(A, ldA, m, k0, kb, r0, r0, top, stage, lane);
-                        mark(kPhaseLUDiag);
-                        if (r0 < m) {
-                            __syncwarp();
-                            factor_diag(A, ldA, m, r0, rpiv, lane, &s_flag);
-                        }
-                        mark(kPhaseLUPanel);
-                    } else {
-                        // unit 0: tile 0 below the next diagonal block; unit u >= 1: tile u
-                        for (int u = warp - 1; u < nct; u += NW - 1) {
-                            if (u == 0) {
-                                if (top < m)
-                                    update_tile<kU12InRegs>(A, ldA, m, k0, kb, r0, top, m, nullptr, lane);
-                            } else {
-                                update_tile<kU12InPlace>(A, ldA, m, k0, kb, r0 + 8 * u, r0, m, nullptr, lane);
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    mark(kPhaseFactor);
-                    if (tid < 64) {  // tile 0 of U12 (rows k0+1 .. k0+kb-1) from the stage
-                        const int j = tid >> 3, c = r0 + (tid & 7);
-                        if (j >= 1 && j < kb && c <= m) A[(k0 + j) * ldA + c] = static_cast<TR>(stage[tid]);
-                    }
-                    if (top < m) solve_l21(A, ldA, m, r0, rpiv, top, tid, NT);
-                    __syncthreads();
-                    mark(kPhaseIntEpilogue);
-                }
+                eliminate_free_block<TR, NT>(A, ldA, m, nrhs, dinv, &s_flag);
+                mark(kPhaseFactor);
+                if (warp < nrhs)
+                    back_substitute_blocks(A, ldA, m, m + warp, dinv, warp == 0 ? xs : x2, lane);
             }
-            // (S4) back substitution U x = y (y in column m): every warp inverts some
-            //      diagonal blocks, then warp 0 substitutes block by block.
-            if (drive) {  // second right-hand side (column m + 1) before U's blocks are inverted
-                if (warp == 0 && m > 0) solve_factored_column(A, ldA, m, m + 1, rpiv, lane);
-                __syncthreads();
-            }
-            for (int b = warp; b * kPanel < m; b += NW) invert_diag_block(A, ldA, m, b * kPanel, rpiv, lane);
-            __syncthreads();
-            if (warp == 0 && m > 0) back_substitute_blocked(A, ldA, m, xs, lane);
-            __syncthreads();
-            if (drive)
-                for (int i = tid; i < m; i += NT) x2[i] = static_cast<double>(A[i * ldA + m + 1]);
             __syncthreads();
         }
         if (drive) {
@@ -3439,7 +3359,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 for (int j = lane; j < n6; j += 32) {
                     const double arj = static_cast<double>(A[(pr + k) * ldA + j]);
                     a1 += arj * xs[j];
-                    a2 += arj * (j < m ? x2[j] : rpiv[j]);
+                    a2 += arj * (j < m ? x2[j] : droot[j]);
                 }
                 for (int o = 16; o > 0; o >>= 1) {
                     a1 += __shfl_xor_sync(0xffffffffu, a1, o);
@@ -3494,7 +3414,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             for (int i = tid; i < m; i += NT) xs[i] += th * x2[i];
             for (int t = tid; t < 6 * nc; t += NT) {
                 const int pr = 6 * pos[KB.con_node[t / 6]];
-                xs[pr + t % 6] += th * rpiv[pr + t % 6];
+                xs[pr + t % 6] += th * droot[pr + t % 6];
             }
             __syncthreads();
         }
