@@ -393,12 +393,14 @@ enum {
 /* Free-block solves of the step kernel (the reference's sparse direct solve,
  * src/step/solve_system.hpp:27-31, after the boundary conditions are
  * eliminated).  Neither pivots.
- * PANEL_LU (default): right-looking LU in shared memory, 8-column look-ahead
- *   panels, trailing updates on the FP64 tensor cores, block back substitution.
+ * PANEL_LU (default): block elimination in shared memory, 8-row panels with
+ *   inverted diagonal blocks, trailing updates on the FP64 tensor cores, block
+ *   back substitution.
  * GAUSS_JORDAN: the block held in registers across the CTA, one barrier per
  *   2x2 pivot block.  FP64 form: the backward error
  *   max|b - A x| / (|A| |x| + |b|) of every solve is measured and counted
- *   (KYN_STAT_SOLVES_CHECKED, _GUARD_TRIPS above 1e-10, _MAX_BACKWARD_ERROR).
+ *   (KYN_STAT_SOLVES_CHECKED, _GUARD_TRIPS above 1e-10, _MAX_BACKWARD_ERROR);
+ *   one above 1e-10 is solved again with row pivoting before it is counted.
  *   FP32 form: the block is inverted in FP32 and every Newton correction is
  *   refined with FP64 residuals of the assembled system until that backward
  *   error is at most 1e-10 (at most 8 sweeps; KYN_STAT_REFINE_*).  Blocks

@@ -25,6 +25,8 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../../include/kynema_b200.h"
 #include "kyn_types.h"
 
@@ -189,7 +191,7 @@ constexpr int x0p = 248;    // [3]
 
 struct Smem {
     int A;              // TR [n6][ldA]; aliased by the per-group QP scratch
-    int G;              // double [4Q][56] weighted quadrature blocks (integration GEMM)
+    int G;              // TR [Q][kGPoint] weighted quadrature blocks (node-pair integration)
     int Fc, Fdig;       // double [Q][6]
     int phi, dphi;      // double [Q][N]
     int dphiJ;          // double [Q][N]
@@ -211,6 +213,25 @@ struct Smem {
     int ldA;
 };
 
+// Position of entry (row, column) of the beam system: inside its group of eight
+// columns an entry's pair moves by the row's place in its group of eight rows,
+// which spreads the node-pair stores (rows 6 apart times an even pitch) and the
+// column reads of the elimination over four times as many banks; pairs stay
+// adjacent.  ldA is a multiple of 8.
+__host__ __device__ __forceinline__ int sys_at(int ldA, int r, int c) { return r * ldA + (c ^ (r & 6)); }
+
+// Weighted quadrature blocks G [Q][6 rows][kGRow]: what a node pair's 6x6 block
+// takes from one point, row r, three columns each.  XI = beta' Muu + gamma' Guu,
+// P, C, O, K the stiffness blocks; L / R the left / right three columns; the
+// pitches keep the four points and two rows of a quarter-warp's loads in
+// different banks.
+namespace gblk {
+constexpr int XIL = 0, PL = 3, CL = 6;                      // left: w J XI, w P, (w / J) C
+constexpr int K = 9, PR = 12, XIR = 15, CR = 18, O = 21;    // right: w J K, w P, w J XI, (w / J) C, w O
+}  // namespace gblk
+constexpr int kGRow = 26;
+constexpr int kGPoint = 6 * kGRow;
+
 // Entries of one slot of the Gauss-Jordan pivot buffers for (storage bytes,
 // threads): 2 (RT * NT/16 + CT * 16) with the tile sizes GJTile below (the
 // pivot pair's column and row entries).
@@ -227,15 +248,20 @@ __host__ __device__ inline int gj_vec_offset(int real_bytes, int nt) {
     return (2 * gj_slot_entries(real_bytes, nt) * real_bytes + 15) & ~15;
 }
 // The block elimination keeps its diagonal-block inverses (64 doubles per 8
-// rows) in the place of the pivot buffers; only a drive train (hub = 2) needs
-// the vectors beside them.
-__host__ __device__ inline int solve_vec_offset(int N, int real_bytes, int nt, int hub) {
-    const int gj = gj_vec_offset(real_bytes, nt), lu = ((6 * N + 7) / 8) * 64 * 8;
-    return hub > 1 && lu > gj ? lu : gj;
+// rows) in the place of the pivot buffers; beside them only a drive train
+// (hub = 2) needs the vectors.  gj_rows: the most rows a Gauss-Jordan grid holds.
+__host__ __device__ constexpr int gj_rows(int real_bytes, int nt) {
+    return real_bytes == 8 ? (nt == 128 ? 56 : nt == 256 ? 96 : 128) : (nt == 128 ? 64 : 128);
 }
-__host__ __device__ inline int solve_scratch_bytes(int N, int real_bytes, int nt, int hub) {
-    const int vec = solve_vec_offset(N, real_bytes, nt, hub) + 4 * 6 * N * 8 + 64 * 8;
-    const int lu = ((6 * N + 7) / 8) * 64 * 8;
+__host__ __device__ inline int solve_vec_offset(int N, int nc, int real_bytes, int nt, int hub) {
+    const int gj = 6 * (N - nc) <= gj_rows(real_bytes, nt) ? gj_vec_offset(real_bytes, nt) : 0;
+    const int lu = hub > 1 ? ((6 * (N - nc) + 7) / 8) * 64 * 8 : 0;
+    return lu > gj ? lu : gj;
+}
+__host__ __device__ inline int solve_scratch_bytes(int N, int nc, int real_bytes, int nt, int hub) {
+    const int off = solve_vec_offset(N, nc, real_bytes, nt, hub);
+    const int vec = off ? off + 4 * 6 * N * 8 + 64 * 8 : 0;
+    const int lu = ((6 * (N - nc) + 7) / 8) * 64 * 8;
     return vec > lu ? vec : lu;
 }
 
@@ -265,11 +291,9 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
         S.A = take(a_bytes > q_bytes ? a_bytes : q_bytes);
         S.sec = S.A + g_bytes;
     }
-    // FP64 form: G in FP64, one k-step per point.  FP32 form: G in FP32 and
-    // k-steps of two points (m16n8k8), so an odd Q gets one zero pad point.
     {
-        const int g_bytes = 4 * (real_bytes == 4 ? (Q + 1) & ~1 : Q) * 56 * real_bytes;
-        const int s_bytes = solve_scratch_bytes(N, real_bytes, nt, hub);
+        const int g_bytes = Q * kGPoint * real_bytes;  // in the form's storage type
+        const int s_bytes = solve_scratch_bytes(N, nc, real_bytes, nt, hub);
         S.G = take(g_bytes > s_bytes ? g_bytes : s_bytes);
     }
     S.Fc = take(Q * 6 * 8);
@@ -296,43 +320,21 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
     return S;
 }
 
-// Leading dimension of the system.  The right-hand sides follow the m free
-// columns, and the elimination's last column tile may reach past them, so a
-// row holds n6 + 1 columns and ceil8(m + 2).  Rows 8 values (mod 16) apart put
-// the two rows of a quarter-warp's pair loads into different halves of the
-// banks; where that padding would cost a resident CTA, or the fit, the rows
-// are packed to the next even length.
+// Leading dimension of the system: n6 columns and one more where every node is
+// free (the right-hand side is column m, a drive train's second one m + 1 with
+// m <= n6 - 6), in whole tiles of eight.  Rows 8 values (mod 16) apart put the
+// two rows of a quarter-warp's pair loads into different halves of the banks;
+// where that padding would cost a resident CTA, or the fit, a row is the next
+// multiple of 8.
 constexpr int kSmemPerSM = 233472;          // 228 KB per SM, 1 KB of it taken per resident CTA
 constexpr int kMaxDynSmem = 232448 - 1024;  // 227 KB per CTA on sm_100, minus static use
 __host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, int nt, int hub = 0) {
-    const int n6 = 6 * N, tile = (n6 - 6 * nc + 9) & ~7;
-    const int tight = n6 + 2 > tile ? n6 + 2 : tile;
+    const int n6 = 6 * N, tight = (n6 + 8) & ~7;
     const Smem P = plan_smem(N, Q, real_bytes, nt, nc, hub, ((n6 + 8) & ~15) + 8);
     const Smem T = plan_smem(N, Q, real_bytes, nt, nc, hub, tight);
     const int most = 512 / nt;  // resident CTAs that the register budget allows
     const int cp = kSmemPerSM / (P.bytes + 1024), ct = kSmemPerSM / (T.bytes + 1024);
     return P.bytes <= kMaxDynSmem && (cp < most ? cp : most) >= (ct < most ? ct : most) ? P : T;
-}
-
-// Column layout of the integration GEMM's B operand G (56 columns).  The 54
-// quantities of a node pair are L[r][c] (left 6x3 block, logical r*3+c),
-// RS[r][k] (right block before the tangent, 18 + r*3+k) and RI[r][c] (right
-// inertia block, 36 + r*3+c).  m8n8k4 leaves column 8*nt + 2*s + e of a tile
-// row in lane s = lane%4, slot 2*nt + e; the layout puts the six values of
-// two right-block rows (RS and RI) in one lane, so SM_ij = C_RS T_j + C_RI is
-// formed from registers: lanes 0..2 own rows {2s, 2s+1} in slots 0..11 and two
-// L values in slots 12..13 (lane 2: padding), lane 3 owns L[0..13].
-__host__ __device__ inline int gcol_slot(int s, int t) { return 8 * (t >> 1) + 2 * s + (t & 1); }
-__host__ __device__ inline int gcol(int logical) {
-    if (logical < 18) {
-        if (logical < 14) return gcol_slot(3, logical);
-        if (logical < 16) return gcol_slot(0, 12 + logical - 14);
-        return gcol_slot(1, 12 + logical - 16);
-    }
-    const bool ri = logical >= 36;
-    const int e = logical - (ri ? 36 : 18);
-    const int r = e / 3, k = e % 3;
-    return gcol_slot(r >> 1, (r & 1) * 6 + (ri ? 3 : 0) + k);
 }
 
 // Constraint record layout inside Smem::con (doubles).
@@ -396,64 +398,118 @@ constexpr int GtL = 47;    // [6] G_target^T lambda
 constexpr int GbL = 53;    // [6] G_base^T lambda
 }  // namespace revrec
 
-// TF32 tensor-core product D += A B for one 16x8x8 tile (mma.sync m16n8k8).
-// Fragment layout per lane l (g = l/4, t = l%4): a = {A[g][t], A[g+8][t],
-// A[g][t+4], A[g+8][t+4]}, b = {B[t][g], B[t+4][g]}, d = {D[g][2t], D[g][2t+1],
-// D[g+8][2t], D[g+8][2t+1]}.
-__device__ __forceinline__ void mma_tf32(float* d, const unsigned* a, const unsigned* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-        "{%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+// Two adjacent values (even position, 16- or 8-byte aligned).
+__device__ __forceinline__ double2 load_pair(const double* p) { return *reinterpret_cast<const double2*>(p); }
+__device__ __forceinline__ double2 load_pair(const float* p) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
+}
+__device__ __forceinline__ void store_pair(double* p, double a, double b) {
+    *reinterpret_cast<double2*>(p) = make_double2(a, b);
+}
+__device__ __forceinline__ void store_pair(float* p, double a, double b) {
+    *reinterpret_cast<float2*>(p) = make_float2(static_cast<float>(a), static_cast<float>(b));
 }
 
-// x = hi + lo with hi, lo representable in TF32 (round to nearest, ties away).
-__device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    const float r = x - __uint_as_float(hi);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
-}
-
-// Writes SM_ij = [C_L | C_RS T_j + C_RI] of node pair (i, j), scaled by the
-// conditioner, into the system matrix from one lane's integration-GEMM slots
-// (column layout: gcol; slot(t) returns the lane's slot t).
-template <typename TR, typename Slot>
-__device__ __forceinline__ void store_pair_block(TR* A, int ldA, const int* pos, const double* sT,
-                                                 int i, int jn, int s4, double cond, Slot slot) {
-    TR* Arow = A + (6 * pos[i]) * ldA + 6 * pos[jn];
-    if (s4 < 3) {
-        const double* Tj = sT + jn * 9;
+// Node-pair blocks SM_ij = S_ij T_j + I_ij (integrate_stiffness_matrix.hpp,
+// integrate_inertia_matrix.hpp, calculate_system_matrix.hpp) of one beam, on the
+// FP64 tensor cores in both forms.  With f = phi_i, g = phi'_i at a point,
+//   SM_ij = sum_q f_q H_jq + g_q H'_jq,
+//   H  = [phi_j XI_L + phi'_j P_L | (phi_j K + phi'_j P_R) T_j + phi_j XI_R],
+//   H' = [phi'_j C_L              | (phi'_j C_R + phi_j O) T_j],
+// so the sum over points is a product [N x 2Q][2Q x 36 N] whose second operand
+// a lane forms in registers, and the result needs no further step.  A unit of
+// work is eight (j, row) lines and one half of the columns: a lane forms its
+// line's three columns of H and H' at its point (line lane / 4, point lane % 4
+// of a step of four) and holds three column tiles by up to three tiles of nodes
+// i.  store(i, j, row, half, v0, v1, v2) gets three adjacent columns.
+//
+// The former product over node pairs [N^2 x 4Q][4Q x 56] took N^2 Q 448
+// multiply-adds where this takes 144, and was bound by the tensor pipe (36k of
+// 55k cycles per iteration at 21 nodes).
+template <int NT, typename TG, typename Tangent, typename Store>
+__device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double* phi, const double* dphi,
+                                                     const TG* G, Tangent tangent, Store store) {
+    constexpr int NW = NT / 32, MT = 3;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g8 = lane >> 2, t = lane & 3;
+    const int lines = 6 * N, blocks = (lines + 7) >> 3;
+    for (int u = warp; u < 2 * blocks; u += NW) {
+        const bool right = u < blocks;  // the longer halves first
+        const int l0 = 8 * (right ? u : u - blocks);
+        const int line = min(l0 + g8, lines - 1);
+        const int j = line / 6, r = line - 6 * j;
+        const TG* gr = G + r * kGRow;
+        double T[9];
+        if (right) {
+            const double* Tj = tangent(j);
 #pragma unroll
-        for (int rr = 0; rr < 2; ++rr) {
-            const int r = 2 * s4 + rr;
-            // slots 6rr..6rr+2: RS[r][0..2]; 6rr+3..6rr+5: RI[r][0..2]
-            double rs[3], ri[3];
+            for (int k = 0; k < 9; ++k) T[k] = Tj[k];
+        }
+        for (int i0 = 0; i0 < N; i0 += 8 * MT) {
+            double acc[MT][3][2];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                rs[k] = slot(6 * rr + k);
-                ri[k] = slot(6 * rr + 3 + k);
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[mt][c][0] = acc[mt][c][1] = 0.;
+            for (int q0 = 0; q0 < Q; q0 += 4) {
+                const int q = min(q0 + t, Q - 1);
+                const bool in = q0 + t < Q;
+                const double pj = phi[q * N + j], dj = dphi[q * N + j];
+                const TG* g = gr + q * kGPoint;
+                double h[3], hp[3];
+                if (right) {
+                    const double2 g8v = load_pair(g + 8), ga = load_pair(g + 10), gb = load_pair(g + 12),
+                                  gc = load_pair(g + 14), gd = load_pair(g + 16), ge = load_pair(g + 18),
+                                  gf = load_pair(g + 20), gg = load_pair(g + 22);
+                    const double s0 = fma(g8v.y, pj, gb.x * dj), s1 = fma(ga.x, pj, gb.y * dj),
+                                 s2 = fma(ga.y, pj, gc.x * dj);
+                    const double p0 = fma(ge.x, dj, gf.y * pj), p1 = fma(ge.y, dj, gg.x * pj),
+                                 p2 = fma(gf.x, dj, gg.y * pj);
+                    const double xi[3] = {gc.y, gd.x, gd.y};
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        h[c] = fma(xi[c], pj, fma(s0, T[c], fma(s1, T[3 + c], s2 * T[6 + c])));
+                        hp[c] = fma(p0, T[c], fma(p1, T[3 + c], p2 * T[6 + c]));
+                    }
+                } else {
+                    const double2 ga = load_pair(g), gb = load_pair(g + 2), gc = load_pair(g + 4),
+                                  gd = load_pair(g + 6), ge = load_pair(g + 8);
+                    h[0] = fma(ga.x, pj, gb.y * dj);
+                    h[1] = fma(ga.y, pj, gc.x * dj);
+                    h[2] = fma(gb.x, pj, gc.y * dj);
+                    hp[0] = gd.x * dj;
+                    hp[1] = gd.y * dj;
+                    hp[2] = ge.x * dj;
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    if (i0 + 8 * mt < N) {  // uniform
+                        const int i = i0 + 8 * mt + g8;
+                        const bool on = in && i < N;
+                        const double f = on ? phi[q * N + i] : 0., fp = on ? dphi[q * N + i] : 0.;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) dmma884(acc[mt][c][0], acc[mt][c][1], f, h[c]);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) dmma884(acc[mt][c][0], acc[mt][c][1], fp, hp[c]);
+                    }
+                }
             }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double val = ri[c];
+            for (int mt = 0; mt < MT; ++mt) {
+                const int i = i0 + 8 * mt + g8;
+                if (i < N) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) val += rs[k] * Tj[k * 3 + c];
-                Arow[r * ldA + 3 + c] = static_cast<TR>(val * cond);
+                    for (int e = 0; e < 2; ++e) {
+                        const int lo = l0 + 2 * t + e;
+                        if (lo < lines) {
+                            const int jo = lo / 6;
+                            store(i, jo, lo - 6 * jo, right ? 1 : 0, acc[mt][0][e], acc[mt][1][e], acc[mt][2][e]);
+                        }
+                    }
+                }
             }
         }
-        if (s4 < 2) {
-            // slots 12, 13: L[14 + 2 s4 + e]
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int l = 14 + 2 * s4 + e;
-                Arow[(l / 3) * ldA + l % 3] = static_cast<TR>(slot(12 + e) * cond);
-            }
-        }
-    } else {
-        // slots 0..13: L[0..13]
-#pragma unroll
-        for (int t = 0; t < 14; ++t) Arow[(t / 3) * ldA + t % 3] = static_cast<TR>(slot(t) * cond);
     }
 }
 
@@ -481,19 +537,6 @@ __device__ __forceinline__ float pivot_rcp(float d) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.f), r);
-}
-
-// Two adjacent values of the system (even column, even leading dimension).
-__device__ __forceinline__ double2 load_pair(const double* p) { return *reinterpret_cast<const double2*>(p); }
-__device__ __forceinline__ double2 load_pair(const float* p) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    return make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
-}
-__device__ __forceinline__ void store_pair(double* p, double a, double b) {
-    *reinterpret_cast<double2*>(p) = make_double2(a, b);
-}
-__device__ __forceinline__ void store_pair(float* p, double a, double b) {
-    *reinterpret_cast<float2*>(p) = make_float2(static_cast<float>(a), static_cast<float>(b));
 }
 
 // In-place inverse of an 8x8 block held by one warp in accumulator layout
@@ -534,7 +577,8 @@ __device__ __forceinline__ void invert_block8(double& v0, double& v1, int lane, 
 // -U^T = -(A_kj^T D_k^-T): the panel's rows are read as they stand.
 template <typename TR>
 __device__ __forceinline__ double2 panel_multiplier(const TR* A, int ldA, int k0, int c0, double2 dinv, int lane) {
-    const TR* a = A + (k0 + 2 * (lane & 3)) * ldA + c0 + (lane >> 2);
+    const int t2 = 2 * (lane & 3);
+    const TR* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));  // rows t2, t2 + 1 share their column shift
     double u0 = 0., u1 = 0.;
     dmma884(u0, u1, static_cast<double>(a[0]), dinv.x);
     dmma884(u0, u1, static_cast<double>(a[ldA]), dinv.y);
@@ -550,16 +594,17 @@ template <typename TR>
 __device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0, const double* dinv_prev,
                                                   double* dinv_out, int lane, int* flag) {
     const int r = k0 + (lane >> 2), c = k0 + 2 * (lane & 3);
-    double2 d = load_pair(A + r * ldA + c);
+    TR* at = A + sys_at(ldA, r, c);
+    double2 d = load_pair(at);
     if (k0 > 0) {
         const double2 dp = load_pair(dinv_prev + 2 * lane);
-        const double2 l = load_pair(A + r * ldA + c - 8);
+        const double2 l = load_pair(at - 8);
         const double2 u = panel_multiplier(A, ldA, k0 - 8, k0, dp, lane);
         dmma884(d.x, d.y, l.x, u.x);
         dmma884(d.x, d.y, l.y, u.y);
     }
     if (k0 + 8 > m) {
-        if (r < m && c >= m) store_pair(A + r * ldA + c, d.x, d.y);
+        if (r < m && c >= m) store_pair(at, d.x, d.y);
         if (r >= m || c >= m) d.x = (r == c) ? 1. : 0.;
         if (r >= m || c + 1 >= m) d.y = (r == c + 1) ? 1. : 0.;
     }
@@ -584,7 +629,7 @@ __device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int 
     constexpr int NWK = NT / 32 - 1;  // warps on the trailing tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (m + 7) >> 3, nct = (m + nrhs + 7) >> 3;
-    const int fr = lane >> 2, fc = 2 * (lane & 3);
+    const int fr = lane >> 2, fc = (2 * (lane & 3)) ^ (fr & 6);
     if (warp == 0) factor_diag_block(A, ldA, m, 0, dinv, dinv, lane, flag);
     __syncthreads();
     for (int k = 0; k + 1 < nb; ++k) {
@@ -633,16 +678,16 @@ __device__ __forceinline__ void back_substitute_blocks(const TR* A, int ldA, int
                                                        double* xs, int lane) {
     constexpr unsigned kAll = 0xffffffffu;
     const int nb = (m + 7) >> 3;
-    const int fr = lane >> 2, t = lane & 3;
+    const int fr = lane >> 2, t = lane & 3, shift = fr & 6;
     double xk = 0.;  // x of the block after, row fr
     for (int k = nb - 1; k >= 0; --k) {
         const int row = 8 * k + fr;
         const TR* ar = A + row * ldA;
         const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
-        double z0 = (t == 0 && row < m) ? static_cast<double>(ar[rhs]) : 0., z1 = 0.;
+        double z0 = (t == 0 && row < m) ? static_cast<double>(ar[rhs ^ shift]) : 0., z1 = 0.;
 #pragma unroll 4
         for (int c = 8 * (k + 2) + 2 * t; c < m; c += 8) {  // m is even: a pair is in or out
-            const double2 a = load_pair(ar + c);
+            const double2 a = load_pair(ar + (c ^ shift));
             const double2 x = load_pair(xs + c);
             z0 = fma(-a.x, x.x, z0);
             z1 = fma(-a.y, x.y, z1);
@@ -650,7 +695,7 @@ __device__ __forceinline__ void back_substitute_blocks(const TR* A, int ldA, int
         if (k + 1 < nb) {
             const double x0 = __shfl_sync(kAll, xk, 8 * t), x1 = __shfl_sync(kAll, xk, 8 * t + 4);
             if (8 * (k + 1) + 2 * t < m) {
-                const double2 a = load_pair(ar + 8 * (k + 1) + 2 * t);
+                const double2 a = load_pair(ar + 8 * (k + 1) + ((2 * t) ^ shift));
                 z0 = fma(-a.x, x0, z0);
                 z1 = fma(-a.y, x1, z1);
             }
@@ -698,6 +743,10 @@ template <typename TR, int NT>
 __host__ __device__ constexpr int gj_slot() {
     return 2 * (GJTile<TR, NT>::RT * (NT / kGJCols) + GJTile<TR, NT>::CT * kGJCols);
 }
+static_assert(gj_rows(8, 128) == GJTile<double, 128>::RT * 8 && gj_rows(8, 256) == GJTile<double, 256>::RT * 16 &&
+                  gj_rows(8, 512) == GJTile<double, 512>::RT * 32 && gj_rows(4, 128) == GJTile<float, 128>::RT * 8 &&
+                  gj_rows(4, 256) == GJTile<float, 256>::RT * 16 && gj_rows(4, 512) == GJTile<float, 512>::RT * 32,
+              "gj_rows must follow GJTile");
 static_assert(gj_slot<double, 128>() == gj_slot_entries(8, 128) &&
                   gj_slot<double, 256>() == gj_slot_entries(8, 256) &&
                   gj_slot<double, 512>() == gj_slot_entries(8, 512) &&
@@ -787,7 +836,7 @@ __device__ __forceinline__ void gj_eliminate(const TR* A, int ldA, int m, int nr
 #pragma unroll
         for (int b = 0; b < CT; ++b) {
             const int j = cj + b * PC;
-            R[a][b] = (i < m && j < ncols) ? A[i * ldA + j] : TR(0);
+            R[a][b] = (i < m && j < ncols) ? A[sys_at(ldA, i, j)] : TR(0);
         }
     }
     // slot 0: columns 0, 1 and rows 0, 1; padding of both slots stays zero
@@ -797,10 +846,10 @@ __device__ __forceinline__ void gj_eliminate(const TR* A, int ldA, int m, int nr
         if (t < SLOT) {
             if (e < ROWS) {
                 const int i = e >> 1, h = e & 1;
-                v = (i < m) ? A[i * ldA + h] : TR(0);
+                v = (i < m) ? A[sys_at(ldA, i, h)] : TR(0);
             } else {
                 const int j = (e - ROWS) >> 1, h = (e - ROWS) & 1;
-                v = (j < ncols) ? A[h * ldA + j] : TR(0);
+                v = (j < ncols) ? A[sys_at(ldA, h, j)] : TR(0);
             }
         }
         buf[t] = v;
@@ -876,6 +925,96 @@ __device__ __forceinline__ void gj_eliminate(const TR* A, int ldA, int m, int nr
     }
 }
 
+// Gauss-Jordan with row pivoting on the same grid, one right-hand side in
+// column m: the solve of a block whose unpivoted elimination lost accuracy to
+// element growth (seen in steps that do not converge, so its three barriers per
+// pivot matter little).  Rows stay in place; the pivot of column k is the
+// largest entry of the rows not yet used.  x to out[0:m].  buf: two rows of the
+// grid's extent and two of its integers.
+template <typename TR, int NT>
+__device__ __noinline__ void gj_solve_pivoted(const TR* A, int ldA, int m, TR* buf, double* out, int* flag) {
+    constexpr int RT = GJTile<TR, NT>::RT, CT = GJTile<TR, NT>::CT;
+    constexpr int PR = NT / kGJCols, PC = kGJCols;
+    const int tid = threadIdx.x, lane = tid & 31, ri = tid / PC, cj = tid % PC;
+    TR* col = buf;                   // [RT * PR]
+    TR* row = col + RT * PR;         // [CT * PC]
+    int* used = reinterpret_cast<int*>(row + CT * PC);  // [RT * PR]
+    int* pivot = used + RT * PR;     // [RT * PR] row that solved column k
+    TR R[RT][CT];
+#pragma unroll
+    for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int b = 0; b < CT; ++b) {
+            const int i = ri + a * PR, j = cj + b * PC;
+            R[a][b] = (i < m && j <= m) ? A[sys_at(ldA, i, j)] : TR(0);
+        }
+    for (int i = tid; i < RT * PR; i += NT) used[i] = i < m ? 0 : 1;
+    for (int k = 0; k < m; ++k) {
+        if (cj == k % PC) {
+#pragma unroll
+            for (int b = 0; b < CT; ++b)
+                if (b == k / PC) {
+#pragma unroll
+                    for (int a = 0; a < RT; ++a) col[ri + a * PR] = R[a][b];
+                }
+        }
+        __syncthreads();
+        TR best = TR(-1);
+        int p = 0;
+        for (int i = lane; i < m; i += 32)
+            if (!used[i] && fabs(col[i]) > best) {
+                best = fabs(col[i]);
+                p = i;
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const TR ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int op = __shfl_xor_sync(0xffffffffu, p, o);
+            if (ob > best || (ob == best && op < p)) {
+                best = ob;
+                p = op;
+            }
+        }
+        if (ri == p % PR) {
+#pragma unroll
+            for (int a = 0; a < RT; ++a)
+                if (a == p / PR) {
+#pragma unroll
+                    for (int b = 0; b < CT; ++b) row[cj + b * PC] = R[a][b];
+                }
+        }
+        if (tid == 0 && !(best > TR(0))) atomicOr(flag, 2);
+        __syncthreads();
+        const TR rd = TR(1) / row[k];
+        if (tid == 0) {
+            used[p] = 1;
+            pivot[k] = p;
+        }
+#pragma unroll
+        for (int a = 0; a < RT; ++a) {
+            const int i = ri + a * PR;
+            const TR l = col[i] * rd;
+#pragma unroll
+            for (int b = 0; b < CT; ++b) {
+                const TR w = row[cj + b * PC];
+                R[a][b] = i == p ? w * rd : R[a][b] - l * w;
+            }
+        }
+        __syncthreads();
+    }
+    if (cj == m % PC) {
+#pragma unroll
+        for (int b = 0; b < CT; ++b)
+            if (b == m / PC) {
+#pragma unroll
+                for (int a = 0; a < RT; ++a) col[ri + a * PR] = R[a][b];
+            }
+    }
+    __syncthreads();
+    for (int k = tid; k < m; k += NT) out[k] = static_cast<double>(col[pivot[k]]);
+    __syncthreads();
+}
+
 // Column `col` (col >= m) of the register grid after the solve form: the
 // solution for that right-hand side, into out[0:m].
 template <typename TR, int NT, typename Out>
@@ -919,7 +1058,8 @@ __device__ __forceinline__ void gj_matvec(const TR (&R)[GJTile<TR, NT>::RT][GJTi
         for (int b = 0; b < CT; ++b) {
             const int j = cj + b * PC;
             if (j < m && i < m) {
-                const double mij = from_regs ? static_cast<double>(R[a][b]) : static_cast<double>(A[i * ldA + j]);
+                const double mij = from_regs ? static_cast<double>(R[a][b])
+                                             : static_cast<double>(A[sys_at(ldA, i, j)]);
                 acc = fma(mij, v[j], acc);
             }
         }
@@ -1138,14 +1278,17 @@ __device__ inline bool joint_target_test(const double* cr, const double* wb, dou
 // rows, and takes its elements in element order.
 // Node n's rows and columns start at pos_mul * pos[n] (6 x the node's position
 // in a beam system; the first-DOF map itself in a dense model).
-template <typename TR>
+template <typename At>
 __device__ void add_lumped_terms(int n, const double* __restrict__ rec, int n_mass, int n_spring,
                                  const double* sq, const double* sv, const double* svd,
                                  const double* sT, const double* grav, double bprime,
-                                 double gprime, double cond, const int* pos, TR* A, int ldA,
+                                 double gprime, double cond, const int* pos, At at,
                                  double* resid, int pos_mul = 6) {
-    TR* Arow = A + (pos_mul * pos[n]) * ldA;
     const int cn = pos_mul * pos[n];
+    auto add = [&](int r, int c, double val) {
+        auto& a = at(cn + r, c);
+        a = static_cast<std::remove_reference_t<decltype(a)>>(static_cast<double>(a) + val);
+    };
     for (int e = 0; e < n_mass; ++e) {
         const double* mr = rec + e * kMassRec;
         if (static_cast<int>(mr[0]) != n) continue;
@@ -1245,8 +1388,7 @@ __device__ void add_lumped_terms(int n, const double* __restrict__ rec, int n_ma
                     val += gprime * G[cc];
                     val += K[0] * Tn[cc] + K[1] * Tn[3 + cc] + K[2] * Tn[6 + cc];
                 }
-                TR* a = Arow + r * ldA + cn + c;
-                *a = static_cast<TR>(static_cast<double>(*a) + val * cond);
+                add(r, cn + c, val * cond);
             }
         }
     }
@@ -1270,10 +1412,8 @@ __device__ void add_lumped_terms(int n, const double* __restrict__ rec, int n_ma
                 double rr = 0.;
                 for (int t = 0; t < 3; ++t) rr += tilde_e(r, i, t) * tilde_e(r, t, j);
                 const double a = ((i == j) ? c1 - c2 * l * l : 0.) - c2 * rr;
-                TR* d = Arow + i * ldA + cn + j;
-                *d = static_cast<TR>(static_cast<double>(*d) + a * cond);
-                TR* o = Arow + i * ldA + co + j;
-                *o = static_cast<TR>(static_cast<double>(*o) - a * cond);
+                add(i, cn + j, a * cond);
+                add(i, co + j, -a * cond);
             }
     }
 }
@@ -1325,7 +1465,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     // scratch and the component's tables and node state (cond_tables)
     auto r16 = [](int b) { return (b + 15) & ~15; };
     const int w_bytes = cond_nd > 0 ? r16(cN * 6 * (cN * 6 + 1) * 8) : 0;
-    const int g_bytes = cond_nd > 0 ? 4 * kCondChunk * 56 * 8 : 0;
+    const int g_bytes = cond_nd > 0 ? kCondChunk * kGPoint * 8 : 0;
     const int s_bytes = cond_nd > 0 ? (nt / 16) * kGroupScratch * 8 : 0;
     const int t_bytes = cond_nd > 0 ? 3 * r16(cQ * cN * 8) + r16(cQ * 4 * 8) + r16(cN * 7 * 8) +
                                           2 * r16(cN * 6 * 8) + 2 * r16(cQ * 6 * 8) : 0;
@@ -1376,7 +1516,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
         S.cq = take(cN * 7 * 8);
         S.cv = take(cN * 6 * 8);
         S.cvd = take(cN * 6 * 8);
-        S.cG = take(4 * cQ * 56 * 8);
+        S.cG = take(cQ * kGPoint * 8);
         S.cFc = take(cQ * 6 * 8);
         S.cFd = take(cQ * 6 * 8);
         S.cgs = take((nt / 16) * kGroupScratch * 8);
@@ -1402,7 +1542,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
 // phi / dphiJ [Q][N], weights qpw [Q][4], node state q [N][7], v, vd [N][6]
 // (shared memory), the system's slab for the sections and reference frames
 // (layout L).  Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the
-// integration GEMM G [4Q][56] (column layout gcol).  gscr: NT/16 groups of
+// integration G [Q][kGPoint] (gblk).  gscr: NT/16 groups of
 // kGroupScratch doubles.  sec: the sections already staged in shared memory
 // (sec_doubles(Q), slab order from x0'), or null to read them from the slab.
 template <typename TG, int NT>
@@ -1455,9 +1595,9 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
                 else v = slab[L.x0p + qp * 3 + (k - 76)];
                 gs[grec::mstar + k] = v;
             }
-            // this point's G rows start at zero (structural zeros, padding)
-            TG* Gq = G + 4 * qp * 56;
-            for (int t = g; t < 4 * 56; t += 16) Gq[t] = TG(0);
+            // P has no translational rows
+            TG* Gq = G + qp * kGPoint;
+            if (g < 9) Gq[(g / 3) * kGRow + gblk::PL + g % 3] = Gq[(g / 3) * kGRow + gblk::PR + g % 3] = TG(0);
         }
         // (1) interpolation: r, u_ddot, omega, omega_dot, u', r'
         if (act) {
@@ -1590,19 +1730,17 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
                 for (int l = 0; l < 3; ++l) inner += Mu[(3 + k) * 6 + 3 + l] * tilde_e(om, l, j);
                 k22 += w_ik * inner;
             }
-            // G rows of this quadrature point (see the integration GEMM):
-            //   4q+1: w [Puu left | Puu right | 0], 4q+3: w [0 | Ouu right | 0]
             const double w = qpw[qp * 4], wJ = qpw[qp * 4 + 2];
-            TG* G1 = G + (4 * qp + 1) * 56;
-            TG* G3 = G + (4 * qp + 3) * 56;
+            TG* Gt = G + qp * kGPoint + i * kGRow + j;  // rows 0..2
+            TG* Gr = Gt + 3 * kGRow;                    // rows 3..5
             O12[g] = o12;
-            G3[gcol(18 + g)] = static_cast<TG>(w * o12);
-            G3[gcol(18 + 9 + g)] = static_cast<TG>(w * o22);
-            G1[gcol(9 + g)] = static_cast<TG>(w * p21);
-            G1[gcol(18 + 9 + g)] = static_cast<TG>(w * p22);
+            Gt[gblk::O] = static_cast<TG>(w * o12);
+            Gr[gblk::O] = static_cast<TG>(w * o22);
+            Gr[gblk::PL] = static_cast<TG>(w * p21);
+            Gr[gblk::PR] = static_cast<TG>(w * p22);
             Gu[g] = g12;
             Gu[9 + g] = g22;
-            G[(4 * qp) * 56 + gcol(18 + g)] = static_cast<TG>(wJ * k12);
+            Gt[gblk::K] = static_cast<TG>(wJ * k12);
             Kk[g] = k22;
         } else if (act && g < 15) {
             // Fd + Fi - Fe - Fg (calculate_force_FD.hpp, calculate_inertial_force.hpp,
@@ -1640,26 +1778,24 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
             Fdig[qp * 6 + c] = fd + fi - fgv;
         }
         __syncwarp();
-        // (6) Quu_22 = SS^T (C11 SS - N~) joins Kuu_22; XI = beta' Muu + gamma' Guu;
-        //     G rows 4q+0: wJ [XI left | XK right | XI right], 4q+2: (w/J) [Cuu]
+        // (6) Quu_22 = SS^T (C11 SS - N~) joins Kuu_22; XI = beta' Muu + gamma' Guu
         if (act) {
             const double wJ = qpw[qp * 4 + 2], wdJ = qpw[qp * 4 + 3];
-            TG* G0 = G + (4 * qp) * 56;
-            TG* G2 = G + (4 * qp + 2) * 56;
+            TG* Gq = G + qp * kGPoint;
             if (g < 9) {
                 const int i = g / 3, j = g % 3;
                 double qv = 0.;
                 for (int k = 0; k < 3; ++k) qv += tilde_e(sv3, k, i) * O12[k * 3 + j];
-                G0[gcol(18 + 9 + g)] = static_cast<TG>(wJ * (Kk[g] + qv));
+                Gq[(3 + i) * kGRow + gblk::K + j] = static_cast<TG>(wJ * (Kk[g] + qv));
             }
             for (int e = g; e < 36; e += 16) {
                 const int i = e / 6, j = e % 6;
                 double gg = 0.;
                 if (j >= 3) gg = Gu[(i < 3 ? 0 : 9) + (i % 3) * 3 + (j - 3)];
                 const double xi = beta_prime * Mu[e] + gamma_prime * gg;
-                const int col = (j < 3) ? i * 3 + j : 36 + i * 3 + (j - 3);
-                G0[gcol(col)] = static_cast<TG>(wJ * xi);
-                G2[gcol((j < 3) ? i * 3 + j : 18 + i * 3 + (j - 3))] = static_cast<TG>(wdJ * Cu[e]);
+                TG* row = Gq + i * kGRow;
+                row[j < 3 ? gblk::XIL + j : gblk::XIR + j - 3] = static_cast<TG>(wJ * xi);
+                row[j < 3 ? gblk::CL + j : gblk::CR + j - 3] = static_cast<TG>(wdJ * Cu[e]);
             }
         }
         __syncwarp();
@@ -1723,37 +1859,15 @@ __device__ void dense_beam_terms(const KBeam& KB, const StepCoeffs& P, const Den
             }
             resid[static_cast<int>(node[n]) * 6 + c] += acc;
         }
-        // one thread per (node pair, row): C_ij[r] = sum_q sum_m coef_m(i, j, q) G[4q+m]
-        // with coef = (phi_i phi_j, phi_i phi'_j, phi'_i phi'_j, phi'_i phi_j)
-        for (int t = tid; t < N * N * 6; t += NT) {
-            const int pr = t / 6, r = t % 6;
-            const int i = pr / N, j = pr % N;
-            double Lr[3] = {0., 0., 0.}, RS[3] = {0., 0., 0.}, RI[3] = {0., 0., 0.};
-            for (int qp = 0; qp < Q; ++qp) {
-                const double pi = phi[qp * N + i], pj = phi[qp * N + j];
-                const double di = dphi[qp * N + i], dj = dphi[qp * N + j];
-                const double coef[4] = {pi * pj, pi * dj, di * dj, di * pj};
-#pragma unroll
-                for (int mm = 0; mm < 4; ++mm) {
-                    const double* g = G + (4 * qp + mm) * 56;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        Lr[c] += coef[mm] * g[gcol(r * 3 + c)];
-                        RS[c] += coef[mm] * g[gcol(18 + r * 3 + c)];
-                        RI[c] += coef[mm] * g[gcol(36 + r * 3 + c)];
-                    }
-                }
-            }
-            const int nj = static_cast<int>(node[j]);
-            const double* Tj = sT + nj * 9;
-            double* row = Md + (fmap[static_cast<int>(node[i])] + r) * nd + fmap[nj];
-            for (int c = 0; c < 3; ++c) row[c] += cond * Lr[c];
-            for (int c = 0; c < 3; ++c) {
-                double v = RI[c];
-                for (int k = 0; k < 3; ++k) v += RS[k] * Tj[k * 3 + c];
-                row[3 + c] += cond * v;
-            }
-        }
+        integrate_node_pairs<NT>(
+            N, Q, phi, dphi, G, [&](int j) { return sT + static_cast<int>(node[j]) * 9; },
+            [&](int i, int j, int r, int half, double v0, double v1, double v2) {
+                double* row = Md + (fmap[static_cast<int>(node[i])] + r) * nd + fmap[static_cast<int>(node[j])] +
+                              3 * half;
+                row[0] += cond * v0;
+                row[1] += cond * v1;
+                row[2] += cond * v2;
+            });
         __syncthreads();
     }
 }
@@ -1943,35 +2057,14 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
                 if (fmap[mn] < 0) W[(lpos[n] * 6 + c) * ldw + mc] -= cond * acc;
                 else resid[mn * 6 + c] += acc;
             }
-            for (int t = tid; t < N * N * 6; t += NT) {
-                const int pr = t / 6, r = t % 6;
-                const int i = pr / N, j = pr % N;
-                double Lr[3] = {0., 0., 0.}, RS[3] = {0., 0., 0.}, RI[3] = {0., 0., 0.};
-                for (int qp = 0; qp < qn; ++qp) {
-                    const int qa = q0 + qp;
-                    const double pi = phi[qa * N + i], pj = phi[qa * N + j];
-                    const double di = dphi[qa * N + i], dj = dphi[qa * N + j];
-                    const double coef[4] = {pi * pj, pi * dj, di * dj, di * pj};
-#pragma unroll
-                    for (int mm = 0; mm < 4; ++mm) {
-                        const double* g = G + (4 * qp + mm) * 56;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            Lr[c] += coef[mm] * g[gcol(r * 3 + c)];
-                            RS[c] += coef[mm] * g[gcol(18 + r * 3 + c)];
-                            RI[c] += coef[mm] * g[gcol(36 + r * 3 + c)];
-                        }
-                    }
-                }
-                const double* Tj = sT + static_cast<int>(node[j]) * 9;
-                double* row = W + (lpos[i] * 6 + r) * ldw + lpos[j] * 6;
-                for (int c = 0; c < 3; ++c) row[c] += cond * Lr[c];
-                for (int c = 0; c < 3; ++c) {
-                    double v = RI[c];
-                    for (int k = 0; k < 3; ++k) v += RS[k] * Tj[k * 3 + c];
-                    row[3 + c] += cond * v;
-                }
-            }
+            integrate_node_pairs<NT>(
+                N, qn, phi + q0 * N, dphi + q0 * N, G, [&](int j) { return sT + static_cast<int>(node[j]) * 9; },
+                [&](int i, int j, int r, int half, double v0, double v1, double v2) {
+                    double* row = W + (lpos[i] * 6 + r) * ldw + lpos[j] * 6 + 3 * half;
+                    row[0] += cond * v0;
+                    row[1] += cond * v1;
+                    row[2] += cond * v2;
+                });
             __syncthreads();
             sub(kPhaseLUDiag);
         }
@@ -2310,7 +2403,8 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         // masses and springs (residual into resid, conditioned blocks into Md)
         for (int n = tid; n < N; n += NT)
             add_lumped_terms(n, KB.lumped, KB.n_mass, KB.n_spring, sq, sv, svd, sT, KB.gravity,
-                             P.beta_prime, P.gamma_prime, cond, fmap, Md, md, resid, 1);
+                             P.beta_prime, P.gamma_prime, cond, fmap,
+                             [&](int r, int c) -> double& { return Md[r * md + c]; }, resid, 1);
         if (KB.n_comps > 0) {  // beam elements, then their node_FX (summed per node)
             __syncthreads();
             if (cnd) cond_add_schur<NT>(KB, S, smem_raw, fmap, Md, md, bc);
@@ -2794,9 +2888,6 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     __syncthreads();
     sec_prefetch();
 
-    if (sizeof(TR) == 4 && (Q & 1))  // zero pad point of the FP32 integration GEMM
-        for (int k = tid; k < 4 * 56; k += NT) G[4 * Q * 56 + k] = TG(0);
-
     // ---- PredictNextState (src/step/predict_next_state.hpp:14-47) ------------
     for (int k = tid; k < N * 7; k += NT) sqp[k] = sq[k];
     for (int k = tid; k < N * 6; k += NT) {
@@ -2887,7 +2978,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         mark(kPhaseQuadrature);
 
         // ---- residual integration (integrate_residual_vector.hpp:33-50) ----------
-        for (int t = tid; t < N * 6; t += NT) {
+        for (int t = NT - 1 - tid; t < N * 6; t += NT) {  // the last warps have fewer pair units
             const int n = t / 6, c = t % 6;
             double acc = 0.;
             for (int qp = 0; qp < Q; ++qp) {
@@ -2898,94 +2989,23 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             resid[t] = acc - slab[L.fx + t];
         }
 
-        // ---- stiffness + inertia integration and S T + I (integrate_*_matrix.hpp,
-        //      calculate_system_matrix.hpp), scaled by the conditioner into A.
-        //      For node pair (i,j):  C_ij = sum_q sum_m coef_m(i,j,q) G[4q+m]  with
-        //      coef = (phi_i phi_j, phi_i phi'_j, phi'_i phi'_j, phi'_i phi_j) and G the
-        //      weighted blocks written by the quadrature phase (K/inertia, P, C, O
-        //      terms).  C_ij holds [S+I left | S right | I right]; then
-        //      SM_ij = [C_L | C_RS T_j + C_RI] (T_j is identity on the translational
-        //      block).  The pair GEMM runs on the FP64 tensor cores: each warp owns
-        //      tiles of 8 pairs and all 7 column tiles, one k-step of 4 (m = 0..3) per
-        //      point, and writes SM_ij from its accumulators (column layout: gcol).
-        __syncthreads();
-        {
-            const int P2 = N * N;
-            const int s4 = lane & 3;
-            const double* fi_tab = (s4 < 2) ? phi : dphi;
-            const double* fj_tab = (s4 == 0 || s4 == 3) ? phi : dphi;
-            const double cond = P.conditioner;
-            if constexpr (sizeof(TR) == 8) {
-                // FP64 tensor cores, m8n8k4: 8 pairs per tile, one point per k-step
-                for (int p0 = 8 * warp; p0 < P2; p0 += 8 * NW) {
-                    const int prow = p0 + (lane >> 2);
-                    const bool valid = prow < P2;
-                    const int i = valid ? prow / N : 0, jn = valid ? prow % N : 0;
-                    double acc[7][2];
-#pragma unroll
-                    for (int nt = 0; nt < 7; ++nt) acc[nt][0] = acc[nt][1] = 0.;
-                    for (int q = 0; q < Q; ++q) {
-                        const double av = valid ? fi_tab[q * N + i] * fj_tab[q * N + jn] : 0.;
-                        const TG* gq = G + (4 * q + s4) * 56 + (lane >> 2);
-#pragma unroll
-                        for (int nt = 0; nt < 7; ++nt) dmma884(acc[nt][0], acc[nt][1], av, gq[nt * 8]);
-                    }
-                    if (valid)
-                        store_pair_block(A, ldA, pos, sT, i, jn, s4, cond,
-                                         [&](int t) { return acc[t >> 1][t & 1]; });
-                }
-            } else {
-                // FP32 form: TF32 tensor cores with the 3-term split (hi*hi + hi*lo +
-                // lo*hi, FP32 accumulation), m16n8k8: 16 pairs per tile, two points
-                // per k-step (an odd Q reads the zero pad point).
-                const int g8 = lane >> 2;
-                const int QK = (Q + 1) >> 1;
-                for (int p0 = 16 * warp; p0 < P2; p0 += 16 * NW) {
-                    const int pa = p0 + g8, pb = p0 + g8 + 8;
-                    const bool va = pa < P2, vb = pb < P2;
-                    const int ia = va ? pa / N : 0, ja = va ? pa % N : 0;
-                    const int ib = vb ? pb / N : 0, jb = vb ? pb % N : 0;
-                    float acc[7][4];
-#pragma unroll
-                    for (int nt = 0; nt < 7; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-                    for (int ks = 0; ks < QK; ++ks) {
-                        const int q0 = 2 * ks, q1 = 2 * ks + 1;
-                        const bool q1ok = q1 < Q;
-                        const int q1c = q1ok ? q1 : q0;
-                        float av[4];
-                        av[0] = va ? static_cast<float>(fi_tab[q0 * N + ia] * fj_tab[q0 * N + ja]) : 0.f;
-                        av[1] = vb ? static_cast<float>(fi_tab[q0 * N + ib] * fj_tab[q0 * N + jb]) : 0.f;
-                        av[2] = (va && q1ok) ? static_cast<float>(fi_tab[q1c * N + ia] * fj_tab[q1c * N + ja]) : 0.f;
-                        av[3] = (vb && q1ok) ? static_cast<float>(fi_tab[q1c * N + ib] * fj_tab[q1c * N + jb]) : 0.f;
-                        unsigned ah[4], al[4];
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) split_tf32(av[r], ah[r], al[r]);
-                        const TG* g0 = G + (4 * q0 + s4) * 56 + g8;
-                        const TG* g1 = G + (4 * q1 + s4) * 56 + g8;
-#pragma unroll
-                        for (int nt = 0; nt < 7; ++nt) {
-                            unsigned bh[2], bl[2];
-                            split_tf32(static_cast<float>(g0[nt * 8]), bh[0], bl[0]);
-                            split_tf32(static_cast<float>(g1[nt * 8]), bh[1], bl[1]);
-                            mma_tf32(acc[nt], al, bh);
-                            mma_tf32(acc[nt], ah, bl);
-                            mma_tf32(acc[nt], ah, bh);
-                        }
-                    }
-                    if (va)
-                        store_pair_block(A, ldA, pos, sT, ia, ja, s4, cond,
-                                         [&](int t) { return static_cast<double>(acc[t >> 1][t & 1]); });
-                    if (vb)
-                        store_pair_block(A, ldA, pos, sT, ib, jb, s4, cond,
-                                         [&](int t) { return static_cast<double>(acc[t >> 1][2 + (t & 1)]); });
-                }
-            }
-        }
+        // ---- stiffness + inertia integration and S T + I, scaled by the conditioner
+        //      into A (the residual's inputs stay untouched)
+        integrate_node_pairs<NT>(
+            N, Q, phi, dphi, G, [&](int j) { return sT + j * 9; },
+            [&](int i, int j, int r, int half, double v0, double v1, double v2) {
+                const int row = 6 * pos[i] + r, col = 6 * pos[j] + 3 * half, sh = row & 6;
+                TR* a = A + row * ldA;
+                a[col ^ sh] = static_cast<TR>(v0 * P.conditioner);
+                a[(col + 1) ^ sh] = static_cast<TR>(v1 * P.conditioner);
+                a[(col + 2) ^ sh] = static_cast<TR>(v2 * P.conditioner);
+            });
         __syncthreads();
         if (LUMP && KB.n_mass + KB.n_spring > 0) {  // point masses and springs at this CTA's nodes
             for (int n = tid; n < N; n += NT)
                 add_lumped_terms(n, KB.lumped, KB.n_mass, KB.n_spring, sq, sv, svd, sT, KB.gravity,
-                                 P.beta_prime, P.gamma_prime, P.conditioner, pos, A, ldA, resid);
+                                 P.beta_prime, P.gamma_prime, P.conditioner, pos,
+                                 [&](int r, int c) -> TR& { return A[sys_at(ldA, r, c)]; }, resid);
             __syncthreads();
         }
         mark(kPhaseIntegrate);
@@ -3029,7 +3049,8 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             double* D = KB.dump;
             for (int t = tid; t < n6 * n6; t += NT) {
                 const int r = t / n6, c = t % n6;
-                D[r * nl + c] = static_cast<double>(A[(6 * pos[r / 6] + r % 6) * ldA + 6 * pos[c / 6] + c % 6]);
+                D[r * nl + c] = static_cast<double>(
+                    A[sys_at(ldA, 6 * pos[r / 6] + r % 6, 6 * pos[c / 6] + c % 6)]);
             }
             for (int t = tid; t < n6; t += NT) D[nl * nl + t] = bp[6 * pos[t / 6] + t % 6];
             if (tid < nc) {
@@ -3167,7 +3188,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         // (S2) free-row right-hand side, folded into column m of A (and kept in
         //      FP64 in bp[0:m]); a drive train adds the second right-hand side
         //      -A_fr d_r in column m + 1 (FP64 copy in rhs2)
-        double* gjv = reinterpret_cast<double*>(smem_raw + S.G + solve_vec_offset(N, sizeof(TR), NT, drive ? 2 : 0));
+        double* gjv = reinterpret_cast<double*>(smem_raw + S.G + solve_vec_offset(N, nc, sizeof(TR), NT, drive ? 2 : 0));
         double* r64 = gjv;                 // [n6] residual of the linear solve
         double* rhs2 = gjv + n6;           // [n6] second right-hand side (drive train)
         double* x2 = gjv + 2 * n6;         // [n6] its solution
@@ -3177,7 +3198,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             const int i = i0 + (lane >> 3), ic = min(i, m - 1);
             double r = 0., r2 = 0.;
             for (int j = m + (lane & 7); j < n6; j += 8) {
-                const double aij = static_cast<double>(A[ic * ldA + j]);
+                const double aij = static_cast<double>(A[sys_at(ldA, ic, j)]);
                 r -= aij * xs[j];
                 if (drive) r2 -= aij * droot[j];
             }
@@ -3188,10 +3209,10 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
             if ((lane & 7) == 0 && i < m) {
                 r += bp[i];
-                A[i * ldA + m] = static_cast<TR>(r);
+                A[sys_at(ldA, i, m)] = static_cast<TR>(r);
                 bp[i] = r;
                 if (drive) {
-                    A[i * ldA + m + 1] = static_cast<TR>(r2);
+                    A[sys_at(ldA, i, m + 1)] = static_cast<TR>(r2);
                     rhs2[i] = r2;
                 }
             }
@@ -3208,7 +3229,8 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         if (use_gj) {
           if constexpr (GJ) {
             TR R[GJTile<TR, NT>::RT][GJTile<TR, NT>::CT];
-            gj_eliminate<TR, NT, kInv>(A, ldA, m, nrhs, reinterpret_cast<TR*>(smem_raw + S.G), &s_flag, R);
+            TR* pivots = reinterpret_cast<TR*>(smem_raw + S.G);
+            gj_eliminate<TR, NT, kInv>(A, ldA, m, nrhs, pivots, &s_flag, R);
             mark(kPhaseFactor);
             // Backward error of a solve: max|b - A x| / (||A|| ||x|| + ||b||),
             // infinity norms, FP64, A as assembled (its FP32 rounding in the
@@ -3226,7 +3248,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                     for (int bb = 0; bb < GJTile<TR, NT>::CT; ++bb) {
                         const int j = cj + bb * kGJCols;
                         if (j < m && i < m) {
-                            const double aij = static_cast<double>(A[i * ldA + j]);
+                            const double aij = static_cast<double>(A[sys_at(ldA, i, j)]);
                             acc = fma(aij, x[j], acc);
                             asum += fabs(aij);
                             if (a == 0) xa = fmax(xa, fabs(x[j]));
@@ -3271,20 +3293,33 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 return den > 0. ? ra / den : 0.;
             };
             if constexpr (!kInv) {
-                gj_extract<TR, NT>(R, m, m, xs);
-                if (drive) gj_extract<TR, NT>(R, m, m + 1, x2);
-                __syncthreads();
                 // guard of the unpivoted elimination: the backward error of the
-                // solve, counted (checked, above kGJBackwardErrorMax, largest)
-                for (int rhs = 0; rhs < nrhs; ++rhs) {
-                    const double eta = backward_error(rhs ? x2 : xs, rhs ? rhs2 : bp, r64);
-                    if (tid == 0 && P.diag) {
-                        atomicAdd(P.diag + kDiagChecked, 1ull);
-                        if (!(eta <= kGJBackwardErrorMax)) atomicAdd(P.diag + kDiagGuardTrips, 1ull);
-                        if (eta == eta)
-                            atomicMax(P.diag + kDiagMaxBackwardError,
-                                      static_cast<unsigned long long>(__double_as_longlong(eta)));
+                // solve; above kGJBackwardErrorMax (element growth) the block,
+                // which shared memory still holds, is solved with row pivoting,
+                // and its residual once more (Gauss-Jordan's residual grows with
+                // the condition number even when pivoted).
+                // (One right-hand side: a drive train runs the LUMP instance.)
+                gj_extract<TR, NT>(R, m, m, xs);
+                __syncthreads();
+                double eta = backward_error(xs, bp, r64);
+                if (eta > kGJBackwardErrorMax) {
+                    double* dx = gjv + 3 * n6;
+                    for (int pass = 0; pass < 2; ++pass) {
+                        gj_solve_pivoted<TR, NT>(A, ldA, m, pivots, pass ? dx : xs, &s_flag);
+                        for (int i = tid; pass && i < m; i += NT) xs[i] += dx[i];
+                        __syncthreads();
+                        eta = backward_error(xs, bp, r64);
+                        for (int i = tid; i < m; i += NT) A[sys_at(ldA, i, m)] = r64[i];
+                        __syncthreads();
                     }
+                }
+                // counted: checked, still above the limit, largest
+                if (tid == 0 && P.diag) {
+                    atomicAdd(P.diag + kDiagChecked, 1ull);
+                    if (!(eta <= kGJBackwardErrorMax)) atomicAdd(P.diag + kDiagGuardTrips, 1ull);
+                    if (eta == eta)
+                        atomicMax(P.diag + kDiagMaxBackwardError,
+                                  static_cast<unsigned long long>(__double_as_longlong(eta)));
                 }
             } else {
                 // FP32 inverse in R; x = R b, then sweeps x += R (b - A x) with
@@ -3357,7 +3392,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 const int pr = 6 * pos[KB.con_node[c]];
                 double a1 = 0., a2 = 0.;
                 for (int j = lane; j < n6; j += 32) {
-                    const double arj = static_cast<double>(A[(pr + k) * ldA + j]);
+                    const double arj = static_cast<double>(A[sys_at(ldA, pr + k, j)]);
                     a1 += arj * xs[j];
                     a2 += arj * (j < m ? x2[j] : droot[j]);
                 }
@@ -3423,7 +3458,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             const int c = rowi / 6, k = rowi % 6;
             const int pr = 6 * pos[KB.con_node[c]];
             double sacc = 0.;
-            for (int j = lane; j < n6; j += 32) sacc += static_cast<double>(A[(pr + k) * ldA + j]) * xs[j];
+            for (int j = lane; j < n6; j += 32) sacc += static_cast<double>(A[sys_at(ldA, pr + k, j)]) * xs[j];
             for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
             if (lane == 0) con[c * kConStride + conrec::yr + k] = bp[pr + k] - sacc;
         }
