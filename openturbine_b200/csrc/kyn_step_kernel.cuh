@@ -160,37 +160,17 @@ __host__ __device__ inline int sec_doubles(int Q) { return ((3 * Q + 1) & ~1) + 
 
 // ---- shared-memory plan of one CTA --------------------------------------------
 // The kernel runs with NT = 128, 256 or 512 threads (up to four, two or one
-// CTAs per SM within the 128-register budget); NT/16 quadrature points are
-// processed per pass and NT/32 warps share the GEMM-shaped phases.  More
+// CTAs per SM within the 128-register budget); four quadrature points per warp
+// are processed at a time and NT/32 warps share the GEMM-shaped phases.  More
 // resident CTAs overlap more beams' serial sections (LU pivots); more warps
 // per CTA shorten the parallel phases of one beam.
-constexpr int kGroupScratch = 256;      // doubles of per-group scratch for QP math
 constexpr int kConStride = 96;          // doubles per constraint record in smem
+constexpr int kQpInterp = 24;           // doubles of interpolated values per quadrature point (qpi)
 constexpr int kHubSmem = 208;           // doubles of the hub record (hubsm)
 constexpr int kDriveSmem = 600;         // doubles of the hub record of a drive train
 
-// Per-group scratch (doubles) of the quadrature phase.
-namespace grec {
-constexpr int interp = 0;   // [20] interpolated sums
-constexpr int rn = 20;      // [4] normalised r
-constexpr int Rx = 24;      // [9] R(r o r0)
-constexpr int Rr = 33;      // [9] R(r)
-constexpr int st = 42;      // [6] strain
-constexpr int Mu = 48;      // [36] Muu
-constexpr int ms = 84;      // mass, eta[3], s = x0'+u' [3] at 88..90
-constexpr int O12 = 92;     // [9]
-constexpr int Gu = 101;     // [18]
-constexpr int Kk = 119;     // [9]
-constexpr int fcv = 128;    // [6]
-constexpr int Cu = 136;     // [36] Cuu (rotated stiffness)
-constexpr int mstar = 172;  // [36] sectional mass (material frame), staged from HBM
-constexpr int cstar = 208;  // [36] sectional stiffness
-constexpr int r0 = 244;     // [4]
-constexpr int x0p = 248;    // [3]
-}  // namespace grec
-
 struct Smem {
-    int A;              // TR [n6][ldA]; aliased by the per-group QP scratch
+    int A;              // TR [n6][ldA]; aliased by the interpolated values
     int G;              // TR [Q][kGPoint] weighted quadrature blocks (node-pair integration)
     int Fc, Fdig;       // double [Q][6]
     int phi, dphi;      // double [Q][N]
@@ -207,7 +187,7 @@ struct Smem {
     int hub;            // double [kHubSmem or kDriveSmem] hub state and records, or -1
     int pos;            // int [N]
     int sec;            // double [sec_doubles(Q)] staged sections, inside A's region after
-                        // the group scratch (quadrature phase only)
+                        // the interpolated values (quadrature phase only)
     int bar;            // uint64 mbarrier of the section copies
     int bytes;
     int ldA;
@@ -286,7 +266,7 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
     S.hub = hub ? take((hub > 1 ? kDriveSmem : kHubSmem) * 8) : -1;
     {
         const int a_bytes = n6 * S.ldA * real_bytes;
-        const int g_bytes = (nt / 16) * kGroupScratch * 8;
+        const int g_bytes = Q * kQpInterp * 8;
         const int q_bytes = g_bytes + sec_doubles(Q) * 8;
         S.A = take(a_bytes > q_bytes ? a_bytes : q_bytes);
         S.sec = S.A + g_bytes;
@@ -1432,7 +1412,7 @@ struct DenseSmem {
     int M, b, x, q, qp, v, vd, a, qd, T, resid, con, act, fmap, red;
     // beam components (dense models with beams): shape tables, weights and
     // node state of one component at a time, its quadrature-point outputs and
-    // the quadrature phase's group scratch
+    // the interpolated values
     int cphi, cdphi, cdphiJ, cqpw, cq, cv, cvd, cG, cFc, cFd, cgs;
     // condensed models: interior solution [6N], interior DOF map [N], the
     // bordered system's right-hand-side corrections [nd], one component's
@@ -1466,7 +1446,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     auto r16 = [](int b) { return (b + 15) & ~15; };
     const int w_bytes = cond_nd > 0 ? r16(cN * 6 * (cN * 6 + 1) * 8) : 0;
     const int g_bytes = cond_nd > 0 ? kCondChunk * kGPoint * 8 : 0;
-    const int s_bytes = cond_nd > 0 ? (nt / 16) * kGroupScratch * 8 : 0;
+    const int s_bytes = cond_nd > 0 ? kCondChunk * kQpInterp * 8 : 0;
     const int t_bytes = cond_nd > 0 ? 3 * r16(cQ * cN * 8) + r16(cQ * 4 * 8) + r16(cN * 7 * 8) +
                                           2 * r16(cN * 6 * 8) + 2 * r16(cQ * 6 * 8) : 0;
     const int c_bytes = w_bytes + g_bytes + s_bytes + t_bytes;
@@ -1519,7 +1499,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
         S.cG = take(cQ * kGPoint * 8);
         S.cFc = take(cQ * 6 * 8);
         S.cFd = take(cQ * 6 * 8);
-        S.cgs = take((nt / 16) * kGroupScratch * 8);
+        S.cgs = take(cQ * kQpInterp * 8);
     }
     S.xi = S.imap = S.bc = S.lpos = S.lnode = S.cx = -1;
     if (cond_nd > 0) {
@@ -1535,270 +1515,303 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
 }
 
 
+// ---- quadrature-point physics -----------------------------------------------------
+// Rows of x times tilde(w): each row crossed with w.
+__device__ __forceinline__ void rows_cross(const double (&x)[9], const double (&w)[3], double (&o)[9]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        o[3 * i] = fma(x[3 * i + 1], w[2], -(x[3 * i + 2] * w[1]));
+        o[3 * i + 1] = fma(x[3 * i + 2], w[0], -(x[3 * i] * w[2]));
+        o[3 * i + 2] = fma(x[3 * i], w[1], -(x[3 * i + 1] * w[0]));
+    }
+}
+// tilde(w) times x: w crossed with each column.
+__device__ __forceinline__ void cols_cross(const double (&w)[3], const double (&x)[9], double (&o)[9]) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        o[j] = fma(w[1], x[6 + j], -(w[2] * x[3 + j]));
+        o[3 + j] = fma(w[2], x[j], -(w[0] * x[6 + j]));
+        o[6 + j] = fma(w[0], x[3 + j], -(w[1] * x[j]));
+    }
+}
+// o += tilde(w)
+__device__ __forceinline__ void add_tilde(double (&o)[9], const double (&w)[3]) {
+    o[1] -= w[2];
+    o[2] += w[1];
+    o[3] += w[2];
+    o[5] -= w[0];
+    o[6] -= w[1];
+    o[7] += w[0];
+}
+__device__ __forceinline__ void mul3(const double (&x)[9], const double (&w)[3], double (&o)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = fma(x[3 * i + 2], w[2], fma(x[3 * i + 1], w[1], x[3 * i] * w[0]));
+}
+
+// Interpolated values of one point in shared memory (doubles): r, u_ddot, omega,
+// omega_dot by the shape values, u' and r' by the shape derivatives.
+namespace qpi {
+constexpr int r = 0, udd = 4, om = 7, omd = 10, up = 16, rp = 19;
+}  // namespace qpi
+
 // Quadrature-point physics of one beam system (calculate_quadrature_point_values.hpp:
-// a6-a10 of the step path): 16 threads per quadrature point, NT/16 points per
-// pass.  Each stage gives every lane of a group the same formula on its own
-// entries, so the half-warps run without divergence.  Inputs: shape tables
-// phi / dphiJ [Q][N], weights qpw [Q][4], node state q [N][7], v, vd [N][6]
-// (shared memory), the system's slab for the sections and reference frames
-// (layout L).  Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the
-// integration G [Q][kGPoint] (gblk).  gscr: NT/16 groups of
-// kGroupScratch doubles.  sec: the sections already staged in shared memory
-// (sec_doubles(Q), slab order from x0'), or null to read them from the slab.
+// a6-a10 of the step path).  Inputs: shape tables phi / dphiJ [Q][N], weights
+// qpw [Q][4], node state q [N][7], v, vd [N][6] (shared memory), the system's
+// slab for the sections and reference frames (layout L), or sec: the sections
+// already staged in shared memory (sec_doubles(Q), slab order from x0').
+// Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the integration
+// G [Q][kGPoint] (gblk).  itp: kQpInterp doubles of scratch per point.
+//
+// The 20 interpolations are products [Q x N][N x 13] and [Q x N][N x 7] on the
+// FP64 tensor cores.  Then eight lanes take a point, one rotated 3x3 block each
+// (C11, C12, C21, C22, M11, M12, M21, M22), with the point's kinematics computed
+// alike in all eight.  Every further matrix is such a block with its rows or
+// columns crossed with a vector, or a dyad, so that one sequence of operations
+// in registers serves all lanes, the operands selected by block:
+//   O12 = C11 S - N~, O22 = C21 S - M~, P21 = S^T C11 + N~, P22 = S^T C12,
+//   Q22 = S^T O12, G22 = w~ rho - (rho w)~,
+//   K22 = rho w'~ - (rho w')~ + u''~ m~ + w~ (rho w~ - (rho w)~),
+//   a~ b~ = b a^T - (a.b) I for G12, K12 and u''~ m~.
+// The former form spent 16 lanes on a point, each entry by index arithmetic on
+// shared memory with the six kinds of lanes one after the other: 23k cycles per
+// iteration at 13 and at 21 nodes.
 template <typename TG, int NT>
 __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const double* dphiJ,
                                          const double* qpw, const double* sq, const double* sv,
                                          const double* svd, const double* __restrict__ slab,
                                          const SlabLayout& L, const double* gravity, double beta_prime,
-                                         double gamma_prime, double* gscr, TG* G, double* Fc, double* Fdig,
+                                         double gamma_prime, double* itp, TG* G, double* Fc, double* Fdig,
                                          const double* sec = nullptr) {
-    constexpr int NG = NT / 16;
-    const int tid = threadIdx.x;
-    const int grp = tid >> 4;
-    const int g = tid & 15;
-    double* gs = gscr + grp * kGroupScratch;
-    double* rn = gs + grec::rn;
-    double* Rx = gs + grec::Rx;
-    double* Rr = gs + grec::Rr;
-    double* st = gs + grec::st;
-    double* Mu = gs + grec::Mu;
-    double* ms = gs + grec::ms;
-    double* O12 = gs + grec::O12;
-    double* Gu = gs + grec::Gu;
-    double* Kk = gs + grec::Kk;
-    double* fcv = gs + grec::fcv;
-    double* Cu = gs + grec::Cu;
-    const double* mst = gs + grec::mstar;
-    const double* cst = gs + grec::cstar;
-    const double* r0 = gs + grec::r0;
-    const double* x0p = gs + grec::x0p;
-    for (int q0 = 0; q0 < Q; q0 += NG) {
-        const int qp = q0 + grp;
-        const bool act = qp < Q;
-        const double* ph_q = phi + qp * N;
-        if (sec) {  // staged by the bulk copy: this point's entries in place
-            const int qc = act ? qp : 0;
-            const int o_r0 = (3 * Q + 1) & ~1;
-            x0p = sec + qc * 3;
-            r0 = sec + o_r0 + qc * 4;
-            mst = sec + o_r0 + 4 * Q + qc * 36;
-            cst = mst + 36 * Q;
-        }
-        if (act) {
-            // stage this point's sections and reference frame from the slab
-            // (read early: the loads overlap the interpolation below)
-            for (int k = g; k < 79 && !sec; k += 16) {
-                double v;
-                if (k < 36) v = slab[L.mstar + qp * 36 + k];
-                else if (k < 72) v = slab[L.cstar + qp * 36 + (k - 36)];
-                else if (k < 76) v = slab[L.r0 + qp * 4 + (k - 72)];
-                else v = slab[L.x0p + qp * 3 + (k - 76)];
-                gs[grec::mstar + k] = v;
-            }
-            // P has no translational rows
-            TG* Gq = G + qp * kGPoint;
-            if (g < 9) Gq[(g / 3) * kGRow + gblk::PL + g % 3] = Gq[(g / 3) * kGRow + gblk::PR + g % 3] = TG(0);
-        }
-        // (1) interpolation: r, u_ddot, omega, omega_dot, u', r'
-        if (act) {
-            for (int k = g; k < 20; k += 16) {
-                // source column of node state and shape table for sum k
-                const double* src = (k < 4) ? sq + 3 + k
-                                  : (k < 7) ? svd + (k - 4)
-                                  : (k < 10) ? sv + 3 + (k - 7)
-                                  : (k < 13) ? svd + 3 + (k - 10)
-                                  : (k < 16) ? sq + (k - 13)
-                                             : sq + 3 + (k - 16);
-                const int stride = (k < 4 || k >= 13) ? 7 : 6;
-                const double* shp = (k < 13) ? ph_q : dphiJ + qp * N;
-                double acc = 0.;
-                for (int n = 0; n < N; ++n) acc += src[n * stride] * shp[n];
-                gs[k] = acc;
-            }
-        }
-        __syncwarp();
-        if (act && g < 4) {
-            const double nr = sqrt(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2] + gs[3] * gs[3]);
-            rn[g] = gs[g] / nr;
-        }
-        __syncwarp();
-        // (2) R(xr), R(r), rotational strain 2 E(r) r', s = x0' + u'
-        if (act) {
-            for (int k = g; k < 24; k += 16) {
-                if (k < 9) {
-                    double xr[4];
-                    quat_compose(rn, r0, xr);
-                    Rx[k] = rot_entry(xr, k / 3, k % 3);
-                } else if (k < 18) {
-                    Rr[k - 9] = rot_entry(rn, (k - 9) / 3, (k - 9) % 3);
-                } else if (k < 21) {
-                    // 2 E(r) r' with E = QuaternionDerivative (3x4)
-                    const int i = k - 18;
-                    const double* rp = gs + 16;
-                    double e;
-                    if (i == 0) e = -rn[1] * rp[0] + rn[0] * rp[1] - rn[3] * rp[2] + rn[2] * rp[3];
-                    else if (i == 1) e = -rn[2] * rp[0] + rn[3] * rp[1] + rn[0] * rp[2] - rn[1] * rp[3];
-                    else e = -rn[3] * rp[0] - rn[2] * rp[1] + rn[1] * rp[2] + rn[0] * rp[3];
-                    st[3 + i] = 2. * e;
-                } else {
-                    ms[4 + (k - 21)] = x0p[k - 21] + gs[13 + (k - 21)];
-                }
-            }
-        }
-        __syncwarp();
-        // (3) Muu = R M* R^T, Cuu = R C* R^T; translational strain
-        if (act) {
-            for (int o = g; o < 75; o += 16) {
-                if (o < 72) {
-                    const int e = o % 36;
-                    const int i = e / 6, j = e % 6;
-                    const int bi = i / 3, bj = j / 3, ii = i % 3, jj = j % 3;
-                    const double* Cs = (o < 36) ? mst : cst;
-                    double acc = 0.;
-                    for (int pp = 0; pp < 3; ++pp) {
-                        double t = 0.;
-                        for (int ss = 0; ss < 3; ++ss)
-                            t += Cs[(3 * bi + pp) * 6 + 3 * bj + ss] * Rx[jj * 3 + ss];
-                        acc += Rx[ii * 3 + pp] * t;
-                    }
-                    if (o < 36) Mu[e] = acc;
-                    else Cu[e] = acc;
-                } else {
-                    // strain[i] = x0' + u' - R(r) x0'  (calculate_strain.hpp:27-46)
-                    const int i = o - 72;
-                    double rx = 0.;
-                    for (int j = 0; j < 3; ++j) rx += Rr[i * 3 + j] * x0p[j];
-                    st[i] = x0p[i] + gs[13 + i] - rx;
-                }
-            }
-        }
-        __syncwarp();
-        // (4) FC = Cuu eps (calculate_force_FC.hpp); mass and eta (CalculateEta)
-        if (act && g < 6) {
-            double f = 0.;
-            for (int j = 0; j < 6; ++j) f += Cu[g * 6 + j] * st[j];
-            fcv[g] = f;
-            Fc[qp * 6 + g] = f;
-        } else if (act && g == 6) {
-            const double mass = Mu[0];
-            ms[0] = mass;
-            ms[1] = Mu[5 * 6 + 1] / mass;
-            ms[2] = -Mu[5 * 6 + 0] / mass;
-            ms[3] = Mu[4 * 6 + 0] / mass;
-        }
-        __syncwarp();
-        const double* ud = gs + 4;
-        const double* om = gs + 7;
-        const double* omd = gs + 10;
-        const double* sv3 = ms + 4;  // x0' + u'
-        if (act && g < 9) {
-            // (5) entry (i,j) of every 3x3 block: Ouu, Puu (calculate_Ouu/Puu.hpp),
-            //     Guu (calculate_gyroscopic_matrix.hpp), Kuu
-            //     (calculate_inertia_stiffness_matrix.hpp)
-            const int i = g / 3, j = g % 3;
-            const double mass = ms[0];
-            const double meta[3] = {mass * ms[1], mass * ms[2], mass * ms[3]};
-            double rw[3], rwd[3], wme[3];
-            for (int r = 0; r < 3; ++r) {
-                rw[r] = Mu[(3 + r) * 6 + 3] * om[0] + Mu[(3 + r) * 6 + 4] * om[1] +
-                        Mu[(3 + r) * 6 + 5] * om[2];
-                rwd[r] = Mu[(3 + r) * 6 + 3] * omd[0] + Mu[(3 + r) * 6 + 4] * omd[1] +
-                         Mu[(3 + r) * 6 + 5] * omd[2];
-            }
-            cross3(om, meta, wme);
-            double o12 = -tilde_e(fcv, i, j), o22 = -tilde_e(fcv + 3, i, j);
-            double p21 = tilde_e(fcv, i, j), p22 = 0.;
-            double g12 = -tilde_e(wme, i, j), g22 = -tilde_e(rw, i, j);
-            double k12 = 0., k22 = -tilde_e(rwd, i, j);
-            for (int k = 0; k < 3; ++k) {
-                const double s_kj = tilde_e(sv3, k, j);
-                const double s_ki = tilde_e(sv3, k, i);
-                o12 += Cu[i * 6 + k] * s_kj;
-                o22 += Cu[(3 + i) * 6 + k] * s_kj;
-                p21 += s_ki * Cu[k * 6 + j];
-                p22 += s_ki * Cu[k * 6 + 3 + j];
-                const double w_ik = tilde_e(om, i, k);
-                const double me_kj = tilde_e(meta, k, j);
-                g12 -= w_ik * me_kj;
-                g22 += w_ik * Mu[(3 + k) * 6 + 3 + j];
-                double ww = 0.;
-                for (int l = 0; l < 3; ++l) ww += tilde_e(om, i, l) * tilde_e(om, l, k);
-                k12 -= (tilde_e(omd, i, k) + ww) * me_kj;
-                k22 += Mu[(3 + i) * 6 + 3 + k] * tilde_e(omd, k, j);
-                k22 += tilde_e(ud, i, k) * me_kj;
-                double inner = -tilde_e(rw, k, j);
-                for (int l = 0; l < 3; ++l) inner += Mu[(3 + k) * 6 + 3 + l] * tilde_e(om, l, j);
-                k22 += w_ik * inner;
-            }
-            const double w = qpw[qp * 4], wJ = qpw[qp * 4 + 2];
-            TG* Gt = G + qp * kGPoint + i * kGRow + j;  // rows 0..2
-            TG* Gr = Gt + 3 * kGRow;                    // rows 3..5
-            O12[g] = o12;
-            Gt[gblk::O] = static_cast<TG>(w * o12);
-            Gr[gblk::O] = static_cast<TG>(w * o22);
-            Gr[gblk::PL] = static_cast<TG>(w * p21);
-            Gr[gblk::PR] = static_cast<TG>(w * p22);
-            Gu[g] = g12;
-            Gu[9 + g] = g22;
-            Gt[gblk::K] = static_cast<TG>(wJ * k12);
-            Kk[g] = k22;
-        } else if (act && g < 15) {
-            // Fd + Fi - Fe - Fg (calculate_force_FD.hpp, calculate_inertial_force.hpp,
-            // calculate_gravity_force.hpp; Fe = 0)
-            const int c = g - 9;
-            const double mass = ms[0];
-            const double eta[3] = {ms[1], ms[2], ms[3]};
-            double fd = 0., fi, fgv;
-            if (c < 3) {
-                double wxe[3], wxwxe[3], wdxe[3];
-                cross3(om, eta, wxe);
-                cross3(om, wxe, wxwxe);
-                cross3(omd, eta, wdxe);
-                fi = mass * ud[c] + mass * (wxwxe[c] + wdxe[c]);
-                fgv = mass * gravity[c];
+    constexpr int NW = NT / 32;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    {
+        const int g8 = lane >> 2, t = lane & 3;
+        const int qt = (Q + 7) >> 3;
+        for (int u = warp; u < 3 * qt; u += NW) {  // (tile of points, tile of columns)
+            const int ct = u / qt, q0 = 8 * (u - ct * qt);
+            const double* tab = (ct < 2 ? phi : dphiJ) + min(q0 + g8, Q - 1) * N;
+            const double* src;
+            int pitch = 6;
+            if (ct == 0) {
+                src = g8 < 4 ? sq + 3 + g8 : g8 < 7 ? svd + g8 - 4 : sv + 3;
+                if (g8 < 4) pitch = 7;
+            } else if (ct == 1) {
+                src = g8 < 2 ? sv + 4 + g8 : svd + min(g8 + 1, 5);
             } else {
-                const int i = c - 3;
-                for (int k = 0; k < 3; ++k) fd += tilde_e(sv3, k, i) * fcv[k];
-                double exu[3], rw[3], rwd[3], wxrw[3];
-                cross3(eta, ud, exu);
-                for (int r = 0; r < 3; ++r) {
-                    rw[r] = Mu[(3 + r) * 6 + 3] * om[0] + Mu[(3 + r) * 6 + 4] * om[1] +
-                            Mu[(3 + r) * 6 + 5] * om[2];
-                    rwd[r] = Mu[(3 + r) * 6 + 3] * omd[0] + Mu[(3 + r) * 6 + 4] * omd[1] +
-                             Mu[(3 + r) * 6 + 5] * omd[2];
+                src = sq + min(g8, 6);
+                pitch = 7;
+            }
+            double d0 = 0., d1 = 0.;
+#pragma unroll 2
+            for (int n0 = 0; n0 < N; n0 += 4) {
+                const int n = n0 + t, nc = min(n, N - 1);
+                dmma884(d0, d1, n < N ? tab[nc] : 0., src[nc * pitch]);
+            }
+            if (q0 + g8 < Q) store_pair(itp + (q0 + g8) * kQpInterp + 8 * ct + 2 * t, d0, d1);
+        }
+    }
+    __syncthreads();
+    const int role = lane & 7, bi = (role >> 1) & 1, bj = role & 1;
+    const bool mass_block = role >= 4;
+    for (int p0 = 4 * warp; p0 < Q; p0 += 4 * NW) {
+        const int qp = p0 + (lane >> 3), qc = min(qp, Q - 1);
+        const double *sx0, *sr0, *sblk;
+        if (sec) {
+            const int o = (3 * Q + 1) & ~1;
+            sx0 = sec + qc * 3;
+            sr0 = sec + o + qc * 4;
+            sblk = sec + o + 4 * Q + (mass_block ? 0 : 36 * Q) + qc * 36;
+        } else {
+            sx0 = slab + L.x0p + qc * 3;
+            sr0 = slab + L.r0 + qc * 4;
+            sblk = slab + (mass_block ? L.mstar : L.cstar) + qc * 36;
+        }
+        sblk += 18 * bi + 3 * bj;
+        const double* it = itp + qc * kQpInterp;
+        double X[9];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) X[e] = sblk[(e / 3) * 6 + e % 3];
+        double s[3], et[3], er[3];
+        {
+            double r[4], R[9], T[9];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r[e] = it[qpi::r + e];
+            const double nr = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]), inv = 1. / nr;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {  // r / nr, its residual put right
+                const double v = r[e] * inv;
+                r[e] = fma(fma(-v, nr, r[e]), inv, v);
+            }
+            // strain x0' + u' - R(r) x0', 2 E(r) r' (calculate_strain.hpp:27-46)
+            const double x0[3] = {sx0[0], sx0[1], sx0[2]};
+            double rx[3];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) R[e] = rot_entry(r, e / 3, e % 3);
+            mul3(R, x0, rx);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                s[e] = x0[e] + it[qpi::up + e];
+                et[e] = s[e] - rx[e];
+            }
+            const double rp[4] = {it[qpi::rp], it[qpi::rp + 1], it[qpi::rp + 2], it[qpi::rp + 3]};
+            er[0] = 2. * (-r[1] * rp[0] + r[0] * rp[1] - r[3] * rp[2] + r[2] * rp[3]);
+            er[1] = 2. * (-r[2] * rp[0] + r[3] * rp[1] + r[0] * rp[2] - r[1] * rp[3]);
+            er[2] = 2. * (-r[3] * rp[0] - r[2] * rp[1] + r[1] * rp[2] + r[0] * rp[3]);
+            // the block in the current frame, R(r o r0) X R^T
+            double xr[4];
+            const double r0[4] = {sr0[0], sr0[1], sr0[2], sr0[3]};
+            quat_compose(r, r0, xr);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) R[e] = rot_entry(xr, e / 3, e % 3);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    T[3 * i + j] = fma(X[3 * i], R[3 * j],
+                                       fma(X[3 * i + 1], R[3 * j + 1], X[3 * i + 2] * R[3 * j + 2]));
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    X[3 * i + j] = fma(R[3 * i], T[j], fma(R[3 * i + 1], T[3 + j], R[3 * i + 2] * T[6 + j]));
+        }
+        // FC = Cuu eps (calculate_force_FC.hpp); rho omega, rho omega'; mass and
+        // mass * eta from the rotated mass matrix
+        double y[3], yd[3], ft[3], fr[3], me[3];
+        {
+            double a[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) a[e] = mass_block ? it[qpi::om + e] : bj ? er[e] : et[e];
+            mul3(X, a, y);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) a[e] = it[qpi::omd + e];
+            mul3(X, a, yd);
+        }
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const double f = y[e] + __shfl_xor_sync(kAll, y[e], 1);
+            ft[e] = __shfl_sync(kAll, f, 0, 8);
+            fr[e] = __shfl_sync(kAll, f, 2, 8);
+        }
+        const double m = __shfl_sync(kAll, X[0], 4, 8);
+        me[0] = __shfl_sync(kAll, X[7], 6, 8);
+        me[1] = -__shfl_sync(kAll, X[6], 6, 8);
+        me[2] = __shfl_sync(kAll, X[3], 6, 8);
+        const bool on = qp < Q;
+        const double w = qpw[qc * 4], wJ = qpw[qc * 4 + 2];
+        TG* Gq = G + qc * kGPoint;
+        // blocks crossed with s (stiffness) or omega (mass): columns first
+        double c[3], om[3], V[9];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            om[e] = it[qpi::om + e];
+            c[e] = mass_block ? om[e] : -s[e];
+        }
+        double wme[3];  // omega x mass eta
+        cross3(om, me, wme);
+        const double wdm = om[0] * me[0] + om[1] * me[1] + om[2] * me[2];
+        {
+            double Z[9], tz[3];
+            cols_cross(c, X, Z);
+            if (role == 5) {  // G12 (calculate_gyroscopic_matrix.hpp)
+#pragma unroll
+                for (int e = 0; e < 9; ++e) Z[e] = (e % 4 == 0 ? wdm : 0.) - me[e / 3] * om[e % 3];
+            }
+#pragma unroll
+            for (int e = 0; e < 3; ++e) tz[e] = role == 0 ? ft[e] : role == 7 ? -y[e] : role == 5 ? -wme[e] : 0.;
+            add_tilde(Z, tz);  // P21, P22; G12, G22
+            if (on) {
+                // C, XI = beta' Muu + gamma' Guu; P (no translational rows)
+                TG* o = Gq + 3 * bi * kGRow + (mass_block ? (bj ? gblk::XIR : gblk::XIL) : (bj ? gblk::CR : gblk::CL));
+                const double sc = mass_block ? wJ * beta_prime : qpw[qc * 4 + 3];
+                const double sg = mass_block && bj ? wJ * gamma_prime : 0.;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) o[(e / 3) * kGRow + e % 3] = static_cast<TG>(fma(sg, Z[e], sc * X[e]));
+                if (role < 4) {
+                    TG* pp = Gq + (role < 2 ? 3 * kGRow : 0) + (bj ? gblk::PR : gblk::PL);
+                    const double wp = role < 2 ? w : 0.;
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) pp[(e / 3) * kGRow + e % 3] = static_cast<TG>(wp * Z[e]);
                 }
-                cross3(om, rw, wxrw);
-                fi = mass * exu[i] + rwd[i] + wxrw[i];
-                const double mg[3] = {mass * gravity[0], mass * gravity[1],
-                                      mass * gravity[2]};
-                double exg[3];
-                cross3(eta, mg, exg);
-                fgv = exg[i];
-            }
-            Fdig[qp * 6 + c] = fd + fi - fgv;
-        }
-        __syncwarp();
-        // (6) Quu_22 = SS^T (C11 SS - N~) joins Kuu_22; XI = beta' Muu + gamma' Guu
-        if (act) {
-            const double wJ = qpw[qp * 4 + 2], wdJ = qpw[qp * 4 + 3];
-            TG* Gq = G + qp * kGPoint;
-            if (g < 9) {
-                const int i = g / 3, j = g % 3;
-                double qv = 0.;
-                for (int k = 0; k < 3; ++k) qv += tilde_e(sv3, k, i) * O12[k * 3 + j];
-                Gq[(3 + i) * kGRow + gblk::K + j] = static_cast<TG>(wJ * (Kk[g] + qv));
-            }
-            for (int e = g; e < 36; e += 16) {
-                const int i = e / 6, j = e % 6;
-                double gg = 0.;
-                if (j >= 3) gg = Gu[(i < 3 ? 0 : 9) + (i % 3) * 3 + (j - 3)];
-                const double xi = beta_prime * Mu[e] + gamma_prime * gg;
-                TG* row = Gq + i * kGRow;
-                row[j < 3 ? gblk::XIL + j : gblk::XIR + j - 3] = static_cast<TG>(wJ * xi);
-                row[j < 3 ? gblk::CL + j : gblk::CR + j - 3] = static_cast<TG>(wdJ * Cu[e]);
             }
         }
-        __syncwarp();
+        {
+            double Y[9], ty[3], a[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                a[e] = mass_block ? om[e] : s[e];
+                ty[e] = -(role == 0 ? ft[e] : role == 2 ? fr[e] : y[e]);
+            }
+            rows_cross(X, a, Y);
+            add_tilde(Y, ty);  // O12, O22; rho w~ - (rho w)~
+            if (on && (role == 0 || role == 2)) {
+                TG* oo = Gq + 3 * bi * kGRow + gblk::O;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) oo[(e / 3) * kGRow + e % 3] = static_cast<TG>(w * Y[e]);
+            }
+            cols_cross(c, Y, V);  // Q22; w~ (rho w~ - (rho w)~)
+        }
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            const double q22 = __shfl_sync(kAll, V[e], 0, 8);
+            if (role == 7) V[e] += q22;
+        }
+        double ff[3] = {0., 0., 0.};
+        if (role == 7) {
+            // K22 (calculate_inertia_stiffness_matrix.hpp) + Q22; rotational part
+            // of Fd + Fi - Fg (calculate_force_FD.hpp, calculate_inertial_force.hpp,
+            // calculate_gravity_force.hpp)
+            double W[9], g3[3], t0[3], t1[3], t2[3], u3[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                u3[e] = it[qpi::udd + e];
+                t0[e] = it[qpi::omd + e];
+            }
+            rows_cross(X, t0, W);
+            const double um = u3[0] * me[0] + u3[1] * me[1] + u3[2] * me[2];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) V[e] += fma(me[e / 3], u3[e % 3], W[e]) - (e % 4 == 0 ? um : 0.);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                t0[e] = -yd[e];
+                g3[e] = u3[e] - gravity[e];
+            }
+            add_tilde(V, t0);
+            cross3(ft, s, t0);
+            cross3(me, g3, t1);
+            cross3(om, y, t2);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) ff[e] = t0[e] + t1[e] + yd[e] + t2[e];
+        } else if (role == 3) {  // K12
+            const double wd3[3] = {it[qpi::omd], it[qpi::omd + 1], it[qpi::omd + 2]};
+            const double wm = wd3[0] * me[0] + wd3[1] * me[1] + wd3[2] * me[2];
+#pragma unroll
+            for (int e = 0; e < 9; ++e)
+                V[e] = (e % 4 == 0 ? wm : 0.) - fma(me[e / 3], wd3[e % 3], wme[e / 3] * om[e % 3]);
+            const double t0[3] = {wdm * om[0], wdm * om[1], wdm * om[2]};
+            add_tilde(V, t0);
+        } else if (role == 6) {  // translational part of the forces
+            const double wd3[3] = {it[qpi::omd], it[qpi::omd + 1], it[qpi::omd + 2]};
+            double t0[3], t1[3];
+            cross3(om, wme, t0);
+            cross3(wd3, me, t1);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) ff[e] = fma(m, it[qpi::udd + e] - gravity[e], t0[e] + t1[e]);
+        }
+        if (on) {
+            if (role == 3 || role == 7) {
+                TG* kk = Gq + (role == 7 ? 3 * kGRow : 0) + gblk::K;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) kk[(e / 3) * kGRow + e % 3] = static_cast<TG>(wJ * V[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                if (role == 0) Fc[qp * 6 + e] = ft[e];
+                if (role == 2) Fc[qp * 6 + 3 + e] = fr[e];
+                if (role >= 6) Fdig[qp * 6 + (role == 7 ? 3 : 0) + e] = ff[e];
+            }
+        }
     }
 }
 
@@ -2745,7 +2758,6 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 int* __restrict__ status_out, int* __restrict__ iters_out) {
     static_assert(NT == 128 || NT == 256 || NT == 512, "step kernel runs with 128, 256 or 512 threads");
     constexpr int NW = NT / 32;  // warps
-    constexpr int NG = NT / 16;  // quadrature-point groups of 16 threads
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const KBeam& KB = beams[blockIdx.x];
     const int N = KB.N, Q = KB.Q, nc = KB.nc;
@@ -2800,7 +2812,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     __shared__ int s_flag;
     __shared__ unsigned long long s_ph[kNumPhases];
     // sections of the next quadrature phase: one bulk copy per Newton
-    // iteration (slab from x0' on -> the A region after the group scratch)
+    // iteration (slab from x0' on -> the A region after the interpolated values)
     uint64_t* sec_bar = reinterpret_cast<uint64_t*>(smem_raw + S.bar);
     double* sec = reinterpret_cast<double*>(smem_raw + S.sec);
     const uint32_t sec_bytes = static_cast<uint32_t>(sec_doubles(Q)) * 8u;
