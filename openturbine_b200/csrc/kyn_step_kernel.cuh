@@ -185,7 +185,7 @@ struct Smem {
     int con;            // double [nc][kConStride]
     int red;            // double [2][NT/32 + 8]  (offset 0: cluster exchange)
     int hub;            // double [kHubSmem or kDriveSmem] hub state and records, or -1
-    int pos;            // int [N]
+    int pos;            // int [2][N] row block of each node, node of each row block
     int sec;            // double [sec_doubles(Q)] staged sections, inside A's region after
                         // the interpolated values (quadrature phase only)
     int bar;            // uint64 mbarrier of the section copies
@@ -294,7 +294,7 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
     S.xs = take(n6 * 8);
     S.droot = hub > 1 ? take(n6 * 8) : -1;
     S.con = take((nc > 0 ? nc : 1) * kConStride * 8);
-    S.pos = take(N * 4);
+    S.pos = take(2 * N * 4);
     S.bar = take(8);
     S.bytes = o;
     return S;
@@ -1560,7 +1560,8 @@ constexpr int r = 0, udd = 4, om = 7, omd = 10, up = 16, rp = 19;
 // slab for the sections and reference frames (layout L), or sec: the sections
 // already staged in shared memory (sec_doubles(Q), slab order from x0').
 // Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the integration
-// G [Q][kGPoint] (gblk).  itp: kQpInterp doubles of scratch per point.
+// G [Q][kGPoint] (gblk).  itp: kQpInterp doubles of scratch per point.  Run by
+// warps 0 .. NW - 1; ALL: they are the whole CTA (else they meet at barrier 1).
 //
 // The 20 interpolations are products [Q x N][N x 13] and [Q x N][N x 7] on the
 // FP64 tensor cores.  Then eight lanes take a point, one rotated 3x3 block each
@@ -1575,14 +1576,13 @@ constexpr int r = 0, udd = 4, om = 7, omd = 10, up = 16, rp = 19;
 // The former form spent 16 lanes on a point, each entry by index arithmetic on
 // shared memory with the six kinds of lanes one after the other: 23k cycles per
 // iteration at 13 and at 21 nodes.
-template <typename TG, int NT>
+template <typename TG, int NW, bool ALL = true>
 __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const double* dphiJ,
                                          const double* qpw, const double* sq, const double* sv,
                                          const double* svd, const double* __restrict__ slab,
                                          const SlabLayout& L, const double* gravity, double beta_prime,
                                          double gamma_prime, double* itp, TG* G, double* Fc, double* Fdig,
                                          const double* sec = nullptr) {
-    constexpr int NW = NT / 32;
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     {
@@ -1611,7 +1611,8 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
             if (q0 + g8 < Q) store_pair(itp + (q0 + g8) * kQpInterp + 8 * ct + 2 * t, d0, d1);
         }
     }
-    __syncthreads();
+    if constexpr (ALL) __syncthreads();
+    else asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
     const int role = lane & 7, bi = (role >> 1) & 1, bj = role & 1;
     const bool mass_block = role >= 4;
     for (int p0 = 4 * warp; p0 < Q; p0 += 4 * NW) {
@@ -1860,7 +1861,7 @@ __device__ void dense_beam_terms(const KBeam& KB, const StepCoeffs& P, const Den
             cvd[k] = svd[n * 6 + k % 6];
         }
         __syncthreads();
-        qp_phase<double, NT>(N, Q, phi, dphiJ, qpw, cq, cv, cvd, cs, L, KB.gravity, P.beta_prime, P.gamma_prime,
+        qp_phase<double, NT / 32>(N, Q, phi, dphiJ, qpw, cq, cv, cvd, cs, L, KB.gravity, P.beta_prime, P.gamma_prime,
                              gscr, G, Fc, Fd);
         __syncthreads();
         for (int t = tid; t < N * 6; t += NT) {
@@ -2054,7 +2055,7 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
             Lc.cstar += 36 * q0;
             Lc.r0 += 4 * q0;
             Lc.x0p += 3 * q0;
-            qp_phase<double, NT>(N, qn, phi + q0 * N, dphiJ + q0 * N, qpw + q0 * 4, cq, cv, cvd, cs, Lc,
+            qp_phase<double, NT / 32>(N, qn, phi + q0 * N, dphiJ + q0 * N, qpw + q0 * 4, cq, cv, cvd, cs, Lc,
                                  KB.gravity, P.beta_prime, P.gamma_prime, gscr, G, Fc, Fd);
             __syncthreads();
             sub(kPhaseQuadrature);
@@ -2806,9 +2807,10 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     double* xs = reinterpret_cast<double*>(smem_raw + S.xs);
     double* droot = drive ? reinterpret_cast<double*>(smem_raw + S.droot) : nullptr;
     double* con = reinterpret_cast<double*>(smem_raw + S.con);
-    double* gscr = reinterpret_cast<double*>(smem_raw + S.A);  // quadrature phase only
+    double* itp = reinterpret_cast<double*>(smem_raw + S.A);  // quadrature phase only
     double* red = reinterpret_cast<double*>(smem_raw + S.red);
     int* pos = reinterpret_cast<int*>(smem_raw + S.pos);
+    int* node_at = pos + N;
     __shared__ int s_flag;
     __shared__ unsigned long long s_ph[kNumPhases];
     // sections of the next quadrature phase: one bulk copy per Newton
@@ -2818,10 +2820,8 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     const uint32_t sec_bytes = static_cast<uint32_t>(sec_doubles(Q)) * 8u;
     uint32_t sec_issued = 0, sec_waited = 0;  // copies issued / completed (thread 0 issues)
     const bool bulk = P.bulk_sections != 0;
-    auto sec_prefetch = [&]() {  // all threads, once every use of the region has ended
+    auto sec_issue = [&]() {  // all threads, after a proxy fence and a barrier behind the region's last use
         if (!bulk) return;
-        proxy_fence_async_smem();
-        __syncthreads();
         if (tid == 0) bulk_copy_g2s(sec, slab + L.x0p, sec_bytes, sec_bar);
         ++sec_issued;
     };
@@ -2885,20 +2885,23 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 hb[hubsm::ah + conrec::lam + k] = 0.;
             }
     }
-    if (tid == 0) {
-        // Free nodes first, constrained nodes last (in constraint order).
-        int p = 0;
-        for (int n = 0; n < N; ++n) {
-            bool constrained = false;
-            for (int c = 0; c < nc; ++c) constrained |= (KB.con_node[c] == n);
-            if (!constrained) pos[n] = p++;
+    if (tid < N) {  // free nodes first, constrained nodes last (in constraint order)
+        int before = 0, at = -1;
+        for (int c = 0; c < nc; ++c) {
+            const int n = KB.con_node[c];
+            before += n < tid;
+            if (n == tid) at = N - nc + c;
         }
-        for (int c = 0; c < nc; ++c) pos[KB.con_node[c]] = p++;
+        if (at < 0) at = tid - before;
+        pos[tid] = at;
+        node_at[at] = tid;
+    }
+    if (tid == 0) {
         s_flag = 0;
         mbar_init(sec_bar);
     }
     __syncthreads();
-    sec_prefetch();
+    sec_issue();
 
     // ---- PredictNextState (src/step/predict_next_state.hpp:14-47) ------------
     for (int k = tid; k < N * 7; k += NT) sqp[k] = sq[k];
@@ -2929,28 +2932,30 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     }
     __syncthreads();
     // CalculateDisplacement (src/state/calculate_displacement.hpp:25-50)
-    auto displacement = [&]() {
-        for (int n = tid; n < N; n += NT) {
-            for (int c = 0; c < 3; ++c) sq[n * 7 + c] = sqp[n * 7 + c] + h * sqd[n * 6 + c];
-            const double d[3] = {h * sqd[n * 6 + 3], h * sqd[n * 6 + 4], h * sqd[n * 6 + 5]};
-            double qd4[4], qn[4];
-            rotvec_to_quat(d, qd4);
-            quat_compose(qd4, sqp + n * 7 + 3, qn);
-            for (int c = 0; c < 4; ++c) sq[n * 7 + 3 + c] = qn[c];
-        }
-        if (hub && chain_rec()) {
-            double* hq = chain_rec() + hubrec::q;
-            const double* hqp = chain_rec() + hubrec::q_prev;
-            const double* hqd = chain_rec() + hubrec::q_delta;
-            for (int c = 0; c < 3; ++c) hq[c] = hqp[c] + h * hqd[c];
-            const double d[3] = {h * hqd[3], h * hqd[4], h * hqd[5]};
-            double qd4[4], qn[4];
-            rotvec_to_quat(d, qd4);
-            quat_compose(qd4, hqp + 3, qn);
-            for (int c = 0; c < 4; ++c) hq[3 + c] = qn[c];
+    auto displaced_rotation = [&](const double* qp, const double* qd, double* qn) {
+        const double d[3] = {h * qd[3], h * qd[4], h * qd[5]};
+        double qd4[4];
+        rotvec_to_quat(d, qd4);
+        quat_compose(qd4, qp + 3, qn);
+    };
+    auto displace = [&](int n, int c) {  // component c of q of node n
+        if (c < 3) {
+            sq[n * 7 + c] = sqp[n * 7 + c] + h * sqd[n * 6 + c];
+        } else {
+            double qn[4];
+            displaced_rotation(sqp + n * 7, sqd + n * 6, qn);
+            sq[n * 7 + c] = c == 3 ? qn[0] : c == 4 ? qn[1] : c == 5 ? qn[2] : qn[3];
         }
     };
-    displacement();
+    auto displace_chain = [&](double* r) {  // hub-chain record
+        for (int c = 0; c < 3; ++c) r[hubrec::q + c] = r[hubrec::q_prev + c] + h * r[hubrec::q_delta + c];
+        double qn[4];
+        displaced_rotation(r + hubrec::q_prev, r + hubrec::q_delta, qn);
+        for (int c = 0; c < 4; ++c) r[hubrec::q + 3 + c] = qn[c];
+    };
+    for (int t = tid; t < 8 * N; t += NT)
+        if ((t & 7) < 7) displace(t >> 3, t & 7);
+    if (hub && chain_rec()) displace_chain(chain_rec());
     __syncthreads();
     mark(kPhaseLoadPredict);
 
@@ -2979,13 +2984,146 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 }
             }
         };
-        for (int n = tid; n < N; n += NT) tangent_op(sqd + n * 6, sT + n * 9);
-        if (hub && chain_rec()) tangent_op(chain_rec() + hubrec::q_delta, chain_rec() + hubrec::tangent);
-
-        // ---- quadrature-point values (calculate_quadrature_point_values.hpp) ---
-        sec_wait();
-        qp_phase<TG, NT>(N, Q, phi, dphiJ, qpw, sq, sv, svd, slab, L, KB.gravity, P.beta_prime,
-                         P.gamma_prime, gscr, G, Fc, Fdig, bulk ? sec : nullptr);
+        // The last warp forms the tangent operators, the constraint records
+        // (calculate_constraint_residual_gradient.hpp:60-320) and the constrained
+        // nodes' corrections B x_r = -Phi while the others do the quadrature
+        // points: none of it needs their values, and its few lanes took 10k
+        // cycles per iteration when the whole CTA waited for them.
+        if (warp == NW - 1) {
+            if (lane < N) tangent_op(sqd + lane * 6, sT + lane * 9);
+            if (hub && chain_rec()) tangent_op(chain_rec() + hubrec::q_delta, chain_rec() + hubrec::tangent);
+            __syncwarp();
+            if (lane < nc) {
+                const int tn = KB.con_node[lane];
+                constraint_record(con + lane * kConStride, KB.con_type[lane], sq + tn * 7, KB.con_X0[lane],
+                                  sT + tn * 9, hub ? hj + hubrec::q : nullptr,
+                                  hub ? hj + hubrec::tangent : nullptr, KB.con_axis[lane]);
+            }
+            if (hub && lane == nc)  // the hub's own boundary condition
+                constraint_record(hb + hubsm::bc, KB.hub_con_type, hb + hubrec::q, hb + hubrec::X0,
+                                  hb + hubrec::tangent, nullptr, nullptr, nullptr);
+            if (drive && lane == nc + 1)  // revolute joint record 0 -> 1
+                revolute_record(hb + hubsm::rev, hb, hA);
+            if (drive && hH && lane == nc + 2)  // rigid joint record 1 -> 2
+                constraint_record(hb + hubsm::ah, KYN_CONSTRAINT_RIGID_JOINT, hH + hubrec::q, hH + hubrec::X0,
+                                  hH + hubrec::tangent, hA + hubrec::q, hA + hubrec::tangent, nullptr);
+            __syncwarp();
+            // With a hub, its correction comes first (its BC rows), then each rigid
+            // joint gives the root correction: B_t x_root = -Phi - B_base x_hub.
+            if (hub) {
+                if (lane == 0) {
+                    const double* br = hb + hubsm::bc;
+                    double* xh = hb + hubsm::xh;
+                    for (int k = 0; k < 3; ++k) xh[k] = -br[conrec::Phi + k];
+                    const double rhs[3] = {-br[conrec::Phi + 3], -br[conrec::Phi + 4], -br[conrec::Phi + 5]};
+                    double y[3] = {0., 0., 0.};
+                    if (!solve3(br + conrec::Brot, rhs, y)) atomicOr(&s_flag, 2);
+                    for (int k = 0; k < 3; ++k) xh[3 + k] = y[k];
+                    if (drive) {
+                        // Drive train: the revolute rows fix record 1's translation and
+                        // two of its rotation components; the third, the shaft rotation
+                        // theta, stays free.  x_1 = cA + theta nA, nA spanning the null
+                        // space of B_t; the chain's later corrections are affine in
+                        // theta as well (cH + theta dH).  Test vectors w (G w = 0 with
+                        // the gradients G, not G T) project the equilibrium rows onto
+                        // the free rotation: w_1 = [0, joint axis].
+                        const double* rv = hb + hubsm::rev;
+                        double* cA = hb + hubsm::cA;
+                        double* nA = hb + hubsm::nA;
+                        double* wA = hb + hubsm::wA;
+                        for (int k = 0; k < 3; ++k) {
+                            cA[k] = -rv[revrec::Phi + k] + xh[k];
+                            nA[k] = 0.;
+                            wA[k] = 0.;
+                            wA[3 + k] = rv[revrec::x + k];
+                        }
+                        const double* b0 = rv + revrec::Bt;
+                        const double* b1 = rv + revrec::Bt + 3;
+                        double r2[2];
+                        for (int i = 0; i < 2; ++i) {
+                            r2[i] = -rv[revrec::Phi + 3 + i];
+                            for (int k = 0; k < 3; ++k) r2[i] -= rv[revrec::Bb + i * 3 + k] * xh[3 + k];
+                        }
+                        // minimum-norm particular solution B_t^T (B_t B_t^T)^-1 r2
+                        const double g00 = b0[0] * b0[0] + b0[1] * b0[1] + b0[2] * b0[2];
+                        const double g01 = b0[0] * b1[0] + b0[1] * b1[1] + b0[2] * b1[2];
+                        const double g11 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
+                        const double det = g00 * g11 - g01 * g01;
+                        if (!(fabs(det) > 0.)) atomicOr(&s_flag, 2);
+                        const double l0 = (g11 * r2[0] - g01 * r2[1]) / det;
+                        const double l1 = (g00 * r2[1] - g01 * r2[0]) / det;
+                        for (int k = 0; k < 3; ++k) cA[3 + k] = b0[k] * l0 + b1[k] * l1;
+                        nA[3] = b0[1] * b1[2] - b0[2] * b1[1];
+                        nA[4] = b0[2] * b1[0] - b0[0] * b1[2];
+                        nA[5] = b0[0] * b1[1] - b0[1] * b1[0];
+                        if (hH) {
+                            const double* ah = hb + hubsm::ah;
+                            bool ok = joint_target_correction(ah, cA, 1., hb + hubsm::cH);
+                            ok &= joint_target_correction(ah, nA, 0., hb + hubsm::dH);
+                            ok &= joint_target_test(ah, wA, hb + hubsm::wH);
+                            if (!ok) atomicOr(&s_flag, 2);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            if (drive && lane < nc) {
+                // roots: x_root = c_r + theta d_r from the corrections of the record
+                // they join; d_r waits in droot for the second right-hand side
+                double* cr = con + lane * kConStride;
+                const int pr = 6 * pos[KB.con_node[lane]];
+                double c6[6], d6[6];
+                if (is_hub_joint(KB.con_type[lane])) {
+                    const double* cb = hb + (hH ? hubsm::cH : hubsm::cA);
+                    const double* db = hb + (hH ? hubsm::dH : hubsm::nA);
+                    bool ok = joint_target_correction(cr, cb, 1., c6);
+                    ok &= joint_target_correction(cr, db, 0., d6);
+                    ok &= joint_target_test(cr, hb + (hH ? hubsm::wH : hubsm::wA), cr + conrec::wr);
+                    if (!ok) atomicOr(&s_flag, 2);
+                } else {
+                    for (int k = 0; k < 3; ++k) {
+                        c6[k] = -cr[conrec::Phi + k];
+                        d6[k] = d6[3 + k] = 0.;
+                    }
+                    const double rr[3] = {-cr[conrec::Phi + 3], -cr[conrec::Phi + 4], -cr[conrec::Phi + 5]};
+                    if (!solve3(cr + conrec::Brot, rr, c6 + 3)) atomicOr(&s_flag, 2);
+                    for (int k = 0; k < 6; ++k) cr[conrec::wr + k] = 0.;
+                }
+                for (int k = 0; k < 6; ++k) {
+                    xs[pr + k] = c6[k];
+                    droot[pr + k] = d6[k];
+                    cr[conrec::dr + k] = d6[k];
+                }
+            } else if (lane < nc) {
+                const double* cr = con + lane * kConStride;
+                const int pr = 6 * pos[KB.con_node[lane]];
+                double rt[3], rr[3];
+                for (int k = 0; k < 3; ++k) {
+                    rt[k] = -cr[conrec::Phi + k];
+                    rr[k] = -cr[conrec::Phi + 3 + k];
+                }
+                if (is_hub_joint(KB.con_type[lane])) {
+                    const double* xh = hb + hubsm::xh;
+                    for (int i = 0; i < 3; ++i) {
+                        rt[i] += xh[i];
+                        for (int k = 0; k < 3; ++k) {
+                            rt[i] -= cr[conrec::Btr + i * 3 + k] * xh[3 + k];
+                            rr[i] -= cr[conrec::Brr + i * 3 + k] * xh[3 + k];
+                        }
+                    }
+                }
+                for (int k = 0; k < 3; ++k) xs[pr + k] = rt[k];
+                double y[3] = {0., 0., 0.};
+                if (!solve3(cr + conrec::Brot, rr, y)) atomicOr(&s_flag, 2);
+                for (int k = 0; k < 3; ++k) xs[pr + 3 + k] = y[k];
+            }
+            sec_wait();
+        } else {
+            // ---- quadrature-point values (calculate_quadrature_point_values.hpp) ---
+            sec_wait();
+            qp_phase<TG, NW - 1, false>(N, Q, phi, dphiJ, qpw, sq, sv, svd, slab, L, KB.gravity, P.beta_prime,
+                                        P.gamma_prime, itp, G, Fc, Fdig, bulk ? sec : nullptr);
+        }
         __syncthreads();
         mark(kPhaseQuadrature);
 
@@ -3022,32 +3160,6 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         }
         mark(kPhaseIntegrate);
 
-        // ---- constraints (calculate_constraint_residual_gradient.hpp:60-320) -------
-        if (warp == NW - 1 && lane < nc) {
-            const int tn = KB.con_node[lane];
-            constraint_record(con + lane * kConStride, KB.con_type[lane], sq + tn * 7, KB.con_X0[lane],
-                              sT + tn * 9, hub ? hj + hubrec::q : nullptr,
-                              hub ? hj + hubrec::tangent : nullptr, KB.con_axis[lane]);
-        }
-        if (hub && warp == NW - 1 && lane == nc)  // the hub's own boundary condition
-            constraint_record(hb + hubsm::bc, KB.hub_con_type, hb + hubrec::q, hb + hubrec::X0,
-                              hb + hubrec::tangent, nullptr, nullptr, nullptr);
-        if (drive && warp == NW - 1 && lane == nc + 1)  // revolute joint record 0 -> 1
-            revolute_record(hb + hubsm::rev, hb, hA);
-        if (drive && hH && warp == NW - 1 && lane == nc + 2)  // rigid joint record 1 -> 2
-            constraint_record(hb + hubsm::ah, KYN_CONSTRAINT_RIGID_JOINT, hH + hubrec::q, hH + hubrec::X0,
-                              hH + hubrec::tangent, hA + hubrec::q, hA + hubrec::tangent, nullptr);
-        __syncthreads();
-
-        // ---- right-hand side: b = -cond (-f + R + G^T lambda) (assemble_system_residual.hpp,
-        //      solve_system.hpp:20-24) in permuted order --------------------------------
-        for (int t = tid; t < n6; t += NT) {
-            const int n = t / 6, c = t % 6;
-            double val = -slab[L.f + t] + resid[t];
-            for (int k = 0; k < nc; ++k)
-                if (KB.con_node[k] == n) val += con[k * kConStride + conrec::Gl + c];
-            bp[6 * pos[n] + c] = -(val * P.conditioner);
-        }
         if (record && KB.dump) {
             // Dump of the assembled local system (natural node order, then constraints):
             // matrix [nl][nl], then rhs [nl], then solution [nl]; nl = n6 + 6 nc.
@@ -3055,7 +3167,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             double* D = KB.dump;
             for (int t = tid; t < nl * nl; t += NT) D[t] = 0.;
         }
-        __syncthreads();
+        if (record) __syncthreads();
         if (record && KB.dump) {
             const int nl = n6 + 6 * nc;
             double* D = KB.dump;
@@ -3064,7 +3176,6 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 D[r * nl + c] = static_cast<double>(
                     A[sys_at(ldA, 6 * pos[r / 6] + r % 6, 6 * pos[c / 6] + c % 6)]);
             }
-            for (int t = tid; t < n6; t += NT) D[nl * nl + t] = bp[6 * pos[t / 6] + t % 6];
             if (tid < nc) {
                 const double* cr = con + tid * kConStride;
                 const int tn = KB.con_node[tid];
@@ -3082,151 +3193,50 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
         }
 
-        __syncthreads();
         mark(kPhaseConstraints);
 
         // ---- solve -----------------------------------------------------------------
-        // (S1) constrained node corrections: B x_r = -Phi.  With a hub, its
-        //      correction comes first (its BC rows), then each rigid joint gives
-        //      the root correction: B_t x_root = -Phi - B_base x_hub.
-        if (hub) {
-            if (tid == 0) {
-                const double* br = hb + hubsm::bc;
-                double* xh = hb + hubsm::xh;
-                for (int k = 0; k < 3; ++k) xh[k] = -br[conrec::Phi + k];
-                const double rhs[3] = {-br[conrec::Phi + 3], -br[conrec::Phi + 4], -br[conrec::Phi + 5]};
-                double y[3] = {0., 0., 0.};
-                if (!solve3(br + conrec::Brot, rhs, y)) atomicOr(&s_flag, 2);
-                for (int k = 0; k < 3; ++k) xh[3 + k] = y[k];
-                if (drive) {
-                    // Drive train: the revolute rows fix record 1's translation and
-                    // two of its rotation components; the third, the shaft rotation
-                    // theta, stays free.  x_1 = cA + theta nA, nA spanning the null
-                    // space of B_t; the chain's later corrections are affine in
-                    // theta as well (cH + theta dH).  Test vectors w (G w = 0 with
-                    // the gradients G, not G T) project the equilibrium rows onto
-                    // the free rotation: w_1 = [0, joint axis].
-                    const double* rv = hb + hubsm::rev;
-                    double* cA = hb + hubsm::cA;
-                    double* nA = hb + hubsm::nA;
-                    double* wA = hb + hubsm::wA;
-                    for (int k = 0; k < 3; ++k) {
-                        cA[k] = -rv[revrec::Phi + k] + xh[k];
-                        nA[k] = 0.;
-                        wA[k] = 0.;
-                        wA[3 + k] = rv[revrec::x + k];
-                    }
-                    const double* b0 = rv + revrec::Bt;
-                    const double* b1 = rv + revrec::Bt + 3;
-                    double r2[2];
-                    for (int i = 0; i < 2; ++i) {
-                        r2[i] = -rv[revrec::Phi + 3 + i];
-                        for (int k = 0; k < 3; ++k) r2[i] -= rv[revrec::Bb + i * 3 + k] * xh[3 + k];
-                    }
-                    // minimum-norm particular solution B_t^T (B_t B_t^T)^-1 r2
-                    const double g00 = b0[0] * b0[0] + b0[1] * b0[1] + b0[2] * b0[2];
-                    const double g01 = b0[0] * b1[0] + b0[1] * b1[1] + b0[2] * b1[2];
-                    const double g11 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
-                    const double det = g00 * g11 - g01 * g01;
-                    if (!(fabs(det) > 0.)) atomicOr(&s_flag, 2);
-                    const double l0 = (g11 * r2[0] - g01 * r2[1]) / det;
-                    const double l1 = (g00 * r2[1] - g01 * r2[0]) / det;
-                    for (int k = 0; k < 3; ++k) cA[3 + k] = b0[k] * l0 + b1[k] * l1;
-                    nA[3] = b0[1] * b1[2] - b0[2] * b1[1];
-                    nA[4] = b0[2] * b1[0] - b0[0] * b1[2];
-                    nA[5] = b0[0] * b1[1] - b0[1] * b1[0];
-                    if (hH) {
-                        const double* ah = hb + hubsm::ah;
-                        bool ok = joint_target_correction(ah, cA, 1., hb + hubsm::cH);
-                        ok &= joint_target_correction(ah, nA, 0., hb + hubsm::dH);
-                        ok &= joint_target_test(ah, wA, hb + hubsm::wH);
-                        if (!ok) atomicOr(&s_flag, 2);
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        if (drive && tid < nc) {
-            // roots: x_root = c_r + theta d_r from the corrections of the record
-            // they join; d_r waits in droot for the second right-hand side
-            double* cr = con + tid * kConStride;
-            const int pr = 6 * pos[KB.con_node[tid]];
-            double c6[6], d6[6];
-            if (is_hub_joint(KB.con_type[tid])) {
-                const double* cb = hb + (hH ? hubsm::cH : hubsm::cA);
-                const double* db = hb + (hH ? hubsm::dH : hubsm::nA);
-                bool ok = joint_target_correction(cr, cb, 1., c6);
-                ok &= joint_target_correction(cr, db, 0., d6);
-                ok &= joint_target_test(cr, hb + (hH ? hubsm::wH : hubsm::wA), cr + conrec::wr);
-                if (!ok) atomicOr(&s_flag, 2);
-            } else {
-                for (int k = 0; k < 3; ++k) {
-                    c6[k] = -cr[conrec::Phi + k];
-                    d6[k] = d6[3 + k] = 0.;
-                }
-                const double rr[3] = {-cr[conrec::Phi + 3], -cr[conrec::Phi + 4], -cr[conrec::Phi + 5]};
-                if (!solve3(cr + conrec::Brot, rr, c6 + 3)) atomicOr(&s_flag, 2);
-                for (int k = 0; k < 6; ++k) cr[conrec::wr + k] = 0.;
-            }
-            for (int k = 0; k < 6; ++k) {
-                xs[pr + k] = c6[k];
-                droot[pr + k] = d6[k];
-                cr[conrec::dr + k] = d6[k];
-            }
-        } else if (tid < nc) {
-            const double* cr = con + tid * kConStride;
-            const int pr = 6 * pos[KB.con_node[tid]];
-            double rt[3], rr[3];
-            for (int k = 0; k < 3; ++k) {
-                rt[k] = -cr[conrec::Phi + k];
-                rr[k] = -cr[conrec::Phi + 3 + k];
-            }
-            if (is_hub_joint(KB.con_type[tid])) {
-                const double* xh = hb + hubsm::xh;
-                for (int i = 0; i < 3; ++i) {
-                    rt[i] += xh[i];
-                    for (int k = 0; k < 3; ++k) {
-                        rt[i] -= cr[conrec::Btr + i * 3 + k] * xh[3 + k];
-                        rr[i] -= cr[conrec::Brr + i * 3 + k] * xh[3 + k];
-                    }
-                }
-            }
-            for (int k = 0; k < 3; ++k) xs[pr + k] = rt[k];
-            double y[3] = {0., 0., 0.};
-            if (!solve3(cr + conrec::Brot, rr, y)) atomicOr(&s_flag, 2);
-            for (int k = 0; k < 3; ++k) xs[pr + 3 + k] = y[k];
-        }
-        __syncthreads();
-        // (S2) free-row right-hand side, folded into column m of A (and kept in
-        //      FP64 in bp[0:m]); a drive train adds the second right-hand side
-        //      -A_fr d_r in column m + 1 (FP64 copy in rhs2)
+        // ---- right-hand side b = -cond (-f + R + G^T lambda) (assemble_system_residual.hpp,
+        //      solve_system.hpp:20-24) in permuted order; the free rows' part
+        //      -A_fr x_r of the constrained corrections folded in, in column m of A
+        //      (and in FP64 in bp[0:m]); a drive train adds the second right-hand
+        //      side -A_fr d_r in column m + 1 (FP64 copy in rhs2)
         double* gjv = reinterpret_cast<double*>(smem_raw + S.G + solve_vec_offset(N, nc, sizeof(TR), NT, drive ? 2 : 0));
         double* r64 = gjv;                 // [n6] residual of the linear solve
         double* rhs2 = gjv + n6;           // [n6] second right-hand side (drive train)
         double* x2 = gjv + 2 * n6;         // [n6] its solution
         double* red4 = gjv + 4 * n6;       // [64] reductions of the refinement
         // (eight lanes per row: the rows start in only two different banks)
-        for (int i0 = 4 * warp; i0 < m; i0 += 4 * NW) {
-            const int i = i0 + (lane >> 3), ic = min(i, m - 1);
+        for (int i0 = 4 * warp; i0 < n6; i0 += 4 * NW) {
+            const int i = i0 + (lane >> 3), ic = min(i, n6 - 1);
             double r = 0., r2 = 0.;
-            for (int j = m + (lane & 7); j < n6; j += 8) {
-                const double aij = static_cast<double>(A[sys_at(ldA, ic, j)]);
-                r -= aij * xs[j];
-                if (drive) r2 -= aij * droot[j];
-            }
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {
-                r += __shfl_xor_sync(0xffffffffu, r, o);
-                if (drive) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-            }
-            if ((lane & 7) == 0 && i < m) {
-                r += bp[i];
-                A[sys_at(ldA, i, m)] = static_cast<TR>(r);
-                bp[i] = r;
-                if (drive) {
-                    A[sys_at(ldA, i, m + 1)] = static_cast<TR>(r2);
-                    rhs2[i] = r2;
+            if (i0 < m) {
+                for (int j = m + (lane & 7); j < n6; j += 8) {
+                    const double aij = static_cast<double>(A[sys_at(ldA, ic, j)]);
+                    r -= aij * xs[j];
+                    if (drive) r2 -= aij * droot[j];
                 }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) {
+                    r += __shfl_xor_sync(0xffffffffu, r, o);
+                    if (drive) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+                }
+            }
+            if ((lane & 7) == 0 && i < n6) {
+                const int t = 6 * node_at[i / 6] + i % 6;
+                double val = -slab[L.f + t] + resid[t];
+                if (i >= m) val += con[((i - m) / 6) * kConStride + conrec::Gl + i % 6];
+                double b = -(val * P.conditioner);
+                if (record && KB.dump) KB.dump[(n6 + 6 * nc) * (n6 + 6 * nc) + t] = b;
+                if (i < m) {
+                    b += r;
+                    A[sys_at(ldA, i, m)] = static_cast<TR>(b);
+                    if (drive) {
+                        A[sys_at(ldA, i, m + 1)] = static_cast<TR>(r2);
+                        rhs2[i] = r2;
+                    }
+                }
+                bp[i] = b;
             }
         }
         __syncthreads();
@@ -3465,90 +3475,108 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
             __syncthreads();
         }
-        // (S5) multipliers from the constrained rows: grad^T x_l = b_r - A_r x
-        for (int rowi = warp; rowi < 6 * nc; rowi += NW) {
-            const int c = rowi / 6, k = rowi % 6;
-            const int pr = 6 * pos[KB.con_node[c]];
-            double sacc = 0.;
-            for (int j = lane; j < n6; j += 32) sacc += static_cast<double>(A[sys_at(ldA, pr + k, j)]) * xs[j];
-            for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-            if (lane == 0) con[c * kConStride + conrec::yr + k] = bp[pr + k] - sacc;
-        }
-        __syncthreads();
-        if (tid < nc) {
-            double* cr = con + tid * kConStride;
-            const double* y = cr + conrec::yr;
-            double yr[3] = {0., 0., 0.};
-            if (!solve3(cr + conrec::AX, y + 3, yr)) atomicOr(&s_flag, 2);
-            // UnconditionSolution (condition_system.hpp): x_lambda /= conditioner
-            for (int k = 0; k < 3; ++k) cr[conrec::xl + k] = y[k] / P.conditioner;
-            for (int k = 0; k < 3; ++k) cr[conrec::xl + 3 + k] = yr[k] / P.conditioner;
-        }
-        __syncthreads();
-        if (hub && tid == 0) {
-            // this beam's part of the hub rows: sum over its joints of
-            // G_base^T (lambda + x_lambda), exchanged over the cluster below
-            double* pub = hb + hubsm::pub + 6 * (iter & 1);
-            for (int k = 0; k < 6; ++k) pub[k] = 0.;
-            for (int c = 0; c < nc; ++c) {
-                if (!is_hub_joint(KB.con_type[c])) continue;
-                const double* cr = con + c * kConStride;
-                double w[6];
-                for (int k = 0; k < 6; ++k) w[k] = cr[conrec::lam + k] + cr[conrec::xl + k];
-                joint_base_transpose_add(cr, w, pub);
-            }
-        }
-        if (record && KB.dump) {
-            const int nl = n6 + 6 * nc;
-            double* D = KB.dump + nl * nl + nl;
-            for (int t = tid; t < n6; t += NT) D[t] = xs[6 * pos[t / 6] + t % 6];
-            if (tid < nc)
-                for (int k = 0; k < 6; ++k) D[n6 + 6 * tid + k] = con[tid * kConStride + conrec::xl + k];
-        }
-
-        __syncthreads();
-        sec_prefetch();  // A is not read again in this iteration
-        mark(kPhaseSubstitute);
-
-        // ---- convergence error (calculate_error_sum_squares.hpp:33-79) --------------
+        // (S5) The last warp: multipliers from the constrained rows, grad^T x_l =
+        //      b_r - A_r x, and their part of the error.  The others: error and
+        //      update of the nodes (calculate_error_sum_squares.hpp:33-79,
+        //      update_dynamic_prediction.hpp, calculate_displacement.hpp), eight
+        //      lanes to a node.
         double part = 0.;
-        for (int t = tid; t < n6; t += NT) {
-            const double pi = xs[6 * pos[t / 6] + t % 6];
-            const double xi = sqd[t] * h;
-            const double e = pi / (P.atol + P.rtol * fabs(xi));
-            part += e * e;
-        }
-        if (tid < 6 * nc) {
-            const double* cr = con + (tid / 6) * kConStride;
-            const double pi = cr[conrec::xl + tid % 6];
-            const double xi = cr[conrec::lam + tid % 6];
-            const double e = pi / (P.atol + P.rtol * fabs(xi));
-            part += e * e;
-        }
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        double* slot = red + (iter & 1) * (NW + 8);
-        if (lane == 0) slot[warp] = part;
-        __syncthreads();
-        if (tid == 0) {
-            double s = 0.;
-            for (int w2 = 0; w2 < NW; ++w2) s += slot[w2];
-            slot[NW] = s;
-            slot[NW + 1] = static_cast<double>(s_flag);
-        }
-        double total, flags;
-        if (clustered) {
-            cluster.sync();
-            total = 0.;
-            flags = 0.;
-            for (int r = 0; r < KB.model_beams; ++r) {
-                const double* peer = cluster.map_shared_rank(slot, r);
-                total += peer[NW];
-                flags = fmax(flags, peer[NW + 1]);
+        if (warp == NW - 1) {
+            for (int c = 0; c < nc; ++c) {
+                const int pr = m + 6 * c;
+                double y[6] = {0., 0., 0., 0., 0., 0.};
+                for (int j = lane; j < n6; j += 32) {
+                    const double xj = xs[j];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) y[k] += static_cast<double>(A[sys_at(ldA, pr + k, j)]) * xj;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) y[k] += __shfl_xor_sync(0xffffffffu, y[k], o);
+                double* cr = con + c * kConStride;
+#pragma unroll
+                for (int k = 0; k < 6; ++k)
+                    if (lane == k) cr[conrec::yr + k] = bp[pr + k] - y[k];
+            }
+            __syncwarp();
+            if (lane < nc) {
+                double* cr = con + lane * kConStride;
+                const double* y = cr + conrec::yr;
+                double yr[3] = {0., 0., 0.};
+                if (!solve3(cr + conrec::AX, y + 3, yr)) atomicOr(&s_flag, 2);
+                // UnconditionSolution (condition_system.hpp): x_lambda /= conditioner
+                const double ic = 1. / P.conditioner;
+                for (int k = 0; k < 3; ++k) {
+                    cr[conrec::xl + k] = y[k] * ic;
+                    cr[conrec::xl + 3 + k] = yr[k] * ic;
+                }
+            }
+            __syncwarp();
+            if (hub && lane == 0) {
+                // this beam's part of the hub rows: sum over its joints of
+                // G_base^T (lambda + x_lambda), exchanged over the cluster below
+                double* pub = hb + hubsm::pub + 6 * (iter & 1);
+                for (int k = 0; k < 6; ++k) pub[k] = 0.;
+                for (int c = 0; c < nc; ++c) {
+                    if (!is_hub_joint(KB.con_type[c])) continue;
+                    const double* cr = con + c * kConStride;
+                    double w[6];
+                    for (int k = 0; k < 6; ++k) w[k] = cr[conrec::lam + k] + cr[conrec::xl + k];
+                    joint_base_transpose_add(cr, w, pub);
+                }
+            }
+            if (record && KB.dump) {
+                const int nl = n6 + 6 * nc;
+                double* D = KB.dump + nl * nl + nl;
+                for (int t = lane; t < n6; t += 32) D[t] = xs[6 * pos[t / 6] + t % 6];
+                if (lane < nc)
+                    for (int k = 0; k < 6; ++k) D[n6 + 6 * lane + k] = con[lane * kConStride + conrec::xl + k];
+            }
+            for (int t = lane; t < 6 * nc; t += 32) {
+                double* cr = con + (t / 6) * kConStride;
+                const double lam = cr[conrec::lam + t % 6], xl = cr[conrec::xl + t % 6];
+                const double e = xl / (P.atol + P.rtol * fabs(lam));
+                part += e * e;
+                if (!hub) cr[conrec::lam + t % 6] = lam + xl;  // update_lambda_prediction.hpp
             }
         } else {
-            __syncthreads();
-            total = slot[NW];
-            flags = slot[NW + 1];
+            for (int n0 = 4 * warp; n0 < N; n0 += 4 * (NW - 1)) {
+                const int n = n0 + (lane >> 3), c = lane & 7, t = 6 * n + c;
+                if (n < N && c < 6) {
+                    const double delta = xs[6 * pos[n] + c], qd = sqd[t];
+                    const double e = delta / (P.atol + P.rtol * fabs(qd * h));
+                    part += e * e;
+                    sqd[t] = qd + delta / h;
+                    if (P.dynamic) {
+                        sv[t] += P.gamma_prime * delta;
+                        svd[t] += P.beta_prime * delta;
+                    }
+                }
+                __syncwarp();
+                if (n < N && c < 7) displace(n, c);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        // per warp its part, then the flags; each CTA of the model sums all of
+        // them in the same order
+        double* slot = red + (iter & 1) * (NW + 8);
+        if (lane == 0) slot[warp] = part;
+        if (tid == NT - 1) slot[NW] = static_cast<double>(*static_cast<volatile int*>(&s_flag));
+        proxy_fence_async_smem();
+        if (clustered) cluster.sync(); else __syncthreads();
+        sec_issue();  // A is not read again in this iteration
+        mark(kPhaseSubstitute);
+        double total = 0., flags = 0.;
+        for (int k = lane; k < KB.model_beams * (NW + 1); k += 32) {
+            const int r = k / (NW + 1), w2 = k - r * (NW + 1);
+            const double v = clustered ? *cluster.map_shared_rank(slot + w2, r) : slot[w2];
+            if (w2 < NW) total += v;
+            else flags = fmax(flags, v);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            total += __shfl_xor_sync(0xffffffffu, total, o);
+            flags = fmax(flags, __shfl_xor_sync(0xffffffffu, flags, o));
         }
         double xlh[6] = {0., 0., 0., 0., 0., 0.};
         if (hub) {
@@ -3637,20 +3665,13 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         if (KB.rank == 0 && tid == 0 && iter < kMaxNewtonIters) KB.conv[iter] = err;
         iters = iter + 1;
 
-        // ---- update (update_dynamic_prediction.hpp, calculate_displacement.hpp,
-        //      update_lambda_prediction.hpp) ----------------------------------------------
-        for (int t = tid; t < n6; t += NT) {
-            const double delta = xs[6 * pos[t / 6] + t % 6];
-            sqd[t] += delta / h;
-            if (P.dynamic) {
-                sv[t] += P.gamma_prime * delta;
-                svd[t] += P.beta_prime * delta;
+        // ---- update of the hub chain and, with a hub, of the multipliers (read by
+        //      the peers' sums above only through pub)
+        if (hub && warp == NW - 1)
+            for (int t = lane; t < 6 * nc; t += 32) {
+                double* cr = con + (t / 6) * kConStride;
+                cr[conrec::lam + t % 6] += cr[conrec::xl + t % 6];
             }
-        }
-        if (tid < 6 * nc) {
-            double* cr = con + (tid / 6) * kConStride;
-            cr[conrec::lam + tid % 6] += cr[conrec::xl + tid % 6];
-        }
         if (hub && tid == NT - 1) {
             const double* xh = hb + hubsm::xh;
             for (int k = 0; k < 6; ++k) {
@@ -3680,9 +3701,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             else
                 for (int k = 0; k < 6; ++k) hb[hubsm::ah + conrec::lam + k] += hb[hubsm::ah + conrec::xl + k];
         }
-        __syncthreads();
-        displacement();
-        __syncthreads();
+        if (hub && chain_rec()) displace_chain(chain_rec());
         mark(kPhaseUpdate);
 
         if (flags != 0.) {
