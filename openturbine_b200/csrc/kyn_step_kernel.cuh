@@ -74,7 +74,7 @@ __device__ __forceinline__ void cross3(const double* a, const double* b, double*
 
 // Exponential map: rotation vector -> quaternion (RotationVectorToQuaternion,
 // device form with factor 0 below 1e-12).
-__device__ __forceinline__ void rotvec_to_quat(const double* phi, double* q) {
+static __device__ __noinline__ void rotvec_to_quat(const double* phi, double* q) {
     const double angle = sqrt(phi[0] * phi[0] + phi[1] * phi[1] + phi[2] * phi[2]);
     double s, c;
     sincos(angle / 2., &s, &c);
@@ -414,6 +414,7 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g8 = lane >> 2, t = lane & 3;
     const int lines = 6 * N, blocks = (lines + 7) >> 3;
+#pragma unroll 1
     for (int u = warp; u < 2 * blocks; u += NW) {
         const bool right = u < blocks;  // the longer halves first
         const int l0 = 8 * (right ? u : u - blocks);
@@ -426,17 +427,19 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
 #pragma unroll
             for (int k = 0; k < 9; ++k) T[k] = Tj[k];
         }
+#pragma unroll 1
         for (int i0 = 0; i0 < N; i0 += 8 * MT) {
             double acc[MT][3][2];
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) acc[mt][c][0] = acc[mt][c][1] = 0.;
-            for (int q0 = 0; q0 < Q; q0 += 4) {
-                const int q = min(q0 + t, Q - 1);
-                const bool in = q0 + t < Q;
-                const double pj = phi[q * N + j], dj = dphi[q * N + j];
-                const TG* g = gr + q * kGPoint;
+            const TG* g = gr + min(t, Q - 1) * kGPoint;
+            const double *pq = phi + min(t, Q - 1) * N, *dq = dphi + min(t, Q - 1) * N;
+#pragma unroll 1
+            for (int q = t; q - t < Q; q += 4) {
+                const bool in = q < Q;
+                const double pj = pq[j], dj = dq[j];
                 double h[3], hp[3];
                 if (right) {
                     const double2 g8v = load_pair(g + 8), ga = load_pair(g + 10), gb = load_pair(g + 12),
@@ -467,13 +470,17 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
                     if (i0 + 8 * mt < N) {  // uniform
                         const int i = i0 + 8 * mt + g8;
                         const bool on = in && i < N;
-                        const double f = on ? phi[q * N + i] : 0., fp = on ? dphi[q * N + i] : 0.;
+                        const double f = on ? pq[i] : 0., fp = on ? dq[i] : 0.;
 #pragma unroll
                         for (int c = 0; c < 3; ++c) dmma884(acc[mt][c][0], acc[mt][c][1], f, h[c]);
 #pragma unroll
                         for (int c = 0; c < 3; ++c) dmma884(acc[mt][c][0], acc[mt][c][1], fp, hp[c]);
                     }
                 }
+                const int step = q + 4 < Q ? 4 : 0;  // past the last point: any, with a zero factor
+                g += step * kGPoint;
+                pq += step * N;
+                dq += step * N;
             }
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
@@ -519,38 +526,52 @@ __device__ __forceinline__ float pivot_rcp(float d) {
     return fmaf(r, fmaf(-d, r, 1.f), r);
 }
 
-// In-place inverse of an 8x8 block held by one warp in accumulator layout
-// (lane l: row l/4, columns 2(l%4) and +1), Gauss-Jordan over four 2x2 pivot
-// blocks D, each inverted through its determinant.  With s the row's pivot
-// entries times adj(D) and u the pivot rows' entries of the lane's columns,
-// every entry becomes base - (s u) / det; pivot rows and columns differ only
-// in s, u and a zero base, so the four steps are free of branches and hold one
-// reciprocal each.  Bound by the latency of that chain (shuffles, two products,
-// the reciprocal, one product per step).  A zero or non-finite determinant
-// sets bit 2 of *flag.
-__device__ __forceinline__ void invert_block8(double& v0, double& v1, int lane, int* flag) {
-    constexpr unsigned kAll = 0xffffffffu;
+// Reciprocal by one third-order step from the hardware's approximation (relative
+// error 2^-23 at most, cubed: below the rounding), a product shorter than two
+// Newton steps.
+__device__ __forceinline__ double block_rcp(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.);
+    return fma(r, fma(e, e, e), r);
+}
+
+// Inverse of an 8x8 block held by one warp in accumulator layout (lane l: row
+// l/4, columns 2(l%4) and +1), into buf (row-major, 64 doubles of shared
+// memory, also the exchange between the steps: a store and five pair loads
+// take half the time of the twenty shuffles they stand for).  Gauss-Jordan over
+// four 2x2 pivot blocks D, each inverted through its determinant.  With s the
+// row's pivot entries times adj(D) and u the pivot rows' entries of the lane's
+// columns, every entry becomes base - (s u) / det; pivot rows (whose pivot
+// entries count as -1 in their own place) and columns (u the identity) differ
+// only in the operands and a zero base, so the four steps are free of branches
+// and hold one reciprocal each.  Bound by the latency of that chain: 966 cycles
+// with shuffles, two Newton steps and a test per step, alone on an SM.  A zero
+// or non-finite determinant sets bit 2 of *flag.
+__device__ __forceinline__ void invert_block8(double v0, double v1, double* buf, int lane, int* flag) {
     const int r = lane >> 2, t = lane & 3;
+    bool bad = false;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        const double a = __shfl_sync(kAll, v0, 9 * p), b = __shfl_sync(kAll, v1, 9 * p);
-        const double c = __shfl_sync(kAll, v0, 9 * p + 4), d = __shfl_sync(kAll, v1, 9 * p + 4);
-        const double x0 = __shfl_sync(kAll, v0, (lane & 28) + p), x1 = __shfl_sync(kAll, v1, (lane & 28) + p);
-        const double w00 = __shfl_sync(kAll, v0, 8 * p + t), w01 = __shfl_sync(kAll, v1, 8 * p + t);
-        const double w10 = __shfl_sync(kAll, v0, 8 * p + 4 + t), w11 = __shfl_sync(kAll, v1, 8 * p + 4 + t);
-        const double det = fma(a, d, -(b * c));
-        const double rd = pivot_rcp(det);
-        if (lane == 0 && (!(fabs(det) > 0.) || !isfinite(rd))) atomicOr(flag, 2);
+        store_pair(buf + 2 * lane, v0, v1);
+        __syncwarp();
+        const double2 ab = load_pair(buf + 18 * p), cd = load_pair(buf + 18 * p + 8);
+        const double2 x = load_pair(buf + 8 * r + 2 * p);
+        const double2 w0 = load_pair(buf + 16 * p + 2 * t), w1 = load_pair(buf + 16 * p + 8 + 2 * t);
+        const double det = fma(ab.x, cd.y, -(ab.y * cd.x));
+        const double rd = block_rcp(det);
+        bad |= !(fabs(det) > 0.) || !isfinite(rd);
         const bool row0 = r == 2 * p, row1 = r == 2 * p + 1, col = t == p;
-        double s0 = fma(x0, d, -(x1 * c)), s1 = fma(x1, a, -(x0 * b));
-        s0 = row0 ? -d : row1 ? c : s0;
-        s1 = row0 ? b : row1 ? -a : s1;
-        const double u00 = col ? 1. : w00, u01 = col ? 0. : w01;
-        const double u10 = col ? 0. : w10, u11 = col ? 1. : w11;
+        const double x0 = row0 ? -1. : row1 ? 0. : x.x, x1 = row1 ? -1. : row0 ? 0. : x.y;
+        const double s0 = fma(x0, cd.y, -(x1 * cd.x)), s1 = fma(x1, ab.x, -(x0 * ab.y));
+        const double e0 = fma(s0, w0.x, s1 * w1.x), e1 = fma(s0, w0.y, s1 * w1.y);
         const bool clear = row0 || row1 || col;
-        v0 = fma(-rd, fma(s0, u00, s1 * u10), clear ? 0. : v0);
-        v1 = fma(-rd, fma(s0, u01, s1 * u11), clear ? 0. : v1);
+        v0 = fma(-rd, col ? s0 : e0, clear ? 0. : v0);
+        v1 = fma(-rd, col ? s1 : e1, clear ? 0. : v1);
+        __syncwarp();
     }
+    store_pair(buf + 2 * lane, v0, v1);
+    if (bad && lane == 0) atomicOr(flag, 2);
 }
 
 // B operands of the update by panel k in column tile c0, the lane's pair of
@@ -588,8 +609,24 @@ __device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0,
         if (r >= m || c >= m) d.x = (r == c) ? 1. : 0.;
         if (r >= m || c + 1 >= m) d.y = (r == c + 1) ? 1. : 0.;
     }
-    invert_block8(d.x, d.y, lane, flag);
-    store_pair(dinv_out + 2 * lane, d.x, d.y);
+    invert_block8(d.x, d.y, dinv_out, lane, flag);
+}
+
+// Replaces tile c0 of panel k0's rows (those below m) by U = D^-1 A.  One warp;
+// no other reads those rows any more.
+template <typename TR>
+__device__ __forceinline__ void normalise_tile(TR* A, int ldA, int m, int k0, int c0, const double* dinv, int lane) {
+    const int t2 = 2 * (lane & 3);
+    const bool in = k0 + t2 < m;  // m is even
+    TR* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));
+    const double2 d = load_pair(dinv + 2 * lane);
+    double u0 = 0., u1 = 0.;
+    dmma884(u0, u1, in ? static_cast<double>(a[0]) : 0., d.x);
+    dmma884(u0, u1, in ? static_cast<double>(a[ldA]) : 0., d.y);
+    if (in) {
+        a[0] = static_cast<TR>(u0);
+        a[ldA] = static_cast<TR>(u1);
+    }
 }
 
 // Eliminates the free block A[0:m][0:m] with its right-hand sides in columns
@@ -598,8 +635,9 @@ __device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0,
 // scratch).  dinv: the inverses of the diagonal blocks, 64 doubles each.
 //
 // Warp 0 runs the serial chain (the next panel's diagonal block: update,
-// inversion) while the other warps share the trailing tiles of panel k in
-// equal contiguous runs down the columns; one barrier per panel.  The former
+// inversion) while the other warps share the trailing tiles of panel k and the
+// rows of panel k - 1, which become U = D^-1 A for the back substitution; one
+// barrier per panel.  The former
 // form (two barriers per panel, an unblocked 8x8 factorisation and a panel of
 // L solved by all threads) spent 62k of 126k cycles per Newton iteration on a
 // 13-node beam and 102k of 187k on a 21-node beam, two thirds of them in warp
@@ -610,85 +648,135 @@ __device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (m + 7) >> 3, nct = (m + nrhs + 7) >> 3;
     const int fr = lane >> 2, fc = (2 * (lane & 3)) ^ (fr & 6);
+    const bool past = 8 * (nb - 1) + fr >= m;  // the lane's row of the last row tile
     if (warp == 0) factor_diag_block(A, ldA, m, 0, dinv, dinv, lane, flag);
     __syncthreads();
+#pragma unroll 1
     for (int k = 0; k + 1 < nb; ++k) {
         const int k0 = 8 * k;
         if (warp == 0) {
             factor_diag_block(A, ldA, m, k0 + 8, dinv + 64 * k, dinv + 64 * (k + 1), lane, flag);
         } else {
-            // trailing tiles in column-major order without the first (warp 0's)
-            const int ni = nb - k - 1, total = ni * (nct - k - 1) - 1;
-            const int lo = total * (warp - 1) / NWK + 1, hi = total * warp / NWK + 1;
+            // equal runs down the columns of the trailing tiles without the first
+            // (warp 0's), then of the tiles of the panel before
+            const int ni = nb - k - 1, total = ni * (nct - k - 1) - 1, both = total + (k > 0 ? nct - k : 0);
+            const int lo = both * (warp - 1) / NWK, hi = both * warp / NWK;
             const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
-            int j = lo / ni, i = lo - j * ni;
-            for (int left = hi - lo; left > 0;) {
-                const int c0 = 8 * (k + 1 + j);
+            int j = static_cast<int>(__fdividef(static_cast<float>(lo) + 1.5f, static_cast<float>(ni)));
+            int i = lo + 1 - j * ni;
+#pragma unroll 1
+            for (int left = min(hi, total) - lo; left > 0;) {
+                const int c0 = 8 * (k + 1 + j), cnt = min(ni - i, left);
                 const double2 u = panel_multiplier(A, ldA, k0, c0, dk, lane);
-                const int cnt = min(ni - i, left);
-                TR* row = A + (8 * (k + 1 + i) + fr) * ldA;
-                const TR* ap = row + k0 + fc;
-                TR* cp = row + c0 + fc;
-                int rows_left = m - 8 * (k + 1 + i) - fr;  // rows from m on are not stored
-#pragma unroll 4
-                for (int e = 0; e < cnt; ++e) {
-                    const double2 l = load_pair(ap);
-                    double2 d = load_pair(cp);
-                    dmma884(d.x, d.y, l.x, u.x);
-                    dmma884(d.x, d.y, l.y, u.y);
-                    if (rows_left > 0) store_pair(cp, d.x, d.y);
-                    ap += 8 * ldA;
-                    cp += 8 * ldA;
-                    rows_left -= 8;
+                const TR* lp = A + (8 * (k + 1 + i) + fr) * ldA + k0 + fc;
+                TR* cp = A + (8 * (k + 1 + i) + fr) * ldA + c0 + fc;
+                const bool last = i + cnt == ni;  // rows from m on are not stored
+#pragma unroll 1
+                for (int e = 0; e < cnt; e += 2) {  // two tiles' loads ahead of their stores
+                    const bool two = e + 1 < cnt;
+                    const int o = two ? 8 * ldA : 0;
+                    const double2 l0 = load_pair(lp), l1 = load_pair(lp + o);
+                    double2 d0 = load_pair(cp), d1 = load_pair(cp + o);
+                    dmma884(d0.x, d0.y, l0.x, u.x);
+                    if (two) dmma884(d1.x, d1.y, l1.x, u.x);
+                    dmma884(d0.x, d0.y, l0.y, u.y);
+                    if (two) dmma884(d1.x, d1.y, l1.y, u.y);
+                    if (!(last && past && e + 1 >= cnt)) store_pair(cp, d0.x, d0.y);
+                    if (two && !(last && past && e + 2 >= cnt)) store_pair(cp + o, d1.x, d1.y);
+                    lp += 16 * ldA;
+                    cp += 16 * ldA;
                 }
                 left -= cnt;
                 ++j;
                 i = 0;
             }
+#pragma unroll 1
+            for (int e = max(lo, total); e < hi; ++e)
+                normalise_tile(A, ldA, m, k0 - 8, 8 * (k + e - total), dinv + 64 * (k - 1), lane);
         }
         __syncthreads();
     }
+    // the last two panels' rows (the last one: its right-hand sides only)
+    const int u0 = nb - 1 + warp;
+    if (nb > 1 && u0 < nct) normalise_tile(A, ldA, m, 8 * (nb - 2), 8 * u0, dinv + 64 * (nb - 2), lane);
+    if (warp == NT / 32 - 1)
+        normalise_tile(A, ldA, m, 8 * (nb - 1), 8 * (nct - 1), dinv + 64 * (nb - 1), lane);
+    __syncthreads();
 }
 
-// Back substitution x_k = D_k^-1 (y_k - sum_{j>k} A_kj x_j) by one warp, y in
-// column rhs, x to xs[0:m].  Lanes (row, column pair) of a block row; the four
-// partial sums of a row and the product with the inverse go through shuffles.
-template <typename TR>
-__device__ __forceinline__ void back_substitute_blocks(const TR* A, int ldA, int m, int rhs, const double* dinv,
-                                                       double* xs, int lane) {
+// Back substitution x_k = y_k - sum_{j>k} U_kj x_j by the CTA, y in column rhs
+// of A, x to xs[0:m], two blocks of rows per step and barrier.  Warp 0 finds the
+// two blocks' x (the pair found before still to be subtracted, then the lower
+// block's from the upper rows), while the other warps subtract the pair found
+// before from all rows above.  All products run on the tensor cores with x
+// spread to the lanes by shuffles: a lane's accumulators are its row's value in
+// every column, so sums need no reduction.  One warp alone took 550 to 830
+// cycles a block (9.3k at 13 nodes, 14.4k at 21): the sums over the older blocks
+// were on its path.
+template <typename TR, int NT>
+__device__ __forceinline__ void back_substitute(const TR* A, int ldA, int m, int rhs, double* xs) {
     constexpr unsigned kAll = 0xffffffffu;
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (m + 7) >> 3;
-    const int fr = lane >> 2, t = lane & 3, shift = fr & 6;
-    double xk = 0.;  // x of the block after, row fr
-    for (int k = nb - 1; k >= 0; --k) {
-        const int row = 8 * k + fr;
-        const TR* ar = A + row * ldA;
-        const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
-        double z0 = (t == 0 && row < m) ? static_cast<double>(ar[rhs ^ shift]) : 0., z1 = 0.;
-#pragma unroll 4
-        for (int c = 8 * (k + 2) + 2 * t; c < m; c += 8) {  // m is even: a pair is in or out
-            const double2 a = load_pair(ar + (c ^ shift));
-            const double2 x = load_pair(xs + c);
-            z0 = fma(-a.x, x.x, z0);
-            z1 = fma(-a.y, x.y, z1);
-        }
-        if (k + 1 < nb) {
-            const double x0 = __shfl_sync(kAll, xk, 8 * t), x1 = __shfl_sync(kAll, xk, 8 * t + 4);
-            if (8 * (k + 1) + 2 * t < m) {
-                const double2 a = load_pair(ar + 8 * (k + 1) + ((2 * t) ^ shift));
-                z0 = fma(-a.x, x0, z0);
-                z1 = fma(-a.y, x1, z1);
+    const int fr = lane >> 2, t2 = 2 * (lane & 3), col = t2 ^ (fr & 6);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += NT) xs[i] = static_cast<double>(A[sys_at(ldA, i, rhs)]);
+    __syncthreads();
+    auto tile = [&](int i, int b) {  // the lane's pair of -U_ib; columns past m count as zero
+        const double2 a = load_pair(A + (8 * i + fr) * ldA + 8 * b + col);
+        const bool in = 8 * b + t2 < m;
+        return make_double2(in ? -a.x : 0., in ? -a.y : 0.);
+    };
+    double2 xh = make_double2(0., 0.), xl = xh;  // warp 0: pairs of the blocks found before
+#pragma unroll 1
+    for (int kh = nb - 1; kh >= 0; kh -= 2) {
+        const bool prev = kh + 2 < nb;  // blocks kh + 1, kh + 2
+        const int kl = kh - 1;
+        if (warp == 0) {
+            const int rh = 8 * kh + fr, rl = 8 * kl + fr;
+            double d0 = rh < m ? xs[rh] : 0., d1 = d0;
+            double e0 = kl >= 0 ? xs[rl] : 0., e1 = e0;
+            double2 c = make_double2(0., 0.);
+            if (kl >= 0) c = tile(kl, kh);
+            if (prev) {
+                const double2 a = tile(kh, kh + 1), b = tile(kh, kh + 2);
+                dmma884(d0, d1, a.x, xl.x);
+                dmma884(d0, d1, a.y, xl.y);
+                dmma884(d0, d1, b.x, xh.x);
+                dmma884(d0, d1, b.y, xh.y);
+                if (kl >= 0) {
+                    const double2 g = tile(kl, kh + 1), h = tile(kl, kh + 2);
+                    dmma884(e0, e1, g.x, xl.x);
+                    dmma884(e0, e1, g.y, xl.y);
+                    dmma884(e0, e1, h.x, xh.x);
+                    dmma884(e0, e1, h.y, xh.y);
+                }
+            }
+            xh = make_double2(__shfl_sync(kAll, d0, 4 * t2), __shfl_sync(kAll, d0, 4 * t2 + 4));
+            dmma884(e0, e1, c.x, xh.x);
+            dmma884(e0, e1, c.y, xh.y);
+            xl = make_double2(__shfl_sync(kAll, e0, 4 * t2), __shfl_sync(kAll, e0, 4 * t2 + 4));
+            if (t2 == 0) {
+                if (rh < m) xs[rh] = d0;
+                if (kl >= 0) xs[rl] = e0;
+            }
+        } else if (prev) {
+            const double2 pl = load_pair(xs + 8 * (kh + 1) + t2);
+            const int ch = 8 * (kh + 2) + t2;  // the last block may be short
+            const double2 ph = ch < m ? load_pair(xs + ch) : make_double2(0., 0.);
+#pragma unroll 1
+            for (int i = warp - 1; i < kl; i += NW - 1) {
+                const double2 a = tile(i, kh + 1), b = tile(i, kh + 2);
+                double d0 = xs[8 * i + fr], d1 = d0;
+                dmma884(d0, d1, a.x, pl.x);
+                dmma884(d0, d1, a.y, pl.y);
+                dmma884(d0, d1, b.x, ph.x);
+                dmma884(d0, d1, b.y, ph.y);
+                if (t2 == 0) xs[8 * i + fr] = d0;
             }
         }
-        z0 += z1;
-        z0 += __shfl_xor_sync(kAll, z0, 1);
-        z0 += __shfl_xor_sync(kAll, z0, 2);
-        const double za = __shfl_sync(kAll, z0, 8 * t), zb = __shfl_sync(kAll, z0, 8 * t + 4);
-        xk = fma(dk.x, za, dk.y * zb);
-        xk += __shfl_xor_sync(kAll, xk, 1);
-        xk += __shfl_xor_sync(kAll, xk, 2);
-        if (t == 0 && row < m) xs[row] = xk;
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -1063,7 +1151,7 @@ __device__ __forceinline__ void gj_matvec(const TR (&R)[GJTile<TR, NT>::RT][GJTi
 // tilde(R1 X0) T_hub and -AX(C) T_hub are kept for the hub elimination.
 // RotationControl puts the commanded rotation Rc = exp(angle * axis) (angle =
 // input[0]) between the target and the hub: C = R(R2 Rc^-1 R1^-1).
-__device__ inline void constraint_record(double* cr, int type, const double* nu, const double* X0,
+static __device__ __noinline__ void constraint_record(double* cr, int type, const double* nu, const double* X0,
                                          const double* Rt, const double* hq, const double* RtHub,
                                          const double* axis) {
     double u1[3] = {0., 0., 0.}, R1[4] = {1., 0., 0., 0.};
@@ -1099,6 +1187,7 @@ __device__ inline void constraint_record(double* cr, int type, const double* nu,
         quat_compose(nu + 3, R1t, R2R1t);
     }
     double C[9];
+#pragma unroll
     for (int e = 0; e < 9; ++e) C[e] = rot_entry(R2R1t, e / 3, e % 3);
     cr[conrec::Phi + 3] = (C[7] - C[5]) / 2.;
     cr[conrec::Phi + 4] = (C[2] - C[6]) / 2.;
@@ -1588,6 +1677,7 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
     {
         const int g8 = lane >> 2, t = lane & 3;
         const int qt = (Q + 7) >> 3;
+#pragma unroll 1
         for (int u = warp; u < 3 * qt; u += NW) {  // (tile of points, tile of columns)
             const int ct = u / qt, q0 = 8 * (u - ct * qt);
             const double* tab = (ct < 2 ? phi : dphiJ) + min(q0 + g8, Q - 1) * N;
@@ -1615,6 +1705,7 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
     else asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
     const int role = lane & 7, bi = (role >> 1) & 1, bj = role & 1;
     const bool mass_block = role >= 4;
+#pragma unroll 1
     for (int p0 = 4 * warp; p0 < Q; p0 += 4 * NW) {
         const int qp = p0 + (lane >> 3), qc = min(qp, Q - 1);
         const double *sx0, *sr0, *sblk;
@@ -2837,6 +2928,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     const bool timing = KB.prof != nullptr;
     long long ph_t = 0;
     if (timing && tid == 0) {
+#pragma unroll 1
         for (int k = 0; k < kNumPhases; ++k) s_ph[k] = 0ull;
         ph_t = clock64();
     }
@@ -2849,14 +2941,18 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     };
 
     // ---- load constants and state ------------------------------------------
+#pragma unroll 1
     for (int k = tid; k < Q * N; k += NT) {
         phi[k] = slab[L.phi + k];
         dphi[k] = slab[L.dphi + k];
         dphiJ[k] = slab[L.dphiJ + k];
     }
+#pragma unroll 1
     for (int k = tid; k < Q * 4; k += NT) qpw[k] = slab[L.qpw + k];
 
+#pragma unroll 1
     for (int k = tid; k < N * 7; k += NT) sq[k] = slab[L.q + k];
+#pragma unroll 1
     for (int k = tid; k < N * 6; k += NT) {
         sv[k] = slab[L.v + k];
         svd[k] = slab[L.vd + k];
@@ -2868,6 +2964,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         for (int k = 0; k < 6; ++k) c[conrec::lam + k] = 0.;  // ResetConstraints
     }
     if (hub) {
+#pragma unroll 1
         for (int k = tid; k < kHubDoubles; k += NT) hb[k] = slab[L.hub + k];
         if (tid == 0) {
             double* br = hb + hubsm::bc;
@@ -2876,6 +2973,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         }
     }
     if (drive) {
+#pragma unroll 1
         for (int k = tid; k < (chain - 1) * kHubDoubles; k += NT)
             hb[hubsm::n1 + (k / kHubDoubles) * (hubsm::n2 - hubsm::n1) + k % kHubDoubles] =
                 slab[L.hub + kHubDoubles + k];
@@ -2887,6 +2985,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     }
     if (tid < N) {  // free nodes first, constrained nodes last (in constraint order)
         int before = 0, at = -1;
+#pragma unroll 1
         for (int c = 0; c < nc; ++c) {
             const int n = KB.con_node[c];
             before += n < tid;
@@ -2904,7 +3003,9 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     sec_issue();
 
     // ---- PredictNextState (src/step/predict_next_state.hpp:14-47) ------------
+#pragma unroll 1
     for (int k = tid; k < N * 7; k += NT) sqp[k] = sq[k];
+#pragma unroll 1
     for (int k = tid; k < N * 6; k += NT) {
         const double v_p = sv[k], vd_p = svd[k], a_p = sa[k];
         svd[k] = 0.;
@@ -2953,6 +3054,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         displaced_rotation(r + hubrec::q_prev, r + hubrec::q_delta, qn);
         for (int c = 0; c < 4; ++c) r[hubrec::q + 3 + c] = qn[c];
     };
+#pragma unroll 1
     for (int t = tid; t < 8 * N; t += NT)
         if ((t & 7) < 7) displace(t >> 3, t & 7);
     if (hub && chain_rec()) displace_chain(chain_rec());
@@ -2965,6 +3067,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     const bool clustered = KB.model_beams > 1;
 
     int extra = 0;  // refinement corrections taken after convergence (FP32 form)
+#pragma unroll 1
     for (int iter = 0; iter < P.max_iter + extra; ++iter) {
         // ---- tangent operator (src/system/calculate_tangent_operator.hpp:26-65)
         // Only the rotational 3x3 block of the stored (transposed) operator is kept.
@@ -3128,9 +3231,11 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         mark(kPhaseQuadrature);
 
         // ---- residual integration (integrate_residual_vector.hpp:33-50) ----------
+#pragma unroll 1
         for (int t = NT - 1 - tid; t < N * 6; t += NT) {  // the last warps have fewer pair units
             const int n = t / 6, c = t % 6;
             double acc = 0.;
+#pragma unroll 1
             for (int qp = 0; qp < Q; ++qp) {
                 const double w = qpw[qp * 4], wJ = qpw[qp * 4 + 2];
                 acc += (w * dphi[qp * N + n]) * Fc[qp * 6 + c] +
@@ -3152,6 +3257,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             });
         __syncthreads();
         if (LUMP && KB.n_mass + KB.n_spring > 0) {  // point masses and springs at this CTA's nodes
+#pragma unroll 1
             for (int n = tid; n < N; n += NT)
                 add_lumped_terms(n, KB.lumped, KB.n_mass, KB.n_spring, sq, sv, svd, sT, KB.gravity,
                                  P.beta_prime, P.gamma_prime, P.conditioner, pos,
@@ -3165,12 +3271,14 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             // matrix [nl][nl], then rhs [nl], then solution [nl]; nl = n6 + 6 nc.
             const int nl = n6 + 6 * nc;
             double* D = KB.dump;
+#pragma unroll 1
             for (int t = tid; t < nl * nl; t += NT) D[t] = 0.;
         }
         if (record) __syncthreads();
         if (record && KB.dump) {
             const int nl = n6 + 6 * nc;
             double* D = KB.dump;
+#pragma unroll 1
             for (int t = tid; t < n6 * n6; t += NT) {
                 const int r = t / n6, c = t % n6;
                 D[r * nl + c] = static_cast<double>(
@@ -3207,10 +3315,12 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         double* x2 = gjv + 2 * n6;         // [n6] its solution
         double* red4 = gjv + 4 * n6;       // [64] reductions of the refinement
         // (eight lanes per row: the rows start in only two different banks)
+#pragma unroll 1
         for (int i0 = 4 * warp; i0 < n6; i0 += 4 * NW) {
             const int i = i0 + (lane >> 3), ic = min(i, n6 - 1);
             double r = 0., r2 = 0.;
             if (i0 < m) {
+#pragma unroll 1
                 for (int j = m + (lane & 7); j < n6; j += 8) {
                     const double aij = static_cast<double>(A[sys_at(ldA, ic, j)]);
                     r -= aij * xs[j];
@@ -3304,6 +3414,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 }
                 __syncthreads();
                 ra = xa = ba = aa = 0.;
+#pragma unroll 1
                 for (int w2 = 0; w2 < NW; ++w2) {
                     ra = fmax(ra, red4[4 * w2]);
                     xa = fmax(xa, red4[4 * w2 + 1]);
@@ -3328,9 +3439,11 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                     double* dx = gjv + 3 * n6;
                     for (int pass = 0; pass < 2; ++pass) {
                         gj_solve_pivoted<TR, NT>(A, ldA, m, pivots, pass ? dx : xs, &s_flag);
+#pragma unroll 1
                         for (int i = tid; pass && i < m; i += NT) xs[i] += dx[i];
                         __syncthreads();
                         eta = backward_error(xs, bp, r64);
+#pragma unroll 1
                         for (int i = tid; i < m; i += NT) A[sys_at(ldA, i, m)] = r64[i];
                         __syncthreads();
                     }
@@ -3347,12 +3460,14 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 // FP32 inverse in R; x = R b, then sweeps x += R (b - A x) with
                 // the residual in FP64 until its backward error is at most
                 // refine_tol (or refine_sweeps sweeps)
+#pragma unroll 1
                 for (int rhs = 0; rhs < nrhs; ++rhs) {
                     double* x = rhs ? x2 : xs;
                     const double* b = rhs ? rhs2 : bp;
                     double amax;
                     gj_matvec<TR, NT, true>(R, A, ldA, m, b, nullptr, x, amax);
                     __syncthreads();
+#pragma unroll 1
                     for (int sweep = 1;; ++sweep) {
                         const double eta = backward_error(x, b, r64);
                         const bool done = eta <= P.refine_tol;
@@ -3391,16 +3506,15 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
           }
         } else {
-            // block elimination, then the back substitution of each right-hand
-            // side by a warp of its own
+            // block elimination, then the back substitution of each right-hand side
             double* dinv = reinterpret_cast<double*>(smem_raw + S.G);
             if (m > 0) {
                 eliminate_free_block<TR, NT>(A, ldA, m, nrhs, dinv, &s_flag);
                 mark(kPhaseFactor);
-                if (warp < nrhs)
-                    back_substitute_blocks(A, ldA, m, m + warp, dinv, warp == 0 ? xs : x2, lane);
+                back_substitute<TR, NT>(A, ldA, m, m, xs);
+                if (drive) back_substitute<TR, NT>(A, ldA, m, m + 1, x2);
             }
-            __syncthreads();
+            mark(kPhaseLUPanel);
         }
         if (drive) {
             // Shaft rotation theta: x = x1 + theta x2 (x1 = (y1, c_r), x2 = (y2, d_r)).
@@ -3409,10 +3523,12 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             //   sum_roots w_r.(b_r - A_r x) + sum_chain w_n.b_n = 0,
             // b_n = -cond (sum of G^T lambda at the node + torque); chain nodes
             // carry no element terms.
+#pragma unroll 1
             for (int rowi = warp; rowi < 6 * nc; rowi += NW) {
                 const int c = rowi / 6, k = rowi % 6;
                 const int pr = 6 * pos[KB.con_node[c]];
                 double a1 = 0., a2 = 0.;
+#pragma unroll 1
                 for (int j = lane; j < n6; j += 32) {
                     const double arj = static_cast<double>(A[sys_at(ldA, pr + k, j)]);
                     a1 += arj * xs[j];
@@ -3431,6 +3547,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             double* xt = hb + hubsm::xt + 8 * (iter & 1);
             if (tid == 0) {  // this beam's roots: w.s1, w.s2 and G_base^T lambda
                 for (int k = 0; k < 8; ++k) xt[k] = 0.;
+#pragma unroll 1
                 for (int c = 0; c < nc; ++c) {
                     const double* cr = con + c * kConStride;
                     for (int k = 0; k < 6; ++k) {
@@ -3445,6 +3562,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 // every CTA sums the beams' parts in rank order, so all find the same theta
                 double num = 0., den = 0.;
                 double gj[6] = {0., 0., 0., 0., 0., 0.};  // roots' G_base^T lambda
+#pragma unroll 1
                 for (int r = 0; r < KB.model_beams; ++r) {
                     const double* peer = clustered ? cluster.map_shared_rank(xt, r) : xt;
                     num += peer[0];
@@ -3468,7 +3586,9 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
             __syncthreads();
             const double th = hb[hubsm::theta];
+#pragma unroll 1
             for (int i = tid; i < m; i += NT) xs[i] += th * x2[i];
+#pragma unroll 1
             for (int t = tid; t < 6 * nc; t += NT) {
                 const int pr = 6 * pos[KB.con_node[t / 6]];
                 xs[pr + t % 6] += th * droot[pr + t % 6];
@@ -3482,9 +3602,11 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         //      lanes to a node.
         double part = 0.;
         if (warp == NW - 1) {
+#pragma unroll 1
             for (int c = 0; c < nc; ++c) {
                 const int pr = m + 6 * c;
                 double y[6] = {0., 0., 0., 0., 0., 0.};
+#pragma unroll 1
                 for (int j = lane; j < n6; j += 32) {
                     const double xj = xs[j];
 #pragma unroll
@@ -3518,6 +3640,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 // G_base^T (lambda + x_lambda), exchanged over the cluster below
                 double* pub = hb + hubsm::pub + 6 * (iter & 1);
                 for (int k = 0; k < 6; ++k) pub[k] = 0.;
+#pragma unroll 1
                 for (int c = 0; c < nc; ++c) {
                     if (!is_hub_joint(KB.con_type[c])) continue;
                     const double* cr = con + c * kConStride;
@@ -3529,10 +3652,12 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             if (record && KB.dump) {
                 const int nl = n6 + 6 * nc;
                 double* D = KB.dump + nl * nl + nl;
+#pragma unroll 1
                 for (int t = lane; t < n6; t += 32) D[t] = xs[6 * pos[t / 6] + t % 6];
                 if (lane < nc)
                     for (int k = 0; k < 6; ++k) D[n6 + 6 * lane + k] = con[lane * kConStride + conrec::xl + k];
             }
+#pragma unroll 1
             for (int t = lane; t < 6 * nc; t += 32) {
                 double* cr = con + (t / 6) * kConStride;
                 const double lam = cr[conrec::lam + t % 6], xl = cr[conrec::xl + t % 6];
@@ -3541,6 +3666,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 if (!hub) cr[conrec::lam + t % 6] = lam + xl;  // update_lambda_prediction.hpp
             }
         } else {
+#pragma unroll 1
             for (int n0 = 4 * warp; n0 < N; n0 += 4 * (NW - 1)) {
                 const int n = n0 + (lane >> 3), c = lane & 7, t = 6 * n + c;
                 if (n < N && c < 6) {
@@ -3568,6 +3694,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         sec_issue();  // A is not read again in this iteration
         mark(kPhaseSubstitute);
         double total = 0., flags = 0.;
+#pragma unroll 1
         for (int k = lane; k < KB.model_beams * (NW + 1); k += 32) {
             const int r = k / (NW + 1), w2 = k - r * (NW + 1);
             const double v = clustered ? *cluster.map_shared_rank(slot + w2, r) : slot[w2];
@@ -3583,6 +3710,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             // Hub rows have no element terms: G_hub^T x_lh = -G_hub^T lambda_hub -
             // sum_j G_base,j^T (lambda_j + x_lj), summed over the beams in rank order.
             double sum[6] = {0., 0., 0., 0., 0., 0.};
+#pragma unroll 1
             for (int r = 0; r < KB.model_beams; ++r) {
                 const double* peer = clustered ? cluster.map_shared_rank(hb + hubsm::pub + 6 * (iter & 1), r)
                                                : hb + hubsm::pub + 6 * (iter & 1);
@@ -3637,6 +3765,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 }
                 // the chain nodes' terms of the error sum
                 const double th = hb[hubsm::theta];
+#pragma unroll 1
                 for (int r = 1; r < chain; ++r) {
                     const double* rec = r == 1 ? hA : hH;
                     const double* c0 = hb + (r == 1 ? hubsm::cA : hubsm::cH);
@@ -3668,6 +3797,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         // ---- update of the hub chain and, with a hub, of the multipliers (read by
         //      the peers' sums above only through pub)
         if (hub && warp == NW - 1)
+#pragma unroll 1
             for (int t = lane; t < 6 * nc; t += 32) {
                 double* cr = con + (t / 6) * kConStride;
                 cr[conrec::lam + t % 6] += cr[conrec::xl + t % 6];
@@ -3730,6 +3860,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     // ---- post-step (step.hpp:86-121) ---------------------------------------------------
     if (status == KYN_OK) {
         const double fac = (1. - P.alpha_f) / (1. - P.alpha_m);
+#pragma unroll 1
         for (int t = tid; t < n6; t += NT) sa[t] += fac * svd[t];
     }
     if (hub && chain_rec()) {
@@ -3747,15 +3878,18 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     }
     __syncthreads();
     if (hub)  // every beam keeps its copy of the hub state (the input is the caller's)
+#pragma unroll 1
         for (int k = tid; k < (drive ? chain : 1) * kHubDoubles; k += NT) {
             const int r = k / kHubDoubles, e = k % kHubDoubles;
             const double* src = r == 0 ? hb : r == 1 ? hA : hH;
             if (e < hubrec::input || e >= hubrec::input + 7) slab[L.hub + k] = src[e];
         }
+#pragma unroll 1
     for (int k = tid; k < N * 7; k += NT) {
         slab[L.q + k] = sq[k];
         slab[L.q_prev + k] = sqp[k];
     }
+#pragma unroll 1
     for (int k = tid; k < N * 6; k += NT) {
         slab[L.v + k] = sv[k];
         slab[L.vd + k] = svd[k];
@@ -3763,6 +3897,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         slab[L.q_delta + k] = sqd[k];
     }
     if (status == KYN_OK) {
+#pragma unroll 1
         for (int n = tid; n < N; n += NT) {
             const double* x0 = slab + L.x0 + n * 7;
             for (int c = 0; c < 3; ++c) slab[L.x + n * 7 + c] = x0[c] + sq[n * 7 + c];
@@ -3771,6 +3906,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             for (int c = 0; c < 4; ++c) slab[L.x + n * 7 + 3 + c] = r[c];
         }
     }
+#pragma unroll 1
     for (int k = tid; k < N * 9; k += NT) slab[L.tangent + k] = sT[k];
     if (tid < 6 * nc) {
         const double* cr = con + (tid / 6) * kConStride;
@@ -3783,6 +3919,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     __syncthreads();
     mark(kPhaseStore);
     if (timing && tid == 0)
+#pragma unroll 1
         for (int k = 0; k < kNumPhases; ++k) atomicAdd(KB.prof + k, s_ph[k]);
     if (clustered) cluster.sync();  // peers may still read this CTA's slot
 }
