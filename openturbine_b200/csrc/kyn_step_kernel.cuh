@@ -402,7 +402,8 @@ __device__ __forceinline__ void store_pair(float* p, double a, double b) {
 // work is eight (j, row) lines and one half of the columns: a lane forms its
 // line's three columns of H and H' at its point (line lane / 4, point lane % 4
 // of a step of four) and holds three column tiles by up to three tiles of nodes
-// i.  store(i, j, row, half, v0, v1, v2) gets three adjacent columns.
+// i.  store(j, row, half) gives put(i, v0, v1, v2), which takes three
+// adjacent columns.
 //
 // The former product over node pairs [N^2 x 4Q][4Q x 56] took N^2 Q 448
 // multiply-adds where this takes 144, and was bound by the tensor pipe (36k of
@@ -438,8 +439,8 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
             const double *pq = phi + min(t, Q - 1) * N, *dq = dphi + min(t, Q - 1) * N;
 #pragma unroll 1
             for (int q = t; q - t < Q; q += 4) {
-                const bool in = q < Q;
-                const double pj = pq[j], dj = dq[j];
+                // past the last point the line's factors are zero; rows i >= N are not stored
+                const double pj = q < Q ? pq[j] : 0., dj = q < Q ? dq[j] : 0.;
                 double h[3], hp[3];
                 if (right) {
                     const double2 g8v = load_pair(g + 8), ga = load_pair(g + 10), gb = load_pair(g + 12),
@@ -468,9 +469,7 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt) {
                     if (i0 + 8 * mt < N) {  // uniform
-                        const int i = i0 + 8 * mt + g8;
-                        const bool on = in && i < N;
-                        const double f = on ? pq[i] : 0., fp = on ? dq[i] : 0.;
+                        const double f = pq[i0 + 8 * mt + g8], fp = dq[i0 + 8 * mt + g8];
 #pragma unroll
                         for (int c = 0; c < 3; ++c) dmma884(acc[mt][c][0], acc[mt][c][1], f, h[c]);
 #pragma unroll
@@ -483,17 +482,15 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
                 dq += step * N;
             }
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                const int i = i0 + 8 * mt + g8;
-                if (i < N) {
+            for (int e = 0; e < 2; ++e) {
+                const int lo = l0 + 2 * t + e;
+                if (lo < lines) {
+                    const int jo = lo / 6;
+                    auto put = store(jo, lo - 6 * jo, right ? 1 : 0);
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int lo = l0 + 2 * t + e;
-                        if (lo < lines) {
-                            const int jo = lo / 6;
-                            store(i, jo, lo - 6 * jo, right ? 1 : 0, acc[mt][0][e], acc[mt][1][e], acc[mt][2][e]);
-                        }
-                    }
+                    for (int mt = 0; mt < MT; ++mt)
+                        if (i0 + 8 * mt + g8 < N)
+                            put(i0 + 8 * mt + g8, acc[mt][0][e], acc[mt][1][e], acc[mt][2][e]);
                 }
             }
         }
@@ -1649,7 +1646,7 @@ constexpr int r = 0, udd = 4, om = 7, omd = 10, up = 16, rp = 19;
 // slab for the sections and reference frames (layout L), or sec: the sections
 // already staged in shared memory (sec_doubles(Q), slab order from x0').
 // Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the integration
-// G [Q][kGPoint] (gblk).  itp: kQpInterp doubles of scratch per point.  Run by
+// G [Q][kGPoint] (gblk), the conditioner cond included.  itp: kQpInterp doubles of scratch per point.  Run by
 // warps 0 .. NW - 1; ALL: they are the whole CTA (else they meet at barrier 1).
 //
 // The 20 interpolations are products [Q x N][N x 13] and [Q x N][N x 7] on the
@@ -1670,7 +1667,7 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
                                          const double* qpw, const double* sq, const double* sv,
                                          const double* svd, const double* __restrict__ slab,
                                          const SlabLayout& L, const double* gravity, double beta_prime,
-                                         double gamma_prime, double* itp, TG* G, double* Fc, double* Fdig,
+                                         double gamma_prime, double cond, double* itp, TG* G, double* Fc, double* Fdig,
                                          const double* sec = nullptr) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1791,7 +1788,7 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
         me[1] = -__shfl_sync(kAll, X[6], 6, 8);
         me[2] = __shfl_sync(kAll, X[3], 6, 8);
         const bool on = qp < Q;
-        const double w = qpw[qc * 4], wJ = qpw[qc * 4 + 2];
+        const double w = cond * qpw[qc * 4], wJ = cond * qpw[qc * 4 + 2];
         TG* Gq = G + qc * kGPoint;
         // blocks crossed with s (stiffness) or omega (mass): columns first
         double c[3], om[3], V[9];
@@ -1816,7 +1813,7 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
             if (on) {
                 // C, XI = beta' Muu + gamma' Guu; P (no translational rows)
                 TG* o = Gq + 3 * bi * kGRow + (mass_block ? (bj ? gblk::XIR : gblk::XIL) : (bj ? gblk::CR : gblk::CL));
-                const double sc = mass_block ? wJ * beta_prime : qpw[qc * 4 + 3];
+                const double sc = mass_block ? wJ * beta_prime : cond * qpw[qc * 4 + 3];
                 const double sg = mass_block && bj ? wJ * gamma_prime : 0.;
 #pragma unroll
                 for (int e = 0; e < 9; ++e) o[(e / 3) * kGRow + e % 3] = static_cast<TG>(fma(sg, Z[e], sc * X[e]));
@@ -1953,7 +1950,7 @@ __device__ void dense_beam_terms(const KBeam& KB, const StepCoeffs& P, const Den
         }
         __syncthreads();
         qp_phase<double, NT / 32>(N, Q, phi, dphiJ, qpw, cq, cv, cvd, cs, L, KB.gravity, P.beta_prime, P.gamma_prime,
-                             gscr, G, Fc, Fd);
+                             cond, gscr, G, Fc, Fd);
         __syncthreads();
         for (int t = tid; t < N * 6; t += NT) {
             const int n = t / 6, c = t % 6;
@@ -1966,12 +1963,14 @@ __device__ void dense_beam_terms(const KBeam& KB, const StepCoeffs& P, const Den
         }
         integrate_node_pairs<NT>(
             N, Q, phi, dphi, G, [&](int j) { return sT + static_cast<int>(node[j]) * 9; },
-            [&](int i, int j, int r, int half, double v0, double v1, double v2) {
-                double* row = Md + (fmap[static_cast<int>(node[i])] + r) * nd + fmap[static_cast<int>(node[j])] +
-                              3 * half;
-                row[0] += cond * v0;
-                row[1] += cond * v1;
-                row[2] += cond * v2;
+            [&](int j, int r, int half) {
+                double* col = Md + r * nd + fmap[static_cast<int>(node[j])] + 3 * half;
+                return [=](int i, double v0, double v1, double v2) {
+                    double* row = col + fmap[static_cast<int>(node[i])] * nd;
+                    row[0] += v0;
+                    row[1] += v1;
+                    row[2] += v2;
+                };
             });
         __syncthreads();
     }
@@ -2147,7 +2146,7 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
             Lc.r0 += 4 * q0;
             Lc.x0p += 3 * q0;
             qp_phase<double, NT / 32>(N, qn, phi + q0 * N, dphiJ + q0 * N, qpw + q0 * 4, cq, cv, cvd, cs, Lc,
-                                 KB.gravity, P.beta_prime, P.gamma_prime, gscr, G, Fc, Fd);
+                                 KB.gravity, P.beta_prime, P.gamma_prime, cond, gscr, G, Fc, Fd);
             __syncthreads();
             sub(kPhaseQuadrature);
             for (int t = tid; t < N * 6; t += NT) {
@@ -2164,11 +2163,14 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
             }
             integrate_node_pairs<NT>(
                 N, qn, phi + q0 * N, dphi + q0 * N, G, [&](int j) { return sT + static_cast<int>(node[j]) * 9; },
-                [&](int i, int j, int r, int half, double v0, double v1, double v2) {
-                    double* row = W + (lpos[i] * 6 + r) * ldw + lpos[j] * 6 + 3 * half;
-                    row[0] += cond * v0;
-                    row[1] += cond * v1;
-                    row[2] += cond * v2;
+                [&](int j, int r, int half) {
+                    double* col = W + r * ldw + lpos[j] * 6 + 3 * half;
+                    return [=](int i, double v0, double v1, double v2) {
+                        double* row = col + lpos[i] * 6 * ldw;
+                        row[0] += v0;
+                        row[1] += v1;
+                        row[2] += v2;
+                    };
                 });
             __syncthreads();
             sub(kPhaseLUDiag);
@@ -3225,7 +3227,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             // ---- quadrature-point values (calculate_quadrature_point_values.hpp) ---
             sec_wait();
             qp_phase<TG, NW - 1, false>(N, Q, phi, dphiJ, qpw, sq, sv, svd, slab, L, KB.gravity, P.beta_prime,
-                                        P.gamma_prime, itp, G, Fc, Fdig, bulk ? sec : nullptr);
+                                        P.gamma_prime, P.conditioner, itp, G, Fc, Fdig, bulk ? sec : nullptr);
         }
         __syncthreads();
         mark(kPhaseQuadrature);
@@ -3248,12 +3250,14 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         //      into A (the residual's inputs stay untouched)
         integrate_node_pairs<NT>(
             N, Q, phi, dphi, G, [&](int j) { return sT + j * 9; },
-            [&](int i, int j, int r, int half, double v0, double v1, double v2) {
-                const int row = 6 * pos[i] + r, col = 6 * pos[j] + 3 * half, sh = row & 6;
-                TR* a = A + row * ldA;
-                a[col ^ sh] = static_cast<TR>(v0 * P.conditioner);
-                a[(col + 1) ^ sh] = static_cast<TR>(v1 * P.conditioner);
-                a[(col + 2) ^ sh] = static_cast<TR>(v2 * P.conditioner);
+            [&](int j, int r, int half) {
+                return [=](int i, double v0, double v1, double v2) {
+                    const int row = 6 * pos[i] + r, col = 6 * pos[j] + 3 * half, sh = row & 6;
+                    TR* a = A + row * ldA;
+                    a[col ^ sh] = static_cast<TR>(v0);
+                    a[(col + 1) ^ sh] = static_cast<TR>(v1);
+                    a[(col + 2) ^ sh] = static_cast<TR>(v2);
+                };
             });
         __syncthreads();
         if (LUMP && KB.n_mass + KB.n_spring > 0) {  // point masses and springs at this CTA's nodes
