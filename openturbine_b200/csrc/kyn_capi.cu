@@ -40,6 +40,7 @@ struct DevModel {
     KBeam* d_kt = nullptr;           // the same records resident on the device (plans gather them)
     std::vector<int> node_base;      // per beam: first global node when its nodes are contiguous, else -1
     int def_nt[2] = {0, 0};          // default threads per CTA, FP64 / FP32 form
+    bool four128[2] = {false, false};  // four CTAs of 128 threads fit an SM (per form)
     int tuned_nt[2] = {0, 0};        // tuned threads per CTA (0: none), cached per form
     int tuned_sv[2] = {-1, -1};      // tuned free-block solver (-1: the context's), cached per form
     unsigned long long tuned_gen[2] = {~0ull, ~0ull};  // tuned-table generation of that cache
@@ -181,6 +182,7 @@ __global__ void xfer_kernel(const XferBeam* __restrict__ beams, const int* __res
 
 struct kyn_ctx {
     int device = 0;
+    int sms = 148;                        // multiprocessors of the device
     size_t budget = 0;
     size_t used = 0;
     cudaStream_t stream = nullptr;
@@ -301,6 +303,13 @@ StepCoeffs make_coeffs(const kyn_ctx* c, const kyn_step_params* p) {
 // Default threads per CTA for a beam: 256 when two such CTAs fit on an SM
 // (their serial phases overlap), else 512 so the one resident CTA has 16
 // warps.  kyn_autotune replaces the default per size class by measurement.
+// A step of more beams than that keeps resident takes 128 threads where four
+// such CTAs fit: the SM has 16 warps either way, and a step's serial chains
+// are shared by four beams instead of two (one B200, 2048 beams: 5 nodes 540
+// -> 375 us, 8 nodes 621 -> 506, 10 nodes 744 -> 661, FP32 form at 14 nodes
+// 1308 -> 1277; with three CTAs, FP64 at 12 nodes, 932 -> 959).  Fewer beams
+// step sooner on 256 (100 beams: 10 nodes 151 against 168 us, FP32 at 14 nodes
+// 208 against 285).
 int beam_threads(int N, int Q, int nc, int real_bytes, int hub = 0) {
     const int s256 = make_smem(N, Q, nc, real_bytes, 256, hub).bytes;
     return (2 * (s256 + 1024) <= kSmemPerSM) ? 256 : 512;
@@ -359,7 +368,9 @@ void prepare_model(DevModel* m) {
     for (int f = 0; f < 2; ++f) {
         const int rb = f ? 4 : 8;
         m->def_nt[f] = 128;
+        m->four128[f] = false;
         for (int k = 0; k < 3; ++k) m->smem_nt[f][k] = 0;
+        bool b0 = true;  // first beam
         for (const HostBeam& hb : H.beams) {
             if (hb.dense) {  // the dense bordered system, FP64 in both forms
                 for (int k = 0; k < 3; ++k)
@@ -377,6 +388,9 @@ void prepare_model(DevModel* m) {
                 continue;
             }
             m->def_nt[f] = std::max(m->def_nt[f], beam_threads(hb.N, hb.Q, hb.nc, rb, hubf));
+            if (b0 || m->four128[f])
+                m->four128[f] = 4 * (beam_smem(hb.N, hb.Q, hb.nc, rb, 128, hubf) + 1024) <= kSmemPerSM;
+            b0 = false;
             for (int k = 0; k < 3; ++k)
                 m->smem_nt[f][k] = std::max(m->smem_nt[f][k], beam_smem(hb.N, hb.Q, hb.nc, rb, 128 << k, hubf));
         }
@@ -500,9 +514,14 @@ int get_plan(kyn_ctx* c, const int* ids, int n, int precision, Plan** out) {
     if (n >= (1 << 26)) return set_err(c, KYN_ERR_UNSUPPORTED, "more than 2^26 models in one step");
     size_t nbeams = 0;
     for (int i = 0; i < n; ++i) {
-        DevModel* m = find_model(c, ids[i]);
+        const DevModel* m = find_model(c, ids[i]);
         if (!m) return set_err(c, KYN_ERR_NOT_FOUND, "unknown model id in step list");
-        int nt = m->def_nt[f];
+        nbeams += m->kt.size();
+    }
+    const bool many = nbeams > static_cast<size_t>(2) * c->sms;  // see beam_threads
+    for (int i = 0; i < n; ++i) {
+        DevModel* m = find_model(c, ids[i]);
+        int nt = many && m->four128[f] ? 128 : m->def_nt[f];
         if (!c->tuned.empty()) {
             if (m->tuned_gen[f] != c->tuned_gen) {  // per-model cache of the tuned table
                 const ClassKey ck = class_key(m->host, precision);
@@ -529,7 +548,6 @@ int get_plan(kyn_ctx* c, const int* ids, int n, int precision, Plan** out) {
                        (static_cast<uint64_t>(std::min(cls, 15)) << 52) |
                        (static_cast<uint64_t>(solver == KYN_SOLVER_GAUSS_JORDAN ? 1 : 0) << 51) |
                        ((1048575ull - work) << 31) | static_cast<uint64_t>(i));
-        nbeams += m->kt.size();
     }
     std::sort(keys.begin(), keys.end());
     std::vector<Entry>& entries = c->plan_sorted_tmp;
@@ -855,6 +873,7 @@ kyn_ctx* kyn_ctx_create(int device, size_t hbm_budget_bytes) {
     auto* c = new kyn_ctx();
     c->device = device;
     c->budget = hbm_budget_bytes;
+    if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) c->sms = 148;
     bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; i < kBucketStreams && ok; ++i) {
         ok = cudaStreamCreateWithFlags(&c->bstream[i], cudaStreamNonBlocking) == cudaSuccess &&
@@ -1827,8 +1846,7 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
     if (n == 0) return KYN_OK;
     KYN_CUDA(c, cudaSetDevice(c->device));
     const int rb = (p->precision == KYN_PRECISION_FP32_REFINED) ? 4 : 8;
-    int sms = 148;
-    KYN_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    const int sms = c->sms;
     const size_t sample_max = 16384;  // copies timed per class at most
     std::map<ClassKey, std::vector<int>> classes;
     for (int i = 0; i < n; ++i) {

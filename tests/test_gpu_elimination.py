@@ -52,3 +52,36 @@ def test_elimination_matches_oracle(nodes, clamped, precision):
     assert np.abs(d - od).max() <= tol
     ctx.close()
 
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_many_small_beams_match_few(precision):
+    """A step of more beams than fill the GPU twice over runs small beams on
+    fewer threads each: the same Newton decisions and states as alone, at the
+    smallest size and at the largest that fits four to an SM."""
+    from openturbine_b200.runtime import Context
+    p = W.batch_params()
+    p.precision = precision
+    ctx = Context(0)
+    sizes = (2, 5, 10)
+    alone, many = [], []
+    for nodes in sizes:
+        pm = _beam(nodes, nodes + 1, True).pack()
+        alone.append(ctx.create_model(pm))
+        many.append([ctx.create_model(pm)])
+        many[-1] += [ctx.clone_model(many[-1][0]) for _ in range(109)]
+    fx = [np.zeros((n, 6)) for n in sizes]
+    for step in range(2):
+        for f, a, ms in zip(fx, alone, many):
+            f[-1] = np.array([200., 300., 400., 10., 20., 30.]) * np.cos(0.3 * step)
+            for i in [a] + ms:
+                ctx.set_node_fx(i, f)
+        sa, ia = ctx.step(alone, p)
+        sm, im = ctx.step([i for ms in many for i in ms], p)
+        assert (sa == 0).all() and (sm == 0).all()
+        assert (im.reshape(len(sizes), -1) == ia[:, None]).all()
+    for a, ms in zip(alone, many):
+        q = ctx.state(a, "q")
+        for i in (ms[0], ms[-1]):
+            assert np.abs(ctx.state(i, "q") - q).max() <= 1e-13 * np.abs(q).max()
+    ctx.close()
