@@ -1043,7 +1043,7 @@ int kyn_model_create(kyn_ctx* c, const kyn_model_desc* desc) {
             // the condensed model's bordered system moves to device memory (the slab's tail)
             if (b.slab.size() & 1) b.slab.push_back(0.);
             b.cond_md_off = static_cast<int>(b.slab.size());
-            b.slab.resize(b.slab.size() + static_cast<size_t>(b.cond_nd) * b.cond_nd, 0.);
+            b.slab.resize(b.slab.size() + static_cast<size_t>(b.cond_nd) * bord_ld(b.cond_nd), 0.);
         }
         const int sm = b.dense ? dense_smem(m->host, b, nt)
                                : std::max(beam_smem(b.N, b.Q, b.nc, sizeof(double), 512, hubf),

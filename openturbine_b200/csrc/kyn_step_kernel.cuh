@@ -1495,7 +1495,7 @@ __device__ void add_lumped_terms(int n, const double* __restrict__ rec, int n_ma
 // in both precision forms: these systems have at most kDenseModelMaxDofs unknowns.
 
 struct DenseSmem {
-    int M, b, x, q, qp, v, vd, a, qd, T, resid, con, act, fmap, red;
+    int M, b, x, q, qp, v, vd, a, qd, T, resid, con, act, fmap, red, rpiv, bord;
     // beam components (dense models with beams): shape tables, weights and
     // node state of one component at a time, its quadrature-point outputs and
     // the interpolated values
@@ -1510,6 +1510,9 @@ struct DenseSmem {
     int cR;  // condensed models: bytes of that region
     int bytes;
 };
+// Row length of a bordered system of nd unknowns: the right-hand side is column
+// nd, rows of even length.
+KYN_HD inline int bord_ld(int nd) { return (nd + 2) & ~1; }
 // Quadrature points per pass of a condensed component's assembly.
 constexpr int kCondChunk = 16;
 // nt, cN, cQ: threads per CTA and the largest beam component (0: none);
@@ -1536,7 +1539,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     const int t_bytes = cond_nd > 0 ? 3 * r16(cQ * cN * 8) + r16(cQ * 4 * 8) + r16(cN * 7 * 8) +
                                           2 * r16(cN * 6 * 8) + 2 * r16(cQ * 6 * 8) : 0;
     const int c_bytes = w_bytes + g_bytes + s_bytes + t_bytes;
-    const int m_bytes = md_global ? 0 : nd * nd * 8;
+    const int m_bytes = md_global ? 0 : nd * bord_ld(nd) * 8;
     const int region = take(m_bytes > c_bytes ? m_bytes : c_bytes);
     S.M = md_global ? -1 : region;
     S.cW = cond_nd > 0 ? region : -1;
@@ -1555,6 +1558,8 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     S.act = take(N * 4);
     S.fmap = take(N * 4);
     S.red = take(64 * 8);  // per-warp partial sums of the error
+    S.rpiv = take(nd * 8);      // reciprocal pivots of the bordered system
+    S.bord = take(1024);        // BordScratch
     S.cphi = S.cdphi = S.cdphiJ = S.cqpw = S.cq = S.cv = S.cvd = S.cG = S.cFc = S.cFd = S.cgs = -1;
     if (cN > 0 && cond_nd > 0) {  // inside the bordered system's region, after the component's system
         int t = region + w_bytes;
@@ -2341,6 +2346,246 @@ __device__ void cond_back_substitute(const KBeam& KB, const DenseSmem& S, unsign
     }
 }
 
+// ---- pivoted LU of a bordered system ------------------------------------------------
+// Md [md][ld], ld even, the right-hand side in column md; partial pivoting
+// (largest entry by its leading 32 bits, lowest row on a tie), eight columns per
+// panel:
+//   1. the first warps factor the panel, a row per thread in registers; a pivot
+//      is found by two integer reductions per warp and an exchange of the warps'
+//      finds, and its row reaches the threads through shared memory;
+//   2. one thread per remaining column brings the pivot rows to the top, the
+//      rows they displace to the places they leave, and solves for U;
+//   3. all warps subtract L U from the rest on the FP64 tensor cores.
+// The unblocked form (pivot search, swap and a rank-1 update of the whole rest
+// per column) was bound by the traffic of those updates and by three barriers a
+// column: 643k cycles for 137 unknowns.  With the panel in one warp, five rows
+// to a lane, a column took 1300 cycles.
+struct BordScratch {
+    double prow[2][8];  // the pivot row, from the pivot on (double-buffered by column)
+    double rp[2];       // the pivot's reciprocal
+    unsigned long long key[2][8];  // per warp: leading bits of its largest entry, row (complemented)
+    double lower[64];   // unit lower triangle of the panel's pivot rows [8][8]
+    int piv[8];         // row each panel column was pivoted on
+    int back[8];        // row (of the panel's eight) that goes where piv[c] was, or -1
+};
+static_assert(sizeof(BordScratch) <= 1024, "DenseSmem::bord");
+
+// Step 1, by warps 0 .. PW - 1 (which meet at barrier 2), RT rows per thread.
+template <int PW, int RT>
+__device__ __forceinline__ void factor_pivoted_panel(double* Md, int ld, int md, int k0, double* rpiv,
+                                                     BordScratch* W, int* flag) {
+    constexpr unsigned kAll = 0xffffffffu;
+    auto meet = [&]() {
+        if constexpr (PW == 1) __syncwarp();
+        else asm volatile("bar.sync 2, %0;" ::"n"(32 * PW) : "memory");
+    };
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kb = min(8, md - k0);
+    double v[RT][8];
+    bool live[RT];
+    double* row[RT];
+#pragma unroll
+    for (int e = 0; e < RT; ++e) {
+        const int i = k0 + tid + 32 * PW * e;
+        live[e] = i < md;
+        row[e] = Md + min(i, md - 1) * ld + k0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[e][c] = c < kb ? row[e][c] : 0.;
+    }
+#pragma unroll 1
+    for (int c = 0; c < kb; ++c) {  // the pivot column is v[.][0]
+        const int h = c & 1;
+        unsigned hi = 0;
+        int at = 0;
+#pragma unroll
+        for (int e = 0; e < RT; ++e) {
+            const double x = fabs(v[e][0]);
+            const unsigned he = live[e] && x > 0. ? static_cast<unsigned>(__double2hiint(x)) + 1u : 0u;  // NaN: 0
+            if (he > hi) {
+                hi = he;
+                at = e;
+            }
+        }
+        double inv[RT];  // every thread's reciprocal, while the reductions run
+#pragma unroll
+        for (int e = 0; e < RT; ++e) inv[e] = 1. / v[e][0];
+        const unsigned mh = __reduce_max_sync(kAll, hi);
+        const unsigned mr = __reduce_min_sync(kAll, hi == mh ? static_cast<unsigned>(tid + 32 * PW * at) : ~0u);
+        unsigned long long key = static_cast<unsigned long long>(mh) << 32 | (~mr);
+        if constexpr (PW > 1) {
+            if (lane == 0) W->key[h][warp] = key;
+            meet();
+            key = W->key[h][0];
+#pragma unroll
+            for (int w = 1; w < PW; ++w) key = max(key, W->key[h][w]);
+        }
+        const bool found = key >> 32 != 0ull;
+        const int r = found ? static_cast<int>(~static_cast<unsigned>(key)) : c;
+#pragma unroll
+        for (int e = 0; e < RT; ++e)
+            if (r == tid + 32 * PW * e) {  // the pivot row's thread
+                W->rp[h] = inv[e];
+                rpiv[k0 + c] = inv[e];
+                W->piv[c] = k0 + r;
+                if (!found) atomicOr(flag, 2);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    W->prow[h][j] = v[e][j];
+                    if (c + j < kb) row[e][c + j] = v[e][j];
+                }
+                live[e] = false;
+            }
+        meet();
+        const double rd = W->rp[h];
+        double u[8];
+#pragma unroll
+        for (int j = 1; j < 8; ++j) u[j] = W->prow[h][j];
+#pragma unroll
+        for (int e = 0; e < RT; ++e) {
+            const double l = v[e][0] * rd;
+            if (live[e]) row[e][c] = l;
+#pragma unroll
+            for (int j = 0; j < 7; ++j) v[e][j] = fma(-l, u[j + 1], v[e][j + 1]);
+            v[e][7] = 0.;
+        }
+    }
+    meet();
+    if (warp == 0) {  // the pivot rows' multipliers, and where the rows they displace go
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int r = lane >> 2, c = 2 * (lane & 3) + x;
+            W->lower[8 * r + c] = r < kb && c < r ? Md[W->piv[r] * ld + k0 + c] : 0.;
+        }
+        const int p = lane < kb ? W->piv[lane] : -1;
+        const unsigned out = __ballot_sync(kAll, p >= k0 + kb);                      // columns pivoted from below
+        unsigned stay = __reduce_or_sync(kAll, p >= k0 && p < k0 + kb ? 1u << (p - k0) : 0u);
+        stay = ~stay & ((1u << kb) - 1u);                                            // panel rows displaced
+        if (lane < 8) {
+            int d = -1;
+            if (out >> lane & 1u) d = __fns(stay, 0, __popc(out & ((1u << lane) - 1u)) + 1);
+            W->back[lane] = d;
+        }
+    }
+}
+
+template <int NT, bool SHARED>
+__device__ __forceinline__ void solve_bordered(double* Mg, int off, int ld, int md, double* x, double* rpiv,
+                                               BordScratch* W, int* flag) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int NW = NT / 32, CS = kCondMaxDofs / 32, PW = NW < CS ? NW : CS;
+    double* Md = SHARED ? reinterpret_cast<double*>(smem_raw + off) : Mg;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int fr = lane >> 2, t = lane & 3, t2 = 2 * t;
+#pragma unroll 1
+    for (int k0 = 0; k0 < md; k0 += 8) {
+        const int kb = min(8, md - k0);
+        // up to 64 rows one warp does it without barriers
+        if (md - k0 <= 64) {
+            if (warp == 0) factor_pivoted_panel<1, 2>(Md, ld, md, k0, rpiv, W, flag);
+        } else if (warp < PW) {
+            factor_pivoted_panel<PW, (kCondMaxDofs + 32 * PW - 1) / (32 * PW)>(Md, ld, md, k0, rpiv, W, flag);
+        }
+        __syncthreads();
+        // 2. rows to their places, U = L^-1 A
+#pragma unroll 1
+        for (int j = k0 + tid; j <= md; j += NT) {
+            double a[8], d[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                a[c] = c < kb ? Md[W->piv[c] * ld + j] : 0.;
+                d[c] = c < kb && W->back[c] >= 0 ? Md[(k0 + W->back[c]) * ld + j] : 0.;
+            }
+            if (j >= k0 + kb) {
+#pragma unroll
+                for (int c = 0; c < 7; ++c)
+#pragma unroll
+                    for (int r = c + 1; r < 8; ++r) a[r] = fma(-W->lower[8 * r + c], a[c], a[r]);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (c < kb) Md[(k0 + c) * ld + j] = a[c];
+                if (c < kb && W->back[c] >= 0) Md[W->piv[c] * ld + j] = d[c];
+            }
+        }
+        __syncthreads();
+        // 3. the rest, in equal runs of tiles down the columns
+        const int r0 = k0 + 8;
+        if (r0 < md) {
+            const int ni = (md - r0 + 7) >> 3, nj = (md + 1 - r0 + 7) >> 3, total = ni * nj;
+            const int lo = total * warp / NW, hi = total * (warp + 1) / NW;
+            int j = static_cast<int>(__fdividef(static_cast<float>(lo) + 0.5f, static_cast<float>(ni)));
+            int i = lo - j * ni;
+#pragma unroll 1
+            for (int left = hi - lo; left > 0;) {
+                const int c0 = r0 + 8 * j, cnt = min(ni - i, left), cu = min(c0 + fr, md), cd = c0 + t2;
+                // products in the order of the columns, as the unblocked elimination takes them
+                const double u0 = -Md[(k0 + t) * ld + cu], u1 = -Md[(k0 + 4 + t) * ld + cu];
+#pragma unroll 1
+                for (int e = 0; e < cnt; e += 2) {  // two tiles' loads ahead of their stores
+                    const int ra = r0 + 8 * (i + e) + fr, rb = ra + 8;
+                    const bool two = e + 1 < cnt;
+                    double* pa = Md + min(ra, md - 1) * ld;
+                    double* pb = Md + min(two ? rb : ra, md - 1) * ld;
+                    const int c1 = min(cd, ld - 2);
+                    const double la0 = pa[k0 + t], la1 = pa[k0 + 4 + t], lb0 = pb[k0 + t], lb1 = pb[k0 + 4 + t];
+                    double2 da = load_pair(pa + c1), db = load_pair(pb + c1);
+                    dmma884(da.x, da.y, la0, u0);
+                    if (two) dmma884(db.x, db.y, lb0, u0);
+                    dmma884(da.x, da.y, la1, u1);
+                    if (two) dmma884(db.x, db.y, lb1, u1);
+                    if (ra < md && cd <= md) store_pair(pa + cd, da.x, da.y);
+                    if (two && rb < md && cd <= md) store_pair(pb + cd, db.x, db.y);
+                }
+                left -= cnt;
+                ++j;
+                i = 0;
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 0 && md <= 64) {
+        // Back substitution by rows.  A small system's chain is short either way,
+        // and a moored platform's step is the rounding of 40 m arms to 1e-9 of
+        // its velocities: the sums keep the order that its results had.
+#pragma unroll 1
+        for (int i = md - 1; i >= 0; --i) {
+            double s2 = 0.;
+#pragma unroll 1
+            for (int j = i + 1 + lane; j < md; j += 32) s2 += Md[i * ld + j] * x[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(kAll, s2, o);
+            if (lane == 0) x[i] = (Md[i * ld + md] - s2) / Md[i * ld + i];
+            __syncwarp();
+        }
+    } else if (warp == 0) {  // by columns, the right-hand side in registers
+        double y[CS], u[CS];
+        const double* row[CS];
+#pragma unroll
+        for (int e = 0; e < CS; ++e) {
+            const int i = lane + 32 * e;
+            row[e] = Md + min(i, md - 1) * ld;
+            y[e] = row[e][md];
+            u[e] = i < md - 1 ? row[e][md - 1] : 0.;
+        }
+#pragma unroll 1
+        for (int k = md - 1; k >= 0; --k) {
+            const int ks = k >> 5;
+            double yk = y[0];
+#pragma unroll
+            for (int e = 1; e < CS; ++e) yk = ks == e ? y[e] : yk;
+            const double xk = __shfl_sync(kAll, yk, k & 31) * rpiv[k];
+            if (lane == 0) x[k] = xk;
+#pragma unroll
+            for (int e = 0; e < CS; ++e) {
+                const int i = lane + 32 * e;
+                if (i < k) y[e] = fma(-u[e], xk, y[e]);
+                if (i < k - 1) u[e] = row[e][k - 1];  // for the next column
+            }
+        }
+    }
+    __syncthreads();
+}
+
 template <int NT>
 __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoeffs& P, int record, int* status_out,
                                  int* iters_out, unsigned char* smem_raw) {
@@ -2369,10 +2614,13 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
     int* act = reinterpret_cast<int*>(smem_raw + S.act);
     int* fmap = reinterpret_cast<int*>(smem_raw + S.fmap);
     double* red = reinterpret_cast<double*>(smem_raw + S.red);
+    double* rpiv = reinterpret_cast<double*>(smem_raw + S.rpiv);
+    BordScratch* bord = reinterpret_cast<BordScratch*>(smem_raw + S.bord);
+    const int ldm = bord_ld(md);
     double* xi = cnd ? reinterpret_cast<double*>(smem_raw + S.xi) : nullptr;
     int* imap = cnd ? reinterpret_cast<int*>(smem_raw + S.imap) : nullptr;
     double* bc = cnd ? reinterpret_cast<double*>(smem_raw + S.bc) : nullptr;
-    __shared__ int s_flag, s_nsys, s_piv;
+    __shared__ int s_flag, s_nsys;
     // phase timers (KYN_OPT_PHASE_TIMING): one CTA's clock, thread 0
     __shared__ unsigned long long s_ph[kNumPhases];
     const bool timing = KB.prof != nullptr;
@@ -2502,7 +2750,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                                      timing ? s_ph : nullptr);
         }
         mark(kPhaseIntegrate);
-        for (int k = tid; k < md * md; k += NT) Md[k] = 0.;
+        for (int k = tid; k < md * ldm; k += NT) Md[k] = 0.;
         for (int k = tid; k < md; k += NT) b[k] = 0.;
         if (cnd)
             for (int k = tid; k < md; k += NT) bc[k] = 0.;
@@ -2511,17 +2759,17 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         for (int n = tid; n < N; n += NT)
             add_lumped_terms(n, KB.lumped, KB.n_mass, KB.n_spring, sq, sv, svd, sT, KB.gravity,
                              P.beta_prime, P.gamma_prime, cond, fmap,
-                             [&](int r, int c) -> double& { return Md[r * md + c]; }, resid, 1);
+                             [&](int r, int c) -> double& { return Md[r * ldm + c]; }, resid, 1);
         if (KB.n_comps > 0) {  // beam elements, then their node_FX (summed per node)
             __syncthreads();
-            if (cnd) cond_add_schur<NT>(KB, S, smem_raw, fmap, Md, md, bc);
-            else dense_beam_terms<NT>(KB, P, S, smem_raw, sq, sv, svd, sT, fmap, Md, nd, resid);
+            if (cnd) cond_add_schur<NT>(KB, S, smem_raw, fmap, Md, ldm, bc);
+            else dense_beam_terms<NT>(KB, P, S, smem_raw, sq, sv, svd, sT, fmap, Md, ldm, resid);
             for (int t = tid; t < N * 6; t += NT) resid[t] -= slab[L.fx + t];
         }
         // constraints: residual, gradients and G^T lambda
-        if (tid < nc) {
-            double* cr = con + tid * kConStride;
-            const int t = KB.con_type[tid], tn = KB.con_node[tid], bn = KB.con_base[tid];
+        if (warp == NW - 1 && lane < nc) {  // beside the masses of the first warps
+            double* cr = con + lane * kConStride;
+            const int t = KB.con_type[lane], tn = KB.con_node[lane], bn = KB.con_base[lane];
             if (t >= KYN_CONSTRAINT_FIXED_BC_3DOF) {
                 // three rows (calculate_*_3DOF_constraint.hpp): u2 + X0 - u1 - R1 X0
                 double u1[3] = {0., 0., 0.}, R1[4] = {1., 0., 0., 0.};
@@ -2532,7 +2780,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                     for (int k = 0; k < 3; ++k) u1[k] = sq[bn * 7 + k];
                     for (int k = 0; k < 4; ++k) R1[k] = sq[bn * 7 + 3 + k];
                 }
-                const double* X0 = KB.con_X0[tid];
+                const double* X0 = KB.con_X0[lane];
                 double r1x0[3];
                 for (int i = 0; i < 3; ++i) {
                     r1x0[i] = 0.;
@@ -2551,98 +2799,110 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                             cr[conrec::Btr + i * 3 + j] = bt;
                         }
             } else if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {
-                revolute_dense_record(cr, sq + bn * 7, sq + tn * 7, KB.con_frames + tid * 9, KB.con_X0[tid],
+                revolute_dense_record(cr, sq + bn * 7, sq + tn * 7, KB.con_frames + lane * 9, KB.con_X0[lane],
                                       sT + bn * 9, sT + tn * 9);
             } else {
-                constraint_record(cr, t, sq + tn * 7, KB.con_X0[tid], sT + tn * 9,
+                constraint_record(cr, t, sq + tn * 7, KB.con_X0[lane], sT + tn * 9,
                                   bn >= 0 ? sq + bn * 7 : nullptr, bn >= 0 ? sT + bn * 9 : nullptr,
-                                  KB.con_axis[tid]);
+                                  KB.con_axis[lane]);
+            }
+            if (bn >= 0 && t != KYN_CONSTRAINT_REVOLUTE_JOINT) {  // G_base^T lambda
+                double* gb = cr + conrec::yr;
+                const double* lam = cr + conrec::lam;
+                for (int k = 0; k < 6; ++k) gb[k] = 0.;
+                if (constraint_rows(t) == 3) {
+                    for (int i = 0; i < 3; ++i) {
+                        gb[i] = -lam[i];
+                        for (int k = 0; k < 3; ++k) gb[3 + i] += tilde_e(cr + conrec::R1X0, k, i) * lam[k];
+                    }
+                } else {
+                    joint_base_transpose_add(cr, lam, gb);
+                }
             }
         }
         __syncthreads();
         // scatter: rows of B = G T, columns G^T, residuals (assemble_constraints_matrix.hpp,
         // assemble_constraints_residual.hpp, assemble_system_residual.hpp)
-        if (tid == 0) {
+        // One thread per constraint: its rows and columns of Md are its own.  The
+        // nodes' forces, which constraints share, are summed per component in
+        // the order of the constraints by six lanes of another warp.
+        if (tid < nc) {
+            const int c = tid;
             int rf = nsys;
-            for (int c = 0; c < nc; ++c) {
-                const double* cr = con + c * kConStride;
-                const int t = KB.con_type[c], tn = KB.con_node[c], bn = KB.con_base[c];
-                const int rows = constraint_rows(t);
-                const int ft = fmap[tn];
-                if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {  // five rows, gradients on both nodes
-                    const int fb = fmap[bn];
-                    for (int r = 0; r < 5; ++r) {
-                        double* row = Md + (rf + r) * md;
-                        if (r < 3) {
-                            row[ft + r] += 1.;
-                            Md[(ft + r) * md + rf + r] += 1.;
-                            row[fb + r] -= 1.;
-                            Md[(fb + r) * md + rf + r] -= 1.;
-                        } else {
-                            const double* v = cr + (r == 3 ? drev::xcz : drev::xcy);
-                            for (int j = 0; j < 3; ++j) {
-                                row[ft + 3 + j] += cr[drev::Bt + (r - 3) * 3 + j];
-                                row[fb + 3 + j] += cr[drev::Bb + (r - 3) * 3 + j];
-                                Md[(ft + 3 + j) * md + rf + r] -= v[j];
-                                Md[(fb + 3 + j) * md + rf + r] += v[j];
-                            }
-                        }
-                        b[rf + r] += cr[drev::Phi + r];
-                    }
-                    for (int e = 0; e < 6; ++e) {
-                        b[ft + e] += cr[drev::GtL + e] + (e >= 3 ? cr[drev::sys + e - 3] : 0.);
-                        b[fb + e] += cr[drev::GbL + e];
-                    }
-                    rf += 5;
-                    continue;
-                }
-                for (int r = 0; r < rows; ++r) {
-                    double* row = Md + (rf + r) * md;
+            for (int e = 0; e < c; ++e) rf += constraint_rows(KB.con_type[e]);
+            const double* cr = con + c * kConStride;
+            const int t = KB.con_type[c], bn = KB.con_base[c];
+            const int rows = constraint_rows(t), ft = fmap[KB.con_node[c]];
+            if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {  // five rows, gradients on both nodes
+                const int fb = fmap[bn];
+#pragma unroll 1
+                for (int r = 0; r < 5; ++r) {
+                    double* row = Md + (rf + r) * ldm;
                     if (r < 3) {
                         row[ft + r] += 1.;
-                        Md[(ft + r) * md + rf + r] += 1.;
+                        Md[(ft + r) * ldm + rf + r] += 1.;
+                        row[fb + r] -= 1.;
+                        Md[(fb + r) * ldm + rf + r] -= 1.;
+                    } else {
+                        const double* v = cr + (r == 3 ? drev::xcz : drev::xcy);
+                        for (int j = 0; j < 3; ++j) {
+                            row[ft + 3 + j] += cr[drev::Bt + (r - 3) * 3 + j];
+                            row[fb + 3 + j] += cr[drev::Bb + (r - 3) * 3 + j];
+                            Md[(ft + 3 + j) * ldm + rf + r] -= v[j];
+                            Md[(fb + 3 + j) * ldm + rf + r] += v[j];
+                        }
+                    }
+                    b[rf + r] += cr[drev::Phi + r];
+                }
+            } else {
+#pragma unroll 1
+                for (int r = 0; r < rows; ++r) {
+                    double* row = Md + (rf + r) * ldm;
+                    if (r < 3) {
+                        row[ft + r] += 1.;
+                        Md[(ft + r) * ldm + rf + r] += 1.;
                     } else {
                         for (int j = 0; j < 3; ++j) {
                             row[ft + 3 + j] += cr[conrec::Brot + (r - 3) * 3 + j];
-                            Md[(ft + 3 + j) * md + rf + r] += cr[conrec::AX + j * 3 + (r - 3)];
+                            Md[(ft + 3 + j) * ldm + rf + r] += cr[conrec::AX + j * 3 + (r - 3)];
                         }
                     }
                     b[rf + r] += cr[conrec::Phi + r];
                 }
-                for (int e = 0; e < (rows == 3 ? 3 : 6); ++e) b[ft + e] += cr[conrec::Gl + e];
                 if (bn >= 0) {  // joint base blocks: B_b = [-I, Btr; 0, Brr], G_b = [-I, tilde; 0, -AX]
                     const int fb = fmap[bn];
-                    const double* r1x0 = cr + conrec::R1X0;
+#pragma unroll 1
                     for (int r = 0; r < rows; ++r) {
-                        double* row = Md + (rf + r) * md;
+                        double* row = Md + (rf + r) * ldm;
                         if (r < 3) {
                             row[fb + r] -= 1.;
-                            Md[(fb + r) * md + rf + r] -= 1.;
+                            Md[(fb + r) * ldm + rf + r] -= 1.;
                             for (int j = 0; j < 3; ++j) {
                                 row[fb + 3 + j] += cr[conrec::Btr + r * 3 + j];
-                                Md[(fb + 3 + j) * md + rf + r] += tilde_e(r1x0, r, j);
+                                Md[(fb + 3 + j) * ldm + rf + r] += tilde_e(cr + conrec::R1X0, r, j);
                             }
                         } else {
                             for (int j = 0; j < 3; ++j) {
                                 row[fb + 3 + j] += cr[conrec::Brr + (r - 3) * 3 + j];
-                                Md[(fb + 3 + j) * md + rf + r] -= cr[conrec::AX + (r - 3) * 3 + j];
+                                Md[(fb + 3 + j) * ldm + rf + r] -= cr[conrec::AX + (r - 3) * 3 + j];
                             }
                         }
                     }
-                    double gb[6] = {0., 0., 0., 0., 0., 0.};
-                    double lam6[6] = {0., 0., 0., 0., 0., 0.};
-                    for (int k = 0; k < rows; ++k) lam6[k] = cr[conrec::lam + k];
-                    if (rows == 3) {
-                        for (int i = 0; i < 3; ++i) {
-                            gb[i] = -lam6[i];
-                            for (int k = 0; k < 3; ++k) gb[3 + i] += tilde_e(r1x0, k, i) * lam6[k];
-                        }
-                    } else {
-                        joint_base_transpose_add(cr, lam6, gb);
-                    }
-                    for (int e = 0; e < 6; ++e) b[fb + e] += gb[e];
                 }
-                rf += rows;
+            }
+        } else if (warp == 1 && lane < 6) {
+            const int e = lane;
+#pragma unroll 1
+            for (int c = 0; c < nc; ++c) {
+                const double* cr = con + c * kConStride;
+                const int t = KB.con_type[c], bn = KB.con_base[c], ft = fmap[KB.con_node[c]];
+                if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {
+                    b[ft + e] += cr[drev::GtL + e] + (e >= 3 ? cr[drev::sys + e - 3] : 0.);
+                    b[fmap[bn] + e] += cr[drev::GbL + e];
+                } else {
+                    if (e < (constraint_rows(t) == 3 ? 3 : 6)) b[ft + e] += cr[conrec::Gl + e];
+                    if (bn >= 0) b[fmap[bn] + e] += cr[conrec::yr + e];
+                }
             }
         }
         __syncthreads();
@@ -2651,76 +2911,14 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
             if (fmap[n] >= 0)
                 for (int c = 0; c < act[n]; ++c) b[fmap[n] + c] += resid[n * 6 + c] - slab[L.f + n * 6 + c];
         __syncthreads();
-        for (int k = tid; k < md; k += NT) b[k] = -(k < nsys ? b[k] * cond : b[k]) + (cnd ? bc[k] : 0.);
+        for (int k = tid; k < md; k += NT)
+            Md[k * ldm + md] = -(k < nsys ? b[k] * cond : b[k]) + (cnd ? bc[k] : 0.);
         __syncthreads();
         mark(kPhaseConstraints);
-        // LU with partial pivoting, in place (the oracle's dense solve)
-        for (int k = 0; k < md; ++k) {
-            if (warp == 0) {
-                double best = -1.;
-                int p = k;
-                for (int i = k + lane; i < md; i += 32) {
-                    const double v = fabs(Md[i * md + k]);
-                    if (v > best) {
-                        best = v;
-                        p = i;
-                    }
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int op = __shfl_xor_sync(0xffffffffu, p, o);
-                    if (ob > best || (ob == best && op < p)) {
-                        best = ob;
-                        p = op;
-                    }
-                }
-                if (lane == 0) {
-                    s_piv = p;
-                    if (!(best > 0.)) s_flag |= 2;
-                }
-            }
-            __syncthreads();
-            const int p = s_piv;
-            if (p != k) {
-                for (int j = tid; j < md; j += NT) {
-                    const double t0 = Md[k * md + j];
-                    Md[k * md + j] = Md[p * md + j];
-                    Md[p * md + j] = t0;
-                }
-                if (tid == 0) {
-                    const double t0 = b[k];
-                    b[k] = b[p];
-                    b[p] = t0;
-                }
-            }
-            __syncthreads();
-            // rows below the pivot over the warps, their columns over the lanes;
-            // each row's warp forms its multiplier (times the pivot's reciprocal),
-            // updates the row and the right-hand side, then stores the multiplier
-            // (no other warp reads it)
-            const double rd = 1. / Md[k * md + k];
-            for (int i = k + 1 + warp; i < md; i += NW) {
-                const double l = Md[i * md + k] * rd;
-                for (int j = k + 1 + lane; j < md; j += 32) Md[i * md + j] -= l * Md[k * md + j];
-                __syncwarp();
-                if (lane == 0) {
-                    Md[i * md + k] = l;
-                    b[i] -= l * b[k];
-                }
-            }
-            __syncthreads();
-        }
+        // (apart, so that the shared system is read by shared-memory loads)
+        if (KB.cond_md) solve_bordered<NT, false>(KB.cond_md, 0, ldm, md, x, rpiv, bord, &s_flag);
+        else solve_bordered<NT, true>(nullptr, S.M, ldm, md, x, rpiv, bord, &s_flag);
         mark(kPhaseFactor);
-        if (warp == 0) {  // back substitution
-            for (int i = md - 1; i >= 0; --i) {
-                double s2 = 0.;
-                for (int j = i + 1 + lane; j < md; j += 32) s2 += Md[i * md + j] * x[j];
-                for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                if (lane == 0) x[i] = (b[i] - s2) / Md[i * md + i];
-                __syncwarp();
-            }
-        }
-        __syncthreads();
         // multipliers unconditioned; convergence error (calculate_convergence_error.hpp)
         for (int k = nsys + tid; k < md; k += NT) x[k] /= cond;
         __syncthreads();
