@@ -350,8 +350,8 @@ ClassKey class_key(const HostModel& h, int precision) {
 }
 
 // Dynamic shared memory of a dense model's CTA.
-int dense_smem(const HostModel& H, const HostBeam& hb, int nt) {
-    return make_dense_smem(hb.N, H.ndofs, nt, hb.comp_maxN, hb.comp_maxQ, hb.cond_nd, hb.cond_md_off >= 0).bytes;
+int dense_smem(const HostModel& H, const HostBeam& hb) {
+    return make_dense_smem(hb.N, H.ndofs, hb.comp_maxN, hb.comp_maxQ, hb.cond_nd, hb.cond_md_off >= 0).bytes;
 }
 
 // Fills the per-model values that plans and transfer plans reuse.
@@ -373,18 +373,11 @@ void prepare_model(DevModel* m) {
         bool b0 = true;  // first beam
         for (const HostBeam& hb : H.beams) {
             if (hb.dense) {  // the dense bordered system, FP64 in both forms
-                for (int k = 0; k < 3; ++k)
-                    m->smem_nt[f][k] = std::max(
-                        m->smem_nt[f][k],
-                        dense_smem(H, hb, 128 << k));
-                // 128 threads, or for a condensed model (elements assembled and
-                // eliminated one after the other in one CTA) the most that fit
-                if (hb.cond_nd > 0)
-                    for (int nt : {512, 256})
-                        if (dense_smem(H, hb, nt) <= kMaxDynSmem) {
-                            m->def_nt[f] = nt;
-                            break;
-                        }
+                for (int k = 0; k < 3; ++k) m->smem_nt[f][k] = std::max(m->smem_nt[f][k], dense_smem(H, hb));
+                // 128 threads; 256 for a condensed model (elements assembled and
+                // eliminated one after the other in one CTA): with 512, whose 128
+                // registers spill, a turbine's iteration took 636k cycles for 545k
+                if (hb.cond_nd > 0) m->def_nt[f] = 256;
                 continue;
             }
             m->def_nt[f] = std::max(m->def_nt[f], beam_threads(hb.N, hb.Q, hb.nc, rb, hubf));
@@ -1039,13 +1032,13 @@ int kyn_model_create(kyn_ctx* c, const kyn_model_desc* desc) {
     for (auto& b : m->host.beams) {
         const int hubf = hub_kind(m->host);
         const int nt = b.dense ? 128 : beam_threads(b.N, b.Q, b.nc, sizeof(double), hubf);
-        if (b.cond_nd > 0 && dense_smem(m->host, b, nt) > kMaxDynSmem) {
+        if (b.cond_nd > 0 && dense_smem(m->host, b) > kMaxDynSmem) {
             // the condensed model's bordered system moves to device memory (the slab's tail)
             if (b.slab.size() & 1) b.slab.push_back(0.);
             b.cond_md_off = static_cast<int>(b.slab.size());
             b.slab.resize(b.slab.size() + static_cast<size_t>(b.cond_nd) * bord_ld(b.cond_nd), 0.);
         }
-        const int sm = b.dense ? dense_smem(m->host, b, nt)
+        const int sm = b.dense ? dense_smem(m->host, b)
                                : std::max(beam_smem(b.N, b.Q, b.nc, sizeof(double), 512, hubf),
                                           beam_smem(b.N, b.Q, b.nc, sizeof(double), nt, hubf));
         if (sm > kMaxDynSmem)
@@ -1893,7 +1886,7 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
         for (int nt : {128, 256, 512}) {
             bool fits = true;
             for (const HostBeam& b : h.beams)
-                fits &= (b.dense ? dense_smem(h, b, nt)
+                fits &= (b.dense ? dense_smem(h, b)
                                  : beam_smem(b.N, b.Q, b.nc, rb, nt, hub_kind(h))) <= kMaxDynSmem;
             if (!fits || (key.beams > 1 && key.beams * nt > 1024 * 8)) continue;
             for (int sv : {c->solver, other}) {

@@ -513,12 +513,10 @@ int build_host_model(const kyn_model_desc* d, HostModel& M, std::string& err) {
             body.insert(body.end(), cb.slab.begin(), cb.slab.end());
             if (body.size() & 1) body.push_back(0.);
         }
-        if (B.cond_nd > 0)  // condensation workspaces [6Nc][6Nc + 1]
+        if (B.cond_nd > 0)  // condensation workspaces
             for (size_t ci = 0; ci < comps.size(); ++ci) {
-                const int mc = 6 * comps[ci].N;
                 head[ci * kCompHead + kCompWork] = static_cast<double>(at + body.size());
-                body.insert(body.end(), static_cast<size_t>(mc) * (mc + 1), 0.);
-                if (body.size() & 1) body.push_back(0.);
+                body.insert(body.end(), static_cast<size_t>(cond_rows(comps[ci].N)) * cond_ld(comps[ci].N, false), 0.);
             }
         head.resize(at, 0.);
         B.slab.insert(B.slab.end(), head.begin(), head.end());

@@ -626,10 +626,14 @@ __device__ __forceinline__ void normalise_tile(TR* A, int ldA, int m, int k0, in
     }
 }
 
-// Eliminates the free block A[0:m][0:m] with its right-hand sides in columns
-// m .. m + nrhs - 1 of a system with leading dimension ldA (a multiple of 8 no
-// smaller than the tiles' extent; columns past the right-hand sides are
-// scratch).  dinv: the inverses of the diagonal blocks, 64 doubles each.
+// Eliminates the leading m unknowns of a system with leading dimension ldA (a
+// multiple of 8 no smaller than the tiles' extent): nrt row tiles, of which the
+// first ceil(m / 8) hold the m pivots (rows from m on are not touched where
+// those are all), and nct column tiles with the right-hand sides behind the
+// unknowns (columns past them are scratch).  With more row tiles than pivots m
+// is a multiple of 8 and the rows below are left with the Schur complement.
+// The pivot rows end as U = D^-1 A.  dinv: the inverses of the diagonal blocks,
+// 64 doubles each.
 //
 // Warp 0 runs the serial chain (the next panel's diagonal block: update,
 // inversion) while the other warps share the trailing tiles of panel k and the
@@ -640,27 +644,29 @@ __device__ __forceinline__ void normalise_tile(TR* A, int ldA, int m, int k0, in
 // 13-node beam and 102k of 187k on a 21-node beam, two thirds of them in warp
 // 0's chain.
 template <typename TR, int NT>
-__device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int nrhs, double* dinv, int* flag) {
+__device__ __forceinline__ void eliminate_blocks(TR* A, int ldA, int m, int nrt, int nct, double* dinv, int* flag) {
     constexpr int NWK = NT / 32 - 1;  // warps on the trailing tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nb = (m + 7) >> 3, nct = (m + nrhs + 7) >> 3;
+    const int nb = (m + 7) >> 3;
+    const bool schur = nrt > nb;
     const int fr = lane >> 2, fc = (2 * (lane & 3)) ^ (fr & 6);
-    const bool past = 8 * (nb - 1) + fr >= m;  // the lane's row of the last row tile
+    const bool past = !schur && 8 * (nb - 1) + fr >= m;  // the lane's row of the last row tile
     if (warp == 0) factor_diag_block(A, ldA, m, 0, dinv, dinv, lane, flag);
     __syncthreads();
 #pragma unroll 1
-    for (int k = 0; k + 1 < nb; ++k) {
+    for (int k = 0; k + (schur ? 0 : 1) < nb; ++k) {
         const int k0 = 8 * k;
+        const int next = k + 1 < nb ? 1 : 0;
         if (warp == 0) {
-            factor_diag_block(A, ldA, m, k0 + 8, dinv + 64 * k, dinv + 64 * (k + 1), lane, flag);
+            if (next) factor_diag_block(A, ldA, m, k0 + 8, dinv + 64 * k, dinv + 64 * (k + 1), lane, flag);
         } else {
             // equal runs down the columns of the trailing tiles without the first
             // (warp 0's), then of the tiles of the panel before
-            const int ni = nb - k - 1, total = ni * (nct - k - 1) - 1, both = total + (k > 0 ? nct - k : 0);
+            const int ni = nrt - k - 1, total = ni * (nct - k - 1) - next, both = total + (k > 0 ? nct - k : 0);
             const int lo = both * (warp - 1) / NWK, hi = both * warp / NWK;
             const double2 dk = load_pair(dinv + 64 * k + 2 * lane);
-            int j = static_cast<int>(__fdividef(static_cast<float>(lo) + 1.5f, static_cast<float>(ni)));
-            int i = lo + 1 - j * ni;
+            int j = static_cast<int>(__fdividef(static_cast<float>(lo + next) + 0.5f, static_cast<float>(ni)));
+            int i = lo + next - j * ni;
 #pragma unroll 1
             for (int left = min(hi, total) - lo; left > 0;) {
                 const int c0 = 8 * (k + 1 + j), cnt = min(ni - i, left);
@@ -693,16 +699,17 @@ __device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int 
         }
         __syncthreads();
     }
-    // the last two panels' rows (the last one: its right-hand sides only)
-    const int u0 = nb - 1 + warp;
-    if (nb > 1 && u0 < nct) normalise_tile(A, ldA, m, 8 * (nb - 2), 8 * u0, dinv + 64 * (nb - 2), lane);
-    if (warp == NT / 32 - 1)
-        normalise_tile(A, ldA, m, 8 * (nb - 1), 8 * (nct - 1), dinv + 64 * (nb - 1), lane);
+    // the panels whose rows are still A: the last but one (none below a Schur
+    // complement) and the last, where the columns behind the pivots count
+    const int n2 = !schur && nb > 1 ? nct - nb + 1 : 0, n1 = schur ? nct - nb : 1;
+    if (warp < n2) normalise_tile(A, ldA, m, 8 * (nb - 2), 8 * (nb - 1 + warp), dinv + 64 * (nb - 2), lane);
+    else if (warp < n2 + n1)
+        normalise_tile(A, ldA, m, 8 * (nb - 1), 8 * (nct - n1 + warp - n2), dinv + 64 * (nb - 1), lane);
     __syncthreads();
 }
 
-// Back substitution x_k = y_k - sum_{j>k} U_kj x_j by the CTA, y in column rhs
-// of A, x to xs[0:m], two blocks of rows per step and barrier.  Warp 0 finds the
+// Back substitution x_k = y_k - sum_{j>k} U_kj x_j by the CTA, y in xs[0:m] on
+// entry (a barrier behind its last write) and x on exit, two blocks of rows per step and barrier.  Warp 0 finds the
 // two blocks' x (the pair found before still to be subtracted, then the lower
 // block's from the upper rows), while the other warps subtract the pair found
 // before from all rows above.  All products run on the tensor cores with x
@@ -711,15 +718,12 @@ __device__ __forceinline__ void eliminate_free_block(TR* A, int ldA, int m, int 
 // cycles a block (9.3k at 13 nodes, 14.4k at 21): the sums over the older blocks
 // were on its path.
 template <typename TR, int NT>
-__device__ __forceinline__ void back_substitute(const TR* A, int ldA, int m, int rhs, double* xs) {
+__device__ __forceinline__ void back_substitute(const TR* A, int ldA, int m, double* xs) {
     constexpr unsigned kAll = 0xffffffffu;
     constexpr int NW = NT / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (m + 7) >> 3;
     const int fr = lane >> 2, t2 = 2 * (lane & 3), col = t2 ^ (fr & 6);
-#pragma unroll 1
-    for (int i = threadIdx.x; i < m; i += NT) xs[i] = static_cast<double>(A[sys_at(ldA, i, rhs)]);
-    __syncthreads();
     auto tile = [&](int i, int b) {  // the lane's pair of -U_ib; columns past m count as zero
         const double2 a = load_pair(A + (8 * i + fr) * ldA + 8 * b + col);
         const bool in = 8 * b + t2 < m;
@@ -1495,31 +1499,30 @@ __device__ void add_lumped_terms(int n, const double* __restrict__ rec, int n_ma
 // in both precision forms: these systems have at most kDenseModelMaxDofs unknowns.
 
 struct DenseSmem {
-    int M, b, x, q, qp, v, vd, a, qd, T, resid, con, act, fmap, red, rpiv, bord;
+    int M, b, x, q, qp, v, vd, a, qd, T, resid, con, act, fmap, red, bord;
     // beam components (dense models with beams): shape tables, weights and
     // node state of one component at a time, its quadrature-point outputs and
     // the interpolated values
     int cphi, cdphi, cdphiJ, cqpw, cq, cv, cvd, cG, cFc, cFd, cgs;
     // condensed models: interior solution [6N], interior DOF map [N], the
-    // bordered system's right-hand-side corrections [nd], one component's
-    // local order (position of each local node, node at each position [32
-    // each]) and its solution [6 cN]; M is -1 when the bordered system lives
-    // in device memory (KBeam::cond_md)
-    int xi, imap, bc, lpos, lnode, cx;
+    // bordered system's right-hand-side corrections [nd], the components'
+    // orders (CompOrder) and one component's solution; M is -1 when the
+    // bordered system lives in device memory (KBeam::cond_md)
+    int xi, imap, bc, order, cx;
     int cW;  // condensed models: one component's system (inside M's region when M is shared)
-    int cR;  // condensed models: bytes of that region
+    int chunk;  // condensed models: quadrature points per pass of a component's assembly,
+    bool tight;  // and whether its rows are as short as whole tiles allow (cond_ld)
     int bytes;
 };
 // Row length of a bordered system of nd unknowns: the right-hand side is column
 // nd, rows of even length.
 KYN_HD inline int bord_ld(int nd) { return (nd + 2) & ~1; }
-// Quadrature points per pass of a condensed component's assembly.
-constexpr int kCondChunk = 16;
-// nt, cN, cQ: threads per CTA and the largest beam component (0: none);
+constexpr int kBordScratch = 1024;  // bytes of a BordScratch
+// cN, cQ: nodes and points of the largest beam component (0: none);
 // cond_nd > 0: a condensed model whose bordered system has cond_nd unknowns
 // (md_global: kept in device memory instead of shared memory).
-__host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128, int cN = 0, int cQ = 0,
-                                                     int cond_nd = 0, bool md_global = false) {
+__host__ __device__ inline DenseSmem plan_dense_smem(int N, int nd, int cN, int cQ, int cond_nd,
+                                                     bool md_global, int chunk, bool tight) {
     DenseSmem S{};
     int o = 0;
     auto take = [&](int bytes) {
@@ -1529,21 +1532,21 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     };
     if (cond_nd > 0) nd = cond_nd;
     // condensed models: the bordered system's region also holds, before the
-    // system is assembled, one component's system [6cN][6cN + 1], the G rows
-    // of one chunk of its quadrature points, the quadrature phase's group
-    // scratch and the component's tables and node state (cond_tables)
+    // system is assembled, one component's system [cond_rows][cond_ld], G and
+    // the interpolated values of one chunk of its quadrature points (then the
+    // inverse diagonal blocks, of which eight points hold twenty), and the
+    // component's tables and node state
     auto r16 = [](int b) { return (b + 15) & ~15; };
-    const int w_bytes = cond_nd > 0 ? r16(cN * 6 * (cN * 6 + 1) * 8) : 0;
-    const int g_bytes = cond_nd > 0 ? kCondChunk * kGPoint * 8 : 0;
-    const int s_bytes = cond_nd > 0 ? kCondChunk * kQpInterp * 8 : 0;
+    const int w_bytes = cond_nd > 0 ? cond_rows(cN) * cond_ld(cN, tight) * 8 : 0;
     const int t_bytes = cond_nd > 0 ? 3 * r16(cQ * cN * 8) + r16(cQ * 4 * 8) + r16(cN * 7 * 8) +
                                           2 * r16(cN * 6 * 8) + 2 * r16(cQ * 6 * 8) : 0;
-    const int c_bytes = w_bytes + g_bytes + s_bytes + t_bytes;
+    const int c_bytes = cond_nd > 0 ? w_bytes + chunk * (kGPoint + kQpInterp) * 8 + t_bytes : 0;
     const int m_bytes = md_global ? 0 : nd * bord_ld(nd) * 8;
+    S.chunk = chunk;
+    S.tight = tight;
     const int region = take(m_bytes > c_bytes ? m_bytes : c_bytes);
     S.M = md_global ? -1 : region;
     S.cW = cond_nd > 0 ? region : -1;
-    S.cR = cond_nd > 0 ? (m_bytes > c_bytes ? m_bytes : c_bytes) : 0;
     S.b = take(nd * 8);
     S.x = take(nd * 8);
     S.q = take(N * 7 * 8);
@@ -1558,8 +1561,7 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
     S.act = take(N * 4);
     S.fmap = take(N * 4);
     S.red = take(64 * 8);  // per-warp partial sums of the error
-    S.rpiv = take(nd * 8);      // reciprocal pivots of the bordered system
-    S.bord = take(1024);        // BordScratch
+    S.bord = take(kBordScratch);
     S.cphi = S.cdphi = S.cdphiJ = S.cqpw = S.cq = S.cv = S.cvd = S.cG = S.cFc = S.cFd = S.cgs = -1;
     if (cN > 0 && cond_nd > 0) {  // inside the bordered system's region, after the component's system
         int t = region + w_bytes;
@@ -1568,8 +1570,8 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
             t += r16(bytes);
             return r;
         };
-        S.cG = at(g_bytes);
-        S.cgs = at(s_bytes);
+        S.cG = at(S.chunk * kGPoint * 8);
+        S.cgs = at(S.chunk * kQpInterp * 8);
         S.cphi = at(cQ * cN * 8);
         S.cdphi = at(cQ * cN * 8);
         S.cdphiJ = at(cQ * cN * 8);
@@ -1592,16 +1594,25 @@ __host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int nt = 128
         S.cFd = take(cQ * 6 * 8);
         S.cgs = take(cQ * kQpInterp * 8);
     }
-    S.xi = S.imap = S.bc = S.lpos = S.lnode = S.cx = -1;
+    S.xi = S.imap = S.bc = S.order = S.cx = -1;
     if (cond_nd > 0) {
         S.xi = take(N * 6 * 8);
         S.imap = take(N * 4);
         S.bc = take(nd * 8);
-        S.lpos = take(32 * 4);
-        S.lnode = take(32 * 4);
-        S.cx = take(cN * 6 * 8);
+        S.order = take(kMaxDenseComps * 164);
+        S.cx = take((cN * 6 + 8) * 8);
     }
     S.bytes = o;
+    return S;
+}
+// A condensed component's points are taken in one pass with the rows of its
+// system on different banks where that fits, otherwise in smaller passes, at
+// last with the rows packed.
+__host__ __device__ inline DenseSmem make_dense_smem(int N, int nd, int cN = 0, int cQ = 0, int cond_nd = 0,
+                                                     bool md_global = false) {
+    DenseSmem S = plan_dense_smem(N, nd, cN, cQ, cond_nd, md_global, cQ > 8 ? cQ : 8, false);
+    for (int chunk = 16; cond_nd > 0 && S.bytes > kMaxDynSmem && chunk >= 4; chunk /= 2)
+        S = plan_dense_smem(N, nd, cN, cQ, cond_nd, md_global, chunk < 8 ? 8 : chunk, chunk < 8);
     return S;
 }
 
@@ -2044,47 +2055,68 @@ __device__ inline void revolute_dense_record(double* cr, const double* bq, const
     }
 }
 
-// ---- condensed beam components of a dense model (KBeam::cond_nd > 0) -------------
-// A component's local order: its interior nodes first (fmap < 0: nodes of this
-// component only, without masses, springs or constraints), then its boundary
-// nodes; lpos[k] = position of local node k, lnode[p] = local node at p.
-// Returns the number of interior nodes.
+// A component's place in shared memory, worked out once per step: its nodes in
+// the model, and their order in the component's own system, interior nodes
+// first.  That system has its interior unknowns padded to a multiple of eight
+// (ones on the diagonal), then the boundary unknowns, then the right-hand side:
+// whole tiles for eliminate_blocks.
+struct CompOrder {
+    short node[32];        // model node of each local node
+    short row[32];         // first row of each local node
+    unsigned char at[32];  // local node at each place (interior first)
+    short ni, nb;          // interior and boundary nodes
+};
+static_assert(sizeof(CompOrder) == 164, "DenseSmem::order");
+__device__ __forceinline__ int comp_pivots(const CompOrder& C) { return (6 * C.ni + 7) & ~7; }
+
+// One warp per component.
 template <int NT>
-__device__ int cond_local_order(const double* node, int N, const int* fmap, int* lpos, int* lnode) {
-    if (threadIdx.x == 0) {
-        int o = 0;
-        for (int pass = 0; pass < 2; ++pass)
-            for (int k = 0; k < N; ++k)
-                if ((fmap[static_cast<int>(node[k])] < 0) == (pass == 0)) {
-                    lpos[k] = o;
-                    lnode[o] = k;
-                    ++o;
-                }
+__device__ __forceinline__ void cond_order(const KBeam& KB, const int* fmap, CompOrder* order) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int ci = warp; ci < KB.n_comps; ci += NT / 32) {
+        const double* hd = KB.comps + ci * kCompHead;
+        const int N = static_cast<int>(hd[1]);
+        CompOrder& C = order[ci];
+        const int node = lane < N ? static_cast<int>(hd[3 + lane]) : 0;
+        const bool inner = lane < N && fmap[node] < 0;
+        const unsigned in = __ballot_sync(kAll, inner), out = __ballot_sync(kAll, lane < N && !inner);
+        const unsigned below = (1u << lane) - 1u;
+        const int ni = __popc(in), place = inner ? __popc(in & below) : ni + __popc(out & below);
+        if (lane < N) {
+            C.node[lane] = static_cast<short>(node);
+            C.row[lane] = static_cast<short>(6 * place + (inner ? 0 : ((6 * ni + 7) & ~7) - 6 * ni));
+            C.at[place] = static_cast<unsigned char>(lane);
+        }
+        if (lane == 0) {
+            C.ni = static_cast<short>(ni);
+            C.nb = static_cast<short>(__popc(out));
+        }
     }
-    int ni = 0;
-    for (int k = 0; k < N; ++k) ni += fmap[static_cast<int>(node[k])] < 0;
-    __syncthreads();
-    return ni;
 }
 
 // Each component's system over its own local nodes, with the element terms of
-// dense_beam_terms (residual, S_ij T_j + I_ij times the conditioner) taken
-// kCondChunk quadrature points at a time.  The interior rows carry their
-// complete right-hand side -conditioner (R - node_FX - f); the boundary
-// nodes' residual goes to resid like the other nodes of the bordered system.
-// Unpivoted elimination of the interior rows (the beam systems' LU) leaves in
-// the boundary rows the Schur complement A_bb - A_bi A_ii^-1 A_ib and the
-// right-hand-side correction -A_bi A_ii^-1 b_i.  The eliminated system is
-// saved to the component's workspace for cond_add_schur and
-// cond_back_substitute.  This is the static condensation of the element
-// groups that the reference's sparse direct solve factors as one matrix
-// (src/solver/compute_system_row_entries.hpp:83-97 gives their overlap).
+// dense_beam_terms (residual, S_ij T_j + I_ij times the conditioner), S.chunk
+// quadrature points at a time.  The interior rows carry their complete
+// right-hand side -conditioner (R - node_FX - f); the boundary nodes' residual
+// goes to resid like the other nodes of the bordered system.  The beam systems'
+// block elimination of the interior rows leaves in the boundary rows the Schur
+// complement A_bb - A_bi A_ii^-1 A_ib and the right-hand-side correction
+// -A_bi A_ii^-1 b_i, and U = D^-1 A in the interior rows.  The eliminated system
+// is saved to the component's workspace for cond_add_schur and
+// cond_back_substitute.  This is the static condensation of the element groups
+// that the reference's sparse direct solve factors as one matrix
+// (src/solver/compute_system_row_entries.hpp:83-97 gives their overlap).  Bound
+// by latency with eight warps on the SM: per iteration of a turbine (four
+// components of 11 nodes) the points take 43k cycles, the assembly 73k, the
+// elimination 42k.  One pivot per barrier with a row update per warp took 332k,
+// and node by node lookups in device memory with sixteen points a pass 190k.
 template <int NT>
-__device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const DenseSmem& S,
-                                     unsigned char* smem_raw, const double* sq, const double* sv,
-                                     const double* svd, const double* sT, const int* fmap,
-                                     const double* mslab, const SlabLayout& ML, double* resid, int* flag,
-                                     unsigned long long* ph = nullptr) {
+__device__ __forceinline__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const DenseSmem& S,
+                                                     const double* sq, const double* sv, const double* svd,
+                                                     const double* sT, const double* mslab, const SlabLayout& ML,
+                                                     double* resid, int* flag, unsigned long long* ph = nullptr) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x;
     // optional sub-phase timers (thread 0): quadrature physics, assembly,
     // elimination, save, in the slots kPhaseQuadrature, kPhaseLUDiag,
@@ -2107,97 +2139,97 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
     double* G = reinterpret_cast<double*>(smem_raw + S.cG);
     double* Fc = reinterpret_cast<double*>(smem_raw + S.cFc);
     double* Fd = reinterpret_cast<double*>(smem_raw + S.cFd);
-    double* gscr = reinterpret_cast<double*>(smem_raw + S.cgs);
+    double* itp = reinterpret_cast<double*>(smem_raw + S.cgs);
     double* W = reinterpret_cast<double*>(smem_raw + S.cW);
-    int* lpos = reinterpret_cast<int*>(smem_raw + S.lpos);
-    int* lnode = reinterpret_cast<int*>(smem_raw + S.lnode);
+    const CompOrder* order = reinterpret_cast<const CompOrder*>(smem_raw + S.order);
     const double cond = P.conditioner;
+#pragma unroll 1
     for (int ci = 0; ci < KB.n_comps; ++ci) {
         const double* hd = KB.comps + ci * kCompHead;
         const double* cs = KB.comps + static_cast<long>(hd[0]);
         double* work = const_cast<double*>(KB.comps) + static_cast<long>(hd[kCompWork]);
         const int N = static_cast<int>(hd[1]), Q = static_cast<int>(hd[2]);
-        const double* node = hd + 3;
+        const CompOrder& C = order[ci];
         const SlabLayout L = make_slab_layout(N, Q);
-        const int mc = 6 * N, ldw = mc + 1;
+        const int mi = 6 * C.ni, mp = comp_pivots(C), rhs = mp + 6 * C.nb;
+        const int rows = (rhs + 7) & ~7, ldw = cond_ld(N, S.tight);
         for (int k = tid; k < Q * N; k += NT) {
             phi[k] = cs[L.phi + k];
             dphi[k] = cs[L.dphi + k];
             dphiJ[k] = cs[L.dphiJ + k];
         }
         for (int k = tid; k < Q * 4; k += NT) qpw[k] = cs[L.qpw + k];
-        for (int k = tid; k < N * 7; k += NT) cq[k] = sq[static_cast<int>(node[k / 7]) * 7 + k % 7];
-        for (int k = tid; k < N * 6; k += NT) {
-            const int n = static_cast<int>(node[k / 6]);
-            cv[k] = sv[n * 6 + k % 6];
-            cvd[k] = svd[n * 6 + k % 6];
-        }
-        const int mi = 6 * cond_local_order<NT>(node, N, fmap, lpos, lnode);
-        for (int k = tid; k < mc * ldw; k += NT) {
-            const int r = k / ldw, c = k % ldw;
-            double v = 0.;
-            if (c == mc && r < mi) {  // interior right-hand side before the element residual
-                const int n = static_cast<int>(node[lnode[r / 6]]) * 6 + r % 6;
-                v = cond * (mslab[ML.fx + n] + mslab[ML.f + n]);
+        for (int k = tid; k < 8 * N; k += NT) {
+            const int l = k >> 3, c = k & 7, n = C.node[l];
+            if (c < 7) cq[l * 7 + c] = sq[n * 7 + c];
+            if (c < 6) {
+                cv[l * 6 + c] = sv[n * 6 + c];
+                cvd[l * 6 + c] = svd[n * 6 + c];
             }
-            W[k] = v;
         }
+#pragma unroll 4
+        for (int k = 2 * tid; k < rows * ldw; k += 2 * NT) store_pair(W + k, 0., 0.);
         __syncthreads();
-        for (int q0 = 0; q0 < Q; q0 += kCondChunk) {
-            const int qn = min(kCondChunk, Q - q0);
+        if (tid < mp) {  // interior right-hand side before the element residual; ones on the padding
+            if (tid < mi) {
+                const int n = C.node[C.at[tid / 6]] * 6 + tid % 6;
+                W[sys_at(ldw, tid, rhs)] = cond * (mslab[ML.fx + n] + mslab[ML.f + n]);
+            } else {
+                W[sys_at(ldw, tid, tid)] = 1.;
+            }
+        }
+#pragma unroll 1
+        for (int q0 = 0; q0 < Q; q0 += S.chunk) {
+            const int qn = min(S.chunk, Q - q0);
             SlabLayout Lc = L;
             Lc.mstar += 36 * q0;
             Lc.cstar += 36 * q0;
             Lc.r0 += 4 * q0;
             Lc.x0p += 3 * q0;
             qp_phase<double, NT / 32>(N, qn, phi + q0 * N, dphiJ + q0 * N, qpw + q0 * 4, cq, cv, cvd, cs, Lc,
-                                 KB.gravity, P.beta_prime, P.gamma_prime, cond, gscr, G, Fc, Fd);
+                                 KB.gravity, P.beta_prime, P.gamma_prime, cond, itp, G, Fc, Fd);
             __syncthreads();
             sub(kPhaseQuadrature);
-            for (int t = tid; t < N * 6; t += NT) {
+            for (int t = NT - 1 - tid; t < N * 6; t += NT) {  // the last warps have fewer pair units
                 const int n = t / 6, c = t % 6;
                 double acc = 0.;
+#pragma unroll 2
                 for (int qp = 0; qp < qn; ++qp) {
                     const int qa = q0 + qp;
                     const double w = qpw[qa * 4], wJ = qpw[qa * 4 + 2];
                     acc += (w * dphi[qa * N + n]) * Fc[qp * 6 + c] + (wJ * phi[qa * N + n]) * Fd[qp * 6 + c];
                 }
-                const int mn = static_cast<int>(node[n]);
-                if (fmap[mn] < 0) W[(lpos[n] * 6 + c) * ldw + mc] -= cond * acc;
-                else resid[mn * 6 + c] += acc;
+                if (C.row[n] < mp) W[sys_at(ldw, C.row[n] + c, rhs)] -= cond * acc;
+                else resid[C.node[n] * 6 + c] += acc;
             }
             integrate_node_pairs<NT>(
-                N, qn, phi + q0 * N, dphi + q0 * N, G, [&](int j) { return sT + static_cast<int>(node[j]) * 9; },
+                N, qn, phi + q0 * N, dphi + q0 * N, G, [&](int j) { return sT + C.node[j] * 9; },
                 [&](int j, int r, int half) {
-                    double* col = W + r * ldw + lpos[j] * 6 + 3 * half;
+                    const short* first = C.row;
+                    const int col = first[j] + 3 * half;
                     return [=](int i, double v0, double v1, double v2) {
-                        double* row = col + lpos[i] * 6 * ldw;
-                        row[0] += v0;
-                        row[1] += v1;
-                        row[2] += v2;
+                        const int row = first[i] + r, sh = row & 6;
+                        double* a = W + row * ldw;
+                        if (q0 > 0) {  // uniform: added to the passes before
+                            v0 += a[col ^ sh];
+                            v1 += a[(col + 1) ^ sh];
+                            v2 += a[(col + 2) ^ sh];
+                        }
+                        a[col ^ sh] = v0;
+                        a[(col + 1) ^ sh] = v1;
+                        a[(col + 2) ^ sh] = v2;
                     };
                 });
             __syncthreads();
             sub(kPhaseLUDiag);
         }
-        // unpivoted elimination of the interior rows, right-hand side included:
-        // rows over the warps, columns over the lanes, one barrier per pivot
-        // (each row's warp stores its own multiplier after using it)
-        const int wid = tid >> 5, wl = tid & 31;
-        for (int k = 0; k < mi; ++k) {
-            const double d = W[k * ldw + k];
-            if (tid == 0 && !(fabs(d) > 0. && isfinite(d))) *flag |= 2;
-            const double rd = 1. / d;
-            for (int i = k + 1 + wid; i < mc; i += NT / 32) {
-                const double l = W[i * ldw + k] * rd;
-                for (int j = k + 1 + wl; j <= mc; j += 32) W[i * ldw + j] -= l * W[k * ldw + j];
-                __syncwarp();
-                if (wl == 0) W[i * ldw + k] = l;
-            }
-            __syncthreads();
-        }
+        if (mp > 0) eliminate_blocks<double, NT>(W, ldw, mp, rows >> 3, (rhs + 8) >> 3, G, flag);
         sub(kPhaseLUPanel);
-        for (int k = tid; k < mc * ldw; k += NT) work[k] = W[k];
+#pragma unroll 4
+        for (int k = 2 * tid; k < rows * ldw; k += 2 * NT) {
+            const double2 v = load_pair(W + k);
+            store_pair(work + k, v.x, v.y);
+        }
         __syncthreads();
         sub(kPhaseIntEpilogue);
     }
@@ -2207,141 +2239,64 @@ __device__ void cond_component_terms(const KBeam& KB, const StepCoeffs& P, const
 // columns of the boundary nodes) into the bordered system Md and its
 // right-hand-side correction into bc, at the boundary nodes' DOF rows.
 template <int NT>
-__device__ void cond_add_schur(const KBeam& KB, const DenseSmem& S, unsigned char* smem_raw, const int* fmap,
-                               double* Md, int md, double* bc) {
+__device__ __forceinline__ void cond_add_schur(const KBeam& KB, const DenseSmem& S, const CompOrder* order, const int* fmap, double* Md, int ldm,
+                               double* bc) {
     const int tid = threadIdx.x;
-    int* lpos = reinterpret_cast<int*>(smem_raw + S.lpos);
-    int* lnode = reinterpret_cast<int*>(smem_raw + S.lnode);
+#pragma unroll 1
     for (int ci = 0; ci < KB.n_comps; ++ci) {
         const double* hd = KB.comps + ci * kCompHead;
         const double* work = KB.comps + static_cast<long>(hd[kCompWork]);
-        const int N = static_cast<int>(hd[1]);
-        const double* node = hd + 3;
-        const int mc = 6 * N, ldw = mc + 1;
-        const int mi = 6 * cond_local_order<NT>(node, N, fmap, lpos, lnode);
-        const int mb = mc - mi;
+        const CompOrder& C = order[ci];
+        const int mp = comp_pivots(C), mb = 6 * C.nb, ldw = cond_ld(static_cast<int>(hd[1]), S.tight);
         for (int e = tid; e < mb * (mb + 1); e += NT) {
-            const int t = mi + e / (mb + 1), u = mi + e % (mb + 1);
-            const int rt = fmap[static_cast<int>(node[lnode[t / 6]])] + t % 6;
-            const double v = work[t * ldw + u];
-            if (u == mc) bc[rt] += v;
-            else Md[rt * md + fmap[static_cast<int>(node[lnode[u / 6]])] + u % 6] += v;
+            const int t = e / (mb + 1), u = e % (mb + 1);
+            const int rt = fmap[C.node[C.at[C.ni + t / 6]]] + t % 6;
+            const double v = work[sys_at(ldw, mp + t, mp + u)];
+            if (u == mb) bc[rt] += v;
+            else Md[rt * ldm + fmap[C.node[C.at[C.ni + u / 6]]] + u % 6] += v;
         }
         __syncthreads();
     }
 }
 
-// The back substitution of cond_back_substitute for all components at once,
-// one warp per component, when every component's eliminated rows and a map
-// of its DOFs fit the condensed region (dead once the bordered system is
-// solved): the rows are staged there together, map[p] is the position of local
-// DOF p in xi (>= 0, interior) or -1 - its position in x (boundary), and each
-// warp sweeps its rows with the sums of the sequential form.  Returns false,
-// having done nothing, when they do not fit.
+// Interior corrections of each condensed component from the bordered system's
+// solution x at its boundary nodes: x_i = y_i - U_ib x_b - U_ii x_i, the rows of
+// the eliminated system staged back into shared memory; the corrections go to
+// xi at the nodes' interior DOFs.
 template <int NT>
-__device__ bool cond_back_substitute_warps(const KBeam& KB, const DenseSmem& S, unsigned char* smem_raw,
-                                           const int* fmap, const int* imap, const double* x, double* xi) {
-    constexpr int NW = NT / 32;
+__device__ __forceinline__ void cond_back_substitute(const KBeam& KB, const DenseSmem& S, const int* fmap,
+                                                     const int* imap, const double* x, double* xi) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    long need = 0;
-    for (int ci = 0; ci < KB.n_comps; ++ci) {
-        const int N = static_cast<int>(KB.comps[ci * kCompHead + 1]);
-        int ni = 0;
-        for (int k = 0; k < N; ++k) ni += fmap[static_cast<int>(KB.comps[ci * kCompHead + 3 + k])] < 0;
-        need += 8L * (6 * ni) * (6 * N + 1) + 4L * 6 * N + 16;
-    }
-    if (need > S.cR) return false;
-    unsigned char* base = smem_raw + S.cW;
-    // per component: rows at a double offset, map at an int offset (tid 0 lays them out)
-    __shared__ int s_roff[kMaxDenseComps], s_moff[kMaxDenseComps], s_mi[kMaxDenseComps];
-    if (tid == 0) {
-        long o = 0;
-        for (int ci = 0; ci < KB.n_comps; ++ci) {
-            const double* hd = KB.comps + ci * kCompHead;
-            const int N = static_cast<int>(hd[1]), mc = 6 * N;
-            int ni = 0;
-            for (int k = 0; k < N; ++k) ni += fmap[static_cast<int>(hd[3 + k])] < 0;
-            s_roff[ci] = static_cast<int>(o / 8);
-            s_mi[ci] = 6 * ni;
-            o += 8L * (6 * ni) * (mc + 1);
-            s_moff[ci] = static_cast<int>(o / 4);
-            int* map = reinterpret_cast<int*>(base) + s_moff[ci];
-            int pi = 0, pb = 6 * ni;  // interior nodes first, then boundary, in local order
-            for (int k = 0; k < N; ++k) {
-                const int n = static_cast<int>(hd[3 + k]);
-                if (fmap[n] < 0)
-                    for (int c = 0; c < 6; ++c) map[pi++] = imap[n] + c;
-                else
-                    for (int c = 0; c < 6; ++c) map[pb++] = -1 - (fmap[n] + c);
-            }
-            o += 4L * mc;
-            o = (o + 15) & ~15L;
-        }
-    }
-    __syncthreads();
-    for (int ci = 0; ci < KB.n_comps; ++ci) {
-        const double* hd = KB.comps + ci * kCompHead;
-        const double* work = KB.comps + static_cast<long>(hd[kCompWork]);
-        const int ldw = 6 * static_cast<int>(hd[1]) + 1;
-        double* R = reinterpret_cast<double*>(base) + s_roff[ci];
-        for (int k = tid; k < s_mi[ci] * ldw; k += NT) R[k] = work[k];
-    }
-    __syncthreads();
-    for (int ci = warp; ci < KB.n_comps; ci += NW) {
-        const int mc = 6 * static_cast<int>(KB.comps[ci * kCompHead + 1]), ldw = mc + 1, mi = s_mi[ci];
-        const double* R = reinterpret_cast<const double*>(base) + s_roff[ci];
-        const int* map = reinterpret_cast<const int*>(base) + s_moff[ci];
-        for (int k = mi - 1; k >= 0; --k) {
-            const double* row = R + k * ldw;
-            double acc = 0.;
-            for (int j = k + 1 + lane; j < mc; j += 32) {
-                const int mj = map[j];
-                acc += row[j] * (mj >= 0 ? xi[mj] : x[-1 - mj]);
-            }
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) xi[map[k]] = (row[mc] - acc) / row[k];
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    return true;
-}
-
-// Interior corrections of each condensed component from the bordered
-// system's solution x at its boundary nodes: U_ii x_i = y_i - U_ib x_b by one
-// warp, rows of the eliminated system (staged back into shared memory in W)
-// from the last up; the corrections go to xi at the nodes' interior DOFs.
-template <int NT>
-__device__ void cond_back_substitute(const KBeam& KB, const DenseSmem& S, unsigned char* smem_raw,
-                                     const int* fmap, const int* imap, const double* x, double* xi) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (cond_back_substitute_warps<NT>(KB, S, smem_raw, fmap, imap, x, xi)) return;
     double* W = reinterpret_cast<double*>(smem_raw + S.cW);
     double* cx = reinterpret_cast<double*>(smem_raw + S.cx);
-    int* lpos = reinterpret_cast<int*>(smem_raw + S.lpos);
-    int* lnode = reinterpret_cast<int*>(smem_raw + S.lnode);
+    const CompOrder* order = reinterpret_cast<const CompOrder*>(smem_raw + S.order);
+#pragma unroll 1
     for (int ci = 0; ci < KB.n_comps; ++ci) {
         const double* hd = KB.comps + ci * kCompHead;
         const double* work = KB.comps + static_cast<long>(hd[kCompWork]);
-        const int N = static_cast<int>(hd[1]);
-        const double* node = hd + 3;
-        const int mc = 6 * N, ldw = mc + 1;
-        const int mi = 6 * cond_local_order<NT>(node, N, fmap, lpos, lnode);
-        for (int k = tid; k < mi * ldw; k += NT) W[k] = work[k];
-        for (int p = mi + tid; p < mc; p += NT) cx[p] = x[fmap[static_cast<int>(node[lnode[p / 6]])] + p % 6];
-        __syncthreads();
-        if (warp == 0) {
-            for (int k = mi - 1; k >= 0; --k) {
-                const double* row = W + k * ldw;
-                double acc = 0.;
-                for (int j = k + 1 + lane; j < mc; j += 32) acc += row[j] * cx[j];
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0) cx[k] = (row[mc] - acc) / row[k];
-                __syncwarp();
-            }
+        const CompOrder& C = order[ci];
+        const int mi = 6 * C.ni, mp = comp_pivots(C), mb = 6 * C.nb, ldw = cond_ld(static_cast<int>(hd[1]), S.tight);
+#pragma unroll 4
+        for (int k = 2 * tid; k < mp * ldw; k += 2 * NT) {
+            const double2 v = load_pair(work + k);
+            store_pair(W + k, v.x, v.y);
         }
         __syncthreads();
-        for (int p = tid; p < mi; p += NT) xi[imap[static_cast<int>(node[lnode[p / 6]])] + p % 6] = cx[p];
+#pragma unroll 1
+        for (int i0 = 4 * warp; i0 < mp; i0 += NT / 8) {  // eight lanes per row
+            const int i = i0 + (lane >> 3);
+            double y = 0.;
+#pragma unroll 1
+            for (int u = lane & 7; u < mb; u += 8)
+                y -= W[sys_at(ldw, i, mp + u)] * x[fmap[C.node[C.at[C.ni + u / 6]]] + u % 6];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+            if ((lane & 7) == 0) cx[i] = W[sys_at(ldw, i, mp + mb)] + y;
+        }
+        __syncthreads();
+        if (mp > 0) back_substitute<double, NT>(W, ldw, mp, cx);
+        for (int p = tid; p < mi; p += NT) xi[imap[C.node[C.at[p / 6]]] + p % 6] = cx[p];
         __syncthreads();
     }
 }
@@ -2368,7 +2323,7 @@ struct BordScratch {
     int piv[8];         // row each panel column was pivoted on
     int back[8];        // row (of the panel's eight) that goes where piv[c] was, or -1
 };
-static_assert(sizeof(BordScratch) <= 1024, "DenseSmem::bord");
+static_assert(sizeof(BordScratch) <= kBordScratch, "DenseSmem::bord");
 
 // Step 1, by warps 0 .. PW - 1 (which meet at barrier 2), RT rows per thread.
 template <int PW, int RT>
@@ -2597,7 +2552,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
     const int nd = KB.model_dofs;                       // the reference's unknowns
     const bool cnd = KB.cond_nd > 0;                    // condensed beam components
     const int md = cnd ? KB.cond_nd : nd;               // unknowns of the bordered system
-    const DenseSmem S = make_dense_smem(N, nd, NT, KB.n_comps > 0 ? KB.comp_maxN : 0, KB.comp_maxQ, KB.cond_nd,
+    const DenseSmem S = make_dense_smem(N, nd, KB.n_comps > 0 ? KB.comp_maxN : 0, KB.comp_maxQ, KB.cond_nd,
                                         KB.cond_md != nullptr);
     double* Md = KB.cond_md ? KB.cond_md : reinterpret_cast<double*>(smem_raw + S.M);
     double* b = reinterpret_cast<double*>(smem_raw + S.b);
@@ -2614,7 +2569,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
     int* act = reinterpret_cast<int*>(smem_raw + S.act);
     int* fmap = reinterpret_cast<int*>(smem_raw + S.fmap);
     double* red = reinterpret_cast<double*>(smem_raw + S.red);
-    double* rpiv = reinterpret_cast<double*>(smem_raw + S.rpiv);
+    CompOrder* order = cnd ? reinterpret_cast<CompOrder*>(smem_raw + S.order) : nullptr;
     BordScratch* bord = reinterpret_cast<BordScratch*>(smem_raw + S.bord);
     const int ldm = bord_ld(md);
     double* xi = cnd ? reinterpret_cast<double*>(smem_raw + S.xi) : nullptr;
@@ -2699,6 +2654,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         s_flag = cnd ? ((o + rows != md || o + oi + rows != nd) ? 2 : 0) : (o > nd) ? 2 : 0;
     }
     __syncthreads();
+    if (cnd) cond_order<NT>(KB, fmap, order);  // read behind the barriers below
     const int nsys = s_nsys;
     // PredictNextState (src/step/predict_next_state.hpp:14-47)
     for (int k = tid; k < N * 7; k += NT) sqp[k] = sq[k];
@@ -2746,7 +2702,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         mark(kPhaseLoadPredict);
         if (cnd) {  // components first: their systems share the bordered system's region
             __syncthreads();
-            cond_component_terms<NT>(KB, P, S, smem_raw, sq, sv, svd, sT, fmap, slab, L, resid, &s_flag,
+            cond_component_terms<NT>(KB, P, S, sq, sv, svd, sT, slab, L, resid, &s_flag,
                                      timing ? s_ph : nullptr);
         }
         mark(kPhaseIntegrate);
@@ -2762,7 +2718,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                              [&](int r, int c) -> double& { return Md[r * ldm + c]; }, resid, 1);
         if (KB.n_comps > 0) {  // beam elements, then their node_FX (summed per node)
             __syncthreads();
-            if (cnd) cond_add_schur<NT>(KB, S, smem_raw, fmap, Md, ldm, bc);
+            if (cnd) cond_add_schur<NT>(KB, S, order, fmap, Md, ldm, bc);
             else dense_beam_terms<NT>(KB, P, S, smem_raw, sq, sv, svd, sT, fmap, Md, ldm, resid);
             for (int t = tid; t < N * 6; t += NT) resid[t] -= slab[L.fx + t];
         }
@@ -2916,13 +2872,13 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         __syncthreads();
         mark(kPhaseConstraints);
         // (apart, so that the shared system is read by shared-memory loads)
-        if (KB.cond_md) solve_bordered<NT, false>(KB.cond_md, 0, ldm, md, x, rpiv, bord, &s_flag);
-        else solve_bordered<NT, true>(nullptr, S.M, ldm, md, x, rpiv, bord, &s_flag);
+        if (KB.cond_md) solve_bordered<NT, false>(KB.cond_md, 0, ldm, md, x, b, bord, &s_flag);
+        else solve_bordered<NT, true>(nullptr, S.M, ldm, md, x, b, bord, &s_flag);
         mark(kPhaseFactor);
         // multipliers unconditioned; convergence error (calculate_convergence_error.hpp)
         for (int k = nsys + tid; k < md; k += NT) x[k] /= cond;
         __syncthreads();
-        if (cnd) cond_back_substitute<NT>(KB, S, smem_raw, fmap, imap, x, xi);
+        if (cnd) cond_back_substitute<NT>(KB, S, fmap, imap, x, xi);
         mark(kPhaseSubstitute);
         // correction of component c of node n
         auto delta_of = [&](int n, int c) { return fmap[n] >= 0 ? x[fmap[n] + c] : xi[imap[n] + c]; };
@@ -3711,10 +3667,15 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             // block elimination, then the back substitution of each right-hand side
             double* dinv = reinterpret_cast<double*>(smem_raw + S.G);
             if (m > 0) {
-                eliminate_free_block<TR, NT>(A, ldA, m, nrhs, dinv, &s_flag);
+                eliminate_blocks<TR, NT>(A, ldA, m, (m + 7) >> 3, (m + nrhs + 7) >> 3, dinv, &s_flag);
                 mark(kPhaseFactor);
-                back_substitute<TR, NT>(A, ldA, m, m, xs);
-                if (drive) back_substitute<TR, NT>(A, ldA, m, m + 1, x2);
+                for (int i = tid; i < m; i += NT) {
+                    xs[i] = static_cast<double>(A[sys_at(ldA, i, m)]);
+                    if (drive) x2[i] = static_cast<double>(A[sys_at(ldA, i, m + 1)]);
+                }
+                __syncthreads();
+                back_substitute<TR, NT>(A, ldA, m, xs);
+                if (drive) back_substitute<TR, NT>(A, ldA, m, x2);
             }
             mark(kPhaseLUPanel);
         }

@@ -40,10 +40,13 @@ constexpr int kMaxDenseComps = 8;
 // of each beam component -- nodes of one component only, without masses,
 // springs or constraints -- inside the component's own system, and solves
 // the bordered system of the remaining nodes and the constraints (at most
-// kCondMaxDofs unknowns).  The workspace of a component holds its system
-// [6Nc][6Nc + 1] during the condensation and its factored interior rows for
-// the back substitution.
+// kCondMaxDofs unknowns).  The workspace of a component holds its eliminated
+// system [cond_rows][cond_ld]: interior unknowns padded to whole tiles of eight
+// rows, boundary unknowns, right-hand side; rows 8 doubles (mod 16) apart, or
+// (tight) as whole tiles.
 constexpr int kCondMaxDofs = 160;
+KYN_HD inline int cond_rows(int N) { return (6 * N + 6 + 7) & ~7; }
+KYN_HD inline int cond_ld(int N, bool tight) { return tight ? (6 * N + 14) & ~7 : ((6 * N + 14) & ~15) + 8; }
 constexpr int kThreads = 256;            // threads per CTA of the step kernel
 
 // Offsets (in doubles) of the arrays inside one beam slab.
