@@ -2308,13 +2308,18 @@ __device__ __forceinline__ void cond_back_substitute(const KBeam& KB, const Dens
 //   1. the first warps factor the panel, a row per thread in registers; a pivot
 //      is found by two integer reductions per warp and an exchange of the warps'
 //      finds, and its row reaches the threads through shared memory;
-//   2. one thread per remaining column brings the pivot rows to the top, the
-//      rows they displace to the places they leave, and solves for U;
+//   2. tiles of eight columns to a warp: the pivot rows to the top, the rows they
+//      displace to the places they leave, and U = L^-1 A with a row to four
+//      lanes and the pivot rows by shuffle;
 //   3. all warps subtract L U from the rest on the FP64 tensor cores.
 // The unblocked form (pivot search, swap and a rank-1 update of the whole rest
 // per column) was bound by the traffic of those updates and by three barriers a
-// column: 643k cycles for 137 unknowns.  With the panel in one warp, five rows
-// to a lane, a column took 1300 cycles.
+// column: 643k cycles for 137 unknowns, now 185k, of which step 1 takes 95k (660
+// cycles a column, a chain of reductions, barriers and a division), step 2 29k
+// (34k with a column to a thread, whose straight-line code was fetched once per
+// panel) and step 3 48k.  Slower: the panel in one warp with five rows to a lane
+// (1100 cycles a column); the next panel beside step 3, whose tensor
+// instructions hold up the panel's chain on the same FP64 pipes.
 struct BordScratch {
     double prow[2][8];  // the pivot row, from the pivot on (double-buffered by column)
     double rp[2];       // the pivot's reciprocal
@@ -2337,33 +2342,37 @@ __device__ __forceinline__ void factor_pivoted_panel(double* Md, int ld, int md,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kb = min(8, md - k0);
     double v[RT][8];
     bool live[RT];
-    double* row[RT];
+    int row[RT];
 #pragma unroll
     for (int e = 0; e < RT; ++e) {
         const int i = k0 + tid + 32 * PW * e;
         live[e] = i < md;
-        row[e] = Md + min(i, md - 1) * ld + k0;
+        row[e] = min(i, md - 1) * ld + k0;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) v[e][c] = c < kb ? row[e][c] : 0.;
+        for (int c = 0; c < 8; c += 2) {  // rows of even length: pairs
+            const double2 x = load_pair(Md + row[e] + (c < kb ? c : 0));
+            v[e][c] = c < kb ? x.x : 0.;
+            v[e][c + 1] = c + 1 < kb ? x.y : 0.;
+        }
     }
 #pragma unroll 1
     for (int c = 0; c < kb; ++c) {  // the pivot column is v[.][0]
         const int h = c & 1;
         unsigned hi = 0;
         int at = 0;
+        double best = v[0][0];
 #pragma unroll
         for (int e = 0; e < RT; ++e) {
-            const double x = fabs(v[e][0]);
-            const unsigned he = live[e] && x > 0. ? static_cast<unsigned>(__double2hiint(x)) + 1u : 0u;  // NaN: 0
+            const unsigned ah = static_cast<unsigned>(__double2hiint(v[e][0])) & 0x7fffffffu;
+            const unsigned he = live[e] && ah <= 0x7ff00000u ? ah : 0u;  // NaN: 0
             if (he > hi) {
                 hi = he;
                 at = e;
+                best = v[e][0];
             }
         }
-        double inv[RT];  // every thread's reciprocal, while the reductions run
-#pragma unroll
-        for (int e = 0; e < RT; ++e) inv[e] = 1. / v[e][0];
         const unsigned mh = __reduce_max_sync(kAll, hi);
+        const double inv = 1. / best;  // every lane's candidate, while the reductions run
         const unsigned mr = __reduce_min_sync(kAll, hi == mh ? static_cast<unsigned>(tid + 32 * PW * at) : ~0u);
         unsigned long long key = static_cast<unsigned long long>(mh) << 32 | (~mr);
         if constexpr (PW > 1) {
@@ -2378,14 +2387,14 @@ __device__ __forceinline__ void factor_pivoted_panel(double* Md, int ld, int md,
 #pragma unroll
         for (int e = 0; e < RT; ++e)
             if (r == tid + 32 * PW * e) {  // the pivot row's thread
-                W->rp[h] = inv[e];
-                rpiv[k0 + c] = inv[e];
+                W->rp[h] = inv;
+                rpiv[k0 + c] = inv;
                 W->piv[c] = k0 + r;
                 if (!found) atomicOr(flag, 2);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     W->prow[h][j] = v[e][j];
-                    if (c + j < kb) row[e][c + j] = v[e][j];
+                    if (c + j < kb) Md[row[e] + c + j] = v[e][j];
                 }
                 live[e] = false;
             }
@@ -2397,28 +2406,29 @@ __device__ __forceinline__ void factor_pivoted_panel(double* Md, int ld, int md,
 #pragma unroll
         for (int e = 0; e < RT; ++e) {
             const double l = v[e][0] * rd;
-            if (live[e]) row[e][c] = l;
+            if (live[e]) Md[row[e] + c] = l;
 #pragma unroll
             for (int j = 0; j < 7; ++j) v[e][j] = fma(-l, u[j + 1], v[e][j + 1]);
             v[e][7] = 0.;
         }
     }
     meet();
-    if (warp == 0) {  // the pivot rows' multipliers, and where the rows they displace go
+    if (warp > 0) return;
+    // the pivot rows' multipliers, and where the rows they displace go
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            const int r = lane >> 2, c = 2 * (lane & 3) + x;
-            W->lower[8 * r + c] = r < kb && c < r ? Md[W->piv[r] * ld + k0 + c] : 0.;
-        }
-        const int p = lane < kb ? W->piv[lane] : -1;
-        const unsigned out = __ballot_sync(kAll, p >= k0 + kb);                      // columns pivoted from below
-        unsigned stay = __reduce_or_sync(kAll, p >= k0 && p < k0 + kb ? 1u << (p - k0) : 0u);
-        stay = ~stay & ((1u << kb) - 1u);                                            // panel rows displaced
-        if (lane < 8) {
-            int d = -1;
-            if (out >> lane & 1u) d = __fns(stay, 0, __popc(out & ((1u << lane) - 1u)) + 1);
-            W->back[lane] = d;
-        }
+    for (int x = 0; x < 2; ++x) {
+        const int r = lane >> 2, c = 2 * (lane & 3) + x;
+        W->lower[8 * r + c] = r < kb && c < r ? Md[W->piv[r] * ld + k0 + c] : 0.;
+    }
+    const int p = lane < kb ? W->piv[lane] : -1;
+    const unsigned out = __ballot_sync(kAll, p >= k0 + kb);                      // columns pivoted from below
+    unsigned stay = __reduce_or_sync(kAll, p >= k0 && p < k0 + kb ? 1u << (p - k0) : 0u);
+    stay = ~stay & ((1u << kb) - 1u);                                            // panel rows displaced
+    if (lane < 8) {
+        int d = -1;
+        if (out >> lane & 1u) d = __fns(stay, 0, __popc(out & ((1u << lane) - 1u)) + 1);
+        W->back[lane] = d;
+        if (lane >= kb) W->piv[lane] = k0;
     }
 }
 
@@ -2431,71 +2441,81 @@ __device__ __forceinline__ void solve_bordered(double* Mg, int off, int ld, int 
     double* Md = SHARED ? reinterpret_cast<double*>(smem_raw + off) : Mg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int fr = lane >> 2, t = lane & 3, t2 = 2 * t;
-#pragma unroll 1
-    for (int k0 = 0; k0 < md; k0 += 8) {
-        const int kb = min(8, md - k0);
+    auto panel = [&](int k0) {
         // up to 64 rows one warp does it without barriers
-        if (md - k0 <= 64) {
-            if (warp == 0) factor_pivoted_panel<1, 2>(Md, ld, md, k0, rpiv, W, flag);
-        } else if (warp < PW) {
-            factor_pivoted_panel<PW, (kCondMaxDofs + 32 * PW - 1) / (32 * PW)>(Md, ld, md, k0, rpiv, W, flag);
+        if (md - k0 > 64) {
+            if (warp < PW) factor_pivoted_panel<PW, (CS + PW - 1) / PW>(Md, ld, md, k0, rpiv, W, flag);
+        } else if (warp == 0) {
+            factor_pivoted_panel<1, 2>(Md, ld, md, k0, rpiv, W, flag);
         }
-        __syncthreads();
-        // 2. rows to their places, U = L^-1 A
-#pragma unroll 1
-        for (int j = k0 + tid; j <= md; j += NT) {
-            double a[8], d[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                a[c] = c < kb ? Md[W->piv[c] * ld + j] : 0.;
-                d[c] = c < kb && W->back[c] >= 0 ? Md[(k0 + W->back[c]) * ld + j] : 0.;
-            }
-            if (j >= k0 + kb) {
-#pragma unroll
-                for (int c = 0; c < 7; ++c)
-#pragma unroll
-                    for (int r = c + 1; r < 8; ++r) a[r] = fma(-W->lower[8 * r + c], a[c], a[r]);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                if (c < kb) Md[(k0 + c) * ld + j] = a[c];
-                if (c < kb && W->back[c] >= 0) Md[W->piv[c] * ld + j] = d[c];
-            }
-        }
-        __syncthreads();
-        // 3. the rest, in equal runs of tiles down the columns
+    };
+    // tiles lo .. hi - 1, counted down columns of ni tiles from column c0 on, less the panel at k0
+    auto update = [&](int k0, int c0, int ni, int lo, int hi) {
         const int r0 = k0 + 8;
-        if (r0 < md) {
-            const int ni = (md - r0 + 7) >> 3, nj = (md + 1 - r0 + 7) >> 3, total = ni * nj;
-            const int lo = total * warp / NW, hi = total * (warp + 1) / NW;
-            int j = static_cast<int>(__fdividef(static_cast<float>(lo) + 0.5f, static_cast<float>(ni)));
-            int i = lo - j * ni;
+        int j = static_cast<int>(__fdividef(static_cast<float>(lo) + 0.5f, static_cast<float>(ni)));
+        int i = lo - j * ni;
 #pragma unroll 1
-            for (int left = hi - lo; left > 0;) {
-                const int c0 = r0 + 8 * j, cnt = min(ni - i, left), cu = min(c0 + fr, md), cd = c0 + t2;
-                // products in the order of the columns, as the unblocked elimination takes them
-                const double u0 = -Md[(k0 + t) * ld + cu], u1 = -Md[(k0 + 4 + t) * ld + cu];
+        for (int left = hi - lo; left > 0;) {
+            const int cj = c0 + 8 * j, cnt = min(ni - i, left), cu = min(cj + fr, md), cd = cj + t2;
+            // products in the order of the columns, as the unblocked elimination takes them
+            const double u0 = -Md[(k0 + t) * ld + cu], u1 = -Md[(k0 + 4 + t) * ld + cu];
 #pragma unroll 1
-                for (int e = 0; e < cnt; e += 2) {  // two tiles' loads ahead of their stores
-                    const int ra = r0 + 8 * (i + e) + fr, rb = ra + 8;
-                    const bool two = e + 1 < cnt;
-                    double* pa = Md + min(ra, md - 1) * ld;
-                    double* pb = Md + min(two ? rb : ra, md - 1) * ld;
-                    const int c1 = min(cd, ld - 2);
-                    const double la0 = pa[k0 + t], la1 = pa[k0 + 4 + t], lb0 = pb[k0 + t], lb1 = pb[k0 + 4 + t];
-                    double2 da = load_pair(pa + c1), db = load_pair(pb + c1);
-                    dmma884(da.x, da.y, la0, u0);
-                    if (two) dmma884(db.x, db.y, lb0, u0);
-                    dmma884(da.x, da.y, la1, u1);
-                    if (two) dmma884(db.x, db.y, lb1, u1);
-                    if (ra < md && cd <= md) store_pair(pa + cd, da.x, da.y);
-                    if (two && rb < md && cd <= md) store_pair(pb + cd, db.x, db.y);
-                }
-                left -= cnt;
-                ++j;
-                i = 0;
+            for (int e = 0; e < cnt; e += 2) {  // two tiles' loads ahead of their stores
+                const int ra = r0 + 8 * (i + e) + fr, rb = ra + 8;
+                const bool two = e + 1 < cnt;
+                double* pa = Md + min(ra, md - 1) * ld;
+                double* pb = Md + min(two ? rb : ra, md - 1) * ld;
+                const int c1 = min(cd, ld - 2);
+                const double la0 = pa[k0 + t], la1 = pa[k0 + 4 + t], lb0 = pb[k0 + t], lb1 = pb[k0 + 4 + t];
+                double2 da = load_pair(pa + c1), db = load_pair(pb + c1);
+                dmma884(da.x, da.y, la0, u0);
+                if (two) dmma884(db.x, db.y, lb0, u0);
+                dmma884(da.x, da.y, la1, u1);
+                if (two) dmma884(db.x, db.y, lb1, u1);
+                if (ra < md && cd <= md) store_pair(pa + cd, da.x, da.y);
+                if (two && rb < md && cd <= md) store_pair(pb + cd, db.x, db.y);
             }
+            left -= cnt;
+            ++j;
+            i = 0;
         }
+    };
+    panel(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0;; k0 += 8) {
+        // 2. rows to their places, U = L^-1 A: a warp takes tiles of eight columns,
+        // the pivot row and the displaced row of panel column fr to a lane
+        const int kb = min(8, md - k0), r0 = k0 + 8;
+        const int piv = W->piv[fr] * ld, back = W->back[fr];
+        double low[7];
+#pragma unroll
+        for (int c = 0; c < 7; ++c) low[c] = -W->lower[8 * fr + c];
+#pragma unroll 1
+        for (int j0 = k0 + 8 * warp; j0 <= md; j0 += 8 * NW) {
+            const int j = min(j0 + t2, ld - 2);
+            const bool in = j0 + t2 <= md;
+            double2 a = load_pair(Md + piv + j);
+            const double2 d = load_pair(Md + (k0 + max(back, 0)) * ld + j);
+            if (j0 > k0 || kb < 8) {
+#pragma unroll
+                for (int c = 0; c < 7; ++c) {
+                    const double px = __shfl_sync(kAll, a.x, 4 * c + t), py = __shfl_sync(kAll, a.y, 4 * c + t);
+                    if (c < fr && j >= k0 + kb) a.x = fma(low[c], px, a.x);
+                    if (c < fr && j + 1 >= k0 + kb) a.y = fma(low[c], py, a.y);
+                }
+            }
+            __syncwarp();
+            if (in && fr < kb) store_pair(Md + (k0 + fr) * ld + j, a.x, a.y);
+            if (in && back >= 0) store_pair(Md + piv + j, d.x, d.y);
+        }
+        __syncthreads();
+        if (r0 >= md) break;
+        // 3. the rest, in equal runs of tiles down the columns
+        const int ni = (md - r0 + 7) >> 3, total = ni * ((md + 1 - r0 + 7) >> 3);
+        update(k0, r0, ni, total * warp / NW, total * (warp + 1) / NW);
+        __syncthreads();
+        panel(r0);
         __syncthreads();
     }
     if (warp == 0 && md <= 64) {
@@ -2514,27 +2534,26 @@ __device__ __forceinline__ void solve_bordered(double* Mg, int off, int ld, int 
         }
     } else if (warp == 0) {  // by columns, the right-hand side in registers
         double y[CS], u[CS];
-        const double* row[CS];
+        int row[CS];
 #pragma unroll
         for (int e = 0; e < CS; ++e) {
             const int i = lane + 32 * e;
-            row[e] = Md + min(i, md - 1) * ld;
-            y[e] = row[e][md];
-            u[e] = i < md - 1 ? row[e][md - 1] : 0.;
+            row[e] = min(i, md - 1) * ld;
+            y[e] = Md[row[e] + md];
+            u[e] = i < md - 1 ? Md[row[e] + md - 1] : 0.;
         }
+#pragma unroll
+        for (int ks = CS - 1; ks >= 0; --ks) {
 #pragma unroll 1
-        for (int k = md - 1; k >= 0; --k) {
-            const int ks = k >> 5;
-            double yk = y[0];
+            for (int k = min(md - 1, 32 * ks + 31); k >= 32 * ks; --k) {
+                const double xk = __shfl_sync(kAll, y[ks] * rpiv[k], k & 31);
+                if (lane == 0) x[k] = xk;
 #pragma unroll
-            for (int e = 1; e < CS; ++e) yk = ks == e ? y[e] : yk;
-            const double xk = __shfl_sync(kAll, yk, k & 31) * rpiv[k];
-            if (lane == 0) x[k] = xk;
-#pragma unroll
-            for (int e = 0; e < CS; ++e) {
-                const int i = lane + 32 * e;
-                if (i < k) y[e] = fma(-u[e], xk, y[e]);
-                if (i < k - 1) u[e] = row[e][k - 1];  // for the next column
+                for (int e = 0; e <= ks; ++e) {
+                    const int i = lane + 32 * e;
+                    if (i < k) y[e] = fma(-u[e], xk, y[e]);
+                    if (i < k - 1) u[e] = Md[row[e] + k - 1];  // for the next column
+                }
             }
         }
     }
@@ -2576,6 +2595,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
     int* imap = cnd ? reinterpret_cast<int*>(smem_raw + S.imap) : nullptr;
     double* bc = cnd ? reinterpret_cast<double*>(smem_raw + S.bc) : nullptr;
     __shared__ int s_flag, s_nsys;
+    __shared__ short4 s_con[kMaxBeamConstraints];  // first row, type, node and base node of each constraint
     // phase timers (KYN_OPT_PHASE_TIMING): one CTA's clock, thread 0
     __shared__ unsigned long long s_ph[kNumPhases];
     const bool timing = KB.prof != nullptr;
@@ -2655,6 +2675,12 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
     }
     __syncthreads();
     if (cnd) cond_order<NT>(KB, fmap, order);  // read behind the barriers below
+    if (tid < nc) {
+        int rf = s_nsys;
+        for (int e = 0; e < tid; ++e) rf += constraint_rows(KB.con_type[e]);
+        s_con[tid] = make_short4(static_cast<short>(rf), static_cast<short>(KB.con_type[tid]),
+                                 static_cast<short>(KB.con_node[tid]), static_cast<short>(KB.con_base[tid]));
+    }
     const int nsys = s_nsys;
     // PredictNextState (src/step/predict_next_state.hpp:14-47)
     for (int k = tid; k < N * 7; k += NT) sqp[k] = sq[k];
@@ -2706,7 +2732,8 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                                      timing ? s_ph : nullptr);
         }
         mark(kPhaseIntegrate);
-        for (int k = tid; k < md * ldm; k += NT) Md[k] = 0.;
+#pragma unroll 4
+        for (int k = 2 * tid; k < md * ldm; k += 2 * NT) store_pair(Md + k, 0., 0.);
         for (int k = tid; k < md; k += NT) b[k] = 0.;
         if (cnd)
             for (int k = tid; k < md; k += NT) bc[k] = 0.;
@@ -2723,9 +2750,11 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
             for (int t = tid; t < N * 6; t += NT) resid[t] -= slab[L.fx + t];
         }
         // constraints: residual, gradients and G^T lambda
-        if (warp == NW - 1 && lane < nc) {  // beside the masses of the first warps
-            double* cr = con + lane * kConStride;
-            const int t = KB.con_type[lane], tn = KB.con_node[lane], bn = KB.con_base[lane];
+        // (one lane each, over the warps behind the masses' first: their types branch apart)
+        const int cc = lane * (NW - 1) + warp - 1;
+        if (warp > 0 && cc < nc) {
+            double* cr = con + cc * kConStride;
+            const int t = s_con[cc].y, tn = s_con[cc].z, bn = s_con[cc].w;
             if (t >= KYN_CONSTRAINT_FIXED_BC_3DOF) {
                 // three rows (calculate_*_3DOF_constraint.hpp): u2 + X0 - u1 - R1 X0
                 double u1[3] = {0., 0., 0.}, R1[4] = {1., 0., 0., 0.};
@@ -2736,7 +2765,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                     for (int k = 0; k < 3; ++k) u1[k] = sq[bn * 7 + k];
                     for (int k = 0; k < 4; ++k) R1[k] = sq[bn * 7 + 3 + k];
                 }
-                const double* X0 = KB.con_X0[lane];
+                const double* X0 = KB.con_X0[cc];
                 double r1x0[3];
                 for (int i = 0; i < 3; ++i) {
                     r1x0[i] = 0.;
@@ -2755,12 +2784,12 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                             cr[conrec::Btr + i * 3 + j] = bt;
                         }
             } else if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {
-                revolute_dense_record(cr, sq + bn * 7, sq + tn * 7, KB.con_frames + lane * 9, KB.con_X0[lane],
+                revolute_dense_record(cr, sq + bn * 7, sq + tn * 7, KB.con_frames + cc * 9, KB.con_X0[cc],
                                       sT + bn * 9, sT + tn * 9);
             } else {
-                constraint_record(cr, t, sq + tn * 7, KB.con_X0[lane], sT + tn * 9,
+                constraint_record(cr, t, sq + tn * 7, KB.con_X0[cc], sT + tn * 9,
                                   bn >= 0 ? sq + bn * 7 : nullptr, bn >= 0 ? sT + bn * 9 : nullptr,
-                                  KB.con_axis[lane]);
+                                  KB.con_axis[cc]);
             }
             if (bn >= 0 && t != KYN_CONSTRAINT_REVOLUTE_JOINT) {  // G_base^T lambda
                 double* gb = cr + conrec::yr;
@@ -2779,33 +2808,30 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         __syncthreads();
         // scatter: rows of B = G T, columns G^T, residuals (assemble_constraints_matrix.hpp,
         // assemble_constraints_residual.hpp, assemble_system_residual.hpp)
-        // One thread per constraint: its rows and columns of Md are its own.  The
+        // One thread per constraint: its rows and columns of Md are its own, zero so far.  The
         // nodes' forces, which constraints share, are summed per component in
         // the order of the constraints by six lanes of another warp.
         if (tid < nc) {
-            const int c = tid;
-            int rf = nsys;
-            for (int e = 0; e < c; ++e) rf += constraint_rows(KB.con_type[e]);
-            const double* cr = con + c * kConStride;
-            const int t = KB.con_type[c], bn = KB.con_base[c];
-            const int rows = constraint_rows(t), ft = fmap[KB.con_node[c]];
+            const double* cr = con + tid * kConStride;
+            const int rf = s_con[tid].x, t = s_con[tid].y, bn = s_con[tid].w;
+            const int rows = constraint_rows(t), ft = fmap[s_con[tid].z];
             if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {  // five rows, gradients on both nodes
                 const int fb = fmap[bn];
 #pragma unroll 1
                 for (int r = 0; r < 5; ++r) {
                     double* row = Md + (rf + r) * ldm;
                     if (r < 3) {
-                        row[ft + r] += 1.;
-                        Md[(ft + r) * ldm + rf + r] += 1.;
-                        row[fb + r] -= 1.;
-                        Md[(fb + r) * ldm + rf + r] -= 1.;
+                        row[ft + r] = 1.;
+                        Md[(ft + r) * ldm + rf + r] = 1.;
+                        row[fb + r] = -1.;
+                        Md[(fb + r) * ldm + rf + r] = -1.;
                     } else {
                         const double* v = cr + (r == 3 ? drev::xcz : drev::xcy);
                         for (int j = 0; j < 3; ++j) {
-                            row[ft + 3 + j] += cr[drev::Bt + (r - 3) * 3 + j];
-                            row[fb + 3 + j] += cr[drev::Bb + (r - 3) * 3 + j];
-                            Md[(ft + 3 + j) * ldm + rf + r] -= v[j];
-                            Md[(fb + 3 + j) * ldm + rf + r] += v[j];
+                            row[ft + 3 + j] = cr[drev::Bt + (r - 3) * 3 + j];
+                            row[fb + 3 + j] = cr[drev::Bb + (r - 3) * 3 + j];
+                            Md[(ft + 3 + j) * ldm + rf + r] = -v[j];
+                            Md[(fb + 3 + j) * ldm + rf + r] = v[j];
                         }
                     }
                     b[rf + r] += cr[drev::Phi + r];
@@ -2815,12 +2841,12 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                 for (int r = 0; r < rows; ++r) {
                     double* row = Md + (rf + r) * ldm;
                     if (r < 3) {
-                        row[ft + r] += 1.;
-                        Md[(ft + r) * ldm + rf + r] += 1.;
+                        row[ft + r] = 1.;
+                        Md[(ft + r) * ldm + rf + r] = 1.;
                     } else {
                         for (int j = 0; j < 3; ++j) {
-                            row[ft + 3 + j] += cr[conrec::Brot + (r - 3) * 3 + j];
-                            Md[(ft + 3 + j) * ldm + rf + r] += cr[conrec::AX + j * 3 + (r - 3)];
+                            row[ft + 3 + j] = cr[conrec::Brot + (r - 3) * 3 + j];
+                            Md[(ft + 3 + j) * ldm + rf + r] = cr[conrec::AX + j * 3 + (r - 3)];
                         }
                     }
                     b[rf + r] += cr[conrec::Phi + r];
@@ -2831,16 +2857,16 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
                     for (int r = 0; r < rows; ++r) {
                         double* row = Md + (rf + r) * ldm;
                         if (r < 3) {
-                            row[fb + r] -= 1.;
-                            Md[(fb + r) * ldm + rf + r] -= 1.;
+                            row[fb + r] = -1.;
+                            Md[(fb + r) * ldm + rf + r] = -1.;
                             for (int j = 0; j < 3; ++j) {
-                                row[fb + 3 + j] += cr[conrec::Btr + r * 3 + j];
-                                Md[(fb + 3 + j) * ldm + rf + r] += tilde_e(cr + conrec::R1X0, r, j);
+                                row[fb + 3 + j] = cr[conrec::Btr + r * 3 + j];
+                                Md[(fb + 3 + j) * ldm + rf + r] = tilde_e(cr + conrec::R1X0, r, j);
                             }
                         } else {
                             for (int j = 0; j < 3; ++j) {
-                                row[fb + 3 + j] += cr[conrec::Brr + (r - 3) * 3 + j];
-                                Md[(fb + 3 + j) * ldm + rf + r] -= cr[conrec::AX + (r - 3) * 3 + j];
+                                row[fb + 3 + j] = cr[conrec::Brr + (r - 3) * 3 + j];
+                                Md[(fb + 3 + j) * ldm + rf + r] = -cr[conrec::AX + (r - 3) * 3 + j];
                             }
                         }
                     }
@@ -2851,7 +2877,7 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
 #pragma unroll 1
             for (int c = 0; c < nc; ++c) {
                 const double* cr = con + c * kConStride;
-                const int t = KB.con_type[c], bn = KB.con_base[c], ft = fmap[KB.con_node[c]];
+                const int t = s_con[c].y, bn = s_con[c].w, ft = fmap[s_con[c].z];
                 if (t == KYN_CONSTRAINT_REVOLUTE_JOINT) {
                     b[ft + e] += cr[drev::GtL + e] + (e >= 3 ? cr[drev::sys + e - 3] : 0.);
                     b[fmap[bn] + e] += cr[drev::GbL + e];
@@ -2883,18 +2909,17 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         // correction of component c of node n
         auto delta_of = [&](int n, int c) { return fmap[n] >= 0 ? x[fmap[n] + c] : xi[imap[n] + c]; };
         double part = 0.;
-        for (int n = tid; n < N; n += NT)
-            for (int c = 0; c < act[n]; ++c) {
-                const double e = delta_of(n, c) / (P.atol + P.rtol * fabs(sqd[n * 6 + c] * h));
+        for (int k = tid; k < N * 6; k += NT) {
+            const int n = k / 6, c = k - 6 * n;
+            if (c < act[n]) {
+                const double e = delta_of(n, c) / (P.atol + P.rtol * fabs(sqd[k] * h));
                 part += e * e;
             }
-        if (tid < nc) {
-            const double* cr = con + tid * kConStride;
-            int rf = nsys;
-            for (int c = 0; c < tid; ++c) rf += constraint_rows(KB.con_type[c]);
-            const int rows = constraint_rows(KB.con_type[tid]);
-            for (int r = 0; r < rows; ++r) {
-                const double e = x[rf + r] / (P.atol + P.rtol * fabs(cr[conrec::lam + r]));
+        }
+        for (int k = NT - 1 - tid; k < nc * 6; k += NT) {
+            const int n = k / 6, r = k - 6 * n;
+            if (r < constraint_rows(s_con[n].y)) {
+                const double e = x[s_con[n].x + r] / (P.atol + P.rtol * fabs(con[n * kConStride + conrec::lam + r]));
                 part += e * e;
             }
         }
@@ -2907,21 +2932,20 @@ __device__ __forceinline__ void dense_model_step(const KBeam& KB, const StepCoef
         if (tid == 0 && iter < kMaxNewtonIters) KB.conv[iter] = err;
         iters = iter + 1;
         // update (update_state_prediction.hpp, update_lambda_prediction.hpp)
-        for (int n = tid; n < N; n += NT)
-            for (int c = 0; c < act[n]; ++c) {
+        for (int k = tid; k < N * 6; k += NT) {
+            const int n = k / 6, c = k - 6 * n;
+            if (c < act[n]) {
                 const double delta = delta_of(n, c);
-                sqd[n * 6 + c] += delta / h;
+                sqd[k] += delta / h;
                 if (P.dynamic) {
-                    sv[n * 6 + c] += P.gamma_prime * delta;
-                    svd[n * 6 + c] += P.beta_prime * delta;
+                    sv[k] += P.gamma_prime * delta;
+                    svd[k] += P.beta_prime * delta;
                 }
             }
-        if (tid < nc) {
-            double* cr = con + tid * kConStride;
-            int rf = nsys;
-            for (int c = 0; c < tid; ++c) rf += constraint_rows(KB.con_type[c]);
-            const int rows = constraint_rows(KB.con_type[tid]);
-            for (int r = 0; r < rows; ++r) cr[conrec::lam + r] += x[rf + r];
+        }
+        for (int k = NT - 1 - tid; k < nc * 6; k += NT) {
+            const int n = k / 6, r = k - 6 * n;
+            if (r < constraint_rows(s_con[n].y)) con[n * kConStride + conrec::lam + r] += x[s_con[n].x + r];
         }
         __syncthreads();
         displacement();
