@@ -2519,18 +2519,43 @@ __device__ __forceinline__ void solve_bordered(double* Mg, int off, int ld, int 
         __syncthreads();
     }
     if (warp == 0 && md <= 64) {
-        // Back substitution by rows.  A small system's chain is short either way,
-        // and a moored platform's step is the rounding of 40 m arms to 1e-9 of
-        // its velocities: the sums keep the order that its results had.
+        // Back substitution by rows.  A moored platform's step is the rounding of
+        // 40 m arms to 1e-9 of its velocities, so the sums keep the order that its
+        // results had: lane l takes columns i + 1 + l and i + 33 + l of row i, the
+        // lanes' sums meet in an xor tree, the quotient is correctly rounded.  Only
+        // lane 0's first term waits for x[i + 1]; what it receives in the tree (R)
+        // is formed a row ahead, beside the row before it: 270 cycles a row for 480
+        // with the tree, the division and x in shared memory one after the other.
+        double xa = 0., xb = 0., m1 = 0., m2 = 0., R[5] = {0., 0., 0., 0., 0.};
 #pragma unroll 1
         for (int i = md - 1; i >= 0; --i) {
-            double s2 = 0.;
-#pragma unroll 1
-            for (int j = i + 1 + lane; j < md; j += 32) s2 += Md[i * ld + j] * x[j];
+            const double d = Md[i * ld + i], rd = rpiv[i];
+            double s2 = fma(m2, xb, fma(m1, xa, 0.));
+            // row i - 1 but for its first term
+            const double *row = Md + max(i - 1, 0) * ld, up = __shfl_sync(kAll, xa, 31);
+            double na = __shfl_up_sync(kAll, xa, 1), nb = __shfl_up_sync(kAll, xb, 1), r[5];
+            if (lane == 0) nb = up;
+            m1 = i + lane < md ? row[i + lane] : 0.;
+            m2 = i + 32 + lane < md ? row[i + 32 + lane] : 0.;
+            double p = fma(m2, nb, fma(m1, na, 0.));
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(kAll, s2, o);
-            if (lane == 0) x[i] = (Md[i * ld + md] - s2) / Md[i * ld + i];
-            __syncwarp();
+            for (int e = 0; e < 5; ++e) {
+                r[e] = __shfl_xor_sync(kAll, p, 16 >> e);
+                p += r[e];
+            }
+#pragma unroll
+            for (int e = 0; e < 5; ++e) s2 += R[e];
+            // the quotient by the correctly rounded reciprocal and two corrections
+            // (Markstein, IBM J. Res. Dev. 34, 1990)
+            const double n = Md[i * ld + md] - s2;
+            double q = n * rd;
+            q = fma(fma(-q, d, n), rd, q);
+            q = fma(fma(-q, d, n), rd, q);
+            if (lane == 0) x[i] = q;
+            xa = lane == 0 ? q : na;
+            xb = nb;
+#pragma unroll
+            for (int e = 0; e < 5; ++e) R[e] = r[e];
         }
     } else if (warp == 0) {  // by columns, the right-hand side in registers
         double y[CS], u[CS];
