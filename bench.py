@@ -503,9 +503,8 @@ def main() -> None:
                 ctx.destroy_model(int(i))
             return out
 
-        prec = {"form": "FP32 tangent (3xTF32 integration GEMM) and FP32 panel LU (pivot chains FP32, "
-                        "trailing updates on FP64 tensor cores), FP64 residual, convergence test and "
-                        "rotation update"
+        prec = {"form": "FP32 tangent blocks and system (integrated and eliminated on the FP64 tensor "
+                        "cores, stored in FP32), FP64 residual, convergence test and rotation update"
                         + (f", {args.refine} extra Newton correction(s) after convergence"
                            if args.refine else "")}
         prec.update(fp32_leg(1))
@@ -655,8 +654,8 @@ def main() -> None:
                        "precision": "plain FP64", "l2": "flushed (256 MB write) before each step",
                        "linear_solver": ("Gauss-Jordan in registers (panel LU where the block "
                                          "exceeds the register grid)" if args.solver == 0 else
-                                         "panel LU (8-column look-ahead panels, FP64 tensor-core "
-                                         "trailing updates)"),
+                                         "block elimination (8x8 blocks, FP64 tensor-core trailing "
+                                         "updates)"),
                        "launch": "direct" if args.no_graph else "CUDA graph replay per step",
                        "threads_per_cta_by_nodes": tuned64,
                        "solver_by_nodes": tuned_solvers.get(0, {}),

@@ -120,7 +120,7 @@ enum {
 /* Arithmetic of the tangent blocks and the linear solve. */
 enum {
     KYN_PRECISION_FP64 = 0,          /* plain form: everything FP64            */
-    KYN_PRECISION_FP32_REFINED = 1   /* FP32 tangent + FP32 LU, FP64 residual,
+    KYN_PRECISION_FP32_REFINED = 1   /* FP32 tangent and system, FP64 residual,
                                         rotation update and refinement        */
 };
 
@@ -314,9 +314,9 @@ KYN_API int kyn_set_loads_batch_static(kyn_ctx* ctx, const int* model_ids, int n
 /* Autotuner (no counterpart in the reference): for every size class of the
  * listed models (beams per model, nodes, quadrature points, constraints,
  * precision), times the step kernel with 128, 256 and 512 threads per CTA --
- * in the FP64 form, for beam systems, each with the panel LU and with the
- * register Gauss-Jordan solve of the free block (the same FP64 accuracy
- * class; Gauss-Jordan is the faster for small beams) -- on temporary copies
+ * in the FP64 form, for beam systems, each with the block elimination and with
+ * the register Gauss-Jordan solve of the free block (the same FP64 accuracy
+ * class) -- on temporary copies
  * of all the class's models (repeated up to 4 x SMs copies, at most 16384;
  * four steps after one warm-up step)
  * and keeps the fastest for later kyn_step calls on this context.  The
@@ -425,8 +425,10 @@ enum {
                                       KYN_OPT_PHASE_TIMING was set: load/predict,
                                       quadrature, integrate, constraints, eliminate,
                                       factor, substitute, update, store, then the
-                                      panel LU's sub-phases (9..11) and the FP32
-                                      form's refinement sweeps (12) */
+                                      sub-phases (9..11: condensed components'
+                                      integration; back substitution, or the
+                                      components' elimination; components saved)
+                                      and the FP32 form's refinement sweeps (12) */
 };
 KYN_API int kyn_ctx_stat(kyn_ctx* ctx, int stat, int64_t* value);
 

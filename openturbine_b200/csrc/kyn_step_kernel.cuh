@@ -18,8 +18,9 @@
 // B = grad*T and transpose grad^T are block-diagonal with an identity
 // translational block (src/constraints/calculate_fixed_bc_constraint.hpp,
 // calculate_prescribed_bc_constraint.hpp), so the constrained node's
-// correction follows from a 3x3 solve, the free-node block is factored by LU
-// in shared memory, and the multipliers follow from the constrained rows.
+// correction follows from a 3x3 solve, the free-node block is eliminated in
+// shared memory by 8x8 blocks, and the multipliers follow from the constrained
+// rows.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -162,8 +163,8 @@ __host__ __device__ inline int sec_doubles(int Q) { return ((3 * Q + 1) & ~1) + 
 // The kernel runs with NT = 128, 256 or 512 threads (up to four, two or one
 // CTAs per SM within the 128-register budget); four quadrature points per warp
 // are processed at a time and NT/32 warps share the GEMM-shaped phases.  More
-// resident CTAs overlap more beams' serial sections (LU pivots); more warps
-// per CTA shorten the parallel phases of one beam.
+// resident CTAs overlap more beams' serial sections (the chain of diagonal
+// blocks); more warps per CTA shorten the parallel phases of one beam.
 constexpr int kConStride = 96;          // doubles per constraint record in smem
 constexpr int kQpInterp = 24;           // doubles of interpolated values per quadrature point (qpi)
 constexpr int kHubSmem = 208;           // doubles of the hub record (hubsm)

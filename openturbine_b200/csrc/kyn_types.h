@@ -186,13 +186,14 @@ enum Phase {
     kPhaseIntegrate = 2,    // residual + stiffness/inertia integration into A
     kPhaseConstraints = 3,  // constraint residual/gradient + right-hand side
     kPhaseEliminate = 4,    // boundary-condition elimination
-    kPhaseFactor = 5,       // LU of the free block
+    kPhaseFactor = 5,       // elimination of the free block; LU of a dense system
     kPhaseSubstitute = 6,   // back substitution + multipliers
     kPhaseUpdate = 7,       // convergence error + Newton update
     kPhaseStore = 8,        // post-step and write-back
-    kPhaseLUDiag = 9,       // LU: diagonal-block factorisation (part of the factor phase)
-    kPhaseLUPanel = 10,     // LU: panel solves (part of the factor phase)
-    kPhaseIntEpilogue = 11, // LU: L21 rows solved by all threads (part of the factor phase)
+    kPhaseLUDiag = 9,       // condensed components: integration (part of the integrate phase)
+    kPhaseLUPanel = 10,     // beams: back substitution (part of the substitute phase);
+                            // condensed components: elimination (part of the integrate phase)
+    kPhaseIntEpilogue = 11, // condensed components: workspace written (part of the integrate phase)
     kPhaseRefine = 12,      // FP32 form: FP64-residual refinement sweeps of the correction
     kNumPhases = 13
 };

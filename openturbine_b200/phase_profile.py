@@ -5,9 +5,10 @@
 Creates a batch of cantilevers (uniform node count, or the mixed batch with
 --nodes 0), takes two untimed steps, switches on KYN_OPT_PHASE_TIMING and
 prints the SM cycles per beam and Newton iteration of each kernel phase (one
-CTA's clock, summed over beams by the kernel).  Phase "factor" is the whole
-Gauss-Jordan elimination (--solver 0) or the panel LU's barrier wait
-(--solver 1, whose own sub-phases follow as lu_*).
+CTA's clock, summed over beams by the kernel).  Phase "factor" is the
+Gauss-Jordan elimination (--solver 0) or the block elimination (--solver 1);
+"back_substitute" is part of "substitute", and in condensed models the
+components' elimination; "components_*" are parts of "integrate_gemm".
 """
 from __future__ import annotations
 
@@ -20,8 +21,8 @@ from . import workloads as W
 from .runtime import LOAD_NODE_FX, OPT_LINEAR_SOLVER, OPT_PHASE_TIMING, Context
 
 PHASES = ["load_predict", "quadrature", "integrate_gemm", "constraints", "eliminate",
-          "factor", "substitute", "update", "store", "lu_warp0_next_rows",
-          "lu_warp0_diag_factor", "lu_l21_all_threads", "refine"]
+          "factor", "substitute", "update", "store", "components_integrate",
+          "back_substitute", "components_save", "refine"]
 
 
 def main() -> None:
@@ -31,7 +32,7 @@ def main() -> None:
     ap.add_argument("--nodes", type=int, default=13, help="0: the mixed batch (U{5..21})")
     ap.add_argument("--precision", type=int, default=0)
     ap.add_argument("--solver", type=int, default=1,
-                    help="1: panel LU (default), 0: Gauss-Jordan in registers where it fits")
+                    help="1: block elimination (default), 0: Gauss-Jordan in registers where it fits")
     ap.add_argument("--bulk-sections", type=int, default=1,
                     help="1: sections staged by one bulk copy per iteration, 0: per-point loads")
     args = ap.parse_args()

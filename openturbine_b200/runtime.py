@@ -149,7 +149,7 @@ class Context:
         self._check(self.lib.kyn_ctx_set_option(self.h, OPT_CUDA_GRAPH, int(on)))
 
     def set_linear_solver(self, solver: int) -> None:
-        """SOLVER_GAUSS_JORDAN (registers, default) or SOLVER_PANEL_LU for the
+        """SOLVER_GAUSS_JORDAN (registers) or SOLVER_PANEL_LU (default) for the
         free-block solve of the step kernel."""
         self._check(self.lib.kyn_ctx_set_option(self.h, OPT_LINEAR_SOLVER, int(solver)))
 
