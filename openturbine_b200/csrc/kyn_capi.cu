@@ -670,12 +670,15 @@ int launch_plan(kyn_ctx* c, Plan* plan, const kyn_step_params* p) {
     const StepCoeffs P = make_coeffs(c, p);
     int rc = configure_smem(c);
     if (rc != KYN_OK) return rc;
-    KYN_CUDA(c, cudaEventRecord(c->fork, c->stream));
     const int nb = static_cast<int>(plan->buckets.size());
+    // one bucket needs no second stream: the events between the two streams and
+    // a copy each for the statuses and the iterations took 7 us of a small step
+    const bool fork = nb > 1;
+    if (fork) KYN_CUDA(c, cudaEventRecord(c->fork, c->stream));
     for (int b = 0; b < nb; ++b) {
         const Bucket& bk = plan->buckets[b];
-        cudaStream_t s = c->bstream[b % kBucketStreams];
-        KYN_CUDA(c, cudaStreamWaitEvent(s, c->fork, 0));
+        cudaStream_t s = fork ? c->bstream[b % kBucketStreams] : c->stream;
+        if (fork) KYN_CUDA(c, cudaStreamWaitEvent(s, c->fork, 0));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(bk.count, 1, 1);
         cfg.blockDim = dim3(bk.nt, 1, 1);
@@ -701,15 +704,15 @@ int launch_plan(kyn_ctx* c, Plan* plan, const kyn_step_params* p) {
         c->launches++;
     }
     c->last_buckets = nb;
-    for (int b = 0; b < std::min(nb, kBucketStreams); ++b) {
+    for (int b = 0; fork && b < std::min(nb, kBucketStreams); ++b) {
         KYN_CUDA(c, cudaEventRecord(c->join[b], c->bstream[b]));
         KYN_CUDA(c, cudaStreamWaitEvent(c->stream, c->join[b], 0));
     }
     const int n = static_cast<int>(plan->ids.size());
-    KYN_CUDA(c, cudaMemcpyAsync(plan->h_status, plan->d_status, sizeof(int) * n,
-                                cudaMemcpyDeviceToHost, c->stream));
-    KYN_CUDA(c, cudaMemcpyAsync(plan->h_iters, plan->d_iters, sizeof(int) * n,
-                                cudaMemcpyDeviceToHost, c->stream));
+    // both arrays are halves of one pool, on the device and on the host
+    const size_t pitch = sizeof(int) * static_cast<size_t>(plan->d_iters - plan->d_status);
+    KYN_CUDA(c, cudaMemcpy2DAsync(plan->h_status, pitch, plan->d_status, pitch, sizeof(int) * n, 2,
+                                  cudaMemcpyDeviceToHost, c->stream));
     return KYN_OK;
 }
 
@@ -1372,9 +1375,14 @@ int kyn_get_state(kyn_ctx* c, int id, int field, double* out) {
         const HostBeam& b = m->host.beams[bi];
         const SlabLayout L = make_slab_layout(b.N, b.Q);
         std::vector<double> h(L.total);
-        KYN_CUDA(c, cudaMemcpy(h.data(), m->d_slab[bi], L.total * sizeof(double),
-                               cudaMemcpyDeviceToHost));
+        // only what the field needs: the slab is mostly constants
+        auto fetch = [&](int at, size_t len) {
+            return cudaMemcpy(h.data() + at, m->d_slab[bi] + at, len * sizeof(double), cudaMemcpyDeviceToHost);
+        };
+        const size_t chain = bi == 0 ? HM.chain.size() * kHubDoubles : 0;
+        if (chain > 0) KYN_CUDA(c, fetch(L.hub, chain));
         if (field == KYN_FIELD_LAMBDA) {
+            if (b.nc > 0) KYN_CUDA(c, fetch(L.lambda, 6 * b.nc));
             for (int s = 0; s < b.nc; ++s)
                 for (int k = 0; k < 6; ++k) out[b.con_row[s] * 6 + k] = h[L.lambda + s * 6 + k];
             // the constraints leading into the hub-chain records: the hub BC, the
@@ -1399,6 +1407,7 @@ int kyn_get_state(kyn_ctx* c, int id, int field, double* out) {
             case KYN_FIELD_TANGENT: src = L.tangent; w = 36; break;
             default: return set_err(c, KYN_ERR_INVALID, "unknown state field");
         }
+        KYN_CUDA(c, fetch(src, static_cast<size_t>(field == KYN_FIELD_TANGENT ? 9 : w) * b.N));
         for (int k = 0; k < b.N; ++k) {
             double* o = out + static_cast<size_t>(b.node_ids[k]) * w;
             if (field == KYN_FIELD_TANGENT) {
