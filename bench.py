@@ -503,8 +503,9 @@ def main() -> None:
                 ctx.destroy_model(int(i))
             return out
 
-        prec = {"form": "FP32 tangent blocks and system (integrated and eliminated on the FP64 tensor "
-                        "cores, stored in FP32), FP64 residual, convergence test and rotation update"
+        prec = {"form": "FP32 tangent (3xTF32 integration GEMM) and FP32 panel LU (pivot chains FP32, "
+                        "trailing updates on FP64 tensor cores), FP64 residual, convergence test and "
+                        "rotation update"
                         + (f", {args.refine} extra Newton correction(s) after convergence"
                            if args.refine else "")}
         prec.update(fp32_leg(1))

@@ -120,7 +120,7 @@ enum {
 /* Arithmetic of the tangent blocks and the linear solve. */
 enum {
     KYN_PRECISION_FP64 = 0,          /* plain form: everything FP64            */
-    KYN_PRECISION_FP32_REFINED = 1   /* FP32 tangent and system, FP64 residual,
+    KYN_PRECISION_FP32_REFINED = 1   /* FP32 tangent + FP32 LU, FP64 residual,
                                         rotation update and refinement        */
 };
 
@@ -395,7 +395,8 @@ enum {
  * eliminated).  Neither pivots.
  * PANEL_LU (default): block elimination in shared memory, 8-row panels with
  *   inverted diagonal blocks, trailing updates on the FP64 tensor cores, block
- *   back substitution.
+ *   back substitution; FP32 form: right-looking LU with 8-column look-ahead
+ *   panels.
  * GAUSS_JORDAN: the block held in registers across the CTA, one barrier per
  *   2x2 pivot block.  FP64 form: the backward error
  *   max|b - A x| / (|A| |x| + |b|) of every solve is measured and counted

@@ -306,10 +306,10 @@ StepCoeffs make_coeffs(const kyn_ctx* c, const kyn_step_params* p) {
 // A step of more beams than that keeps resident takes 128 threads where four
 // such CTAs fit: the SM has 16 warps either way, and a step's serial chains
 // are shared by four beams instead of two (one B200, 2048 beams: 5 nodes 540
-// -> 375 us, 8 nodes 621 -> 506, 10 nodes 744 -> 661, FP32 form at 14 nodes
-// 1308 -> 1277; with three CTAs, FP64 at 12 nodes, 932 -> 959).  Fewer beams
-// step sooner on 256 (100 beams: 10 nodes 151 against 168 us, FP32 at 14 nodes
-// 208 against 285).
+// -> 375 us, 8 nodes 621 -> 506, 10 nodes 744 -> 661, FP32 form at 5 nodes 990
+// -> 613, at 14 nodes 2175 -> 2106; with three CTAs, FP64 at 12 nodes, 932 ->
+// 959, FP32 at 15 nodes 2513 -> 2539).  Fewer beams step sooner on 256 (100
+// beams: 10 nodes 151 against 168 us, FP32 at 14 nodes 333 against 424).
 int beam_threads(int N, int Q, int nc, int real_bytes, int hub = 0) {
     const int s256 = make_smem(N, Q, nc, real_bytes, 256, hub).bytes;
     return (2 * (s256 + 1024) <= kSmemPerSM) ? 256 : 512;

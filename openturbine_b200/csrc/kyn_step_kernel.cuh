@@ -19,8 +19,8 @@
 // translational block (src/constraints/calculate_fixed_bc_constraint.hpp,
 // calculate_prescribed_bc_constraint.hpp), so the constrained node's
 // correction follows from a 3x3 solve, the free-node block is eliminated in
-// shared memory by 8x8 blocks, and the multipliers follow from the constrained
-// rows.
+// shared memory (FP64 form: by 8x8 blocks; FP32 form: panel LU), and the
+// multipliers follow from the constrained rows.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -172,7 +172,8 @@ constexpr int kDriveSmem = 600;         // doubles of the hub record of a drive 
 
 struct Smem {
     int A;              // TR [n6][ldA]; aliased by the interpolated values
-    int G;              // TR [Q][kGPoint] weighted quadrature blocks (node-pair integration)
+    int G;              // weighted quadrature blocks (node-pair integration): FP64 form double
+                        // [Q][kGPoint], FP32 form float [4 (Q rounded up to even)][kGCols32]
     int Fc, Fdig;       // double [Q][6]
     int phi, dphi;      // double [Q][N]
     int dphiJ;          // double [Q][N]
@@ -198,8 +199,12 @@ struct Smem {
 // columns an entry's pair moves by the row's place in its group of eight rows,
 // which spreads the node-pair stores (rows 6 apart times an even pitch) and the
 // column reads of the elimination over four times as many banks; pairs stay
-// adjacent.  ldA is a multiple of 8.
-__host__ __device__ __forceinline__ int sys_at(int ldA, int r, int c) { return r * ldA + (c ^ (r & 6)); }
+// adjacent.  ldA is a multiple of 8.  The FP32 form keeps its rows as they are,
+// an odd number of values apart.
+template <typename TR = double>
+__host__ __device__ __forceinline__ int sys_at(int ldA, int r, int c) {
+    return r * ldA + (sizeof(TR) == 4 ? c : c ^ (r & 6));
+}
 
 // Weighted quadrature blocks G [Q][6 rows][kGRow]: what a node pair's 6x6 block
 // takes from one point, row r, three columns each.  XI = beta' Muu + gamma' Guu,
@@ -212,6 +217,26 @@ constexpr int K = 9, PR = 12, XIR = 15, CR = 18, O = 21;    // right: w J K, w P
 }  // namespace gblk
 constexpr int kGRow = 26;
 constexpr int kGPoint = 6 * kGRow;
+
+// FP32 form: the weighted blocks of a point are four rows of 54 quantities of a
+// node pair (56 columns), one row per product of shape factors (phi_i phi_j,
+// phi_i phi'_j, phi'_i phi'_j, phi'_i phi_j): L[r][c] (left 6x3 block, logical
+// r*3+c), RS[r][k] (right block before the tangent, 18 + r*3+k) and RI[r][c]
+// (right inertia block, 36 + r*3+c).  The tensor instruction leaves column
+// 8*nt + 2*s + e of a tile row in lane s = lane%4, slot 2*nt + e; the layout
+// puts the six values of two right-block rows (RS and RI) in one lane, so
+// SM_ij = C_RS T_j + C_RI is formed from registers: lanes 0..2 own rows
+// {2s, 2s+1} in slots 0..11 and two L values in slots 12..13 (lane 2: padding),
+// lane 3 owns L[0..13].
+constexpr int kGCols32 = 56;
+__host__ __device__ constexpr int gcol_slot(int s, int t) { return 8 * (t >> 1) + 2 * s + (t & 1); }
+__host__ __device__ constexpr int gcol(int logical) {
+    return logical < 14   ? gcol_slot(3, logical)
+           : logical < 16 ? gcol_slot(0, 12 + logical - 14)
+           : logical < 18 ? gcol_slot(1, 12 + logical - 16)
+                          : gcol_slot((logical - 18) % 18 / 6,
+                                      (logical - 18) % 18 / 3 % 2 * 6 + (logical >= 36 ? 3 : 0) + logical % 3);
+}
 
 // Entries of one slot of the Gauss-Jordan pivot buffers for (storage bytes,
 // threads): 2 (RT * NT/16 + CT * 16) with the tile sizes GJTile below (the
@@ -229,20 +254,27 @@ __host__ __device__ inline int gj_vec_offset(int real_bytes, int nt) {
     return (2 * gj_slot_entries(real_bytes, nt) * real_bytes + 15) & ~15;
 }
 // The block elimination keeps its diagonal-block inverses (64 doubles per 8
-// rows) in the place of the pivot buffers; beside them only a drive train
-// (hub = 2) needs the vectors.  gj_rows: the most rows a Gauss-Jordan grid holds.
+// rows) in the place of the pivot buffers, the FP32 form's LU its reciprocal
+// pivots and a staged tile; beside them only a drive train (hub = 2) needs the
+// vectors.  gj_rows: the most rows a Gauss-Jordan grid holds.
 __host__ __device__ constexpr int gj_rows(int real_bytes, int nt) {
     return real_bytes == 8 ? (nt == 128 ? 56 : nt == 256 ? 96 : 128) : (nt == 128 ? 64 : 128);
 }
+__host__ __device__ inline int factor_scratch_bytes(int N, int nc, int real_bytes) {
+    return real_bytes == 4 ? 6 * N * 8 + 64 * 8 : ((6 * (N - nc) + 7) / 8) * 64 * 8;
+}
+__host__ __device__ inline bool solve_vectors(int N, int nc, int real_bytes, int nt, int hub) {
+    return hub > 1 || 6 * (N - nc) <= gj_rows(real_bytes, nt);
+}
 __host__ __device__ inline int solve_vec_offset(int N, int nc, int real_bytes, int nt, int hub) {
     const int gj = 6 * (N - nc) <= gj_rows(real_bytes, nt) ? gj_vec_offset(real_bytes, nt) : 0;
-    const int lu = hub > 1 ? ((6 * (N - nc) + 7) / 8) * 64 * 8 : 0;
+    const int lu = hub > 1 ? factor_scratch_bytes(N, nc, real_bytes) : 0;
     return lu > gj ? lu : gj;
 }
 __host__ __device__ inline int solve_scratch_bytes(int N, int nc, int real_bytes, int nt, int hub) {
-    const int off = solve_vec_offset(N, nc, real_bytes, nt, hub);
-    const int vec = off ? off + 4 * 6 * N * 8 + 64 * 8 : 0;
-    const int lu = ((6 * (N - nc) + 7) / 8) * 64 * 8;
+    const int vec = solve_vectors(N, nc, real_bytes, nt, hub)
+                        ? solve_vec_offset(N, nc, real_bytes, nt, hub) + 4 * 6 * N * 8 + 64 * 8 : 0;
+    const int lu = factor_scratch_bytes(N, nc, real_bytes);
     return vec > lu ? vec : lu;
 }
 
@@ -273,7 +305,8 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
         S.sec = S.A + g_bytes;
     }
     {
-        const int g_bytes = Q * kGPoint * real_bytes;  // in the form's storage type
+        // FP32 form: k-steps of two points, so an odd Q gets one zero pad point
+        const int g_bytes = real_bytes == 4 ? 4 * ((Q + 1) & ~1) * kGCols32 * 4 : Q * kGPoint * 8;
         const int s_bytes = solve_scratch_bytes(N, nc, real_bytes, nt, hub);
         S.G = take(g_bytes > s_bytes ? g_bytes : s_bytes);
     }
@@ -306,11 +339,12 @@ __host__ __device__ inline Smem plan_smem(int N, int Q, int real_bytes, int nt, 
 // m <= n6 - 6), in whole tiles of eight.  Rows 8 values (mod 16) apart put the
 // two rows of a quarter-warp's pair loads into different halves of the banks;
 // where that padding would cost a resident CTA, or the fit, a row is the next
-// multiple of 8.
+// multiple of 8.  The FP32 form's rows are n6 + 1 values.
 constexpr int kSmemPerSM = 233472;          // 228 KB per SM, 1 KB of it taken per resident CTA
 constexpr int kMaxDynSmem = 232448 - 1024;  // 227 KB per CTA on sm_100, minus static use
 __host__ __device__ inline Smem make_smem(int N, int Q, int nc, int real_bytes, int nt, int hub = 0) {
     const int n6 = 6 * N, tight = (n6 + 8) & ~7;
+    if (real_bytes == 4) return plan_smem(N, Q, real_bytes, nt, nc, hub, n6 + 1);
     const Smem P = plan_smem(N, Q, real_bytes, nt, nc, hub, ((n6 + 8) & ~15) + 8);
     const Smem T = plan_smem(N, Q, real_bytes, nt, nc, hub, tight);
     const int most = 512 / nt;  // resident CTAs that the register budget allows
@@ -381,20 +415,13 @@ constexpr int GbL = 53;    // [6] G_base^T lambda
 
 // Two adjacent values (even position, 16- or 8-byte aligned).
 __device__ __forceinline__ double2 load_pair(const double* p) { return *reinterpret_cast<const double2*>(p); }
-__device__ __forceinline__ double2 load_pair(const float* p) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    return make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
-}
 __device__ __forceinline__ void store_pair(double* p, double a, double b) {
     *reinterpret_cast<double2*>(p) = make_double2(a, b);
-}
-__device__ __forceinline__ void store_pair(float* p, double a, double b) {
-    *reinterpret_cast<float2*>(p) = make_float2(static_cast<float>(a), static_cast<float>(b));
 }
 
 // Node-pair blocks SM_ij = S_ij T_j + I_ij (integrate_stiffness_matrix.hpp,
 // integrate_inertia_matrix.hpp, calculate_system_matrix.hpp) of one beam, on the
-// FP64 tensor cores in both forms.  With f = phi_i, g = phi'_i at a point,
+// FP64 tensor cores (FP64 form and dense models).  With f = phi_i, g = phi'_i at a point,
 //   SM_ij = sum_q f_q H_jq + g_q H'_jq,
 //   H  = [phi_j XI_L + phi'_j P_L | (phi_j K + phi'_j P_R) T_j + phi_j XI_R],
 //   H' = [phi'_j C_L              | (phi'_j C_R + phi_j O) T_j],
@@ -409,9 +436,9 @@ __device__ __forceinline__ void store_pair(float* p, double a, double b) {
 // The former product over node pairs [N^2 x 4Q][4Q x 56] took N^2 Q 448
 // multiply-adds where this takes 144, and was bound by the tensor pipe (36k of
 // 55k cycles per iteration at 21 nodes).
-template <int NT, typename TG, typename Tangent, typename Store>
+template <int NT, typename Tangent, typename Store>
 __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double* phi, const double* dphi,
-                                                     const TG* G, Tangent tangent, Store store) {
+                                                     const double* G, Tangent tangent, Store store) {
     constexpr int NW = NT / 32, MT = 3;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g8 = lane >> 2, t = lane & 3;
@@ -422,7 +449,7 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
         const int l0 = 8 * (right ? u : u - blocks);
         const int line = min(l0 + g8, lines - 1);
         const int j = line / 6, r = line - 6 * j;
-        const TG* gr = G + r * kGRow;
+        const double* gr = G + r * kGRow;
         double T[9];
         if (right) {
             const double* Tj = tangent(j);
@@ -436,7 +463,7 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) acc[mt][c][0] = acc[mt][c][1] = 0.;
-            const TG* g = gr + min(t, Q - 1) * kGPoint;
+            const double* g = gr + min(t, Q - 1) * kGPoint;
             const double *pq = phi + min(t, Q - 1) * N, *dq = dphi + min(t, Q - 1) * N;
 #pragma unroll 1
             for (int q = t; q - t < Q; q += 4) {
@@ -498,10 +525,138 @@ __device__ __forceinline__ void integrate_node_pairs(int N, int Q, const double*
     }
 }
 
-// ---- block elimination of the free block in shared memory --------------------------
-// Right-looking elimination in 8-row panels on the FP64 tensor cores, in both
-// forms (FP32 operands are exact in FP64; a result is rounded once to TR on
-// store).  Panel k multiplies its rows by the inverse of its 8x8 diagonal
+// TF32 tensor-core product D += A B for one 16x8x8 tile (mma.sync m16n8k8).
+// Fragment layout per lane l (g = l/4, t = l%4): a = {A[g][t], A[g+8][t],
+// A[g][t+4], A[g+8][t+4]}, b = {B[t][g], B[t+4][g]}, d = {D[g][2t], D[g][2t+1],
+// D[g+8][2t], D[g+8][2t+1]}.
+__device__ __forceinline__ void mma_tf32(float* d, const unsigned* a, const unsigned* b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+        "{%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// x = hi + lo with hi, lo representable in TF32 (round to nearest, ties away).
+__device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    const float r = x - __uint_as_float(hi);
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+}
+
+// Writes SM_ij = [C_L | C_RS T_j + C_RI] of node pair (i, j), scaled by the
+// conditioner, into the system matrix from one lane's integration-GEMM slots
+// (column layout: gcol; slot(t) returns the lane's slot t).
+template <typename Slot>
+__device__ __forceinline__ void store_pair_block(float* A, int ldA, const int* pos, const double* sT,
+                                                 int i, int jn, int s4, double cond, Slot slot) {
+    float* Arow = A + (6 * pos[i]) * ldA + 6 * pos[jn];
+    if (s4 < 3) {
+        const double* Tj = sT + jn * 9;
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+            const int r = 2 * s4 + rr;
+            // slots 6rr..6rr+2: RS[r][0..2]; 6rr+3..6rr+5: RI[r][0..2]
+            double rs[3], ri[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                rs[k] = slot(6 * rr + k);
+                ri[k] = slot(6 * rr + 3 + k);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double val = ri[c];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) val += rs[k] * Tj[k * 3 + c];
+                Arow[r * ldA + 3 + c] = static_cast<float>(val * cond);
+            }
+        }
+        if (s4 < 2) {
+            // slots 12, 13: L[14 + 2 s4 + e]
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int l = 14 + 2 * s4 + e;
+                Arow[(l / 3) * ldA + l % 3] = static_cast<float>(slot(12 + e) * cond);
+            }
+        }
+    } else {
+        // slots 0..13: L[0..13]
+#pragma unroll
+        for (int t = 0; t < 14; ++t) Arow[(t / 3) * ldA + t % 3] = static_cast<float>(slot(t) * cond);
+    }
+}
+
+// Node-pair blocks of the FP32 form.  For node pair (i, j):
+//   C_ij = sum_q sum_m coef_m(i, j, q) G[4q + m]
+// with coef = (phi_i phi_j, phi_i phi'_j, phi'_i phi'_j, phi'_i phi_j) and G the
+// weighted blocks of the quadrature phase (K / inertia, P, C, O terms); then
+// SM_ij = [C_L | C_RS T_j + C_RI], times the conditioner.  TF32 tensor cores with
+// the 3-term split (hi*hi + hi*lo + lo*hi, FP32 accumulation), m16n8k8: 16 pairs
+// per tile, two points per k-step (an odd Q reads the zero pad point).
+//
+// The form's states follow its roundings: a closing correction contracts by
+// only 1e-3 on the worst beams, so another order of the integration or the
+// factorisation moves the positions (by up to 6e-8 m in three steps, on some
+// ensembles several times further from the 64-bit step).  Both therefore keep
+// their order of operations, although the FP64 tensor cores' product
+// (integrate_node_pairs) and the block elimination take less time: 4096 beams of
+// 5 to 21 nodes step in 4313 us for 2617.  This takes 42k cycles an iteration at
+// 13 nodes (four CTAs to an SM), 69k at 21, factor_fp32 53k and 100k.
+template <int NT>
+__device__ __forceinline__ void integrate_node_pairs_fp32(int N, int Q, const double* phi, const double* dphi,
+                                                          const float* G, float* A, int ldA, const int* pos,
+                                                          const double* sT, double cond) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int P2 = N * N, s4 = lane & 3, g8 = lane >> 2, QK = (Q + 1) >> 1;
+    const double* fi_tab = (s4 < 2) ? phi : dphi;
+    const double* fj_tab = (s4 == 0 || s4 == 3) ? phi : dphi;
+#pragma unroll 1
+    for (int p0 = 16 * warp; p0 < P2; p0 += 16 * NW) {
+        const int pa = p0 + g8, pb = p0 + g8 + 8;
+        const bool va = pa < P2, vb = pb < P2;
+        const int ia = va ? pa / N : 0, ja = va ? pa % N : 0;
+        const int ib = vb ? pb / N : 0, jb = vb ? pb % N : 0;
+        float acc[7][4];
+#pragma unroll
+        for (int nt = 0; nt < 7; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+#pragma unroll 1
+        for (int ks = 0; ks < QK; ++ks) {
+            const int q0 = 2 * ks, q1 = 2 * ks + 1;
+            const bool q1ok = q1 < Q;
+            const int q1c = q1ok ? q1 : q0;
+            float av[4];
+            av[0] = va ? static_cast<float>(fi_tab[q0 * N + ia] * fj_tab[q0 * N + ja]) : 0.f;
+            av[1] = vb ? static_cast<float>(fi_tab[q0 * N + ib] * fj_tab[q0 * N + jb]) : 0.f;
+            av[2] = (va && q1ok) ? static_cast<float>(fi_tab[q1c * N + ia] * fj_tab[q1c * N + ja]) : 0.f;
+            av[3] = (vb && q1ok) ? static_cast<float>(fi_tab[q1c * N + ib] * fj_tab[q1c * N + jb]) : 0.f;
+            unsigned ah[4], al[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) split_tf32(av[r], ah[r], al[r]);
+            const float* g0 = G + (4 * q0 + s4) * kGCols32 + g8;
+            const float* g1 = G + (4 * q1 + s4) * kGCols32 + g8;
+#pragma unroll
+            for (int nt = 0; nt < 7; ++nt) {
+                unsigned bh[2], bl[2];
+                split_tf32(g0[nt * 8], bh[0], bl[0]);
+                split_tf32(g1[nt * 8], bh[1], bl[1]);
+                mma_tf32(acc[nt], al, bh);
+                mma_tf32(acc[nt], ah, bl);
+                mma_tf32(acc[nt], ah, bh);
+            }
+        }
+        if (va)
+            store_pair_block(A, ldA, pos, sT, ia, ja, s4, cond,
+                             [&](int t) { return static_cast<double>(acc[t >> 1][t & 1]); });
+        if (vb)
+            store_pair_block(A, ldA, pos, sT, ib, jb, s4, cond,
+                             [&](int t) { return static_cast<double>(acc[t >> 1][2 + (t & 1)]); });
+    }
+}
+
+// ---- block elimination of the free block in shared memory (FP64 form) --------------
+// Right-looking elimination in 8-row panels on the FP64 tensor cores.  Panel k
+// multiplies its rows by the inverse of its 8x8 diagonal
 // block, U_kj = D_k^-1 A_kj, in registers, and subtracts A_ik U_kj from the
 // rows below; A_kj and A_ik stay as they are, so no panel of L is solved and
 // nothing but trailing tiles is stored.  Fragments use the k order
@@ -574,13 +729,12 @@ __device__ __forceinline__ void invert_block8(double v0, double v1, double* buf,
 
 // B operands of the update by panel k in column tile c0, the lane's pair of
 // -U^T = -(A_kj^T D_k^-T): the panel's rows are read as they stand.
-template <typename TR>
-__device__ __forceinline__ double2 panel_multiplier(const TR* A, int ldA, int k0, int c0, double2 dinv, int lane) {
+__device__ __forceinline__ double2 panel_multiplier(const double* A, int ldA, int k0, int c0, double2 dinv, int lane) {
     const int t2 = 2 * (lane & 3);
-    const TR* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));  // rows t2, t2 + 1 share their column shift
+    const double* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));  // rows t2, t2 + 1 share their column shift
     double u0 = 0., u1 = 0.;
-    dmma884(u0, u1, static_cast<double>(a[0]), dinv.x);
-    dmma884(u0, u1, static_cast<double>(a[ldA]), dinv.y);
+    dmma884(u0, u1, a[0], dinv.x);
+    dmma884(u0, u1, a[ldA], dinv.y);
     return make_double2(-u0, -u1);
 }
 
@@ -589,11 +743,10 @@ __device__ __forceinline__ double2 panel_multiplier(const TR* A, int ldA, int k0
 // writes the inverse (row-major 8x8) to dinv_out.  A last block of fewer than
 // eight columns shares its tile with right-hand sides, whose update is stored.
 // One warp.
-template <typename TR>
-__device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0, const double* dinv_prev,
+__device__ __forceinline__ void factor_diag_block(double* A, int ldA, int m, int k0, const double* dinv_prev,
                                                   double* dinv_out, int lane, int* flag) {
     const int r = k0 + (lane >> 2), c = k0 + 2 * (lane & 3);
-    TR* at = A + sys_at(ldA, r, c);
+    double* at = A + sys_at(ldA, r, c);
     double2 d = load_pair(at);
     if (k0 > 0) {
         const double2 dp = load_pair(dinv_prev + 2 * lane);
@@ -612,18 +765,17 @@ __device__ __forceinline__ void factor_diag_block(TR* A, int ldA, int m, int k0,
 
 // Replaces tile c0 of panel k0's rows (those below m) by U = D^-1 A.  One warp;
 // no other reads those rows any more.
-template <typename TR>
-__device__ __forceinline__ void normalise_tile(TR* A, int ldA, int m, int k0, int c0, const double* dinv, int lane) {
+__device__ __forceinline__ void normalise_tile(double* A, int ldA, int m, int k0, int c0, const double* dinv, int lane) {
     const int t2 = 2 * (lane & 3);
     const bool in = k0 + t2 < m;  // m is even
-    TR* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));
+    double* a = A + sys_at(ldA, k0 + t2, c0 + (lane >> 2));
     const double2 d = load_pair(dinv + 2 * lane);
     double u0 = 0., u1 = 0.;
-    dmma884(u0, u1, in ? static_cast<double>(a[0]) : 0., d.x);
-    dmma884(u0, u1, in ? static_cast<double>(a[ldA]) : 0., d.y);
+    dmma884(u0, u1, in ? a[0] : 0., d.x);
+    dmma884(u0, u1, in ? a[ldA] : 0., d.y);
     if (in) {
-        a[0] = static_cast<TR>(u0);
-        a[ldA] = static_cast<TR>(u1);
+        a[0] = u0;
+        a[ldA] = u1;
     }
 }
 
@@ -644,8 +796,8 @@ __device__ __forceinline__ void normalise_tile(TR* A, int ldA, int m, int k0, in
 // L solved by all threads) spent 62k of 126k cycles per Newton iteration on a
 // 13-node beam and 102k of 187k on a 21-node beam, two thirds of them in warp
 // 0's chain.
-template <typename TR, int NT>
-__device__ __forceinline__ void eliminate_blocks(TR* A, int ldA, int m, int nrt, int nct, double* dinv, int* flag) {
+template <int NT>
+__device__ __forceinline__ void eliminate_blocks(double* A, int ldA, int m, int nrt, int nct, double* dinv, int* flag) {
     constexpr int NWK = NT / 32 - 1;  // warps on the trailing tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = (m + 7) >> 3;
@@ -672,8 +824,8 @@ __device__ __forceinline__ void eliminate_blocks(TR* A, int ldA, int m, int nrt,
             for (int left = min(hi, total) - lo; left > 0;) {
                 const int c0 = 8 * (k + 1 + j), cnt = min(ni - i, left);
                 const double2 u = panel_multiplier(A, ldA, k0, c0, dk, lane);
-                const TR* lp = A + (8 * (k + 1 + i) + fr) * ldA + k0 + fc;
-                TR* cp = A + (8 * (k + 1 + i) + fr) * ldA + c0 + fc;
+                const double* lp = A + (8 * (k + 1 + i) + fr) * ldA + k0 + fc;
+                double* cp = A + (8 * (k + 1 + i) + fr) * ldA + c0 + fc;
                 const bool last = i + cnt == ni;  // rows from m on are not stored
 #pragma unroll 1
                 for (int e = 0; e < cnt; e += 2) {  // two tiles' loads ahead of their stores
@@ -718,8 +870,8 @@ __device__ __forceinline__ void eliminate_blocks(TR* A, int ldA, int m, int nrt,
 // every column, so sums need no reduction.  One warp alone took 550 to 830
 // cycles a block (9.3k at 13 nodes, 14.4k at 21): the sums over the older blocks
 // were on its path.
-template <typename TR, int NT>
-__device__ __forceinline__ void back_substitute(const TR* A, int ldA, int m, double* xs) {
+template <int NT>
+__device__ __forceinline__ void back_substitute(const double* A, int ldA, int m, double* xs) {
     constexpr unsigned kAll = 0xffffffffu;
     constexpr int NW = NT / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -778,6 +930,290 @@ __device__ __forceinline__ void back_substitute(const TR* A, int ldA, int m, dou
                 if (t2 == 0) xs[8 * i + fr] = d0;
             }
         }
+        __syncthreads();
+    }
+}
+
+// ---- panel LU of the FP32 form's free block in shared memory -----------------------
+// The pivot chains (diagonal blocks, panel solves, block back substitution)
+// compute in FP32.  Trailing updates run on the FP64 tensor cores (FP32
+// operands are exact in FP64; the result is rounded once to FP32 on store).
+constexpr int kPanel = 8;  // panel width
+
+// Warp-level factorisation of the kb x kb diagonal block of the panel of
+// columns [p0, p0+kb): lane r holds row p0+r; pivots broadcast by shuffles.
+__device__ __forceinline__ void factor_diag(float* A, int ldA, int m, int p0, double* rpiv, int lane,
+                                            int* flag) {
+    const int kb = min(kPanel, m - p0);
+    float v[kPanel];
+#pragma unroll
+    for (int c = 0; c < kPanel; ++c) v[c] = (lane < kb && c < kb) ? A[(p0 + lane) * ldA + p0 + c] : float(0);
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) {
+        if (j < kb) {
+            const float d = __shfl_sync(0xffffffffu, v[j], j);
+            float u[kPanel];
+#pragma unroll
+            for (int c = j + 1; c < kPanel; ++c) u[c] = __shfl_sync(0xffffffffu, v[c], j);
+            const float rp = pivot_rcp(d);
+            if (lane == 0) {
+                rpiv[p0 + j] = static_cast<double>(rp);
+                if (!(fabs(d) > float(0)) || !isfinite(rp)) *flag |= 2;
+            }
+            if (lane > j) {
+                const float l = v[j] * rp;
+                v[j] = l;
+#pragma unroll
+                for (int c = j + 1; c < kPanel; ++c) v[c] -= l * u[c];
+            }
+        }
+    }
+    if (lane < kb) {
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c)
+            if (c < kb) A[(p0 + lane) * ldA + p0 + c] = v[c];
+    }
+}
+
+// L21 = A21 U11^{-1} for rows [r_begin, m) of the panel [p0, p0+kb), rows
+// strided by `stride` starting at r_begin + idx.
+__device__ __forceinline__ void solve_l21(float* A, int ldA, int m, int p0, const double* rpiv,
+                                          int r_begin, int idx, int stride) {
+    const int kb = min(kPanel, m - p0);
+#pragma unroll 2
+    for (int r = r_begin + idx; r < m; r += stride) {
+        float u[kPanel];
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) u[c] = (c < kb) ? A[r * ldA + p0 + c] : float(0);
+#pragma unroll
+        for (int j = 0; j < kPanel; ++j) {
+            if (j < kb) {
+                u[j] *= static_cast<float>(rpiv[p0 + j]);
+#pragma unroll
+                for (int k = j + 1; k < kPanel; ++k)
+                    if (k < kb) u[k] -= u[j] * A[(p0 + j) * ldA + p0 + k];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c)
+            if (c < kb) A[r * ldA + p0 + c] = u[c];
+    }
+}
+
+// One warp applies panel [k0, k0+kb) to the column tile [c0, c0+8) (columns
+// beyond m masked) for rows [rb0, rb1): U12 = L11^{-1} A12 for the tile, then
+// A22 -= L21 U12 on the FP64 tensor cores (8x8x4 tiles, two k-steps).
+// Where U12 goes:
+//   kU12InPlace  - lanes 0..7 solve one column each and overwrite A12 (the
+//                  tile of U12 is part of the factorisation);
+//   kU12ToStage  - same, but into stage[8][8]; the caller copies it into A once
+//                  no other warp reads that A12 tile any more;
+//   kU12InRegs   - every lane solves column c0 + lane/4 in registers and
+//                  nothing is written (a helper warp on rows of a tile whose
+//                  U12 another warp stores).
+enum U12Mode { kU12InPlace = 0, kU12ToStage = 1, kU12InRegs = 2 };
+
+template <int kMode>
+__device__ __forceinline__ void update_tile(float* A, int ldA, int m, int k0, int kb, int c0, int rb0,
+                                            int rb1, double* stage, int lane) {
+    const int r0 = k0 + kb;
+    const int s4 = lane & 3;
+    const int kk0 = k0 + s4, kk1 = k0 + 4 + s4;
+    double b0, b1;
+    if (kMode != kU12InRegs) {
+        if (lane < 8 && c0 + lane <= m) {
+            const int c = c0 + lane;
+            float u[kPanel];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) u[j] = (j < kb) ? A[(k0 + j) * ldA + c] : float(0);
+#pragma unroll
+            for (int q = 0; q < kPanel - 1; ++q) {
+#pragma unroll
+                for (int j = q + 1; j < kPanel; ++j)
+                    if (j < kb) u[j] -= A[(k0 + j) * ldA + k0 + q] * u[q];
+            }
+            if (kMode == kU12InPlace) {
+#pragma unroll
+                for (int j = 1; j < kPanel; ++j)
+                    if (j < kb) A[(k0 + j) * ldA + c] = u[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < kPanel; ++j) stage[j * 8 + lane] = static_cast<double>(u[j]);
+            }
+        }
+        __syncwarp();
+        const int bcol = c0 + (lane >> 2);
+        const bool bok = bcol <= m;
+        if (kMode == kU12InPlace) {
+            b0 = (kk0 < r0 && bok) ? static_cast<double>(A[kk0 * ldA + bcol]) : 0.;
+            b1 = (kk1 < r0 && bok) ? static_cast<double>(A[kk1 * ldA + bcol]) : 0.;
+        } else {
+            b0 = (kk0 < r0 && bok) ? stage[s4 * 8 + (lane >> 2)] : 0.;
+            b1 = (kk1 < r0 && bok) ? stage[(4 + s4) * 8 + (lane >> 2)] : 0.;
+        }
+    } else {
+        const int col = c0 + (lane >> 2);
+        const bool cok = col <= m;
+        float u[kPanel];
+#pragma unroll
+        for (int j = 0; j < kPanel; ++j) u[j] = (j < kb && cok) ? A[(k0 + j) * ldA + (cok ? col : c0)] : float(0);
+#pragma unroll
+        for (int q = 0; q < kPanel - 1; ++q) {
+#pragma unroll
+            for (int j = q + 1; j < kPanel; ++j)
+                if (j < kb) u[j] -= A[(k0 + j) * ldA + k0 + q] * u[q];
+        }
+        b0 = u[0];
+        b1 = u[4];
+#pragma unroll
+        for (int t = 1; t < 4; ++t) {
+            b0 = (s4 == t) ? u[t] : b0;
+            b1 = (s4 == t) ? u[4 + t] : b1;
+        }
+        if (kk0 >= r0) b0 = 0.;
+        if (kk1 >= r0) b1 = 0.;
+    }
+    const int dcol = c0 + 2 * s4;
+    const bool c0ok = dcol <= m, c1ok = dcol + 1 <= m;
+#pragma unroll 2
+    for (int rb = rb0; rb < rb1; rb += 8) {
+        const int row = rb + (lane >> 2);
+        const bool rv = row < rb1;
+        const double a0 = (rv && kk0 < r0) ? -static_cast<double>(A[row * ldA + kk0]) : 0.;
+        const double a1 = (rv && kk1 < r0) ? -static_cast<double>(A[row * ldA + kk1]) : 0.;
+        double d0 = (rv && c0ok) ? static_cast<double>(A[row * ldA + dcol]) : 0.;
+        double d1 = (rv && c1ok) ? static_cast<double>(A[row * ldA + dcol + 1]) : 0.;
+        dmma884(d0, d1, a0, b0);
+        dmma884(d0, d1, a1, b1);
+        if (rv && c0ok) A[row * ldA + dcol] = static_cast<float>(d0);
+        if (rv && c1ok) A[row * ldA + dcol + 1] = static_cast<float>(d1);
+    }
+}
+
+// Solves L U y = r for the right-hand side in column rc (rows [0, m)) by one
+// warp, in place, with the factors as the LU leaves them (unit L below the
+// diagonal, U with its pivots on it, reciprocal pivots in rpiv): forward then
+// back substitution, one column per step.
+__device__ inline void solve_factored_column(float* A, int ldA, int m, int rc, const double* rpiv, int lane) {
+    for (int j = 0; j < m; ++j) {
+        const double yj = static_cast<double>(A[j * ldA + rc]);
+        for (int i = j + 1 + lane; i < m; i += 32)
+            A[i * ldA + rc] = static_cast<float>(static_cast<double>(A[i * ldA + rc]) -
+                                              static_cast<double>(A[i * ldA + j]) * yj);
+        __syncwarp();
+    }
+    for (int j = m - 1; j >= 0; --j) {
+        const double yj = static_cast<double>(A[j * ldA + rc]) * rpiv[j];
+        __syncwarp();
+        if (lane == 0) A[j * ldA + rc] = static_cast<float>(yj);
+        for (int i = lane; i < j; i += 32)
+            A[i * ldA + rc] = static_cast<float>(static_cast<double>(A[i * ldA + rc]) -
+                                              static_cast<double>(A[i * ldA + j]) * yj);
+        __syncwarp();
+    }
+}
+
+// Replaces the kb x kb upper-triangular diagonal block of panel p0 (pivots in
+// rpiv) by its inverse; lane j < kb computes column j by back substitution
+// (lanes >= kb compute on padding and store nothing).
+__device__ __forceinline__ void invert_diag_block(float* A, int ldA, int m, int p0, const double* rpiv,
+                                                  int lane) {
+    const int kb = min(kPanel, m - p0);
+    const int jc = lane & 7;
+    float x[kPanel];
+#pragma unroll
+    for (int i = 0; i < kPanel; ++i) x[i] = (i == jc) ? float(1) : float(0);
+#pragma unroll
+    for (int c = kPanel - 1; c >= 0; --c) {
+        if (c < kb) {  // warp-uniform; x[c] = 0 for c > jc, so no lane test is needed
+            x[c] *= static_cast<float>(rpiv[p0 + c]);
+#pragma unroll
+            for (int i = 0; i < c; ++i) x[i] -= A[(p0 + i) * ldA + p0 + c] * x[c];
+        }
+    }
+    __syncwarp();
+    if (lane < kb) {
+#pragma unroll
+        for (int i = 0; i < kPanel; ++i)
+            if (i <= lane) A[(p0 + i) * ldA + p0 + lane] = x[i];
+    }
+}
+
+// Block back substitution U x = y by one warp (y in column m), with the
+// diagonal blocks already inverted: x_b = U_bb^{-1} y_b, then the rows above
+// the block take y_i -= U_i,b x_b.  Arithmetic in FP32; the solution is written
+// to xs in FP64.
+__device__ __forceinline__ void back_substitute_blocked(const float* A, int ldA, int m, double* xs, int lane) {
+    for (int i = lane; i < m; i += 32) xs[i] = static_cast<double>(A[i * ldA + m]);
+    __syncwarp();
+    const int nblk = (m + kPanel - 1) / kPanel;
+    for (int b = nblk - 1; b >= 0; --b) {
+        const int k0 = b * kPanel, kb = min(kPanel, m - k0);
+        float xv = float(0);
+        if (lane < kb) {
+#pragma unroll
+            for (int c = 0; c < kPanel; ++c)
+                if (c >= lane && c < kb) xv += A[(k0 + lane) * ldA + k0 + c] * static_cast<float>(xs[k0 + c]);
+        }
+        __syncwarp();
+        if (lane < kb) xs[k0 + lane] = static_cast<double>(xv);
+        __syncwarp();
+        float xb[kPanel];
+#pragma unroll
+        for (int c = 0; c < kPanel; ++c) xb[c] = (c < kb) ? static_cast<float>(xs[k0 + c]) : float(0);
+#pragma unroll 2
+        for (int i = lane; i < k0; i += 32) {
+            float acc = static_cast<float>(xs[i]);
+#pragma unroll
+            for (int c = 0; c < kPanel; ++c)
+                if (c < kb) acc -= A[i * ldA + k0 + c] * xb[c];
+            xs[i] = static_cast<double>(acc);
+        }
+        __syncwarp();
+    }
+}
+
+// Factors the leading m unknowns of A (right-hand side in column m): warp 0 takes
+// the next diagonal block (update, factorisation) while the others share the
+// trailing tiles; then all threads form the next panel's L21.  rpiv: m reciprocal
+// pivots; stage: 64 doubles.
+template <int NT>
+__device__ __forceinline__ void factor_fp32(float* A, int ldA, int m, double* rpiv, double* stage, int* flag) {
+    constexpr int NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (warp == 0) factor_diag(A, ldA, m, 0, rpiv, lane, flag);
+    __syncthreads();
+    solve_l21(A, ldA, m, 0, rpiv, min(kPanel, m), tid, NT);
+    __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0; k0 < m; k0 += kPanel) {
+        const int kb = min(kPanel, m - k0);
+        const int r0 = k0 + kb;
+        const int nct = (m + 1 - r0 + 7) / 8;  // column tiles of [r0, m], rhs included
+        const int top = min(r0 + kPanel, m);   // rows of the next diagonal block
+        if (warp == 0) {
+            update_tile<kU12ToStage>(A, ldA, m, k0, kb, r0, r0, top, stage, lane);
+            if (r0 < m) {
+                __syncwarp();
+                factor_diag(A, ldA, m, r0, rpiv, lane, flag);
+            }
+        } else {
+            // unit 0: tile 0 below the next diagonal block; unit u >= 1: tile u
+#pragma unroll 1
+            for (int u = warp - 1; u < nct; u += NW - 1) {
+                if (u == 0) {
+                    if (top < m) update_tile<kU12InRegs>(A, ldA, m, k0, kb, r0, top, m, nullptr, lane);
+                } else {
+                    update_tile<kU12InPlace>(A, ldA, m, k0, kb, r0 + 8 * u, r0, m, nullptr, lane);
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 64) {  // tile 0 of U12 (rows k0+1 .. k0+kb-1) from the stage
+            const int j = tid >> 3, c = r0 + (tid & 7);
+            if (j >= 1 && j < kb && c <= m) A[(k0 + j) * ldA + c] = static_cast<float>(stage[tid]);
+        }
+        if (top < m) solve_l21(A, ldA, m, r0, rpiv, top, tid, NT);
         __syncthreads();
     }
 }
@@ -906,7 +1342,7 @@ __device__ __forceinline__ void gj_eliminate(const TR* A, int ldA, int m, int nr
 #pragma unroll
         for (int b = 0; b < CT; ++b) {
             const int j = cj + b * PC;
-            R[a][b] = (i < m && j < ncols) ? A[sys_at(ldA, i, j)] : TR(0);
+            R[a][b] = (i < m && j < ncols) ? A[sys_at<TR>(ldA, i, j)] : TR(0);
         }
     }
     // slot 0: columns 0, 1 and rows 0, 1; padding of both slots stays zero
@@ -916,10 +1352,10 @@ __device__ __forceinline__ void gj_eliminate(const TR* A, int ldA, int m, int nr
         if (t < SLOT) {
             if (e < ROWS) {
                 const int i = e >> 1, h = e & 1;
-                v = (i < m) ? A[sys_at(ldA, i, h)] : TR(0);
+                v = (i < m) ? A[sys_at<TR>(ldA, i, h)] : TR(0);
             } else {
                 const int j = (e - ROWS) >> 1, h = (e - ROWS) & 1;
-                v = (j < ncols) ? A[sys_at(ldA, h, j)] : TR(0);
+                v = (j < ncols) ? A[sys_at<TR>(ldA, h, j)] : TR(0);
             }
         }
         buf[t] = v;
@@ -1016,7 +1452,7 @@ __device__ __noinline__ void gj_solve_pivoted(const TR* A, int ldA, int m, TR* b
 #pragma unroll
         for (int b = 0; b < CT; ++b) {
             const int i = ri + a * PR, j = cj + b * PC;
-            R[a][b] = (i < m && j <= m) ? A[sys_at(ldA, i, j)] : TR(0);
+            R[a][b] = (i < m && j <= m) ? A[sys_at<TR>(ldA, i, j)] : TR(0);
         }
     for (int i = tid; i < RT * PR; i += NT) used[i] = i < m ? 0 : 1;
     for (int k = 0; k < m; ++k) {
@@ -1129,7 +1565,7 @@ __device__ __forceinline__ void gj_matvec(const TR (&R)[GJTile<TR, NT>::RT][GJTi
             const int j = cj + b * PC;
             if (j < m && i < m) {
                 const double mij = from_regs ? static_cast<double>(R[a][b])
-                                             : static_cast<double>(A[sys_at(ldA, i, j)]);
+                                             : static_cast<double>(A[sys_at<TR>(ldA, i, j)]);
                 acc = fma(mij, v[j], acc);
             }
         }
@@ -1662,9 +2098,10 @@ constexpr int r = 0, udd = 4, om = 7, omd = 10, up = 16, rp = 19;
 // qpw [Q][4], node state q [N][7], v, vd [N][6] (shared memory), the system's
 // slab for the sections and reference frames (layout L), or sec: the sections
 // already staged in shared memory (sec_doubles(Q), slab order from x0').
-// Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the integration
-// G [Q][kGPoint] (gblk), the conditioner cond included.  itp: kQpInterp doubles of scratch per point.  Run by
-// warps 0 .. NW - 1; ALL: they are the whole CTA (else they meet at barrier 1).
+// Outputs: Fc, Fd + Fi - Fg [Q][6] and the weighted blocks of the integration, in
+// FP64 G [Q][kGPoint] (gblk), the conditioner cond included, in FP32 G [4 Q][kGCols32]
+// (gcol) without it.  itp: kQpInterp doubles of scratch per point.  Run by warps
+// 0 .. NW - 1; ALL: they are the whole CTA (else they meet at barrier 1).
 //
 // The 20 interpolations are products [Q x N][N x 13] and [Q x N][N x 7] on the
 // FP64 tensor cores.  Then eight lanes take a point, one rotated 3x3 block each
@@ -1805,8 +2242,16 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
         me[1] = -__shfl_sync(kAll, X[6], 6, 8);
         me[2] = __shfl_sync(kAll, X[3], 6, 8);
         const bool on = qp < Q;
-        const double w = cond * qpw[qc * 4], wJ = cond * qpw[qc * 4 + 2];
-        TG* Gq = G + qc * kGPoint;
+        constexpr bool wide = sizeof(TG) == 8;
+        const double cw = wide ? cond : 1.;
+        const double w = cw * qpw[qc * 4], wJ = cw * qpw[qc * 4 + 2];
+        TG* Gq = G + qc * (wide ? kGPoint : 4 * kGCols32);
+        if constexpr (!wide) {  // structural zeros, padding; the pad point of an odd Q
+            if (on)
+                for (int k = role; k < kGCols32 * ((Q & 1) && qp == Q - 1 ? 2 : 1); k += 8)
+                    reinterpret_cast<float4*>(Gq)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();
+        }
         // blocks crossed with s (stiffness) or omega (mass): columns first
         double c[3], om[3], V[9];
 #pragma unroll
@@ -1827,7 +2272,20 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
 #pragma unroll
             for (int e = 0; e < 3; ++e) tz[e] = role == 0 ? ft[e] : role == 7 ? -y[e] : role == 5 ? -wme[e] : 0.;
             add_tilde(Z, tz);  // P21, P22; G12, G22
-            if (on) {
+            if (on && !wide) {
+                // the same, XI by the sum that the form's rounding follows; left blocks at
+                // 9 bi, right ones at 18 (C, K, O, P) or 36 (XI)
+                TG* o = Gq + (mass_block ? 0 : 2 * kGCols32);
+                const double wd = qpw[qc * 4 + 3];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    const int l = bi ? gcol(9 + e) : gcol(e), rs = bi ? gcol(27 + e) : gcol(18 + e),
+                              ri = bi ? gcol(45 + e) : gcol(36 + e);
+                    const double xi = beta_prime * X[e] + gamma_prime * (bj ? Z[e] : 0.);
+                    o[!bj ? l : mass_block ? ri : rs] = static_cast<TG>(mass_block ? wJ * xi : wd * X[e]);
+                    if (role < 2) Gq[kGCols32 + (bj ? gcol(27 + e) : gcol(9 + e))] = static_cast<TG>(w * Z[e]);
+                }
+            } else if (on) {
                 // C, XI = beta' Muu + gamma' Guu; P (no translational rows)
                 TG* o = Gq + 3 * bi * kGRow + (mass_block ? (bj ? gblk::XIR : gblk::XIL) : (bj ? gblk::CR : gblk::CL));
                 const double sc = mass_block ? wJ * beta_prime : cond * qpw[qc * 4 + 3];
@@ -1852,9 +2310,10 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
             rows_cross(X, a, Y);
             add_tilde(Y, ty);  // O12, O22; rho w~ - (rho w)~
             if (on && (role == 0 || role == 2)) {
-                TG* oo = Gq + 3 * bi * kGRow + gblk::O;
+                TG* oo = wide ? Gq + 3 * bi * kGRow + gblk::O : Gq + 3 * kGCols32;
 #pragma unroll
-                for (int e = 0; e < 9; ++e) oo[(e / 3) * kGRow + e % 3] = static_cast<TG>(w * Y[e]);
+                for (int e = 0; e < 9; ++e)
+                    oo[wide ? (e / 3) * kGRow + e % 3 : bi ? gcol(27 + e) : gcol(18 + e)] = static_cast<TG>(w * Y[e]);
             }
             cols_cross(c, Y, V);  // Q22; w~ (rho w~ - (rho w)~)
         }
@@ -1907,9 +2366,11 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
         }
         if (on) {
             if (role == 3 || role == 7) {
-                TG* kk = Gq + (role == 7 ? 3 * kGRow : 0) + gblk::K;
+                TG* kk = wide ? Gq + (role == 7 ? 3 * kGRow : 0) + gblk::K : Gq;
 #pragma unroll
-                for (int e = 0; e < 9; ++e) kk[(e / 3) * kGRow + e % 3] = static_cast<TG>(wJ * V[e]);
+                for (int e = 0; e < 9; ++e)
+                    kk[wide ? (e / 3) * kGRow + e % 3 : role == 7 ? gcol(27 + e) : gcol(18 + e)] =
+                        static_cast<TG>(wJ * V[e]);
             }
 #pragma unroll
             for (int e = 0; e < 3; ++e) {
@@ -2224,7 +2685,7 @@ __device__ __forceinline__ void cond_component_terms(const KBeam& KB, const Step
             __syncthreads();
             sub(kPhaseLUDiag);
         }
-        if (mp > 0) eliminate_blocks<double, NT>(W, ldw, mp, rows >> 3, (rhs + 8) >> 3, G, flag);
+        if (mp > 0) eliminate_blocks<NT>(W, ldw, mp, rows >> 3, (rhs + 8) >> 3, G, flag);
         sub(kPhaseLUPanel);
 #pragma unroll 4
         for (int k = 2 * tid; k < rows * ldw; k += 2 * NT) {
@@ -2296,7 +2757,7 @@ __device__ __forceinline__ void cond_back_substitute(const KBeam& KB, const Dens
             if ((lane & 7) == 0) cx[i] = W[sys_at(ldw, i, mp + mb)] + y;
         }
         __syncthreads();
-        if (mp > 0) back_substitute<double, NT>(W, ldw, mp, cx);
+        if (mp > 0) back_substitute<NT>(W, ldw, mp, cx);
         for (int p = tid; p < mi; p += NT) xi[imap[C.node[C.at[p / 6]]] + p % 6] = cx[p];
         __syncthreads();
     }
@@ -3452,24 +3913,27 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
 
         // ---- stiffness + inertia integration and S T + I, scaled by the conditioner
         //      into A (the residual's inputs stay untouched)
-        integrate_node_pairs<NT>(
-            N, Q, phi, dphi, G, [&](int j) { return sT + j * 9; },
-            [&](int j, int r, int half) {
-                return [=](int i, double v0, double v1, double v2) {
-                    const int row = 6 * pos[i] + r, col = 6 * pos[j] + 3 * half, sh = row & 6;
-                    TR* a = A + row * ldA;
-                    a[col ^ sh] = static_cast<TR>(v0);
-                    a[(col + 1) ^ sh] = static_cast<TR>(v1);
-                    a[(col + 2) ^ sh] = static_cast<TR>(v2);
-                };
-            });
+        if constexpr (sizeof(TR) == 4)
+            integrate_node_pairs_fp32<NT>(N, Q, phi, dphi, G, A, ldA, pos, sT, P.conditioner);
+        else
+            integrate_node_pairs<NT>(
+                N, Q, phi, dphi, G, [&](int j) { return sT + j * 9; },
+                [&](int j, int r, int half) {
+                    return [=](int i, double v0, double v1, double v2) {
+                        const int row = 6 * pos[i] + r, col = 6 * pos[j] + 3 * half, sh = row & 6;
+                        double* a = A + row * ldA;
+                        a[col ^ sh] = v0;
+                        a[(col + 1) ^ sh] = v1;
+                        a[(col + 2) ^ sh] = v2;
+                    };
+                });
         __syncthreads();
         if (LUMP && KB.n_mass + KB.n_spring > 0) {  // point masses and springs at this CTA's nodes
 #pragma unroll 1
             for (int n = tid; n < N; n += NT)
                 add_lumped_terms(n, KB.lumped, KB.n_mass, KB.n_spring, sq, sv, svd, sT, KB.gravity,
                                  P.beta_prime, P.gamma_prime, P.conditioner, pos,
-                                 [&](int r, int c) -> TR& { return A[sys_at(ldA, r, c)]; }, resid);
+                                 [&](int r, int c) -> TR& { return A[sys_at<TR>(ldA, r, c)]; }, resid);
             __syncthreads();
         }
         mark(kPhaseIntegrate);
@@ -3490,7 +3954,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             for (int t = tid; t < n6 * n6; t += NT) {
                 const int r = t / n6, c = t % n6;
                 D[r * nl + c] = static_cast<double>(
-                    A[sys_at(ldA, 6 * pos[r / 6] + r % 6, 6 * pos[c / 6] + c % 6)]);
+                    A[sys_at<TR>(ldA, 6 * pos[r / 6] + r % 6, 6 * pos[c / 6] + c % 6)]);
             }
             if (tid < nc) {
                 const double* cr = con + tid * kConStride;
@@ -3530,7 +3994,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             if (i0 < m) {
 #pragma unroll 1
                 for (int j = m + (lane & 7); j < n6; j += 8) {
-                    const double aij = static_cast<double>(A[sys_at(ldA, ic, j)]);
+                    const double aij = static_cast<double>(A[sys_at<TR>(ldA, ic, j)]);
                     r -= aij * xs[j];
                     if (drive) r2 -= aij * droot[j];
                 }
@@ -3548,9 +4012,9 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 if (record && KB.dump) KB.dump[(n6 + 6 * nc) * (n6 + 6 * nc) + t] = b;
                 if (i < m) {
                     b += r;
-                    A[sys_at(ldA, i, m)] = static_cast<TR>(b);
+                    A[sys_at<TR>(ldA, i, m)] = static_cast<TR>(b);
                     if (drive) {
-                        A[sys_at(ldA, i, m + 1)] = static_cast<TR>(r2);
+                        A[sys_at<TR>(ldA, i, m + 1)] = static_cast<TR>(r2);
                         rhs2[i] = r2;
                     }
                 }
@@ -3588,7 +4052,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                     for (int bb = 0; bb < GJTile<TR, NT>::CT; ++bb) {
                         const int j = cj + bb * kGJCols;
                         if (j < m && i < m) {
-                            const double aij = static_cast<double>(A[sys_at(ldA, i, j)]);
+                            const double aij = static_cast<double>(A[sys_at<TR>(ldA, i, j)]);
                             acc = fma(aij, x[j], acc);
                             asum += fabs(aij);
                             if (a == 0) xa = fmax(xa, fabs(x[j]));
@@ -3652,7 +4116,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                         __syncthreads();
                         eta = backward_error(xs, bp, r64);
 #pragma unroll 1
-                        for (int i = tid; i < m; i += NT) A[sys_at(ldA, i, m)] = r64[i];
+                        for (int i = tid; i < m; i += NT) A[sys_at<TR>(ldA, i, m)] = r64[i];
                         __syncthreads();
                     }
                 }
@@ -3714,18 +4178,36 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
             }
           }
         } else {
-            // block elimination, then the back substitution of each right-hand side
-            double* dinv = reinterpret_cast<double*>(smem_raw + S.G);
             if (m > 0) {
-                eliminate_blocks<TR, NT>(A, ldA, m, (m + 7) >> 3, (m + nrhs + 7) >> 3, dinv, &s_flag);
-                mark(kPhaseFactor);
-                for (int i = tid; i < m; i += NT) {
-                    xs[i] = static_cast<double>(A[sys_at(ldA, i, m)]);
-                    if (drive) x2[i] = static_cast<double>(A[sys_at(ldA, i, m + 1)]);
+                if constexpr (sizeof(TR) == 4) {
+                    // panel LU; the back substitution with the diagonal blocks of U inverted
+                    // (every warp some of them), by warp 0 block by block; a drive train's
+                    // second right-hand side before they are
+                    double* rpiv = reinterpret_cast<double*>(smem_raw + S.G);
+                    factor_fp32<NT>(A, ldA, m, rpiv, rpiv + n6, &s_flag);
+                    mark(kPhaseFactor);
+                    if (drive) {
+                        if (warp == 0) solve_factored_column(A, ldA, m, m + 1, rpiv, lane);
+                        __syncthreads();
+                        for (int i = tid; i < m; i += NT) x2[i] = static_cast<double>(A[i * ldA + m + 1]);
+                    }
+                    for (int b = warp; b * kPanel < m; b += NW) invert_diag_block(A, ldA, m, b * kPanel, rpiv, lane);
+                    __syncthreads();
+                    if (warp == 0) back_substitute_blocked(A, ldA, m, xs, lane);
+                    __syncthreads();
+                } else {
+                    // block elimination, then the back substitution of each right-hand side
+                    double* dinv = reinterpret_cast<double*>(smem_raw + S.G);
+                    eliminate_blocks<NT>(A, ldA, m, (m + 7) >> 3, (m + nrhs + 7) >> 3, dinv, &s_flag);
+                    mark(kPhaseFactor);
+                    for (int i = tid; i < m; i += NT) {
+                        xs[i] = A[sys_at<TR>(ldA, i, m)];
+                        if (drive) x2[i] = A[sys_at<TR>(ldA, i, m + 1)];
+                    }
+                    __syncthreads();
+                    back_substitute<NT>(A, ldA, m, xs);
+                    if (drive) back_substitute<NT>(A, ldA, m, x2);
                 }
-                __syncthreads();
-                back_substitute<TR, NT>(A, ldA, m, xs);
-                if (drive) back_substitute<TR, NT>(A, ldA, m, x2);
             }
             mark(kPhaseLUPanel);
         }
@@ -3743,7 +4225,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 double a1 = 0., a2 = 0.;
 #pragma unroll 1
                 for (int j = lane; j < n6; j += 32) {
-                    const double arj = static_cast<double>(A[sys_at(ldA, pr + k, j)]);
+                    const double arj = static_cast<double>(A[sys_at<TR>(ldA, pr + k, j)]);
                     a1 += arj * xs[j];
                     a2 += arj * (j < m ? x2[j] : droot[j]);
                 }
@@ -3823,7 +4305,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 for (int j = lane; j < n6; j += 32) {
                     const double xj = xs[j];
 #pragma unroll
-                    for (int k = 0; k < 6; ++k) y[k] += static_cast<double>(A[sys_at(ldA, pr + k, j)]) * xj;
+                    for (int k = 0; k < 6; ++k) y[k] += static_cast<double>(A[sys_at<TR>(ldA, pr + k, j)]) * xj;
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1)
