@@ -4490,7 +4490,12 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         iters = iter + 1;
 
         // ---- update of the hub chain and, with a hub, of the multipliers (read by
-        //      the peers' sums above only through pub)
+        //      the peers' sums above only through pub).  Every thread formed the sums
+        //      above from this CTA's hub record, which the last warp now changes and,
+        //      in the next iteration, forms anew beside the quadrature points: it
+        //      waits until all have read it, else they could find another error and
+        //      leave the loop at another iteration.
+        if (hub) __syncthreads();
         if (hub && warp == NW - 1)
 #pragma unroll 1
             for (int t = lane; t < 6 * nc; t += 32) {
