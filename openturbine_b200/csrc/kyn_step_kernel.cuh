@@ -2635,12 +2635,13 @@ __device__ __forceinline__ void cond_component_terms(const KBeam& KB, const Step
 #pragma unroll 4
         for (int k = 2 * tid; k < rows * ldw; k += 2 * NT) store_pair(W + k, 0., 0.);
         __syncthreads();
-        if (tid < mp) {  // interior right-hand side before the element residual; ones on the padding
-            if (tid < mi) {
-                const int n = C.node[C.at[tid / 6]] * 6 + tid % 6;
-                W[sys_at(ldw, tid, rhs)] = cond * (mslab[ML.fx + n] + mslab[ML.f + n]);
+#pragma unroll 1
+        for (int i = tid; i < mp; i += NT) {  // interior right-hand side before the element residual; ones on the padding
+            if (i < mi) {
+                const int n = C.node[C.at[i / 6]] * 6 + i % 6;
+                W[sys_at(ldw, i, rhs)] = cond * (mslab[ML.fx + n] + mslab[ML.f + n]);
             } else {
-                W[sys_at(ldw, tid, tid)] = 1.;
+                W[sys_at(ldw, i, i)] = 1.;
             }
         }
 #pragma unroll 1

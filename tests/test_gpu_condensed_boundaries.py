@@ -1,8 +1,10 @@
 """Condensed beam elements with many boundary nodes (point masses along the
 element, its clamped root, a joint at its tip): the eliminated system's boundary
 and right-hand-side columns take more tiles than the CTA has warps from eleven
-boundary nodes on at 256 threads, from six on at 128.  With the default threads
-and with the tuned ones, against the oracle's dense solve."""
+boundary nodes on at 256 threads, from six on at 128.  And an element whose root
+alone is a boundary node, of 22 interior nodes: more rows than 128 threads.
+With the default threads and with the tuned ones, against the oracle's dense
+solve."""
 import numpy as np
 import pytest
 
@@ -14,7 +16,8 @@ pytestmark = pytest.mark.gpu
 
 def _model(order, points, masses):
     """A clamped element of `order` with point masses at its first `masses`
-    interior nodes, and a second beam on a rigid joint at its tip."""
+    interior nodes, and a second beam on a rigid joint at its tip; without
+    masses, a beam of two nodes on a rigid joint at its root."""
     m = Model()
     m.SetGravity(0., 0., -9.81)
     secs = [BeamSection(0., COMPOSITE_MASS, COMPOSITE_STIFF), BeamSection(1., COMPOSITE_MASS, COMPOSITE_STIFF)]
@@ -23,18 +26,21 @@ def _model(order, points, masses):
         return [[x, w] for x, w in zip(*np.polynomial.legendre.leggauss(n))]
 
     along, _ = chain_beam(m, 1, order, 10., [1., 0., 0., 0.], secs, rule(points))
-    tail, _ = chain_beam(m, 1, 12, 6., [1., 0., 0., 0.], secs, rule(13), origin=(10., 0., 1.))
+    joint, rest = (along[-1], 12) if masses else (along[0], 1)
+    tail, _ = chain_beam(m, 1, rest, 6., [1., 0., 0., 0.], secs, rule(rest + 1),
+                         origin=(10. if masses else 0., 0., 1.))
     for k in range(masses):
         m.AddMassElement(along[1 + k], np.diag([0.02] * 3 + [1e-4, 2e-4, 2e-4]) * (1. + 0.1 * k))
     m.AddFixedBC(along[0])
-    m.AddRigidJointConstraint([along[-1], tail[0]])
+    m.AddRigidJointConstraint([joint, tail[0]])
     return m, along, tail
 
 
 # (order, points, masses, boundary nodes of the first element)
 @pytest.mark.parametrize("tuned", [False, True])
 @pytest.mark.parametrize("order, points, masses, boundary", [
-    (20, 21, 4, 6), (20, 21, 8, 10), (20, 21, 9, 11), (20, 21, 10, 12), (20, 21, 14, 16), (12, 13, 10, 12)])
+    (20, 21, 4, 6), (20, 21, 8, 10), (20, 21, 9, 11), (20, 21, 10, 12), (20, 21, 14, 16), (12, 13, 10, 12),
+    (22, 12, 0, 1)])
 def test_condensed_boundaries_match_oracle(order, points, masses, boundary, tuned):
     from openturbine_b200.runtime import Context
     from oracle.oracle_py import OracleModel
