@@ -41,6 +41,7 @@ struct DevModel {
     std::vector<int> node_base;      // per beam: first global node when its nodes are contiguous, else -1
     int def_nt[2] = {0, 0};          // default threads per CTA, FP64 / FP32 form
     bool four128[2] = {false, false};  // four CTAs of 128 threads fit an SM (per form)
+    bool grid128[2] = {false, false};  // every free block fits the 128-thread Gauss-Jordan grid (per form)
     int tuned_nt[2] = {0, 0};        // tuned threads per CTA (0: none), cached per form
     int tuned_sv[2] = {-1, -1};      // tuned free-block solver (-1: the context's), cached per form
     unsigned long long tuned_gen[2] = {~0ull, ~0ull};  // tuned-table generation of that cache
@@ -310,6 +311,9 @@ StepCoeffs make_coeffs(const kyn_ctx* c, const kyn_step_params* p) {
 // -> 613, at 14 nodes 2175 -> 2106; with three CTAs, FP64 at 12 nodes, 932 ->
 // 959, FP32 at 15 nodes 2513 -> 2539).  Fewer beams step sooner on 256 (100
 // beams: 10 nodes 151 against 168 us, FP32 at 14 nodes 333 against 424).
+// Beams whose free block only a larger Gauss-Jordan grid holds keep 256 with that
+// solver: on 128 they would run the elimination in shared memory instead, in the
+// FP32 form without the FP64-residual refinement that the caller asked for.
 int beam_threads(int N, int Q, int nc, int real_bytes, int hub = 0) {
     const int s256 = make_smem(N, Q, nc, real_bytes, 256, hub).bytes;
     return (2 * (s256 + 1024) <= kSmemPerSM) ? 256 : 512;
@@ -354,6 +358,13 @@ int dense_smem(const HostModel& H, const HostBeam& hb) {
     return make_dense_smem(hb.N, H.ndofs, hb.comp_maxN, hb.comp_maxQ, hb.cond_nd, hb.cond_md_off >= 0).bytes;
 }
 
+// Threads per CTA of an untuned model in a step of `many` beams (more than two per
+// SM) or fewer, with the solver that it runs (see beam_threads).
+int default_threads(const DevModel* m, int form, bool many, int solver) {
+    const bool grid = solver == KYN_SOLVER_GAUSS_JORDAN && m->lump == 0;  // others run no Gauss-Jordan
+    return many && m->four128[form] && (!grid || m->grid128[form]) ? 128 : m->def_nt[form];
+}
+
 // Fills the per-model values that plans and transfer plans reuse.
 void prepare_model(DevModel* m) {
     const HostModel& H = m->host;
@@ -369,6 +380,7 @@ void prepare_model(DevModel* m) {
         const int rb = f ? 4 : 8;
         m->def_nt[f] = 128;
         m->four128[f] = false;
+        m->grid128[f] = true;
         for (int k = 0; k < 3; ++k) m->smem_nt[f][k] = 0;
         bool b0 = true;  // first beam
         for (const HostBeam& hb : H.beams) {
@@ -384,6 +396,7 @@ void prepare_model(DevModel* m) {
             if (b0 || m->four128[f])
                 m->four128[f] = 4 * (beam_smem(hb.N, hb.Q, hb.nc, rb, 128, hubf) + 1024) <= kSmemPerSM;
             b0 = false;
+            m->grid128[f] &= 6 * (hb.N - hb.nc) <= gj_rows(rb, 128);
             for (int k = 0; k < 3; ++k)
                 m->smem_nt[f][k] = std::max(m->smem_nt[f][k], beam_smem(hb.N, hb.Q, hb.nc, rb, 128 << k, hubf));
         }
@@ -514,7 +527,7 @@ int get_plan(kyn_ctx* c, const int* ids, int n, int precision, Plan** out) {
     const bool many = nbeams > static_cast<size_t>(2) * c->sms;  // see beam_threads
     for (int i = 0; i < n; ++i) {
         DevModel* m = find_model(c, ids[i]);
-        int nt = many && m->four128[f] ? 128 : m->def_nt[f];
+        int tuned_nt = 0;
         if (!c->tuned.empty()) {
             if (m->tuned_gen[f] != c->tuned_gen) {  // per-model cache of the tuned table
                 const ClassKey ck = class_key(m->host, precision);
@@ -524,9 +537,10 @@ int get_plan(kyn_ctx* c, const int* ids, int n, int precision, Plan** out) {
                 m->tuned_sv[f] = (tsv != c->tuned_solver.end()) ? tsv->second : -1;
                 m->tuned_gen[f] = c->tuned_gen;
             }
-            if (m->tuned_nt[f] > 0) nt = m->tuned_nt[f];
+            tuned_nt = m->tuned_nt[f];
         }
         const int solver = (!c->tuned.empty() && m->tuned_sv[f] >= 0) ? m->tuned_sv[f] : c->solver;
+        const int nt = tuned_nt > 0 ? tuned_nt : default_threads(m, f, many, solver);
         const int smem = m->smem_nt[f][nt_index(nt)];
         const int cluster = static_cast<int>(m->kt.size());
         const int cls = ctas_per_sm(rbytes, nt, smem);
