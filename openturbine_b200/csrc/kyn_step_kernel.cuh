@@ -853,13 +853,18 @@ __device__ __forceinline__ void eliminate_blocks(double* A, int ldA, int m, int 
         __syncthreads();
     }
     // the panels whose rows are still A: the last but one (none below a Schur
-    // complement) and the last, where the columns behind the pivots count (a
-    // Schur complement has as many tiles of them as its boundary unknowns take)
-    const int n2 = !schur && nb > 1 ? nct - nb + 1 : 0, n1 = schur ? nct - nb : 1;
+    // complement) and the last, where the columns behind the pivots count: at
+    // most three tiles, or with a Schur complement as many as the boundary
+    // unknowns and the right-hand side take, in turns
+    if (schur) {
 #pragma unroll 1
-    for (int e = warp; e < n2 + n1; e += NT / 32) {
-        const int kn = e < n2 ? nb - 2 : nb - 1;
-        normalise_tile(A, ldA, m, 8 * kn, 8 * (e < n2 ? nb - 1 + e : nct - n1 + e - n2), dinv + 64 * kn, lane);
+        for (int j = nb + warp; j < nct; j += NT / 32)
+            normalise_tile(A, ldA, m, 8 * (nb - 1), 8 * j, dinv + 64 * (nb - 1), lane);
+    } else {
+        const int n2 = nb > 1 ? nct - nb + 1 : 0;
+        if (warp < n2) normalise_tile(A, ldA, m, 8 * (nb - 2), 8 * (nb - 1 + warp), dinv + 64 * (nb - 2), lane);
+        else if (warp < n2 + 1)
+            normalise_tile(A, ldA, m, 8 * (nb - 1), 8 * (nct - 1 + warp - n2), dinv + 64 * (nb - 1), lane);
     }
     __syncthreads();
 }
