@@ -323,7 +323,11 @@ KYN_API int kyn_set_loads_batch_static(kyn_ctx* ctx, const int* model_ids, int n
  * listed models' states are not changed. */
 KYN_API int kyn_autotune(kyn_ctx* ctx, const int* model_ids, int n, const kyn_step_params* params);
 
-/* Threads per CTA kyn_step uses for a model at a precision (tuned or default). */
+/* Threads per CTA kyn_step uses for a model at a precision: the tuned number, else
+ * the default of a step of at most two beams per multiprocessor.  Untuned, a step
+ * of more beams runs a beam on 128 threads where four such CTAs fit a
+ * multiprocessor (with the Gauss-Jordan solver: and its grid of 128 threads holds
+ * the beam's free block). */
 KYN_API int kyn_tuned_threads(kyn_ctx* ctx, int model_id, int precision);
 
 /* Free-block solver (KYN_SOLVER_*) kyn_step uses for a model at a precision:

@@ -1888,7 +1888,9 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
         }
         if (clones.empty()) continue;
         const HostModel& h = find_model(c, clones[0])->host;
-        const int def_nt = find_model(c, clones[0])->def_nt[rb == 4 ? 1 : 0];
+        // what an untuned step of the copies runs with
+        const bool many = clones.size() * h.beams.size() > static_cast<size_t>(2) * sms;
+        const int def_nt = default_threads(find_model(c, clones[0]), rb == 4 ? 1 : 0, many, c->solver);
         // Every candidate is timed on the same two steps from the sources'
         // current state (the clones are reset before the warm-up and before the
         // timed steps), so that Newton iteration counts match across candidates.
@@ -1970,10 +1972,7 @@ extern "C" int kyn_tuned_threads(kyn_ctx* c, int model_id, int precision) {
     if (!m) return set_err(c, KYN_ERR_NOT_FOUND, "unknown model id");
     const auto it = c->tuned.find(class_key(m->host, precision));
     if (it != c->tuned.end()) return it->second;
-    const int rb = (precision == KYN_PRECISION_FP32_REFINED) ? 4 : 8;
-    int nt = 128;
-    for (const HostBeam& b : m->host.beams) nt = std::max(nt, beam_threads(b.N, b.Q, b.nc, rb, hub_kind(m->host)));
-    return nt;
+    return m->def_nt[precision == KYN_PRECISION_FP32_REFINED ? 1 : 0];
 }
 
 extern "C" int kyn_tuned_solver(kyn_ctx* c, int model_id, int precision) {
