@@ -2249,6 +2249,8 @@ __device__ __forceinline__ void qp_phase(int N, int Q, const double* phi, const 
         me[0] = __shfl_sync(kAll, X[7], 6, 8);
         me[1] = -__shfl_sync(kAll, X[6], 6, 8);
         me[2] = __shfl_sync(kAll, X[3], 6, 8);
+        // a section without mass has no centre of mass (eta = M/m): its step is refused
+        if (m == 0.) me[0] = __longlong_as_double(0x7ff8000000000000ll);
         const bool on = qp < Q;
         constexpr bool wide = sizeof(TG) == 8;
         const double cw = wide ? cond : 1.;
