@@ -1906,6 +1906,8 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
         // Gauss-Jordan: the same FP64 accuracy class, different speeds by size)
         const bool try_solver = p->precision == KYN_PRECISION_FP64 && find_model(c, clones[0])->lump == 0;
         const int other = c->solver == KYN_SOLVER_PANEL_LU ? KYN_SOLVER_GAUSS_JORDAN : KYN_SOLVER_PANEL_LU;
+        const DevModel* m0 = find_model(c, clones[0]);
+        const bool no_grid128 = c->solver == KYN_SOLVER_GAUSS_JORDAN && m0->lump == 0 && !m0->grid128[rb == 4 ? 1 : 0];
         int best_nt = -1, best_sv = c->solver;
         float best_ms = 0.f, def_ms = -1.f;
         for (int nt : {128, 256, 512}) {
@@ -1916,6 +1918,8 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
             if (!fits || (key.beams > 1 && key.beams * nt > 1024 * 8)) continue;
             for (int sv : {c->solver, other}) {
                 if (sv != c->solver && !try_solver) continue;
+                // FP32 form: without its grid the solver would lose the refinement
+                if (rb == 4 && nt == 128 && no_grid128) continue;
                 c->tuned[key] = nt;
                 c->tuned_solver[key] = sv;
                 ++c->tuned_gen;

@@ -53,3 +53,26 @@ def test_gauss_jordan_alone_and_in_a_large_step(nodes, clamped, precision):
     for i in (many[0], many[-1]):
         assert np.abs(ctx.state(i, "q") - q).max() <= 1e-10 * np.abs(q).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("nodes", [5, 12, 16, 18])
+def test_tuned_fp32_gauss_jordan_keeps_its_refinement(nodes):
+    """The autotuner trades no refinement for speed: every solve of the FP32 form
+    with the solver is still checked."""
+    from openturbine_b200.runtime import SOLVER_GAUSS_JORDAN, Context
+    ctx = Context(0)
+    ctx.set_linear_solver(SOLVER_GAUSS_JORDAN)
+    ids = [ctx.create_model(_beam(nodes, True))]
+    ids += [ctx.clone_model(ids[0]) for _ in range(319)]
+    p = W.batch_params()
+    p.precision = 1
+    fx = np.zeros((nodes, 6))
+    fx[-1] = [200., 300., 400., 10., 20., 30.]
+    for i in ids:
+        ctx.set_node_fx(i, fx)
+    ctx.autotune(ids, p)
+    before = ctx.stat(STAT_SOLVES_CHECKED)
+    st, it = ctx.step(ids, p)
+    assert (st == 0).all()
+    assert ctx.stat(STAT_SOLVES_CHECKED) - before == int(it.sum())
+    ctx.close()
