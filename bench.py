@@ -39,9 +39,9 @@ L2_FLUSH_BYTES = 256 << 20
 
 
 # DRAM bytes per beam-step of the step kernel from the ncu capture of
-# profiles/step_kernel_fp64_batch.md (53.2 MB for 2048 beams: the slab read once
-# and the state written once per step).
-DRAM_BYTES_PER_BEAM_STEP = 53.2e6 / 2048
+# profiles/kernel_counters.md (43.1 MB for 2048 beams: the slab read once per
+# step; most of the state written stays in L2).
+DRAM_BYTES_PER_BEAM_STEP = 43.1e6 / 2048
 
 
 def _hbm_peak() -> float | None:
@@ -67,11 +67,12 @@ def qp_flops(N: int) -> float:
 
 
 def algorithmic_flops(N: int, Q: int, iters: int) -> float:
-    """FLOPs of one beam for `iters` Newton iterations (per-iteration count:
-    Q*F_qp(N) + 410 N^2 Q + 468 N^2 + 48 N Q + (2/3) n^3 + 2 n^2, n = 6N + 6)."""
-    n = 6 * N + 6
-    per = (Q * qp_flops(N) + 410.0 * N * N * Q + 468.0 * N * N + 48.0 * N * Q + (2.0 / 3.0) * n ** 3
-           + 2.0 * n * n)
+    """FLOPs of one clamped beam for `iters` Newton iterations (per-iteration count:
+    Q*F_qp(N) + 144 N^2 Q + 200 N Q + (2/3) m^3 + 2 m^2, m = 6N - 6): the points;
+    the node-pair product [N x 2Q][2Q x 36N]; its second factor and the residual;
+    elimination and substitution of the free block."""
+    m = 6 * N - 6
+    per = Q * qp_flops(N) + 144.0 * N * N * Q + 200.0 * N * Q + (2.0 / 3.0) * m ** 3 + 2.0 * m * m
     return per * iters
 
 
@@ -317,8 +318,8 @@ def main() -> None:
     ap.add_argument("--refine", type=int, default=0,
                     help="refinement corrections of the FP32 form after convergence")
     ap.add_argument("--solver", type=int, default=1,
-                    help="free-block solve of the headline legs: 1 panel LU (default), 0 Gauss-Jordan "
-                         "in registers (panel LU where the block does not fit)")
+                    help="free-block solve of the headline legs: 1 elimination in shared memory (default), 0 "
+                         "Gauss-Jordan in registers (elimination where the block does not fit)")
     ap.add_argument("--single-models", action="store_true",
                     help="time the single cantilever and rotor configurations instead")
     ap.add_argument("--bulk-sections", type=int, default=1,
@@ -392,7 +393,8 @@ def main() -> None:
         for i, d in enumerate(draws):
             out.setdefault(int(d.num_nodes), ctx.tuned_threads(int(step_ids[i]), step_params.precision))
             sv.setdefault(int(d.num_nodes), "gauss-jordan" if ctx.tuned_solver(
-                int(step_ids[i]), step_params.precision) == 0 else "panel LU")
+                int(step_ids[i]), step_params.precision) == 0 else
+                "panel LU" if step_params.precision else "block elimination")
         tuned_solvers[step_params.precision] = dict(sorted(sv.items()))
         return dict(sorted(out.items()))
 
@@ -653,7 +655,7 @@ def main() -> None:
                        "beams_per_gpu": args.beams, "h": 0.01, "rho_inf": 0.9,
                        "max_iter": params.max_iter, "a_tol": 1e-7, "r_tol": 1e-3,
                        "precision": "plain FP64", "l2": "flushed (256 MB write) before each step",
-                       "linear_solver": ("Gauss-Jordan in registers (panel LU where the block "
+                       "linear_solver": ("Gauss-Jordan in registers (block elimination where the block "
                                          "exceeds the register grid)" if args.solver == 0 else
                                          "block elimination (8x8 blocks, FP64 tensor-core trailing "
                                          "updates)"),
@@ -677,7 +679,7 @@ def main() -> None:
                          "traffic": DRAM_BYTES_PER_BEAM_STEP * len(ids),
                          "peak_source": "cuBLAS FP64 GEMM 8192^3 (FP64 tensor cores) measured in this run",
                          "traffic_source": "ncu dram bytes read+write per beam-step (2048 beams x 13 nodes, "
-                                           "profiles/step_kernel_fp64_batch.md) x beams per step",
+                                           "profiles/kernel_counters.md) x beams per step",
                          "hbm": {"achieved_gbs": DRAM_BYTES_PER_BEAM_STEP * len(ids) / (t_value_ms / args.steps * 1e-3) / 1e9,
                                  "peak_gbs": _hbm_peak(), "peak_source": "MEASURED_PEAKS.json hbm_gbs"}},
             "gpu_launches": launches,

@@ -1902,7 +1902,7 @@ extern "C" int kyn_autotune(kyn_ctx* c, const int* ids, int n, const kyn_step_pa
             return static_cast<int>(KYN_OK);
         };
         // candidates: threads per CTA, and in the FP64 form for plain beam
-        // systems also the free-block solver (panel LU or register
+        // systems also the free-block solver (elimination in shared memory or register
         // Gauss-Jordan: the same FP64 accuracy class, different speeds by size)
         const bool try_solver = p->precision == KYN_PRECISION_FP64 && find_model(c, clones[0])->lump == 0;
         const int other = c->solver == KYN_SOLVER_PANEL_LU ? KYN_SOLVER_GAUSS_JORDAN : KYN_SOLVER_PANEL_LU;

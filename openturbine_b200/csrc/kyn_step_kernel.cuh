@@ -679,9 +679,10 @@ __device__ __forceinline__ float pivot_rcp(float d) {
     return fmaf(r, fmaf(-d, r, 1.f), r);
 }
 
-// Reciprocal by one third-order step from the hardware's approximation (relative
-// error 2^-23 at most, cubed: below the rounding), a product shorter than two
-// Newton steps.
+// Reciprocal by one third-order step from the hardware's approximation, a product
+// shorter than two Newton steps.  The approximation takes the operand's and gives
+// the result's upper 32 bits, 20 of them mantissa: a relative error below 2^-18,
+// cubed below 2^-54, half of the rounding.
 __device__ __forceinline__ double block_rcp(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
@@ -700,7 +701,9 @@ __device__ __forceinline__ double block_rcp(double d) {
 // only in the operands and a zero base, so the four steps are free of branches
 // and hold one reciprocal each.  Bound by the latency of that chain: 966 cycles
 // with shuffles, two Newton steps and a test per step, alone on an SM.  A zero
-// or non-finite determinant sets bit 2 of *flag.
+// or non-finite determinant sets bit 2 of *flag; three entries are multiplied
+// before the reciprocal comes in, so that a system whose entries lie outside
+// 1e-100 .. 1e100 counts as singular.
 __device__ __forceinline__ void invert_block8(double v0, double v1, double* buf, int lane, int* flag) {
     const int r = lane >> 2, t = lane & 3;
     bool bad = false;
@@ -1238,7 +1241,7 @@ __device__ __forceinline__ void factor_fp32(float* A, int ldA, int m, double* rp
 // the triangular solves of an LU disappear (Gauss-Jordan eliminates above the
 // pivot as well), so the chain is m steps of ~one barrier each.
 // Tile sizes per (type, threads): the registers a thread can spend on the block
-// within its launch budget.  Blocks that do not fit take the panel LU.
+// within its launch budget.  Blocks that do not fit are eliminated in shared memory.
 template <typename TR, int NT>
 struct GJTile;
 template <> struct GJTile<double, 128> { static constexpr int RT = 7, CT = 4; };
@@ -2591,8 +2594,8 @@ __device__ __forceinline__ void cond_component_terms(const KBeam& KB, const Step
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x;
     // optional sub-phase timers (thread 0): quadrature physics, assembly,
-    // elimination, save, in the slots kPhaseQuadrature, kPhaseLUDiag,
-    // kPhaseLUPanel, kPhaseIntEpilogue of ph
+    // elimination, save, in the slots kPhaseQuadrature, kPhaseCompIntegrate,
+    // kPhaseCompEliminate, kPhaseCompSave of ph
     long long pt = (ph && tid == 0) ? clock64() : 0;
     auto sub = [&](int slot) {
         if (ph && tid == 0) {
@@ -2694,17 +2697,17 @@ __device__ __forceinline__ void cond_component_terms(const KBeam& KB, const Step
                     };
                 });
             __syncthreads();
-            sub(kPhaseLUDiag);
+            sub(kPhaseCompIntegrate);
         }
         if (mp > 0) eliminate_blocks<NT>(W, ldw, mp, rows >> 3, (rhs + 8) >> 3, G, flag);
-        sub(kPhaseLUPanel);
+        sub(kPhaseCompEliminate);
 #pragma unroll 4
         for (int k = 2 * tid; k < rows * ldw; k += 2 * NT) {
             const double2 v = load_pair(W + k);
             store_pair(work + k, v.x, v.y);
         }
         __syncthreads();
-        sub(kPhaseIntEpilogue);
+        sub(kPhaseCompSave);
     }
 }
 
@@ -3520,8 +3523,8 @@ __host__ __device__ constexpr int step_min_blocks(int real_bytes, int nt) {
 // beams without them run the instance compiled without that code, whose
 // registers it would otherwise crowd.
 // GJ: the instance that also carries the register Gauss-Jordan solve
-// (KYN_SOLVER_GAUSS_JORDAN); the default instances carry only the panel LU,
-// whose register allocation the Gauss-Jordan tile would otherwise crowd.
+// (KYN_SOLVER_GAUSS_JORDAN); the default instances carry only the
+// elimination in shared memory, whose register allocation the Gauss-Jordan tile would otherwise crowd.
 template <typename TR, int NT, bool LUMP, bool GJ = false>
 __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
     step_kernel(const KBeam* __restrict__ beams, StepCoeffs P, int record,
@@ -4036,7 +4039,8 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
         mark(kPhaseEliminate);
         // (S3) the free block: Gauss-Jordan in registers where it fits the grid
         //      (FP64 form: solve; FP32 form: inverse, then FP64-residual
-        //      refinement), else the panel LU.  x1 -> xs[0:m], x2 -> x2[0:m].
+        //      refinement), else the elimination in shared memory (FP64 form: by 8x8
+        //      blocks; FP32 form: panel LU).  x1 -> xs[0:m], x2 -> x2[0:m].
         constexpr bool kInv = sizeof(TR) == 4;
         const int nrhs = drive ? 2 : 1;
         const bool use_gj = GJ && P.solver == KYN_SOLVER_GAUSS_JORDAN && m > 0 && (m & 1) == 0 &&
@@ -4220,7 +4224,7 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                     if (drive) back_substitute<NT>(A, ldA, m, x2);
                 }
             }
-            mark(kPhaseLUPanel);
+            mark(kPhaseBackSubstitute);
         }
         if (drive) {
             // Shaft rotation theta: x = x1 + theta x2 (x1 = (y1, c_r), x2 = (y2, d_r)).

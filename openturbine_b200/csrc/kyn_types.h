@@ -190,10 +190,10 @@ enum Phase {
     kPhaseSubstitute = 6,   // back substitution + multipliers
     kPhaseUpdate = 7,       // convergence error + Newton update
     kPhaseStore = 8,        // post-step and write-back
-    kPhaseLUDiag = 9,       // condensed components: integration (part of the integrate phase)
-    kPhaseLUPanel = 10,     // beams: back substitution (part of the substitute phase);
-                            // condensed components: elimination (part of the integrate phase)
-    kPhaseIntEpilogue = 11, // condensed components: workspace written (part of the integrate phase)
+    kPhaseCompIntegrate = 9,  // condensed components: integration (part of the integrate phase)
+    kPhaseBackSubstitute = 10,  // beams: back substitution (part of the substitute phase);
+    kPhaseCompEliminate = 10,   // condensed components: elimination (part of the integrate phase)
+    kPhaseCompSave = 11,    // condensed components: workspace written (part of the integrate phase)
     kPhaseRefine = 12,      // FP32 form: FP64-residual refinement sweeps of the correction
     kNumPhases = 13
 };
@@ -205,7 +205,7 @@ struct StepCoeffs {
     int32_t max_iter;
     int32_t dynamic;
     int32_t refine_iters;  // extra corrections after convergence (FP32 form)
-    int32_t solver;        // KYN_SOLVER_*: free-block solve (register Gauss-Jordan or panel LU)
+    int32_t solver;        // KYN_SOLVER_*: free-block solve (register Gauss-Jordan or the elimination in shared memory)
     int32_t refine_sweeps; // FP32 form: most refinement sweeps of one linear solve
     double refine_tol;     // FP32 form: target relative FP64 residual of the linear solve
     unsigned long long* diag;  // solve counters (kDiag*), or null
