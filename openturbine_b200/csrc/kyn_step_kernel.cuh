@@ -4499,18 +4499,19 @@ __global__ void __launch_bounds__(NT, step_min_blocks(sizeof(TR), NT))
                 const double e2 = xlh[k] / (P.atol + P.rtol * fabs(br[conrec::lam + k]));
                 total += e1 * e1 + e2 * e2;
             }
+            // Every thread formed these sums from this CTA's hub record, which the
+            // last warp changes below and, in the next iteration, forms anew beside
+            // the quadrature points: it waits until all have read it, else they could
+            // find another error and leave the loop at another iteration.  (As a
+            // branch of its own the barrier cost models without a hub 2 %.)
+            __syncthreads();
         }
         const double err = sqrt(total / static_cast<double>(KB.model_dofs));
         if (KB.rank == 0 && tid == 0 && iter < kMaxNewtonIters) KB.conv[iter] = err;
         iters = iter + 1;
 
         // ---- update of the hub chain and, with a hub, of the multipliers (read by
-        //      the peers' sums above only through pub).  Every thread formed the sums
-        //      above from this CTA's hub record, which the last warp now changes and,
-        //      in the next iteration, forms anew beside the quadrature points: it
-        //      waits until all have read it, else they could find another error and
-        //      leave the loop at another iteration.
-        if (hub) __syncthreads();
+        //      the peers' sums above only through pub)
         if (hub && warp == NW - 1)
 #pragma unroll 1
             for (int t = lane; t < 6 * nc; t += 32) {
